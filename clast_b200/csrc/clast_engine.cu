@@ -375,7 +375,7 @@ struct DevHitsSink : HitSink {
 // CDeviceHitList for every query window of `qb` against the window whose
 // seeds are in z: seed filters, DP, result order.
 int64_t search_seeded(clast_ctx* c, Workspace& ws, const clast_params* p, const QueryRef& qb, int32_t q_first,
-                      SeedSet& z, bool tune, HitSink& sink) {
+                      SeedSet& z, HitSink& sink) {
   cudaStream_t st = c->st;
   const clast_index* ix = z.ix;
   const QueryView q = qb.q;
@@ -442,88 +442,44 @@ int64_t search_seeded(clast_ctx* c, Workspace& ws, const clast_params* p, const 
   DpParams dp{p->lmer, p->stride, p->gap, p->local, p->cutoff, p->total_db, p->K, p->lambda};
   // Reads of different lengths: the DP takes the hits longest first, so that a
   // warp's hits have about the same number of rows (the reference sorts them
-  // by rows before aligning too, CDeviceHitList_alignmentHits.cu:10-58), by
-  // an exact sort or by length buckets; the kernel runs over a grid of all
-  // hits or as a persistent grid taking hits from a queue.  Which of these
-  // runs fastest is measured once per context and kind of batch (gap, mode,
-  // uneven or not) on a batch of at least kDpTuneHits hits; every variant
-  // writes the same results.
+  // by rows before aligning too, CDeviceHitList_alignmentHits.cu:10-58), by an
+  // exact sort of the row counts.  (Length buckets in one counting pass take
+  // 0.10 against 0.15 ms for 130,000 hits, but their DP 3.68 against 3.66 ms,
+  // and 17.3 against 17.0 ms on 200,000 reads of 50 bp - 10 kbp; a persistent
+  // grid taking hits from a queue is slower than the plain one, 17.7 and 4.2 ms.)
   // The longest hits of the order may run one per warp (banded_dp decides
   // from the length buckets, or for equal lengths from the row count).
   const bool uneven = qb.max_len != qb.min_len && H > 1;
-  const int warp_mode = dp_warp_mode_from_env(c->dp_warp);
-  DpBuckets buckets;  // of the order last made
-  auto make_order = [&](int kind) -> const uint64_t* {
-    buckets = DpBuckets();
-    if (kind == 0) return nullptr;
-    if (kind == 1) {
-      const int rows_max = std::max(1, qb.max_len - p->lmer + 1);
-      int bits = 1;
-      while ((1ll << bits) <= rows_max) ++bits;
-      uint64_t* ok = ws.get<uint64_t>("h_order", H);
-      uint64_t* ok2 = ws.get<uint64_t>("h_order2", H);
-      dp_order_keys(hs, q.len, H, p->lmer, rows_max, ok, st);
-      const uint64_t* sorted = radix_sort_u64(ws, ok, nullptr, ok2, nullptr, H, 32, 32 + bits, st) ? ok2 : ok;
-      if (warp_mode == kDpWarpAuto) buckets = dp_bucket_count(ws, hs, q.len, H, p->lmer, st);
-      return sorted;
-    }
-    uint64_t* ob = ws.get<uint64_t>("h_border", H);
-    buckets = dp_bucket_order(ws, hs, q.len, H, p->lmer, ob, st);
-    return ob;
-  };
-  unsigned long long* dp_head = ws.get<unsigned long long>("dp_head", 1);
+  const int warp_mode = qb.max_len > kDpMaxThreadLen ? kDpWarpAll : dp_warp_mode_from_env(c->dp_warp);
   long long* dp_warp_n = ws.get<long long>("dp_warp_n", 1);
   int* dp_bad = ws.get<int>("dp_bad", 1);
   CLAST_CK(cudaMemsetAsync(dp_bad, 0, sizeof(int), st));
-  auto launch_of = [&](const DpChoice& ch) {
-    DpLaunch m;
-    if (ch.queue) {
-      m.head = dp_head;
-      m.chunk = ch.chunk;
-    }
-    m.warp = warp_mode;
-    m.buckets = buckets;
-    m.warp_n = dp_warp_n;
-    m.aux = c->st_dp;
-    m.ev_fork = c->ev_dp_fork;
-    m.ev_join = c->ev_dp_join;
-    m.bad = dp_bad;
-    if (!uneven) m.uniform_rows = std::max(0, qb.max_len - p->lmer);
-    return m;
-  };
-  const int tune_key = (p->gap << 2) | (p->local ? 2 : 0) | (uneven ? 1 : 0);
-  auto it = c->dp_tuned.find(tune_key);
-  if (tune && it == c->dp_tuned.end() && H >= kDpTuneHits && !std::getenv("CLAST_DP_NO_TUNE")) {
-    std::vector<DpChoice> cands;
-    for (int ord : (uneven ? std::vector<int>{1, 2} : std::vector<int>{0}))
-      for (int q_ : {0, 1})
-        for (int chunk : (q_ ? std::vector<int>{1, 2} : std::vector<int>{1})) cands.push_back(DpChoice{ord, q_ != 0, chunk});
-    float best = 1e30f;
-    DpChoice pick = cands[0];
-    for (const DpChoice& ch : cands) {
-      CLAST_CK(cudaEventRecord(c->ev_t0, st));
-      const uint64_t* order = make_order(ch.order);
-      banded_dp(tv, q, hk, hq, hs, order, H, dp, o, st, launch_of(ch));
-      CLAST_CK(cudaEventRecord(c->ev_t1, st));
-      CLAST_CK(cudaEventSynchronize(c->ev_t1));
-      float ms = 0;
-      CLAST_CK(cudaEventElapsedTime(&ms, c->ev_t0, c->ev_t1));
-      if (ms < best) {
-        best = ms;
-        pick = ch;
-      }
-    }
-    it = c->dp_tuned.emplace(tune_key, pick).first;
-  }
-  DpChoice ch = it != c->dp_tuned.end() ? it->second : DpChoice{uneven ? 1 : 0, false, 1};
-  if (ch.order != 0 && !uneven) ch.order = 0;
-  c->stats.dp_order_kind = ch.order;
-  c->stats.dp_queue_chunk = ch.queue ? ch.chunk : 0;
+  c->stats.dp_order_kind = uneven ? 1 : 0;
+  c->stats.dp_queue_chunk = 0;
+  DpBuckets buckets;
+  const uint64_t* order = nullptr;
   tm.begin(st);
-  const uint64_t* order = make_order(ch.order);
+  if (uneven) {
+    const int rows_max = std::max(1, qb.max_len - p->lmer + 1);
+    int bits = 1;
+    while ((1ll << bits) <= rows_max) ++bits;
+    uint64_t* ok = ws.get<uint64_t>("h_order", H);
+    uint64_t* ok2 = ws.get<uint64_t>("h_order2", H);
+    dp_order_keys(hs, q.len, H, p->lmer, rows_max, ok, st);
+    order = radix_sort_u64(ws, ok, nullptr, ok2, nullptr, H, 32, 32 + bits, st) ? ok2 : ok;
+    if (warp_mode == kDpWarpAuto) buckets = dp_bucket_count(ws, hs, q.len, H, p->lmer, st);
+  }
   tm.end(StageTimer::DPORDER, st);
   tm.begin(st);
-  const DpLaunch dl = launch_of(ch);
+  DpLaunch dl;
+  dl.warp = warp_mode;
+  dl.buckets = buckets;
+  dl.warp_n = dp_warp_n;
+  dl.aux = c->st_dp;
+  dl.ev_fork = c->ev_dp_fork;
+  dl.ev_join = c->ev_dp_join;
+  dl.bad = dp_bad;
+  if (!uneven) dl.uniform_rows = std::max(0, qb.max_len - p->lmer);
   const long long warp_fixed = banded_dp(tv, q, hk, hq, hs, order, H, dp, o, st, dl);
   tm.end(StageTimer::DP, st);
   if (warp_fixed >= 0) c->stats.dp_warp_hits += warp_fixed;
@@ -562,7 +518,7 @@ void search_batch(clast_ctx* c, const clast_index* ix, const clast_params* p, co
   std::vector<SeedSet> sets(1);
   sets[0].ix = ix;
   seed_windows(c, p, qb, sets);
-  search_seeded(c, c->ws, p, qb, q_first, sets[0], true, sink);
+  search_seeded(c, c->ws, p, qb, q_first, sets[0], sink);
 }
 
 template <class T>
@@ -663,8 +619,7 @@ int clast_ctx_create(int device, clast_ctx** out) {
     (void)cudaGetLastError();
   }
   if (cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
-      cudaEventCreate(&c->ev2) != cudaSuccess || cudaEventCreate(&c->ev3) != cudaSuccess ||
-      cudaEventCreate(&c->ev_t0) != cudaSuccess || cudaEventCreate(&c->ev_t1) != cudaSuccess)
+      cudaEventCreate(&c->ev2) != cudaSuccess || cudaEventCreate(&c->ev3) != cudaSuccess)
     return CLAST_ERR_CUDA;
   *out = c.release();
   return CLAST_OK;
@@ -691,8 +646,6 @@ void clast_ctx_destroy(clast_ctx* ctx) {
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->ev2) cudaEventDestroy(ctx->ev2);
   if (ctx->ev3) cudaEventDestroy(ctx->ev3);
-  if (ctx->ev_t0) cudaEventDestroy(ctx->ev_t0);
-  if (ctx->ev_t1) cudaEventDestroy(ctx->ev_t1);
   if (ctx->ev_dp_fork) cudaEventDestroy(ctx->ev_dp_fork);
   if (ctx->ev_dp_join) cudaEventDestroy(ctx->ev_dp_join);
   if (ctx->st_dp) {
@@ -1097,7 +1050,7 @@ static int map_impl(clast_ctx* ctx, const clast_targets* T, const clast_params* 
       seed_windows(ctx, p, qr, sets);
       for (size_t j = 0; j < sets.size(); ++j) {
         DevHitsSink sink(per_win[idx[j]]);
-        search_seeded(ctx, ctx->ws, p, qr, 0, sets[j], true, sink);
+        search_seeded(ctx, ctx->ws, p, qr, 0, sets[j], sink);
       }
     }
     // fixResult: stable merge by (read, score desc) over the windows, on the device
@@ -1434,9 +1387,8 @@ extern "C" int clast_search_noalloc(clast_ctx* ctx, const clast_index* ix, const
       part_cap = most;
     }
     if (S == 0) return finish(0);
-    // the stages after seeding are clast_search's, on the fixed scratch (no
-    // autotuner runs: its trial orders would need more of it); the hits go
-    // to slots of the scratch, then to the caller's arrays
+    // the stages after seeding are clast_search's, on the fixed scratch; the
+    // hits go to slots of the scratch, then to the caller's arrays
     int32_t lmin = INT32_MAX, lmax = 0;
     for (int32_t i = 0; i < n_qseqs; ++i) {
       lmin = std::min(lmin, q_lengths[i]);
@@ -1477,7 +1429,7 @@ extern "C" int clast_search_noalloc(clast_ctx* ctx, const clast_index* ix, const
         return fo;
       }
     } sink(ws, capacity, out);
-    const int64_t F = search_seeded(ctx, ws, p, qr, q_begin, z, false, sink);
+    const int64_t F = search_seeded(ctx, ws, p, qr, q_begin, z, sink);
     if (F == 0) return finish(0);
     const FinalOut& fo = sink.fo;
     int32_t* const dst[8] = {out->t_id, out->t_idx, out->q_id, out->q_idx, out->t_len, out->q_len, out->match,

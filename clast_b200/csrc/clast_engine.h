@@ -161,15 +161,6 @@ struct PinnedArena {
   } dev;
 };
 
-// How the banded DP of one kind of batch runs (measured, see search_seeded):
-// order 0 = none, 1 = exact sort by rows, 2 = length buckets; queue = the
-// persistent grid with `chunk` hits per lane per take.
-struct DpChoice {
-  int order = 0;
-  bool queue = false;
-  int chunk = 1;
-};
-constexpr int64_t kDpTuneHits = 1 << 16;
 constexpr int kBuildStreams = 2;  // target windows indexed at once by clast_targets_create
 
 }  // namespace clast
@@ -193,8 +184,6 @@ struct clast_ctx {
   clast_stats stats{};
   StageTimer timer;
   int64_t seed_hint = 0;  // seed buffer capacity that sufficed before
-  std::map<int, clast::DpChoice> dp_tuned;  // by (gap, local, uneven)
-  cudaEvent_t ev_t0 = nullptr, ev_t1 = nullptr;  // DP tuning
   // the DP's one-hit-per-warp kernel runs on st_dp beside the one-per-thread
   // kernels on st (forked and joined by these events)
   cudaStream_t st_dp = nullptr;

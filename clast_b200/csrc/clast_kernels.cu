@@ -18,6 +18,7 @@
 #include <cstdint>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <utility>
 
 #include "clast_device.cuh"
@@ -1926,90 +1927,192 @@ __device__ __forceinline__ int2 cell_score(int t, int q) {
   return make_int2(-3, 0);
 }
 
+// Scores of the band are kept as potentials: after row r (from 0) of a pass,
+// column c holds S + 4 (r + 1) + 2 c (likewise for V and H).  A vertical step
+// (r - 1, c + 1) -> (r, c) and a horizontal one (r, c - 1) -> (r, c) both raise
+// 4 (r + 1) + 2 c by 2, which cancels the gap extension, so that extending a
+// gap costs nothing and opening one costs 5 from either side:
+//   V = max(s_up - 5, v_up)   H = max(s_left - 5, h_left)   diagonal: s_diag + POINT + 4
+// (calcutlateCell, krnlAlignment.cu:42-77, with every difference unchanged, so
+// every comparison and tie is too).  With P = max(diagonal, V), S = max(P, H)
+// and S - 5 <= max(P - 5, H), the horizontal state is a running maximum along
+// the row, H' = max(P - 5, H): one operation per cell on the row's dependent
+// chain.  H wins iff H >= P (it wins ties over V, and both win them over the
+// diagonal); otherwise V wins iff V >= diagonal.
+constexpr int kStepRow = 4, kStepCol = 2;
+constexpr int kOpenPot = kGapOpen + kGapExtend + kStepCol;  // -5
+
+// Shared memory of a DP block: the letter-pair table (POINT + 4, match
+// increment) by class, and the classes' byte offsets into it by letter byte
+// (target offset in the low byte, query offset in the high half).  The four
+// bases of target and query take the table's first 16 entries, which are the
+// 32 banks once: lanes that look up different base pairs never conflict.
+template <class T2>
+struct DpTab {
+  T2 w[128];
+  uint16_t q_off[256];
+  uint8_t t_off[256];
+};
+__host__ __device__ constexpr int dp_t_class_off(int c) { return 32 * c; }                          // < 256
+__host__ __device__ constexpr int dp_q_class_off(int c) { return c < 4 ? 8 * c : 256 * (c - 3); }
+
+__device__ __forceinline__ int2 dp_pair_of(int2, int x, int y) { return make_int2(x, y); }
+__device__ __forceinline__ float2 dp_pair_of(float2, int x, int y) { return make_float2((float)x, (float)y); }
+
+template <class T2>
+__device__ __forceinline__ void dp_table_init(DpTab<T2>& tab) {
+  for (int i = threadIdx.x; i < 49; i += blockDim.x) {
+    const int t = i / 7, q = i % 7;
+    const int2 w = cell_score(t, q);
+    tab.w[(dp_t_class_off(t) + dp_q_class_off(q)) / 8] = dp_pair_of(T2(), w.x + kStepRow, w.y);
+  }
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) {
+    const int c = class_of_letter(base_class((char)i));
+    tab.t_off[i] = (uint8_t)dp_t_class_off(c);
+    tab.q_off[i] = (uint16_t)dp_q_class_off(c);
+  }
+}
+template <class T2>
+__device__ __forceinline__ uint32_t dp_t_off(const DpTab<T2>& tab, char b) {
+  return tab.t_off[(unsigned char)b];
+}
+template <class T2>
+__device__ __forceinline__ uint32_t dp_q_off(const DpTab<T2>& tab, char b) {
+  return tab.q_off[(unsigned char)b];
+}
+template <class T2>
+__device__ __forceinline__ T2 dp_pair(const DpTab<T2>& tab, uint32_t off) {
+  return *reinterpret_cast<const T2*>(reinterpret_cast<const char*>(tab.w) + off);
+}
+
+// initTempNodeArray, krnlAlignment.cu:6-38 (band rows 1..W): state of column c
+// before row 0.  u is the vertical state the column hands to the row below.
+template <int GAP>
+__device__ __forceinline__ void dp_init_col(int c, int& s, int& u, int& m) {
+  const int sc = c < GAP ? kMarginScore : c == GAP ? 0 : (c - GAP) * kGapExtend + kGapOpen;
+  s = sc + kStepCol * c;
+  u = c < GAP ? s : s + kOpenPot;  // max(S - 5, V): V is the margin itself left of the middle, S - 5 elsewhere
+  m = c < GAP ? kMarginScore : 0;
+}
+// Left margin's H and the fixed band row's V (below the last column) of row 0;
+// both rise by kStepRow per row.
+template <int GAP>
+constexpr int kDpLeftH = kMarginScore + kGapExtend + kStepRow;
+template <int GAP>
+constexpr int kDpBottomV =
+    (GAP + 1) * kGapExtend + kGapOpen + kGapOpen + kGapExtend + kStepRow + kStepCol * 2 * GAP;
+
+__device__ __forceinline__ float max3_f32(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
 // Banded DP of one hit, backward pass then forward pass, in ONE row loop of
 // rows_b + rows_f iterations: every hit of a read has qLen - l rows in total,
 // so the threads of a warp stay converged although each switches from the
 // backward to the forward pass at its own row.
 //
-// Per band column the registers hold A = S - 7 (score minus gap open +
-// extend), B = V - 2 (vertical state minus gap extend) and M (matches); along
-// a row the chain carries hA = S - 7 and hB = H - 2 of the previous column.
-// Then, exactly as calcutlateCell (krnlAlignment.cu:42-77):
-//   V = max(Sv - 7, Vv - 2) = max(A_v, B_v)        H = max(Sh - 7, Hh - 2) = max(hA, hB)
-//   pt = S_diag + POINT = A_diag + (POINT + 7)      (the table stores POINT + 7)
-//   H wins over V iff H >= V; the diagonal wins iff pt > max(V, H)
-// Storing S itself and folding the "- 7" into a fused add-and-max per
-// maximum takes one add per cell less, but the row's chain through it is
-// slower: a lone thread took 6.8 against 2.7 ms on one 5 kbp hit, with no gain
-// on full batches of 150 bp reads.  A long hit's chain sets the latency of
-// small batches, so the band keeps S - 7.
+// Bound by the ALU pipe (79 % busy on 2 kbp reads), where a warp instruction
+// takes two cycles and where maxima, compares and selects run whatever their
+// type.  So the whole numbers are held in floats (exact: see kDpMaxThreadLen):
+// their additions run on the FMA pipe instead, at twice the rate, and a cell's
+// ALU work is one three-way and two two-way maxima, two compares and two
+// selects.  The columns' letters are packed four to a word, one dp4a makes a
+// table address of them, and each pair is looked up a row ahead of its use
+// (without that, a lone hit waits 2.1 against 1.1 ms on 5 kbp).  Measured
+// against the integer form with a spread table that this replaced: 1,172 to
+// 1,980 GCUPS on uneven reads of 50 bp - 10 kbp (28.7 to 17.0 ms), 1,185 to
+// 1,590 on a million reads of 150 bp (4.55 to 3.39 ms), 599 to 1,200 at gap 16.
+// (Tried: packed f32x2 additions, arithmetic selects by saturated differences
+// on the FMA pipe, the row in two loops; all slower or within the noise.)
 template <int GAP>
 struct Band {
   static constexpr int W = 2 * GAP + 1;
-  int A[W], B[W], M[W], tc[W];
+  static constexpr int kWords = (W + 3) / 4;
+  float2 sm[W];         // score potential, matches
+  float u[W];           // the vertical state each column hands to the row below
+  uint32_t tw[kWords];  // the columns' target letters: byte c = class offset in the table
 
-  // initTempNodeArray, krnlAlignment.cu:6-38 (band rows 1..W), and the first W
-  // target bases of a pass: index ib0 + step * c, 'X' outside [lo, hi).
-  __device__ __forceinline__ void init(const char* __restrict__ tb, int64_t tstart, int64_t ib0, int step,
-                                       int64_t lo, int64_t hi) {
+  // The band before row 0, and the first W target bases of a pass: index ib0 +
+  // step * c, 'X' outside [lo, hi).
+  __device__ __forceinline__ void init(const DpTab<float2>& tab, const char* __restrict__ tb, int64_t tstart,
+                                       int64_t ib0, int step, int64_t lo, int64_t hi) {
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) tw[i] = 0;
 #pragma unroll
     for (int c = 0; c < W; ++c) {
-      const int r = c + 1;
-      int sc, v, m;
-      if (r < GAP + 1) { sc = kMarginScore; v = kMarginScore; m = kMarginScore; }
-      else if (r == GAP + 1) { sc = 0; v = kGapOpen; m = 0; }
-      else { sc = (r - GAP - 1) * kGapExtend + kGapOpen; v = sc + kGapOpen; m = 0; }
-      A[c] = sc + kGapOpen + kGapExtend;
-      B[c] = v + kGapExtend;
-      M[c] = m;
+      int s, v, m;
+      dp_init_col<GAP>(c, s, v, m);
+      sm[c] = make_float2((float)s, (float)m);
+      u[c] = (float)v;
       const int64_t ib = ib0 + (int64_t)step * c;
-      tc[c] = ((ib < lo || ib >= hi) ? kBadClass : base_class(tb[tstart + ib])) << 8;  // byte offset of its table row
+      tw[c / 4] |= dp_t_off(tab, (ib < lo || ib >= hi) ? 'X' : tb[tstart + ib]) << (8 * (c % 4));
     }
   }
-  // select end node (global mode), krnlAlignment.cu:170-185
-  __device__ __forceinline__ void end_node(int& best, int& best_m, int& ep) const {
+  __device__ __forceinline__ void shift_in(uint32_t t) {
+#pragma unroll
+    for (int i = 0; i + 1 < kWords; ++i) tw[i] = __funnelshift_r(tw[i], tw[i + 1], 8);
+    tw[kWords - 1] = (tw[kWords - 1] >> 8) | (t << (8 * ((W - 1) % 4)));
+  }
+  // select end node (global mode) after `rows` rows, krnlAlignment.cu:170-185
+  __device__ __forceinline__ void end_node(int rows, int& best, int& best_m, int& ep) const {
     best = kMarginScore;
     best_m = kMarginScore;
     ep = -1;
 #pragma unroll
     for (int c = 0; c < W; ++c) {
-      const int sc = A[c] - (kGapOpen + kGapExtend);
-      if (best < sc) { best = sc; best_m = M[c]; ep = c; }
+      const int sc = (int)sm[c].x - kStepRow * rows - kStepCol * c;
+      if (best < sc) { best = sc; best_m = (int)sm[c].y; ep = c; }
     }
   }
 };
 
 template <int GAP, bool LOCAL>
-__device__ __forceinline__ void banded_hit(const int2* __restrict__ tab, const char* __restrict__ tb, int64_t tstart,
+__device__ __forceinline__ void banded_hit(const DpTab<float2>& tab, const char* __restrict__ tb, int64_t tstart,
                                            int tlen, const char* __restrict__ qb, int64_t qstart, int qlen, int tidx,
                                            int qidx, int l, int& t_hl, int& q_hl, int& match, int& score,
                                            int& o_tidx, int& o_qidx) {
   constexpr int W = Band<GAP>::W;
-  constexpr int kGapSO = kGapOpen + kGapExtend;  // -7
-  constexpr int kBotA = (GAP + 1) * kGapExtend + kGapOpen + kGapSO;  // fixed band row 2*GAP+2
-  constexpr int kBotB = (GAP + 1) * kGapExtend + kGapOpen + kGapOpen + kGapExtend;
-  constexpr int kMarginA = kMarginScore + kGapSO, kMarginB = kMarginScore + kGapExtend;
   constexpr int kNoLow = INT_MIN / 2, kNoHigh = INT_MAX / 2;
+  constexpr float kOpen = (float)kOpenPot;
   const int rows_b = qlen - (qidx + l);  // alignmentSize of the backward pass
   const int rows_f = qidx;              // rows of the forward pass
   const int rows = rows_b + rows_f;
   Band<GAP> bd;
-  const char* __restrict__ t_seq = tb + tstart;
   // backward pass (globalAlignBackward / localAlignBackward): target bases
-  // tIdx + l - gap + q + c ('X' at or past tLen), query bases qIdx + l + q
-  const char* q_ptr = qb + qstart + qidx + l;  // query base of the current row
-  int q_step = 1;
-  int t_ib = tidx + l + GAP + 1;  // next target base to shift in
-  int t_step = 1;
-  int t_lo = kNoLow, t_hi = tlen;
-  int row_end = rows_b;  // last row + 1 of the current pass
-  bd.init(tb, tstart, (int64_t)tidx + l - GAP, 1, t_lo, t_hi);
-  int bs = 0, bm = 0, calc = -1, ep = GAP, qrow = 0;
+  // tIdx + l - gap + q + c ('X' at or past tLen), query bases qIdx + l + q.
+  // tp, qp: letters of the row after the next; they hold while r < t_end, q_end.
+  int64_t step = 1;
+  const char* __restrict__ tp = tb + tstart + tidx + l + GAP + 1;
+  const char* __restrict__ qp = qb + qstart + qidx + l;
+  int t_end = tlen - (tidx + l + GAP + 1), q_end = rows_b;
+  float2 w[W];  // the row's letter pairs, looked up one row ahead
+  uint32_t qo = 0;   // the row's query letter
+  char t_n, q_n;     // letters of the next row
+  // r0: the pass's first row
+  auto enter = [&](int r0) {
+    const char q0 = r0 < q_end ? *qp : 'N';
+    qp += step;
+    qo = dp_q_off(tab, q0);
+#pragma unroll
+    for (int c = 0; c < W; ++c) w[c] = dp_pair(tab, __dp4a(bd.tw[c / 4], 1u << (8 * (c % 4)), qo));
+    t_n = r0 < t_end ? *tp : 'X';
+    q_n = r0 + 1 < q_end ? *qp : 'N';
+    tp += step;
+    qp += step;
+    --t_end;
+    q_end -= 2;
+  };
+  bd.init(tab, tb, tstart, (int64_t)tidx + l - GAP, 1, kNoLow, tlen);
+  enter(0);
+  int bs = 0, bm = 0, calc = -1, ep = GAP;
   int pass = 0;
+  float lift = kStepRow;  // potential of the row's column 0: kStepRow * (row of the pass + 1)
   auto finish = [&](int pass_rows) {  // result of the pass that just ended
     int move, best, best_m, e;
     if (LOCAL) { best = bs; best_m = bm; e = ep; move = calc + 1; }
-    else { bd.end_node(best, best_m, e); move = pass_rows; }
+    else { bd.end_node(pass_rows, best, best_m, e); move = pass_rows; }
     e -= GAP;
     if (pass_rows != 0) {
       if (pass == 1) {  // forward: the hit's start moves
@@ -2022,63 +2125,56 @@ __device__ __forceinline__ void banded_hit(const int2* __restrict__ tab, const c
       score += best;
     }
   };
-  char q_cur = (rows_b > 0) ? *q_ptr : 'N';
+#pragma unroll 1
   for (int r = 0; r < rows; ++r) {
     if (r == rows_b) {  // switch to the forward pass (globalAlignForward / localAlignForward)
       finish(rows_b);
       pass = 1;
-      q_ptr = qb + qstart + qidx - 1;  // query bases qIdx - q - 1
-      q_step = -1;
-      t_ib = tidx - GAP - 2;  // target bases tIdx + gap - 1 - q - c ('X' below 0)
-      t_step = -1;
-      t_lo = 0;
-      t_hi = kNoHigh;
-      row_end = rows;
-      bd.init(tb, tstart, (int64_t)tidx + GAP - 1, -1, t_lo, t_hi);
-      bs = 0; bm = 0; calc = -1; ep = GAP; qrow = 0;
-      q_cur = *q_ptr;
+      step = -1;
+      qp = qb + qstart + qidx - 1;           // query bases qIdx - q - 1
+      tp = tb + tstart + tidx - GAP - 2;     // target bases tIdx + gap - 1 - q - c ('X' below 0)
+      t_end = r + tidx - GAP - 1;
+      q_end = rows;
+      bd.init(tab, tb, tstart, (int64_t)tidx + GAP - 1, -1, 0, kNoHigh);
+      enter(r);
+      bs = 0; bm = 0; calc = -1; ep = GAP;
+      lift = kStepRow;
     }
-    // loads for the next row go out first; their latency hides behind this row
-    const char t_next = (t_ib < t_lo || t_ib >= t_hi) ? 'X' : t_seq[t_ib];
-    t_ib += t_step;
-    const char q_next = (r + 1 < row_end) ? q_ptr[q_step] : 'N';
-    q_ptr += q_step;
-    // the query letter's column in every target row: one add per cell finds
-    // the (point + 7, match) pair (byte offsets; no index arithmetic)
-    const char* rowp = reinterpret_cast<const char*>(tab) + (base_class(q_cur) << 3);
-    int hA = kMarginA, hB = kMarginB, hM = kMarginScore;  // row 0 of the band (left margin)
+    // letters two rows ahead go out first
+    const char t_nn = r < t_end ? *tp : 'X', q_nn = r < q_end ? *qp : 'N';
+    tp += step;
+    qp += step;
+    bd.shift_in(dp_t_off(tab, t_n));  // 'X' is the bad-area letter itself
+    qo = dp_q_off(tab, q_n);
+    float h = lift + (float)(kDpLeftH<GAP> - kStepRow), mh = kMarginScore;  // row 0 of the band (left margin)
+    float top = -3e38f;                                                     // highest score of the row + lift (local)
+    const float vbot = lift + (float)(kDpBottomV<GAP> - kStepRow);
 #pragma unroll
     for (int c = 0; c < W; ++c) {
-      const int vA = (c + 1 < W) ? bd.A[(c + 1) % W] : kBotA;
-      const int vB = (c + 1 < W) ? bd.B[(c + 1) % W] : kBotB;
-      const int vM = (c + 1 < W) ? bd.M[(c + 1) % W] : 0;
-      const int nV = max(vA, vB);
-      const int nH = max(hA, hB);
-      const int2 w = *reinterpret_cast<const int2*>(rowp + bd.tc[c]);  // (POINT + 7, match increment)
-      const int pt = bd.A[c] + w.x;
-      // (plain compares and maxima: fewer instructions than __vibmax_s32 here)
-      const bool h_wins = nH >= nV;
-      const int mx = max(nH, nV);
-      const bool not_diag = mx >= pt;
-      const int nS = max(mx, pt);
-      const int side_m = h_wins ? hM : vM;
-      const int nM = not_diag ? side_m : (bd.M[c] + w.y);
-      const int nA = nS + kGapSO;
-      bd.A[c] = nA;
-      bd.B[c] = nV + kGapExtend;
-      bd.M[c] = nM;
-      hA = nA;
-      hB = nH + kGapExtend;
-      hM = nM;
-      if (LOCAL) {
-        if (bs < nS) { bs = nS; bm = nM; calc = qrow; ep = c; }
-      }
+      const float v = (c + 1 < W) ? bd.u[(c + 1) % W] : vbot;
+      const float vm = (c + 1 < W) ? bd.sm[(c + 1) % W].y : 0.0f;
+      const float2 d = make_float2(bd.sm[c].x + w[c].x, bd.sm[c].y + w[c].y);
+      w[c] = dp_pair(tab, __dp4a(bd.tw[c / 4], 1u << (8 * (c % 4)), qo));
+      const float S = max3_f32(d.x, v, h);
+      const float open = S + kOpen;
+      const float Q = S == v ? vm : d.y;
+      const float M = S == h ? mh : Q;
+      bd.sm[c] = make_float2(S, M);
+      bd.u[c] = fmaxf(open, v);
+      h = fmaxf(open, h);
+      mh = M;
+      if (LOCAL) top = fmaxf(S - (float)(kStepCol * c), top);
     }
+    if (LOCAL && top - lift > (float)bs) {  // the first column with the row's highest score
+      bs = (int)(top - lift);
+      calc = (int)lift / kStepRow - 1;
 #pragma unroll
-    for (int c = 0; c < W - 1; ++c) bd.tc[c] = bd.tc[c + 1];
-    bd.tc[W - 1] = base_class(t_next) << 8;  // 'X' above is the bad-area letter itself
-    q_cur = q_next;
-    ++qrow;
+      for (int c = W - 1; c >= 0; --c)
+        if (bd.sm[c].x - (float)(kStepCol * c) == top) { bm = (int)bd.sm[c].y; ep = c; }
+    }
+    t_n = t_nn;
+    q_n = q_nn;
+    lift += (float)kStepRow;
   }
   if (rows_b == rows) {  // the loop never switched: close the backward pass (rows_f == 0)
     finish(rows_b);
@@ -2087,36 +2183,31 @@ __device__ __forceinline__ void banded_hit(const int2* __restrict__ tab, const c
   }
 }
 
-// The same extension with one warp per hit: the band's anti-diagonal
-// wavefront.  Cell (r, c) of the band needs (r, c-1), (r-1, c+1) and (r-1, c),
+// The same extension with one warp per hit, in 32-bit integers: the band's
+// anti-diagonal wavefront.  Cell (r, c) of the band needs (r, c-1), (r-1, c+1) and (r-1, c),
 // so the cells with equal 2r + c are independent.  Lane j owns band columns 2j
 // and 2j + 1 and runs row r - j while lane 0 runs row r: column 2j at the even
-// step, taking its left neighbour from lane j - 1 (shuffle) and its upper-right
-// one from its own odd column; column 2j + 1 at the odd step, with its left
-// neighbour its own even column and its upper-right one from lane j + 1
-// (shuffle).  A row costs two steps instead of W dependent cells, which is
+// step, taking H and the match count left of it from lane j - 1 (shuffles) and
+// the vertical state from its own odd column; column 2j + 1 at the odd step,
+// with the vertical state and match count from lane j + 1 (shuffles).  A row's
+// dependent chain is two shuffles and four maxima instead of W cells, which is
 // what one long hit in a small batch waits for.  Same cell arithmetic as
 // banded_hit, same tie rules (the local best is the first maximum in
 // row-major order, the global end node the first maximum in column order),
 // so every output equals banded_hit's.  Results are returned in every lane.
+// A row takes 217 cycles alone (275 before H became a running maximum and the
+// letter pairs were looked up a row ahead): the two shuffles and the selects
+// between them.
 template <int GAP, bool LOCAL>
-__device__ __forceinline__ void banded_hit_warp(const int2* __restrict__ tab, const char* __restrict__ tb,
+__device__ __forceinline__ void banded_hit_warp(const DpTab<int2>& tab, const char* __restrict__ tb,
                                                 int64_t tstart, int tlen, const char* __restrict__ qb, int64_t qstart,
                                                 int qlen, int tidx, int qidx, int l, int& t_hl, int& q_hl, int& match,
                                                 int& score, int& o_tidx, int& o_qidx) {
   constexpr int W = 2 * GAP + 1;
-  constexpr int kGapSO = kGapOpen + kGapExtend;  // -7
-  constexpr int kBotA = (GAP + 1) * kGapExtend + kGapOpen + kGapSO;
-  constexpr int kBotB = (GAP + 1) * kGapExtend + kGapOpen + kGapOpen + kGapExtend;
-  constexpr int kMarginA = kMarginScore + kGapSO, kMarginB = kMarginScore + kGapExtend;
   const int lane = threadIdx.x & 31;
   const int ce = 2 * lane, co = 2 * lane + 1;  // this lane's band columns
   const bool has_e = ce < W, has_o = co < W;
-  // lane 0's left neighbour is lane 31 (GAP <= 16 leaves it idle), which holds
-  // the band's left margin; lane GAP, without an odd column, holds the fixed
-  // band row below the last column there instead
   const int left = (lane + 31) & 31, right = (lane + 1) & 31;
-  const char* tabb = reinterpret_cast<const char*>(tab);
   const char* __restrict__ t_seq = tb + tstart;
   const char* __restrict__ q_seq = qb + qstart;
   const int rows_b = qlen - (qidx + l);
@@ -2133,102 +2224,90 @@ __device__ __forceinline__ void banded_hit_warp(const int2* __restrict__ tab, co
     const int qi0 = pass == 0 ? qidx + l : qidx - 1;
     auto t_byte = [&](int ib) -> char { return (ib < lo || ib >= hi) ? 'X' : t_seq[ib]; };
     auto q_byte = [&](int r) -> char { return (unsigned)r < (unsigned)rows_p ? q_seq[qi0 + step * r] : 'N'; };
-    // initTempNodeArray for this lane's two columns (the state before row 0)
-    auto init_col = [&](int c, int& A, int& B, int& M) {
-      const int rr = c + 1;
-      int sc, v, m;
-      if (rr < GAP + 1) { sc = kMarginScore; v = kMarginScore; m = kMarginScore; }
-      else if (rr == GAP + 1) { sc = 0; v = kGapOpen; m = 0; }
-      else { sc = (rr - GAP - 1) * kGapExtend + kGapOpen; v = sc + kGapOpen; m = 0; }
-      A = sc + kGapSO;
-      B = v + kGapExtend;
-      M = m;
-    };
-    int eA, eB, eM, oA = 0, oB = 0, oM = 0, eH = 0, oH = 0;
-    init_col(ce, eA, eB, eM);
-    if (has_o) {
-      init_col(co, oA, oB, oM);
-    } else if (lane == 31) {
-      oA = kMarginA;
-      oH = kMarginB;
-      oM = kMarginScore;
-    } else {
-      oA = kBotA;
-      oB = kBotB;
-      oM = 0;
-    }
+    int se, ue, me, so, uo, mo;  // score, vertical state for the row below, matches of the two columns
+    dp_init_col<GAP>(ce, se, ue, me);
+    dp_init_col<GAP>(co, so, uo, mo);
+    int ho = 0;
     int bs = 0, bm = 0, calc = -1, ep = GAP;
     // Row r of this lane uses the target bases r + 2j (even column; the odd
     // column's base of row r - 1) and r + 2j + 1, and query base r.  Bytes are
-    // loaded four rows ahead and turned into table offsets one row ahead, so
-    // that no load's latency falls inside a row.
+    // loaded five rows ahead, turned into table offsets two rows ahead and
+    // into pairs one row ahead, so that no load's latency falls inside a row.
     int r = -lane;
-    int te = base_class(t_byte(ib0 + step * (r + ce))) << 8;
-    int to = base_class(t_byte(ib0 + step * (r + co))) << 8;
-    char t1 = t_byte(ib0 + step * (r + 1 + co)), t2 = t_byte(ib0 + step * (r + 2 + co));
-    char t3 = t_byte(ib0 + step * (r + 3 + co));
-    int qc = base_class(q_byte(r)) << 3;
-    char q1 = q_byte(r + 1), q2 = q_byte(r + 2), q3 = q_byte(r + 3);
-    int tk = ib0 + step * (r + 4 + co);
-    const int n_iter = rows_p + GAP;  // lane GAP runs the last row at rows_p - 1 + GAP
-#pragma unroll 2
-    for (int it = 0; it < n_iter; ++it, ++r) {
-      const char t4 = t_byte(tk);
+    const uint32_t t_a = dp_t_off(tab, t_byte(ib0 + step * (r + ce)));
+    const uint32_t t_b = dp_t_off(tab, t_byte(ib0 + step * (r + co)));
+    uint32_t t_c = dp_t_off(tab, t_byte(ib0 + step * (r + 1 + co)));  // odd column of row r + 1
+    const uint32_t q_a = dp_q_off(tab, q_byte(r));
+    uint32_t q_c = dp_q_off(tab, q_byte(r + 1));
+    int2 we = dp_pair(tab, t_a + q_a), wo = dp_pair(tab, t_b + q_a);
+    uint32_t t_even = t_b;  // even column of row r + 1
+    char t2 = t_byte(ib0 + step * (r + 2 + co)), t3 = t_byte(ib0 + step * (r + 3 + co));
+    char t4 = t_byte(ib0 + step * (r + 4 + co));
+    char q2 = q_byte(r + 2), q3 = q_byte(r + 3), q4 = q_byte(r + 4);
+    int tk = ib0 + step * (r + 5 + co);
+    int lift = kStepRow * (r + 1);
+    // One row.  EDGE: some lanes may be outside the pass's rows and keep their state.
+    auto row = [&](auto edge) {
+      constexpr bool EDGE = decltype(edge)::value;
+      const int hl = __shfl_sync(kFull, ho, left), ml = __shfl_sync(kFull, mo, left);
+      const char t5 = t_byte(tk);
+      const char q5 = q_byte(r + 5);
       tk += step;
-      const char q4 = q_byte(r + 4);
-      const bool on = (unsigned)r < (unsigned)rows_p;
-      {  // even step: column 2j of row r; left neighbour from lane j - 1, upper right from our odd column
-        const int hA = __shfl_sync(kFull, oA, left);
-        const int hB = __shfl_sync(kFull, oH, left);
-        const int hM = __shfl_sync(kFull, oM, left);
-        const int nV = max(oA, oB);
-        const int nH = max(hA, hB);
-        const int2 w = *reinterpret_cast<const int2*>(tabb + te + qc);
-        const int pt = eA + w.x;
-        const bool h_wins = nH >= nV;
-        const int mx = max(nH, nV);
-        const bool not_diag = mx >= pt;
-        const int nS = max(mx, pt);
-        const int nM = not_diag ? (h_wins ? hM : oM) : (eM + w.y);
-        if (on && has_e) {
-          eA = nS + kGapSO;
-          eB = nV + kGapExtend;
-          eH = nH + kGapExtend;
-          eM = nM;
-          if (LOCAL && bs < nS) { bs = nS; bm = nM; calc = r; ep = ce; }
+      const int2 we_n = dp_pair(tab, t_even + q_c), wo_n = dp_pair(tab, t_c + q_c);
+      const bool on = !EDGE || (unsigned)r < (unsigned)rows_p;
+      // even step: column 2j; H from lane j - 1, the vertical state from our
+      // odd column (below the last column: the fixed band row)
+      const int ve = has_o ? uo : kDpBottomV<GAP> - kStepRow + lift;
+      const int Pe = __viaddmax_s32(se, we.x, ve);
+      const int Qe = Pe == ve ? (has_o ? mo : 0) : me + we.y;
+      const int h = lane == 0 ? kDpLeftH<GAP> - kStepRow + lift : hl;
+      const int mh = lane == 0 ? kMarginScore : ml;
+      const int Se = max(Pe, h);
+      const int Me = Se == h ? mh : Qe;
+      const int Ue = __viaddmax_s32(Se, kOpenPot, ve);
+      const int he = __viaddmax_s32(Pe, kOpenPot, h);
+      if (on) {
+        se = Se;
+        ue = Ue;
+        me = Me;
+      }
+      // odd step: column 2j + 1; the vertical state from lane j + 1
+      const int vo = __shfl_sync(kFull, ue, right), vm = __shfl_sync(kFull, me, right);
+      const int Po = __viaddmax_s32(so, wo.x, vo);
+      const int Qo = Po == vo ? vm : mo + wo.y;
+      const int So = max(Po, he);
+      const int Mo = So == he ? Me : Qo;
+      if (on) {
+        so = So;
+        uo = __viaddmax_s32(So, kOpenPot, vo);
+        mo = Mo;
+        ho = __viaddmax_s32(Po, kOpenPot, he);
+        if (LOCAL) {
+          const int xe = Se - lift - kStepCol * ce, xo = So - lift - kStepCol * co;
+          if (has_e && xe > bs) { bs = xe; bm = Me; calc = r; ep = ce; }
+          if (has_o && xo > bs) { bs = xo; bm = Mo; calc = r; ep = co; }
         }
       }
-      {  // odd step: column 2j + 1 of row r; left neighbour our even column, upper right from lane j + 1
-        const int vA = __shfl_sync(kFull, eA, right);
-        const int vB = __shfl_sync(kFull, eB, right);
-        const int vM = __shfl_sync(kFull, eM, right);
-        const int nV = max(vA, vB);
-        const int nH = max(eA, eH);
-        const int2 w = *reinterpret_cast<const int2*>(tabb + to + qc);
-        const int pt = oA + w.x;
-        const bool h_wins = nH >= nV;
-        const int mx = max(nH, nV);
-        const bool not_diag = mx >= pt;
-        const int nS = max(mx, pt);
-        const int nM = not_diag ? (h_wins ? eM : vM) : (oM + w.y);
-        if (on && has_o) {
-          oA = nS + kGapSO;
-          oB = nV + kGapExtend;
-          oH = nH + kGapExtend;
-          oM = nM;
-          if (LOCAL && bs < nS) { bs = nS; bm = nM; calc = r; ep = co; }
-        }
-      }
-      te = to;
-      to = base_class(t1) << 8;
-      t1 = t2;
+      we = we_n;
+      wo = wo_n;
+      t_even = t_c;
+      t_c = dp_t_off(tab, t2);
+      q_c = dp_q_off(tab, q2);
       t2 = t3;
       t3 = t4;
-      qc = base_class(q1) << 3;
-      q1 = q2;
+      t4 = t5;
       q2 = q3;
       q3 = q4;
-    }
+      q4 = q5;
+      lift += kStepRow;
+      ++r;
+    };
+    // lane GAP starts GAP rows after lane 0 and ends GAP rows after it
+    const int n_ramp = min(GAP, rows_p);
+    for (int it = 0; it < n_ramp; ++it) row(std::true_type());
+#pragma unroll 2
+    for (int it = n_ramp; it < rows_p; ++it) row(std::false_type());
+    for (int it = 0; it < GAP; ++it) row(std::true_type());
     int best, best_m, e, move;
     if (LOCAL) {  // first maximum in row-major order: (score desc, row asc, column asc)
 #pragma unroll
@@ -2243,8 +2322,9 @@ __device__ __forceinline__ void banded_hit_warp(const int2* __restrict__ tab, co
       move = calc + 1;
     } else {  // end node: the first column of the last row with the highest score above the margin
       int sc = INT_MIN, c = W, m = 0;
-      if (has_e) { sc = eA - kGapSO; c = ce; m = eM; }
-      if (has_o && oA - kGapSO > sc) { sc = oA - kGapSO; c = co; m = oM; }
+      if (has_e) { sc = se - kStepRow * rows_p - kStepCol * ce; c = ce; m = me; }
+      const int sco = so - kStepRow * rows_p - kStepCol * co;
+      if (has_o && sco > sc) { sc = sco; c = co; m = mo; }
 #pragma unroll
       for (int off = 16; off; off >>= 1) {
         const int xs = __shfl_xor_sync(kFull, sc, off), xc = __shfl_xor_sync(kFull, c, off);
@@ -2296,16 +2376,6 @@ __device__ __forceinline__ int64_t dp_warp_hits(const DpKernelArgs& a) {
   return w < a.n ? w : a.n;
 }
 
-// The letter-pair table (POINT + 7, match increment) of krnlMatrix.cuh in
-// shared memory: [target letter][query letter], letters 'A'..'Z'.
-__device__ __forceinline__ void dp_table_init(int2* tab) {
-  for (int i = threadIdx.x; i < 32 * 32; i += blockDim.x) {
-    const int2 w = cell_score(class_of_letter((i >> 5) < 26 ? (i >> 5) : kNClass),
-                              class_of_letter((i & 31) < 26 ? (i & 31) : kNClass));
-    tab[i] = make_int2(w.x - (kGapOpen + kGapExtend), w.y);
-  }
-}
-
 // calculateEvalue (krnlCalculateEvalue.cu:21, same operation order) and the
 // two hit filters of deleteBadHits, then the hit's outputs at its own index.
 __device__ __forceinline__ void dp_store(const DpKernelArgs& a, int64_t h, int qlen, int o_tidx, int o_qidx, int t_hl,
@@ -2332,7 +2402,7 @@ __device__ __forceinline__ void dp_skip(const DpKernelArgs& a, int64_t h) {
 // Extension of the hit at position i of the order (alignmentHits +
 // calculateEvalue + the two hit filters of deleteBadHits).
 template <int GAP, bool LOCAL>
-__device__ __forceinline__ void dp_one(const DpKernelArgs& a, const int2* tab, int64_t i) {
+__device__ __forceinline__ void dp_one(const DpKernelArgs& a, const DpTab<float2>& tab, int64_t i) {
   const int64_t h = a.order ? (int64_t)(uint32_t)a.order[i] : i;
   const uint64_t k = a.hk[h];
   const int qidx = a.hq[h];
@@ -2355,38 +2425,48 @@ __device__ __forceinline__ void dp_one(const DpKernelArgs& a, const int2* tab, i
   dp_store(a, h, qlen, o_tidx, o_qidx, t_hl, q_hl, match, score);
 }
 
-template <int GAP, bool LOCAL>
-__global__ void __launch_bounds__(128, GAP <= 9 ? 4 : (GAP <= 12 ? 3 : 2)) k_banded_dp(DpKernelArgs a) {
-  __shared__ int2 tab[32 * 32];
-  dp_table_init(tab);
-  __syncthreads();
-  const int64_t i = dp_warp_hits(a) + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  dp_one<GAP, LOCAL>(a, tab, i);
-}
+// A block extends kDpThreads * rounds consecutive hits of the order.  With
+// `by_rows` (hits of equal length, in no order of their own) it first sorts
+// them by the rows of the forward pass, so that the lanes of a warp leave the
+// backward pass at the same row: the switch (end node, new band, its letters)
+// is some 350 instructions that every lane leaving at a row of its own would
+// run alone (3.63 to 3.44 ms on a million reads of 150 bp).
+constexpr int kDpThreads = 128, kDpMaxRounds = 4;
+// Blocks per SM by the registers the band takes (natural: 96 at gap 2, 194 at
+// gap 8, 254 at gap 16).  At gap 8, three blocks of up to 168 registers run
+// the uneven reads in 16.1 ms against 17.2 for four of 128: what the fourth
+// block hides, its register moves cost again.
+template <int GAP>
+constexpr int kDpBlocksPerSm = GAP <= 4 ? 4 : (GAP <= 9 ? 3 : 2);
 
-// Persistent form: a grid that fills the GPU once; each warp takes the next
-// `chunk` x 32 hits of the order (longest first) from a queue head until the
-// queue is empty, so that warps which drew short hits go on to take more
-// while the long ones run.  No warp waits on another.
 template <int GAP, bool LOCAL>
-__global__ void __launch_bounds__(128, GAP <= 9 ? 4 : (GAP <= 12 ? 3 : 2))
-    k_banded_dp_queue(DpKernelArgs a, unsigned long long* __restrict__ head, int chunk) {
-  __shared__ int2 tab[32 * 32];
+__global__ void __launch_bounds__(kDpThreads, kDpBlocksPerSm<GAP>)
+    k_banded_dp(DpKernelArgs a, int rounds, int by_rows) {
+  __shared__ DpTab<float2> tab;
+  __shared__ uint32_t key[kDpThreads * kDpMaxRounds];  // forward rows << 16 | hit within the block
   dp_table_init(tab);
+  const int64_t base = dp_warp_hits(a) + (int64_t)blockIdx.x * (kDpThreads * rounds);
+  const int n = kDpThreads * rounds;  // a power of two
+  if (by_rows) {
+    for (int i = threadIdx.x; i < n; i += kDpThreads)
+      key[i] = base + i < a.n ? ((uint32_t)min(a.hq[base + i], 0xfffe) << 16) | (uint32_t)i : ~0u;
+    for (int size = 2; size <= n; size <<= 1)
+      for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < n / 2; i += kDpThreads) {
+          const int lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
+          const uint32_t x = key[lo], y = key[hi];
+          if ((x > y) == ((lo & size) == 0)) {
+            key[lo] = y;
+            key[hi] = x;
+          }
+        }
+      }
+  }
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const unsigned long long take = 32ull * (unsigned long long)chunk;
-  const int64_t first = dp_warp_hits(a);  // the hits before it run one per warp
-  for (;;) {
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(head, take);
-    base = __shfl_sync(kFull, base, 0);
-    if (first + (int64_t)base >= a.n) break;
-    for (int c = 0; c < chunk; ++c) {
-      const int64_t i = first + (int64_t)base + 32 * c + lane;
-      if (i < a.n) dp_one<GAP, LOCAL>(a, tab, i);
-    }
+  for (int i = threadIdx.x; i < n; i += kDpThreads) {
+    const int64_t at = base + (by_rows ? (int64_t)(key[i] & 0xffffu) : (int64_t)i);
+    if (at < a.n && !(by_rows && key[i] == ~0u)) dp_one<GAP, LOCAL>(a, tab, at);
   }
 }
 
@@ -2394,7 +2474,7 @@ __global__ void __launch_bounds__(128, GAP <= 9 ? 4 : (GAP <= 12 ? 3 : 2))
 // the longest ones: a grid-stride loop over them, one warp each.
 template <int GAP, bool LOCAL>
 __global__ void __launch_bounds__(128) k_banded_dp_warp(DpKernelArgs a) {
-  __shared__ int2 tab[32 * 32];
+  __shared__ DpTab<int2> tab;
   dp_table_init(tab);
   __syncthreads();
   const int64_t nw = dp_warp_hits(a);
@@ -2424,7 +2504,7 @@ __global__ void __launch_bounds__(128) k_banded_dp_warp(DpKernelArgs a) {
   }
 }
 
-// Length buckets of the hits for the DP order: 16 buckets per power of two of
+// Length buckets of the hits for the warp / thread split: 16 buckets per power of two of
 // the row count (rows within a bucket differ by at most 1/16), numbered so
 // that ascending bucket = longest first.
 constexpr int kDpBuckets = 16 * 33;
@@ -2483,10 +2563,10 @@ __host__ __device__ __forceinline__ long long dp_bucket_hi(int b) {
 // sub-partition, and the GPU cannot issue faster than I).  Forking the second
 // stream and the launch cost kDpLaunchCycles.  Only the split depends on
 // these; results do not.
-constexpr double kDpThreadCellCycles = 34.0;
-constexpr double kDpThreadCellsPerCycle = 490.0;
-constexpr double kDpWarpRowCycles = 289.0;
-constexpr double kDpWarpRowsPerCycle = 4.7;
+constexpr double kDpThreadCellCycles = 26.0;
+constexpr double kDpThreadCellsPerCycle = 1000.0;
+constexpr double kDpWarpRowCycles = 217.0;
+constexpr double kDpWarpRowsPerCycle = 6.0;
 constexpr double kDpLaunchCycles = 10000.0;
 constexpr long long kDpWarpMinRows = 16;
 
@@ -2533,33 +2613,10 @@ __global__ void k_dp_warp_split(const unsigned int* __restrict__ count, const un
   *warp_n = best_s;
 }
 
-// exclusive scan of the bucket counts in one block (kDpBuckets <= 1024)
-__global__ void k_dp_bucket_scan(const unsigned int* __restrict__ count, unsigned long long* __restrict__ cursor) {
-  __shared__ unsigned long long v[1024];
-  const int i = threadIdx.x;
-  v[i] = i < kDpBuckets ? count[i] : 0;
-  __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    const unsigned long long x = i >= o ? v[i - o] : 0;
-    __syncthreads();
-    v[i] += x;
-    __syncthreads();
-  }
-  if (i < kDpBuckets) cursor[i] = v[i] - count[i];
-}
-
-__global__ void k_dp_bucket_scatter(const int32_t* __restrict__ hs, const int32_t* __restrict__ q_len, int64_t n,
-                                    int l, unsigned long long* __restrict__ cursor, uint64_t* __restrict__ order) {
-  const int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (h >= n) return;
-  const unsigned long long at = atomicAdd(&cursor[dp_bucket(max(0, q_len[hs[h]] - l))], 1ull);
-  order[at] = (uint64_t)h;
-}
-
 template <int GAP, bool LOCAL>
 long long launch_dp_mode(DpKernelArgs a, const DpLaunch& m, cudaStream_t st) {
   constexpr int W = 2 * GAP + 1;
-  const int threads = 128;
+  const int threads = kDpThreads;
   struct Occupancy {
     int sms = 0, per_sm = 1, warp_per_sm = 1;
   };
@@ -2568,8 +2625,8 @@ long long launch_dp_mode(DpKernelArgs a, const DpLaunch& m, cudaStream_t st) {
     int dev = 0;
     CLAST_CK(cudaGetDevice(&dev));
     CLAST_CK(cudaDeviceGetAttribute(&o.sms, cudaDevAttrMultiProcessorCount, dev));
-    CLAST_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.per_sm, k_banded_dp_queue<GAP, LOCAL>, 128, 0));
-    CLAST_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.warp_per_sm, k_banded_dp_warp<GAP, LOCAL>, 128, 0));
+    CLAST_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.per_sm, k_banded_dp<GAP, LOCAL>, kDpThreads, 0));
+    CLAST_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.warp_per_sm, k_banded_dp_warp<GAP, LOCAL>, kDpThreads, 0));
     o.per_sm = std::max(1, o.per_sm);
     o.warp_per_sm = std::max(1, o.warp_per_sm);
     return o;
@@ -2612,17 +2669,12 @@ long long launch_dp_mode(DpKernelArgs a, const DpLaunch& m, cudaStream_t st) {
   }
   const long long warp_hits = a.warp_n ? -1 : a.warp_fixed;
   if (rest <= 0) return warp_hits;
-  // a batch that fits in one wave of the grid runs one hit per thread: the
-  // queue's takes of several hits per lane would only lengthen the longest
-  if (m.head == nullptr || rest <= (int64_t)sms * per_sm * threads) {
-    const unsigned grid = (unsigned)((rest + threads - 1) / threads);
-    k_banded_dp<GAP, LOCAL><<<grid, threads, 0, st>>>(a);
-  } else {
-    const int64_t need = (rest + 32 * m.chunk - 1) / (32 * m.chunk) / (threads / 32) + 1;
-    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)sms * per_sm, need));
-    CLAST_CK(cudaMemsetAsync(m.head, 0, sizeof(unsigned long long), st));
-    k_banded_dp_queue<GAP, LOCAL><<<grid, threads, 0, st>>>(a, m.head, m.chunk);
-  }
+  // blocks of several rounds sort more hits together; short batches need the blocks
+  const bool by_rows = m.uniform_rows >= 0;
+  const int64_t waves = rest / ((int64_t)sms * per_sm * threads);
+  const int rounds = !by_rows ? 1 : waves >= 8 ? kDpMaxRounds : waves >= 4 ? 2 : 1;
+  const unsigned grid = (unsigned)((rest + threads * rounds - 1) / (threads * rounds));
+  k_banded_dp<GAP, LOCAL><<<grid, threads, 0, st>>>(a, rounds, by_rows);
   CLAST_LAUNCHED();
   if (joined) CLAST_CK(cudaStreamWaitEvent(st, m.ev_join, 0));
   return warp_hits;
@@ -3059,18 +3111,6 @@ DpBuckets dp_bucket_count(Workspace& ws, const int32_t* hs, const int32_t* q_len
   DpBuckets b;
   b.count = count;
   b.rows = rows;
-  return b;
-}
-
-DpBuckets dp_bucket_order(Workspace& ws, const int32_t* hs, const int32_t* q_len, int64_t n_hits, int l,
-                          uint64_t* order, cudaStream_t st) {
-  const DpBuckets b = dp_bucket_count(ws, hs, q_len, n_hits, l, st);
-  if (n_hits <= 0) return b;
-  unsigned long long* cursor = ws.get<unsigned long long>("dpb_cursor", kDpBuckets);
-  k_dp_bucket_scan<<<1, 1024, 0, st>>>(b.count, cursor);
-  CLAST_LAUNCHED();
-  k_dp_bucket_scatter<<<blocks_for(n_hits, 256), 256, 0, st>>>(hs, q_len, n_hits, l, cursor, order);
-  CLAST_LAUNCHED();
   return b;
 }
 

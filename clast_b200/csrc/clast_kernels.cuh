@@ -132,12 +132,10 @@ struct DpParams {
   int l, stride, gap, local;
   double cutoff, total_db, K, lambda;
 };
-// How the DP kernel is launched: one thread per hit over a grid of all hits
-// (head null), or a persistent grid whose warps take `chunk` x 32 hits at a
-// time from a queue (head: a device counter the launch zeroes).  Results are
-// the same either way.
+// How the DP is launched: one thread per hit over a grid of all hits, in blocks
+// that sort hits of one length (uniform_rows) by the rows of their forward pass.
 //
-// Independently of that, the first hits of the order (the longest, when the
+// The first hits of the order (the longest, when the
 // order is longest first) may run one per warp (an anti-diagonal wavefront
 // over the band) instead of one per thread: a long hit alone takes about 1/7
 // of the time there, at a lower throughput per cell.  `warp` says how many:
@@ -147,13 +145,16 @@ struct DpParams {
 // none on the host; kDpWarpOff runs every hit one per thread, kDpWarpAll one
 // per warp.  Results are the same either way.
 constexpr int kDpWarpAuto = 0, kDpWarpOff = 1, kDpWarpAll = 2;
+// Longest read the one-per-thread kernel takes: it holds whole numbers in
+// floats, which are exact below 2^24, and a pass of r rows stays within
+// 5 r + 34,000 of zero (potentials rise by up to 5 per row from margins of
+// -30,000).  Longer reads run one hit per warp, in 32-bit integers.
+constexpr int kDpMaxThreadLen = 1 << 20;
 struct DpBuckets {
   const unsigned int* count = nullptr;      // hits per length bucket (longest first)
   const unsigned long long* rows = nullptr;  // their rows, summed
 };
 struct DpLaunch {
-  unsigned long long* head = nullptr;
-  int chunk = 1;
   int warp = kDpWarpAuto;
   DpBuckets buckets;
   long long* warp_n = nullptr;  // device word for the split (with buckets)
@@ -177,10 +178,6 @@ long long banded_dp(const TargetView& t, const QueryView& q, const uint64_t* hk,
 // first) and their row sums, in the workspace.
 DpBuckets dp_bucket_count(Workspace& ws, const int32_t* hs, const int32_t* q_len, int64_t n_hits, int l,
                           cudaStream_t st);
-// DP order by length buckets: order[k] = hit index, in one counting pass
-// instead of a sort (the counts of dp_bucket_count, which it runs).
-DpBuckets dp_bucket_order(Workspace& ws, const int32_t* hs, const int32_t* q_len, int64_t n_hits, int l,
-                          uint64_t* order, cudaStream_t st);
 // CLAST_DP_WARP=off|all, else `fallback` (the environment overrides a
 // context's setting, for tests and measurements).
 int dp_warp_mode_from_env(int fallback);
