@@ -198,35 +198,49 @@ clast_index* make_index(clast_ctx* c, const clast_params* p, const char* bases, 
   return ix.release();
 }
 
-// Device-resident query strands of one batch, packed once for every index.
+// Device-resident query strands of one batch, packed once for every index: one
+// allocation with the padded bases, the 2-bit words and the strand tables.
 struct QueryRef;
 
 struct QueryBatch {
-  DevArray<char> bases;  // padded
+  DevArray<char> mem;
+  char* bases = nullptr;  // padded
   int64_t n = 0;
-  DevArray<int64_t> start;
-  DevArray<int32_t> len;
-  DevArray<uint64_t> packed, nmask;
+  int64_t* start = nullptr;
+  int32_t* len = nullptr;
+  uint64_t *packed = nullptr, *nmask = nullptr;
   int32_t nstrands = 0;
-  DevArray<int32_t> wstart;  // strand index where each window starts, plus the end
+  char* meta = nullptr;             // the caller's tables, directly behind len
+  const int32_t* wstart = nullptr;  // strand index where each window starts, plus the end
   int32_t nwin = 0;
   int32_t min_len = 0, max_len = 0;  // strand lengths (the DP orders hits by rows when they differ)
+  static size_t al(size_t b) { return (b + 255) & ~size_t(255); }
+  void alloc(int64_t n_bases, int64_t strands, size_t meta_bytes) {
+    n = n_bases;
+    nstrands = (int32_t)strands;
+    const size_t sz[5] = {al((size_t)n + 2 * kPad), al((size_t)(n / 32 + 4) * 8), al((size_t)(n / 64 + 4) * 8),
+                          al((size_t)strands * 8), al((size_t)strands * 4)};
+    mem.alloc(sz[0] + sz[1] + sz[2] + sz[3] + sz[4] + meta_bytes);
+    char* at = mem.p;
+    bases = at;
+    packed = reinterpret_cast<uint64_t*>(at += sz[0]);
+    nmask = reinterpret_cast<uint64_t*>(at += sz[1]);
+    start = reinterpret_cast<int64_t*>(at += sz[2]);
+    len = reinterpret_cast<int32_t*>(at += sz[3]);
+    meta = at + sz[4];
+  }
   QueryView view() const {
     QueryView q;
-    q.bases = bases.p + kPad;
+    q.bases = bases + kPad;
     q.n = n;
-    q.packed = packed.p;
-    q.nmask = nmask.p;
-    q.start = start.p;
-    q.len = len.p;
+    q.packed = packed;
+    q.nmask = nmask;
+    q.start = start;
+    q.len = len;
     q.nstrands = nstrands;
     return q;
   }
-  void pack(cudaStream_t st) {
-    packed.alloc((size_t)(n / 32 + 4));
-    nmask.alloc((size_t)(n / 64 + 4));
-    pack_bases(bases.p + kPad, n, packed.p, nmask.p, st);
-  }
+  void pack(cudaStream_t st) { pack_bases(bases + kPad, n, packed, nmask, st); }
   QueryRef ref() const;
 };
 
@@ -238,197 +252,142 @@ struct QueryRef {
   const int32_t* wstart = nullptr;   // strand where each query window starts, plus the end
   int32_t nwin = 0;
   int32_t min_len = 0, max_len = 0;  // strand lengths (the DP orders hits by rows when they differ)
+  const int32_t* lens = nullptr;     // the same on the host once the stream has run so far, when given
 };
 
 QueryRef QueryBatch::ref() const {
   QueryRef r;
   r.q = view();
   r.n = n;
-  r.wstart = wstart.p;
+  r.wstart = wstart;
   r.nwin = nwin;
   r.min_len = min_len;
   r.max_len = max_len;
   return r;
 }
 
-// Host copy of one batch's result (reference order within each query window).
-// One batch's hits on the device, reads ascending (reference order within
-// every query window), with per-read offsets.
-struct DevHits {
-  int64_t n = 0;
-  DevArray<int32_t> t_id, t_idx, q_id, q_idx, t_len, q_len, match, score;
-  DevArray<double> evalue;
-  DevArray<int64_t> foff;
-};
-
-// Seeds of one target window for a query batch (createRawSeedList +
-// deleteSeedsOnSequenceBoundary), in the workspace slots of `slot`.
-struct SeedSet {
-  const clast_index* ix = nullptr;
-  int64_t* off = nullptr;
-  int32_t* len32 = nullptr;
-  int32_t* nvalid = nullptr;
-  unsigned long long* counters = nullptr;  // [1] DP cells, then seed_parts() cursors and l-mer counters
-  uint64_t* skey = nullptr;
-  uint32_t* sq = nullptr;
-  int64_t part_cap = 0;
-  int64_t S = 0;
-};
-
-// Seeds of up to kMaxSeedWins windows (all of `sets`) in one pass over the
-// query: the 2-bit words are read once and every l-mer's lookups in all the
-// windows are issued together.  A window whose seed partition overflowed is
-// seeded again (alone with the others that overflowed) with partitions sized
-// from the exact counts.
-void seed_windows(clast_ctx* c, const clast_params* p, const QueryRef& qb, std::vector<SeedSet>& sets) {
-  cudaStream_t st = c->st;
-  Workspace& ws = c->ws;
-  const QueryView q = qb.q;
-  const int64_t ns = q.nstrands;
-  const int parts = seed_parts();
-  StageTimer& tm = c->timer;
-  std::vector<int> todo;
-  for (size_t k = 0; k < sets.size(); ++k) {
-    SeedSet& z = sets[k];
-    const std::string tag = "#" + std::to_string(k);
-    z.off = ws.get<int64_t>("s_off" + tag, ns + 1);
-    z.len32 = ws.get<int32_t>("s_len32" + tag, ns);
-    z.nvalid = ws.get<int32_t>("s_nvalid" + tag, ns);
-    z.counters = ws.get<unsigned long long>("s_counters" + tag, 2 + 2 * parts);
-    z.part_cap = std::max<int64_t>(c->seed_hint, qb.n / 16 + (1 << 20)) / parts + 1;
-    todo.push_back((int)k);
-  }
-  for (int attempt = 0; attempt < 2 && !todo.empty(); ++attempt) {
-    SeedWins W{};
-    for (size_t j = 0; j < todo.size(); ++j) {
-      SeedSet& z = sets[todo[j]];
-      const std::string tag = "#" + std::to_string(todo[j]);
-      z.skey = ws.get<uint64_t>("s_key" + tag, (size_t)z.part_cap * parts);
-      z.sq = ws.get<uint32_t>("s_q" + tag, (size_t)z.part_cap * parts);
-      CLAST_CK(cudaMemsetAsync(z.counters, 0, (2 + 2 * parts) * sizeof(unsigned long long), st));
-      W.w[j] = SeedWin{z.ix->view(), z.ix->tview(), z.counters + 2, z.counters + 2 + parts, z.off, z.len32,
-                       z.nvalid, z.skey, z.sq, z.part_cap};
-    }
-    tm.begin(st);
-    static const bool force_multi = std::getenv("CLAST_SEED_MULTI_ONLY") != nullptr;
-    if (todo.size() == 1 && !force_multi) {  // one window: the single-window kernel (round 0 staged while its range is reserved)
-      const SeedWin& w = W.w[0];
-      seed_fused(q, w.ix, w.t, p->gap, p->local, w.cursor, w.n_kmers, w.off, w.cnt, w.nvalid, w.skey, w.sq,
-                 w.part_cap, st);
-    } else {
-      seed_multi(q, W, (int)todo.size(), p->gap, p->local, st);
-    }
-    tm.end(StageTimer::SEED, st);
-    std::vector<unsigned long long> cur(todo.size() * 2 * parts);
-    for (size_t j = 0; j < todo.size(); ++j)
-      CLAST_CK(cudaMemcpyAsync(cur.data() + j * 2 * parts, sets[todo[j]].counters + 2,
-                               2 * parts * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    CLAST_CK(cudaStreamSynchronize(st));
-    std::vector<int> again;
-    for (size_t j = 0; j < todo.size(); ++j) {
-      SeedSet& z = sets[todo[j]];
-      const unsigned long long* cj = cur.data() + j * 2 * parts;
-      int64_t S = 0, most = 0, kmers = 0;
-      for (int i = 0; i < parts; ++i) {
-        S += (int64_t)cj[i];
-        most = std::max<int64_t>(most, (int64_t)cj[i]);
-        kmers += (int64_t)cj[parts + i];
-      }
-      z.S = S;
-      if (most <= z.part_cap) {
-        c->stats.query_kmers += kmers;
-        c->seed_hint = std::max<int64_t>(c->seed_hint, S + S / 4);
-      } else {
-        z.part_cap = most;  // strands past a full partition wrote nothing: run again
-        again.push_back(todo[j]);
-      }
-    }
-    todo.swap(again);
-  }
-  if (!todo.empty()) throw std::runtime_error("seed partitions overflowed twice");
-}
-
-// Where search_seeded puts a window's final hits: take(F, foff, nr) returns
-// the arrays for its F hits (and may keep the nr + 1 per-read offsets), or
-// throws when they do not fit.
+// Where search_group puts a group's final hits: take(F, foff, nr) returns the
+// arrays for its F hits (and may keep the nr + 1 per-read offsets), or throws
+// when they do not fit.
 struct HitSink {
   virtual ~HitSink() = default;
-  virtual FinalOut take(int64_t F, const int64_t* foff, int64_t nr, cudaStream_t st) = 0;
+  virtual OutView take(int64_t F, const int64_t* foff, int64_t nr, cudaStream_t st) = 0;
 };
 
-// Device arrays of their own, with the per-read offsets (clast_search,
-// clast_map).
-struct DevHitsSink : HitSink {
-  DevHits& out;
-  explicit DevHitsSink(DevHits& o) : out(o) { out = DevHits(); }
-  FinalOut take(int64_t F, const int64_t* foff, int64_t nr, cudaStream_t st) override {
-    out.n = F;
-    out.t_id.alloc(F); out.t_idx.alloc(F); out.q_id.alloc(F); out.q_idx.alloc(F); out.t_len.alloc(F);
-    out.q_len.alloc(F); out.match.alloc(F); out.score.alloc(F); out.evalue.alloc(F);
-    out.foff.alloc(nr + 1);
-    CLAST_CK(cudaMemcpyAsync(out.foff.p, foff, (nr + 1) * sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
-    return FinalOut{out.t_id.p, out.t_idx.p, out.q_id.p, out.q_idx.p, out.t_len.p, out.q_len.p, out.match.p,
-                    out.score.p, out.evalue.p};
-  }
+// A group of target windows searched together, and the limits of its seed
+// partitions.
+struct Group {
+  int nw = 0;
+  const clast_index* ix[kMaxSeedWins] = {};
+  int32_t load[kMaxSeedWins] = {};
+  int64_t part_cap = 0;           // seeds per partition to begin with
+  int64_t part_fit = INT64_MAX;   // most the scratch holds (arena mode)
 };
 
-// CDeviceHitList for every query window of `qb` against the window whose
-// seeds are in z: seed filters, DP, result order.
-int64_t search_seeded(clast_ctx* c, Workspace& ws, const clast_params* p, const QueryRef& qb, int32_t q_first,
-                      SeedSet& z, HitSink& sink) {
+// Host copy of the group's counters: waits for the stream.
+const GroupCtl& read_ctl(clast_ctx* c, const GroupCtl* dev, cudaStream_t st) {
+  if (!c->ctl) CLAST_CK(cudaMallocHost(reinterpret_cast<void**>(&c->ctl), sizeof(GroupCtl)));
+  CLAST_CK(cudaMemcpyAsync(c->ctl, dev, sizeof(GroupCtl), cudaMemcpyDeviceToHost, st));
+  CLAST_CK(cudaStreamSynchronize(st));
+  return *c->ctl;
+}
+
+// CDeviceHitList for every query window of `qb` against every window of the
+// group: seeds, seed filters, DP, result order.  The host waits twice, for the
+// hit count and for the result count; every stage runs once for all windows of
+// the group, so a small batch pays for some fifteen launches instead of
+// twenty-odd per window.  A group whose seed partitions overflowed is seeded
+// again with partitions sized from the exact counts.  Returns the results.
+int64_t search_group(clast_ctx* c, Workspace& ws, const clast_params* p, const QueryRef& qb, Group& g, HitSink& sink) {
   cudaStream_t st = c->st;
-  const clast_index* ix = z.ix;
   const QueryView q = qb.q;
-  const TargetView tv = ix->tview();
-  const int64_t ns = q.nstrands, nr = ns / 2;
+  const int nw = g.nw;
+  const int64_t nv = (int64_t)q.nstrands * nw, nr = q.nstrands / 2;
   StageTimer& tm = c->timer;
-  const int64_t S = z.S;
-  int64_t* off = z.off;
-  int32_t* len32 = z.len32;
-  int32_t* nvalid = z.nvalid;
-  unsigned long long* counters = z.counters;
-  uint64_t* skey = z.skey;
-  uint32_t* sq = z.sq;
-  const long long* warp_dev = nullptr;  // the DP's split, when it was made on the device
-  const int* bad_dev = nullptr;         // the DP's flag of hits outside the window, once it ran
-  auto add_counters = [&]() {
-    unsigned long long cells = 0;
-    long long warp = 0;
-    int bad = 0;
-    CLAST_CK(cudaMemcpyAsync(&cells, counters + 1, sizeof(cells), cudaMemcpyDeviceToHost, st));
-    if (warp_dev) CLAST_CK(cudaMemcpyAsync(&warp, warp_dev, sizeof(warp), cudaMemcpyDeviceToHost, st));
-    if (bad_dev) CLAST_CK(cudaMemcpyAsync(&bad, bad_dev, sizeof(bad), cudaMemcpyDeviceToHost, st));
-    CLAST_CK(cudaStreamSynchronize(st));
-    c->stats.dp_cells += (int64_t)cells;
-    c->stats.dp_warp_hits += warp;
+  const size_t mark = ws.arena_used;  // arena mode: everything below is this group's
+  // counters and scan states, zeroed together
+  const int64_t st1 = scan_state_words(nv), st2 = scan_state_words(nr);
+  const size_t ctl_bytes = (sizeof(GroupCtl) + 255) & ~size_t(255);
+  const size_t zero_bytes = ctl_bytes + (size_t)(st1 + st2) * sizeof(unsigned long long);
+  GroupCtl* ctl = nullptr;
+  unsigned long long *state1 = nullptr, *state2 = nullptr;
+  int64_t *off = nullptr, *hoff = nullptr;
+  int32_t *cnt = nullptr, *nvalid = nullptr, *hcnt = nullptr;
+  uint64_t* skey = nullptr;
+  uint32_t* sq = nullptr;
+  int64_t H = 0;
+  for (int attempt = 0;; ++attempt) {
+    off = ws.get<int64_t>("s_off", nv);
+    cnt = ws.get<int32_t>("s_cnt", nv);
+    nvalid = ws.get<int32_t>("s_nvalid", nv);
+    skey = ws.get<uint64_t>("s_key", (size_t)g.part_cap * kSeedParts * nw);
+    sq = ws.get<uint32_t>("s_q", (size_t)g.part_cap * kSeedParts * nw);
+    char* zero = ws.get<char>("s_ctl", zero_bytes);
+    ctl = reinterpret_cast<GroupCtl*>(zero);
+    state1 = reinterpret_cast<unsigned long long*>(zero + ctl_bytes);
+    state2 = state1 + st1;
+    hcnt = ws.get<int32_t>("s_hcnt", nv);
+    hoff = ws.get<int64_t>("s_hoff", nv + 1);
+    uint32_t* lists = ws.get<uint32_t>("s_lists", 3 * nv);
+    CLAST_CK(cudaMemsetAsync(zero, 0, zero_bytes, st));
+    tm.begin(st);
+    static const bool force_multi = std::getenv("CLAST_SEED_MULTI_ONLY") != nullptr;
+    if (nw == 1 && !force_multi) {  // the single-window kernel (round 0 staged while its range is reserved)
+      seed_fused(q, g.ix[0]->view(), g.ix[0]->tview(), p->gap, p->local, ctl->cursor[0], ctl->kmers[0], off, cnt,
+                 nvalid, skey, sq, g.part_cap, st);
+    } else {
+      SeedWins W{};
+      for (int w = 0; w < nw; ++w)
+        W.w[w] = SeedWin{g.ix[w]->view(), g.ix[w]->tview(), ctl->cursor[w], ctl->kmers[w]};
+      W.off = off;
+      W.cnt = cnt;
+      W.nvalid = nvalid;
+      W.skey = skey;
+      W.sq = sq;
+      W.part_cap = g.part_cap;
+      seed_multi(q, W, nw, p->gap, p->local, st);
+    }
+    tm.end(StageTimer::SEED, st);
+    // sortSeeds, deletingIsolateSeeds, deleteDuplicateSeeds
+    tm.begin(st);
+    seed_filter(skey, sq, off, cnt, nvalid, qb.wstart, qb.nwin, nw, p->width, p->gap, nv, lists, hcnt, ctl, st);
+    tm.end(StageTimer::SORT, st, 4);
+    scan_i32_to(hcnt, nv, hoff, state1, &ctl->hits, st);
+    const GroupCtl& h = read_ctl(c, ctl, st);
     tm.flush();
-    if (bad) throw std::runtime_error("internal: a hit named a target sequence or strand outside the window");
-  };
-  c->stats.seeds += S;
-  if (S == 0) {
-    add_counters();
-    return 0;
+    int64_t most = 0, kmers = 0, S = 0, most_win = 0;
+    for (int w = 0; w < nw; ++w) {
+      int64_t sw = 0;
+      for (int i = 0; i < kSeedParts; ++i) {
+        sw += (int64_t)h.cursor[w][i];
+        most = std::max<int64_t>(most, (int64_t)h.cursor[w][i]);
+        kmers += (int64_t)h.kmers[w][i];
+      }
+      S += sw;
+      most_win = std::max(most_win, sw);
+    }
+    if (most <= g.part_cap) {
+      c->stats.query_kmers += kmers;
+      c->stats.seeds += S;
+      c->seed_hint = std::max<int64_t>(c->seed_hint, most_win + most_win / 4);
+      H = h.hits;
+      break;
+    }
+    if (attempt > 0) throw std::runtime_error("seed partitions overflowed twice");
+    if (most > g.part_fit)  // the partitions this window needs do not fit the scratch
+      throw std::invalid_argument("query window needs seed partitions of " + std::to_string(most) +
+                                  " seeds; clast_search_noalloc's scratch holds " + std::to_string(g.part_fit) +
+                                  " (use clast_search)");
+    if (ws.arena) ws.arena_rewind(mark);
+    g.part_cap = most;  // strands past a full partition wrote nothing: run again
   }
-  int32_t* wfirst = ws.get<int32_t>("s_wfirst", qb.nwin);
-  window_first(nvalid, qb.wstart, qb.nwin, wfirst, st);
-  // sortSeeds, deletingIsolateSeeds, deleteDuplicateSeeds
-  tm.begin(st);
-  int32_t* hcnt = ws.get<int32_t>("s_hcnt", ns);
-  seed_sort_filter(ws, skey, sq, off, len32, nvalid, qb.wstart, qb.nwin, wfirst, p->width, p->gap, ns, hcnt, st);
-  tm.end(StageTimer::SORT, st, 4);
-  int64_t* hoff = ws.get<int64_t>("s_hoff", ns + 1);
-  scan_i32(ws, hcnt, ns, hoff, st);
-  const int64_t H = read_scalar(hoff + ns, st);
   if (H >= ((int64_t)1 << 32)) throw std::invalid_argument("more than 2^32 hits in one window");  // DP order words
   c->stats.hits += H;
-  if (H == 0) {
-    add_counters();
-    return 0;
-  }
+  if (H == 0) return 0;
   uint64_t* hk = ws.get<uint64_t>("h_key", H);
   int32_t* hq = ws.get<int32_t>("h_q", H);
-  int32_t* hs = ws.get<int32_t>("h_s", H);
-  gather_hits(skey, sq, off, hcnt, hoff, ns, hk, hq, hs, q.len, p->lmer, 2 * p->gap + 1, counters + 1, st);
+  uint32_t* hs = ws.get<uint32_t>("h_s", H);
+  gather_hits(skey, sq, off, hcnt, hoff, nv, nw, hk, hq, hs, q.len, p->lmer, 2 * p->gap + 1, ctl, st);
   // alignmentHits + calculateEvalue + deleteHits_lowEValue / _tooShort
   DpOut o;
   o.t_idx = ws.get<int32_t>("d_tidx", H);
@@ -449,86 +408,91 @@ int64_t search_seeded(clast_ctx* c, Workspace& ws, const clast_params* p, const 
   // grid taking hits from a queue is slower than the plain one, 17.7 and 4.2 ms.)
   // The longest hits of the order may run one per warp (banded_dp decides
   // from the length buckets, or for equal lengths from the row count).
-  const bool uneven = qb.max_len != qb.min_len && H > 1;
-  const int warp_mode = qb.max_len > kDpMaxThreadLen ? kDpWarpAll : dp_warp_mode_from_env(c->dp_warp);
-  long long* dp_warp_n = ws.get<long long>("dp_warp_n", 1);
-  int* dp_bad = ws.get<int>("dp_bad", 1);
-  CLAST_CK(cudaMemsetAsync(dp_bad, 0, sizeof(int), st));
+  const int min_len = qb.lens ? qb.lens[0] : qb.min_len, max_len = qb.lens ? qb.lens[1] : qb.max_len;
+  const bool uneven = max_len != min_len && H > 1;
+  const int warp_mode = max_len > kDpMaxThreadLen ? kDpWarpAll : dp_warp_mode_from_env(c->dp_warp);
   c->stats.dp_order_kind = uneven ? 1 : 0;
   c->stats.dp_queue_chunk = 0;
   DpBuckets buckets;
   const uint64_t* order = nullptr;
-  tm.begin(st);
   if (uneven) {
-    const int rows_max = std::max(1, qb.max_len - p->lmer + 1);
+    tm.begin(st);
+    const int rows_max = std::max(1, max_len - p->lmer + 1);
     int bits = 1;
     while ((1ll << bits) <= rows_max) ++bits;
     uint64_t* ok = ws.get<uint64_t>("h_order", H);
     uint64_t* ok2 = ws.get<uint64_t>("h_order2", H);
-    dp_order_keys(hs, q.len, H, p->lmer, rows_max, ok, st);
+    dp_order_keys(hs, nw, q.len, H, p->lmer, rows_max, ok, st);
     order = radix_sort_u64(ws, ok, nullptr, ok2, nullptr, H, 32, 32 + bits, st) ? ok2 : ok;
-    if (warp_mode == kDpWarpAuto) buckets = dp_bucket_count(ws, hs, q.len, H, p->lmer, st);
+    if (warp_mode == kDpWarpAuto) buckets = dp_bucket_count(ws, hs, nw, q.len, H, p->lmer, st);
+    tm.end(StageTimer::DPORDER, st);
   }
-  tm.end(StageTimer::DPORDER, st);
   tm.begin(st);
   DpLaunch dl;
   dl.warp = warp_mode;
   dl.buckets = buckets;
-  dl.warp_n = dp_warp_n;
+  dl.warp_n = &ctl->dp_warp;
   dl.aux = c->st_dp;
   dl.ev_fork = c->ev_dp_fork;
   dl.ev_join = c->ev_dp_join;
-  dl.bad = dp_bad;
-  if (!uneven) dl.uniform_rows = std::max(0, qb.max_len - p->lmer);
-  const long long warp_fixed = banded_dp(tv, q, hk, hq, hs, order, H, dp, o, st, dl);
+  dl.bad = &ctl->bad;
+  if (!uneven) dl.uniform_rows = std::max(0, max_len - p->lmer);
+  TargetView tv[kMaxSeedWins];
+  for (int w = 0; w < nw; ++w) tv[w] = g.ix[w]->tview();
+  const long long warp_fixed = banded_dp(tv, nw, q, hk, hq, hs, order, H, dp, o, st, dl);
   tm.end(StageTimer::DP, st);
-  if (warp_fixed >= 0) c->stats.dp_warp_hits += warp_fixed;
-  else warp_dev = dl.warp_n;
-  bad_dev = dp_bad;
   // resultSorting + deleteHits_duplicateResult, per read
-  uint64_t* k1 = ws.get<uint64_t>("f_k1", H);
-  uint64_t* k2 = ws.get<uint64_t>("f_k2", H);
-  int32_t* idx = ws.get<int32_t>("f_idx", H);
-  final_keys(hk, hq, hs, o, H, k1, k2, idx, st);
   tm.begin(st);
-  int64_t* roff = ws.get<int64_t>("f_roff", nr);
-  int32_t* rlen = ws.get<int32_t>("f_rlen", nr);
-  read_ranges(hoff, nr, roff, rlen, st);
-  segmented_sort_u64(ws, k1, k2, idx, roff, rlen, nr, st, 1);
-  int32_t* fcnt = ws.get<int32_t>("f_cnt", nr);
+  uint64_t* g1 = ws.get<uint64_t>("f_g1", H);
+  uint64_t* g2 = ws.get<uint64_t>("f_g2", H);
   int32_t* fsel = ws.get<int32_t>("f_sel", H);
-  final_dedupe(k1, k2, idx, hk, hs, o, roff, rlen, nr, fcnt, fsel, st);
+  int32_t* fcnt = ws.get<int32_t>("f_cnt", nr);
+  uint32_t* flist = ws.get<uint32_t>("f_list", nr);
+  final_order(hk, hq, hs, o, hoff, nr, nw, g1, g2, flist, fcnt, fsel, ctl, st);
   int64_t* foff = ws.get<int64_t>("f_off", nr + 1);
-  scan_i32(ws, fcnt, nr, foff, st);
-  tm.end(StageTimer::FINAL, st, 9);
-  const int64_t F = read_scalar(foff + nr, st);
+  scan_i32_to(fcnt, nr, foff, state2, &ctl->results, st);
+  tm.end(StageTimer::FINAL, st, 3);
+  const GroupCtl& h = read_ctl(c, ctl, st);
+  tm.flush();
+  const int64_t F = h.results;
   c->stats.results += F;
-  add_counters();
+  c->stats.dp_cells += (int64_t)h.cells;
+  c->stats.dp_warp_hits += warp_fixed >= 0 ? warp_fixed : h.dp_warp;
+  if (h.bad) throw std::runtime_error("internal: a hit named a target sequence or strand outside the window");
   if (F == 0) return 0;
-  const FinalOut fo = sink.take(F, foff, nr, st);
-  final_compact(fsel, roff, fcnt, foff, nr, hk, hs, o, ix->t_begin, q_first, fo, st);
+  OutView out = sink.take(F, foff, nr, st);
+  for (int w = 0; w < nw; ++w) {
+    out.t_first[w] = g.ix[w]->t_begin;
+    out.load[w] = g.load[w];
+  }
+  final_write(hk, hs, o, hoff, nr, nw, fcnt, fsel, foff, out, st);
   return F;
 }
 
-// CDeviceHitList for every query window of `qb` against one index.
-void search_batch(clast_ctx* c, const clast_index* ix, const clast_params* p, const QueryRef& qb,
-                  int32_t q_first, DevHits& out) {
-  DevHitsSink sink(out);
-  if (qb.q.nstrands == 0 || ix->n_keys == 0) return;
-  std::vector<SeedSet> sets(1);
-  sets[0].ix = ix;
-  seed_windows(c, p, qb, sets);
-  search_seeded(c, c->ws, p, qb, q_first, sets[0], sink);
+// Seeds per partition that a group begins with.
+int64_t first_part_cap(const clast_ctx* c, int64_t n_bases) {
+  return std::max<int64_t>(c->seed_hint, n_bases / 16 + (1 << 20)) / kSeedParts + 1;
 }
 
-template <class T>
-T* host_copy(const std::vector<T>& v) {
-  T* p = static_cast<T*>(std::malloc((v.size() ? v.size() : 1) * sizeof(T)));
-  if (!p) throw std::bad_alloc();
-  if (!v.empty()) std::memcpy(p, v.data(), v.size() * sizeof(T));
-  return p;
-}
-
+// One search's results in device memory of their own, with the per-read
+// offsets kept when the results are to be merged.
+struct SlabSink : HitSink {
+  ResultSlab slab;
+  int32_t n_loads;
+  bool keep_offsets;
+  const int64_t* foff = nullptr;  // the group's per-read offsets (scratch), until the next group
+  DevArray<int64_t> offsets;
+  SlabSink(int32_t loads, bool keep) : n_loads(loads), keep_offsets(keep) {}
+  OutView take(int64_t F, const int64_t* f, int64_t nr, cudaStream_t st) override {
+    slab.alloc(F, n_loads);
+    foff = f;
+    if (keep_offsets) {
+      offsets.alloc(nr + 1);
+      CLAST_CK(cudaMemcpyAsync(offsets.p, f, (nr + 1) * sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
+    }
+    return slab.view();
+  }
+};
 
 }  // namespace
 
@@ -567,19 +531,21 @@ namespace {
 // One read window list per query load (moveQueryWindow, CHostSchedular.cu:12-23):
 // the window [qb, qe) grows while gateway(2*qe+2) - gateway(2*qb) < q_vram,
 // where every read adds two strands of len + l - 1 bases.  With the prefix
-// sums cum[], qe = clamp(first j with cum[j] >= cum[qb] + q_vram, minus one,
-// to [qb + 1, n]).
+// sums cum(j), which the read offsets give, qe = clamp(first j with cum(j) >=
+// cum(qb) + q_vram, minus one, to [qb + 1, n]).
 void query_windows(const int64_t* offsets, int64_t r0, int64_t r1, int l, int32_t q_vram,
                    std::vector<int64_t>& win_first_read) {
   const int64_t n = r1 - r0;
-  std::vector<int64_t> cum(n + 1);
-  cum[0] = 0;
-  for (int64_t r = 0; r < n; ++r)
-    cum[r + 1] = cum[r] + 2 * ((offsets[r0 + r + 1] - offsets[r0 + r]) + (l - 1));
+  auto cum = [&](int64_t j) { return 2 * ((offsets[r0 + j] - offsets[r0]) + j * (l - 1)); };
   for (int64_t qb = 0; qb < n;) {
-    const int64_t lim = cum[qb] + (int64_t)q_vram;
-    const int64_t j = std::lower_bound(cum.begin() + qb, cum.end(), lim) - cum.begin();
-    const int64_t qe = std::max(qb + 1, std::min(n, j - 1));
+    const int64_t lim = cum(qb) + (int64_t)q_vram;
+    int64_t lo = qb, hi = n + 1;  // first j in [qb, n] with cum(j) >= lim, n + 1 when there is none
+    while (lo < hi) {
+      const int64_t mid = (lo + hi) >> 1;
+      if (mid <= n && cum(mid) < lim) lo = mid + 1;
+      else hi = mid;
+    }
+    const int64_t qe = std::max(qb + 1, std::min(n, lo - 1));
     win_first_read.push_back(r0 + qb);
     qb = qe;
   }
@@ -605,7 +571,8 @@ int clast_ctx_create(int device, clast_ctx** out) {
   if (cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking) != cudaSuccess) return CLAST_ERR_CUDA;
   if (cudaStreamCreateWithFlags(&c->st_copy, cudaStreamNonBlocking) != cudaSuccess) return CLAST_ERR_CUDA;
   if (cudaStreamCreateWithFlags(&c->st_dp, cudaStreamNonBlocking) != cudaSuccess) return CLAST_ERR_CUDA;
-  if (cudaEventCreateWithFlags(&c->ev_dp_fork, cudaEventDisableTiming) != cudaSuccess ||
+  if (cudaEventCreateWithFlags(&c->ev_stage, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->ev_dp_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_dp_join, cudaEventDisableTiming) != cudaSuccess)
     return CLAST_ERR_CUDA;
   for (int b = 0; b < kBuildStreams; ++b)
@@ -628,11 +595,7 @@ int clast_ctx_create(int device, clast_ctx** out) {
 void clast_ctx_destroy(clast_ctx* ctx) {
   if (!ctx) return;
   cudaSetDevice(ctx->device);
-  for (auto& a : ctx->arenas) {  // device copies of results, freed on the stream before it goes
-    for (auto& f : a->dev.f) f.release();
-    a->dev.evalue.release();
-    a->dev.load_offsets.release();
-  }
+  for (auto& a : ctx->arenas) a->dev.slab.mem.release();  // device copies of results, freed on the stream before it goes
   if (ctx->st) cudaStreamSynchronize(ctx->st);
   for (int b = 0; b < kBuildStreams; ++b)
     if (ctx->st_build[b]) cudaStreamSynchronize(ctx->st_build[b]);
@@ -642,6 +605,10 @@ void clast_ctx_destroy(clast_ctx* ctx) {
     if (a->p) cudaFreeHost(a->p);
   for (auto& a : ctx->tsv_arenas)
     if (a->p) cudaFreeHost(a->p);
+  if (ctx->st_copy) cudaStreamSynchronize(ctx->st_copy);
+  if (ctx->staging) cudaFreeHost(ctx->staging);
+  if (ctx->ctl) cudaFreeHost(ctx->ctl);
+  if (ctx->ev_stage) cudaEventDestroy(ctx->ev_stage);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->ev2) cudaEventDestroy(ctx->ev2);
@@ -704,44 +671,75 @@ int clast_search(clast_ctx* ctx, const clast_index* ix, const clast_params* p, c
     g_alloc_stream = ctx->st;
     g_kernel_launches = 0;
     cudaStream_t st = ctx->st;
-    QueryBatch qb;
-    qb.n = n_qbases;
-    qb.nstrands = n_qseqs;
-    upload_padded(q_bases, n_qbases, qb.bases, st);
-    std::vector<int64_t> start(n_qseqs);
-    qb.min_len = n_qseqs ? INT32_MAX : 0;
+    int32_t min_len = n_qseqs ? INT32_MAX : 0, max_len = 0;
+    // strand starts and lengths and the one query window, staged behind each other as on the device
+    const size_t len_at = QueryBatch::al((size_t)n_qseqs * sizeof(int64_t));
+    const size_t win_at = len_at + QueryBatch::al((size_t)n_qseqs * sizeof(int32_t));
+    const size_t table_bytes = win_at + 2 * sizeof(int32_t);
+    char* host_tables = ctx->stage(table_bytes);
+    int64_t* start = reinterpret_cast<int64_t*>(host_tables);
     for (int32_t i = 0; i < n_qseqs; ++i) {
       start[i] = q_gateway[i];
       if (q_gateway[i] < 0 || q_lengths[i] < 0 || (int64_t)q_gateway[i] + q_lengths[i] > n_qbases)
         throw std::invalid_argument("query sequence outside the base array");
-      qb.min_len = std::min(qb.min_len, q_lengths[i]);
-      qb.max_len = std::max(qb.max_len, q_lengths[i]);
+      min_len = std::min(min_len, q_lengths[i]);
+      max_len = std::max(max_len, q_lengths[i]);
     }
-    qb.start.alloc(n_qseqs);
-    qb.len.alloc(n_qseqs);
-    if (n_qseqs) {
-      CLAST_CK(cudaMemcpyAsync(qb.start.p, start.data(), n_qseqs * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-      CLAST_CK(cudaMemcpyAsync(qb.len.p, q_lengths, n_qseqs * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    }
+    if (n_qseqs) std::memcpy(host_tables + len_at, q_lengths, n_qseqs * sizeof(int32_t));
     const int32_t ws2[2] = {0, n_qseqs};
+    std::memcpy(host_tables + win_at, ws2, sizeof(ws2));
+    QueryBatch qb;
+    qb.alloc(n_qbases, n_qseqs, sizeof(ws2));
+    qb.min_len = min_len;
+    qb.max_len = max_len;
     qb.nwin = 1;
-    qb.wstart.alloc(2);
-    CLAST_CK(cudaMemcpyAsync(qb.wstart.p, ws2, sizeof(ws2), cudaMemcpyHostToDevice, st));
+    qb.wstart = reinterpret_cast<const int32_t*>(qb.meta);
+    CLAST_CK(cudaMemcpyAsync(qb.start, host_tables, table_bytes, cudaMemcpyHostToDevice, st));
+    ctx->staged(st);
+    CLAST_CK(cudaMemsetAsync(qb.bases, 'N', kPad, st));
+    CLAST_CK(cudaMemsetAsync(qb.bases + kPad + n_qbases, 'N', kPad, st));
+    if (n_qbases > 0)
+      CLAST_CK(cudaMemcpyAsync(qb.bases + kPad, q_bases, (size_t)n_qbases, cudaMemcpyHostToDevice, st));
     qb.pack(st);
-    DevHits h;
-    search_batch(ctx, ix, p, qb.ref(), q_begin, h);
-    const int64_t F = h.n;
+    struct SearchSink : HitSink {
+      ResultSlab slab;
+      int32_t q_first;
+      explicit SearchSink(int32_t q) : q_first(q) {}
+      OutView take(int64_t F, const int64_t*, int64_t, cudaStream_t) override {
+        slab.alloc(F, 0);
+        OutView v = slab.view();
+        v.q_id = v.read;
+        v.q_first = q_first;
+        return v;
+      }
+    } sink(q_begin);
+    int64_t F = 0;
+    if (n_qseqs > 0 && ix->n_keys != 0) {
+      Group g;
+      g.nw = 1;
+      g.ix[0] = ix;
+      g.part_cap = first_part_cap(ctx, n_qbases);
+      F = search_group(ctx, ctx->ws, p, qb.ref(), g, sink);
+    }
     out->n = F;
-    auto d2h32 = [&](int32_t*& dst, const DevArray<int32_t>& src) {
-      dst = static_cast<int32_t*>(std::malloc((F ? F : 1) * sizeof(int32_t)));
+    // small results: one download into the pinned staging buffer
+    const ResultSlab& h = sink.slab;  // q_id in the place of read
+    const char* host = nullptr;
+    if (F && h.bytes <= kStageMax) {
+      char* to = ctx->stage(h.bytes);
+      CLAST_CK(cudaMemcpyAsync(to, h.mem.p, h.bytes, cudaMemcpyDeviceToHost, st));
+      CLAST_CK(cudaStreamSynchronize(st));
+      host = to;
+    }
+    auto copy = [&](auto*& dst, const auto* dev) {
+      dst = static_cast<std::remove_reference_t<decltype(dst)>>(std::malloc((F ? F : 1) * sizeof(*dst)));
       if (!dst) throw std::bad_alloc();
-      if (F) CLAST_CK(cudaMemcpyAsync(dst, src.p, F * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+      if (host) std::memcpy(dst, host + (reinterpret_cast<const char*>(dev) - h.mem.p), F * sizeof(*dst));
+      else if (F) CLAST_CK(cudaMemcpyAsync(dst, dev, F * sizeof(*dst), cudaMemcpyDeviceToHost, st));
     };
-    d2h32(out->t_id, h.t_id); d2h32(out->t_idx, h.t_idx); d2h32(out->q_id, h.q_id); d2h32(out->q_idx, h.q_idx);
-    d2h32(out->t_len, h.t_len); d2h32(out->q_len, h.q_len); d2h32(out->match, h.match); d2h32(out->score, h.score);
-    out->evalue = static_cast<double*>(std::malloc((F ? F : 1) * sizeof(double)));
-    if (!out->evalue) throw std::bad_alloc();
-    if (F) CLAST_CK(cudaMemcpyAsync(out->evalue, h.evalue.p, F * sizeof(double), cudaMemcpyDeviceToHost, st));
+    copy(out->t_id, h.f[3]); copy(out->t_idx, h.f[4]); copy(out->q_id, h.f[0]); copy(out->q_idx, h.f[5]);
+    copy(out->t_len, h.f[6]); copy(out->q_len, h.f[7]); copy(out->match, h.f[8]); copy(out->score, h.f[9]);
+    copy(out->evalue, h.evalue);
     CLAST_CK(cudaStreamSynchronize(st));
     ctx->last_launches = g_kernel_launches;
     return CLAST_OK;
@@ -986,113 +984,129 @@ static int map_impl(clast_ctx* ctx, const clast_targets* T, const clast_params* 
     for (int32_t k = 0; k < n_loads; ++k)
       query_windows(reads->offsets, load_first[k], load_first[k + 1], p->lmer, q_vram, wfirst);
     wfirst.push_back(nreads);
-    std::vector<int32_t> wstart(wfirst.size());
-    for (size_t i = 0; i < wfirst.size(); ++i) wstart[i] = (int32_t)(2 * wfirst[i]);
-    // every read uploaded once; strands are built on the device
-    std::vector<int64_t> off0;
-    const int64_t* offs_rel = reads->offsets;  // offsets relative to the first read
-    if (reads->offsets[0] != 0) {
-      off0.resize(nreads + 1);
-      for (int64_t i = 0; i <= nreads; ++i) off0[i] = reads->offsets[i] - reads->offsets[0];
-      offs_rel = off0.data();
-    }
-    DevArray<int64_t> doff;
-    g_alloc_stream = cs;
-    doff.alloc((size_t)nreads + 1);
-    QueryBatch qb;
-    qb.wstart.alloc(wstart.size());
-    g_alloc_stream = st;
-    doff.st = qb.wstart.st = st;
-    qb.n = 2 * nb;
-    qb.nstrands = (int32_t)(2 * nreads);
-    qb.min_len = nreads ? INT32_MAX : 0;
-    for (int64_t r = 0; r < nreads; ++r) {
+    // read lengths: of a large batch on the device (a pass over a million
+    // offsets takes the host 1-2 ms), unless one may exceed 32 bits
+    const bool dev_lengths = nreads > kHostLengths && nb <= INT32_MAX;
+    int32_t min_len = nreads ? INT32_MAX : 0, max_len = 0;
+    for (int64_t r = 0; r < nreads && !dev_lengths; ++r) {
       const int64_t len = reads->offsets[r + 1] - reads->offsets[r];
       if (len > INT32_MAX) throw std::invalid_argument("read longer than 2^31 bases");
-      qb.min_len = std::min<int32_t>(qb.min_len, (int32_t)len);
-      qb.max_len = std::max<int32_t>(qb.max_len, (int32_t)len);
+      min_len = std::min<int32_t>(min_len, (int32_t)len);
+      max_len = std::max<int32_t>(max_len, (int32_t)len);
     }
-    qb.bases.alloc((size_t)qb.n + 2 * kPad);
-    qb.start.alloc(2 * nreads);
-    qb.len.alloc(2 * nreads);
+    // The tables of the batch behind its strands: first reads of the loads,
+    // strands where the query windows start, read offsets relative to the first
+    // read.  They are staged in pinned memory and go up in one copy; the
+    // offsets of a large batch come straight from the caller's array.
+    const size_t win_at = QueryBatch::al(((size_t)n_loads + 1) * sizeof(int64_t));
+    const size_t len_at = win_at + QueryBatch::al(wfirst.size() * sizeof(int32_t));
+    const size_t off_at = len_at + QueryBatch::al(2 * sizeof(int32_t));  // shortest, longest read
+    const size_t off_bytes = ((size_t)nreads + 1) * sizeof(int64_t);
+    const bool offs_staged = off_bytes <= kStageMax / 16 || reads->offsets[0] != 0;
+    QueryBatch qb;
+    g_alloc_stream = cs;
+    qb.alloc(2 * nb, 2 * nreads, off_at + off_bytes);
+    g_alloc_stream = st;
+    qb.mem.st = st;
+    qb.min_len = min_len;
+    qb.max_len = max_len;
     qb.nwin = (int32_t)wfirst.size() - 1;
+    qb.wstart = reinterpret_cast<const int32_t*>(qb.meta + win_at);
+    const int64_t* dlf = reinterpret_cast<const int64_t*>(qb.meta);
+    const int64_t* doff = reinterpret_cast<const int64_t*>(qb.meta + off_at);
+    char* tables = ctx->stage(off_at + (offs_staged ? off_bytes : 0));
+    std::memcpy(tables, load_first.data(), load_first.size() * sizeof(int64_t));
+    int32_t* wstart = reinterpret_cast<int32_t*>(tables + win_at);
+    for (size_t i = 0; i < wfirst.size(); ++i) wstart[i] = (int32_t)(2 * wfirst[i]);
+    const int32_t lens[2] = {min_len, max_len};
+    std::memcpy(tables + len_at, lens, sizeof(lens));
+    if (offs_staged) {
+      int64_t* o = reinterpret_cast<int64_t*>(tables + off_at);
+      for (int64_t i = 0; i <= nreads; ++i) o[i] = reads->offsets[i] - reads->offsets[0];
+    }
     S.map_prep_ms = wall_ms() - w0;
-    CLAST_CK(cudaMemcpyAsync(doff.p, offs_rel, (nreads + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, cs));
-    CLAST_CK(cudaMemcpyAsync(qb.wstart.p, wstart.data(), wstart.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
-                             cs));
+    CLAST_CK(cudaMemcpyAsync(qb.meta, tables, off_at + (offs_staged ? off_bytes : 0), cudaMemcpyHostToDevice, cs));
+    ctx->staged(cs);
+    if (!offs_staged)
+      CLAST_CK(cudaMemcpyAsync(qb.meta + off_at, reads->offsets, off_bytes, cudaMemcpyHostToDevice, cs));
     CLAST_CK(cudaEventRecord(ctx->ev3, cs));
     CLAST_CK(cudaStreamWaitEvent(st, ctx->ev3, 0));
     CLAST_CK(cudaEventRecord(ctx->ev1, st));  // the reads are resident and the compute stream is free
-    CLAST_CK(cudaMemsetAsync(qb.bases.p, 'N', (size_t)qb.n + 2 * kPad, st));
-    build_strands(rsrc, doff.p, nreads, nb, qb.bases.p + kPad, qb.start.p, qb.len.p, st);
-    qb.pack(st);
+    build_strands(rsrc, doff, nreads, qb.bases + kPad, qb.start, qb.len, st);
+    if (nreads > 0) qb.pack(st);
+    int32_t* dlen = reinterpret_cast<int32_t*>(qb.meta + len_at);
+    if (dev_lengths) {
+      read_lengths(doff, nreads, dlen, dlen + 1, st);
+      CLAST_CK(cudaMemcpyAsync(tables + len_at, dlen, sizeof(lens), cudaMemcpyDeviceToHost, st));
+    }
     S.query_bases = qb.n;
     // the index builds of clast_targets_create end before the first search
     settle_targets(ctx, T);
     CLAST_CK(cudaStreamWaitEvent(st, T->ev_done, 0));
-    // every target window, in holder order (target load, window)
-    std::vector<DevHits> per_win(T->wins.size());
-    const QueryRef qr = qb.ref();
-    // windows seeded per pass over the query (CLAST_SEED_WINDOWS, 1..4)
+    QueryRef qr = qb.ref();
+    if (dev_lengths) qr.lens = reinterpret_cast<const int32_t*>(tables + len_at);
+    // windows searched per group (CLAST_SEED_WINDOWS, 1..4), as long as the
+    // group's slots have 32-bit numbers
     int group = 2;
     if (const char* e = std::getenv("CLAST_SEED_WINDOWS")) group = std::max(1, std::min(kMaxSeedWins, std::atoi(e)));
-    for (size_t g0 = 0; g0 < T->wins.size(); g0 += (size_t)group) {
-      std::vector<SeedSet> sets;
-      std::vector<size_t> idx;
+    while (group > 1 && (int64_t)group * qr.q.nstrands >= INT32_MAX) --group;
+    // every target window, in holder order (target load, window)
+    std::vector<Group> groups;
+    for (size_t g0 = 0; g0 < T->wins.size() && qr.q.nstrands > 0; g0 += (size_t)group) {
+      Group g;
       for (size_t w = g0; w < std::min(T->wins.size(), g0 + (size_t)group); ++w) {
-        const clast_index* ix = T->wins[w].ix.get();
-        if (qr.q.nstrands == 0 || ix->n_keys == 0) continue;
-        sets.emplace_back();
-        sets.back().ix = ix;
-        idx.push_back(w);
+        if (T->wins[w].ix->n_keys == 0) continue;
+        g.load[g.nw] = T->wins[w].load;
+        g.ix[g.nw++] = T->wins[w].ix.get();
       }
-      if (sets.empty()) continue;
-      seed_windows(ctx, p, qr, sets);
-      for (size_t j = 0; j < sets.size(); ++j) {
-        DevHitsSink sink(per_win[idx[j]]);
-        search_seeded(ctx, ctx->ws, p, qr, 0, sets[j], sink);
+      if (g.nw > 0) groups.push_back(g);
+    }
+    std::vector<std::unique_ptr<SlabSink>> found;
+    int64_t F = 0;
+    for (Group& g : groups) {
+      std::unique_ptr<SlabSink> sink(new SlabSink(n_loads, groups.size() > 1));
+      g.part_cap = first_part_cap(ctx, qr.n);
+      const int64_t f = search_group(ctx, ctx->ws, p, qr, g, *sink);
+      if (f == 0) continue;
+      F += f;
+      found.push_back(std::move(sink));
+    }
+    ResultSlab res_dev;
+    const int64_t* roff = nullptr;  // per-read offsets of the result
+    if (groups.size() == 1 && found.size() == 1) {
+      res_dev = std::move(found[0]->slab);
+      roff = found[0]->foff;
+    } else {
+      // fixResult: stable merge by (read, score desc) over the groups, on the device
+      res_dev.alloc(F, n_loads);
+      if (F > 0) {
+        std::vector<GroupHits> gh;
+        int64_t base = 0;
+        for (const auto& x : found) {
+          GroupHits h{};
+          for (int k = 0; k < 10; ++k) h.f[k] = x->slab.f[k];
+          h.evalue = x->slab.evalue;
+          h.foff = x->offsets.p;
+          h.base = base;
+          base += x->slab.n;
+          gh.push_back(h);
+        }
+        GroupHits* dgh = ctx->ws.get<GroupHits>("m_groups", gh.size());
+        CLAST_CK(cudaMemcpyAsync(dgh, gh.data(), gh.size() * sizeof(GroupHits), cudaMemcpyHostToDevice, st));
+        int32_t* mcnt = ctx->ws.get<int32_t>("m_cnt", nreads + 1);
+        int64_t* moff = ctx->ws.get<int64_t>("m_off", nreads + 1);
+        merge_groups(dgh, (int)gh.size(), F, nreads, mcnt, moff, res_dev.view(), ctx->ws, st);
+        roff = moff;
       }
     }
-    // fixResult: stable merge by (read, score desc) over the windows, on the device
-    std::vector<WinHits> wh;
-    int64_t n_items = 0;
-    for (size_t w = 0; w < T->wins.size(); ++w) {
-      const DevHits& h = per_win[w];
-      if (h.n == 0) continue;
-      wh.push_back(WinHits{h.t_id.p, h.t_idx.p, h.q_id.p, h.q_idx.p, h.t_len.p, h.q_len.p, h.match.p, h.score.p,
-                           h.evalue.p, h.foff.p, n_items, T->wins[w].load});
-      n_items += h.n;
-    }
-    DevArray<WinHits> dwh;
-    dwh.alloc(wh.size());
-    if (!wh.empty())
-      CLAST_CK(cudaMemcpyAsync(dwh.p, wh.data(), wh.size() * sizeof(WinHits), cudaMemcpyHostToDevice, st));
-    const int64_t F = n_items;
-    DevArray<int32_t> m_read, m_strand, m_load, m_seq, m_tidx, m_qidx, m_tlen, m_qlen, m_match, m_score;
-    DevArray<double> m_e;
-    for (auto* a : {&m_read, &m_strand, &m_load, &m_seq, &m_tidx, &m_qidx, &m_tlen, &m_qlen, &m_match, &m_score})
-      a->alloc(F);
-    m_e.alloc(F);
-    int32_t* mcnt = ctx->ws.get<int32_t>("m_cnt", nreads + 1);
-    int64_t* moff = ctx->ws.get<int64_t>("m_off", nreads + 1);
-    MapOut mo{m_read.p, m_strand.p, m_load.p, m_seq.p, m_tidx.p, m_qidx.p, m_tlen.p, m_qlen.p, m_match.p,
-              m_score.p, m_e.p};
-    merge_windows(dwh.p, (int)wh.size(), n_items, nreads, mcnt, moff, mo, ctx->ws, st);
     // per query load offsets
-    std::vector<int64_t> lf(load_first.begin(), load_first.end());
-    DevArray<int64_t> dlf, dlo;
-    dlf.alloc(lf.size());
-    dlo.alloc(lf.size());
-    CLAST_CK(cudaMemcpyAsync(dlf.p, lf.data(), lf.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-    if (nreads > 0) gather_i64(moff, dlf.p, (int)lf.size(), dlo.p, st);
-    else CLAST_CK(cudaMemsetAsync(dlo.p, 0, lf.size() * sizeof(int64_t), st));
+    if (roff) gather_i64(roff, dlf, n_loads + 1, res_dev.load_offsets, st);
+    else CLAST_CK(cudaMemsetAsync(res_dev.load_offsets, 0, ((size_t)n_loads + 1) * sizeof(int64_t), st));
     clast_map_result res;
     std::memset(&res, 0, sizeof(res));
     res.n = F;
-    // one pinned arena: load offsets, ten int32 arrays, evalue
-    auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-    const size_t need = al((n_loads + 1) * sizeof(int64_t)) + 10 * al((F ? F : 1) * sizeof(int32_t)) +
-                        al((F ? F : 1) * sizeof(double));
+    // one pinned arena laid out as the device's result: one download
+    const size_t need = res_dev.bytes;
     PinnedArena* arena = nullptr;
     for (auto& a : ctx->arenas)
       if (!a->in_use && (arena == nullptr || a->bytes > arena->bytes)) arena = a.get();
@@ -1104,40 +1118,28 @@ static int map_impl(clast_ctx* ctx, const clast_targets* T, const clast_params* 
       if (arena->p) CLAST_CK(cudaFreeHost(arena->p));
       arena->p = nullptr;
       arena->bytes = 0;
-      const size_t nb = need + need / 4;
-      if (cudaMallocHost(&arena->p, nb) != cudaSuccess) {
+      const size_t want = need + need / 4;
+      if (cudaMallocHost(&arena->p, want) != cudaSuccess) {
         (void)cudaGetLastError();
         throw std::bad_alloc();
       }
-      arena->bytes = nb;
+      arena->bytes = want;
     }
     arena->in_use = true;
     res.owner = arena;
-    char* cur = static_cast<char*>(arena->p);
-    auto take = [&](size_t b) { char* q = cur; cur += al(b); return q; };
-    res.load_offsets = reinterpret_cast<int64_t*>(take((n_loads + 1) * sizeof(int64_t)));
-    std::memset(res.load_offsets, 0, (n_loads + 1) * sizeof(int64_t));
-    if (nreads > 0)
-      CLAST_CK(cudaMemcpyAsync(res.load_offsets, dlo.p, (n_loads + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost,
-                               st));
-    auto d2h32 = [&](int32_t*& dst, const DevArray<int32_t>& src) {
-      dst = reinterpret_cast<int32_t*>(take((F ? F : 1) * sizeof(int32_t)));
-      if (F) CLAST_CK(cudaMemcpyAsync(dst, src.p, F * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    };
-    d2h32(res.read, m_read); d2h32(res.strand, m_strand); d2h32(res.t_load, m_load); d2h32(res.t_seq, m_seq);
-    d2h32(res.t_idx, m_tidx); d2h32(res.q_idx, m_qidx); d2h32(res.t_len, m_tlen); d2h32(res.q_len, m_qlen);
-    d2h32(res.match, m_match); d2h32(res.score, m_score);
-    res.evalue = reinterpret_cast<double*>(take((F ? F : 1) * sizeof(double)));
-    if (F) CLAST_CK(cudaMemcpyAsync(res.evalue, m_e.p, F * sizeof(double), cudaMemcpyDeviceToHost, st));
-    {  // the device copy stays with the arena for clast_format_tsv
-      PinnedArena::Device& d = arena->dev;
-      DevArray<int32_t>* src[10] = {&m_read, &m_strand, &m_load, &m_seq, &m_tidx, &m_qidx, &m_tlen, &m_qlen,
-                                    &m_match, &m_score};
-      for (int k = 0; k < 10; ++k) d.f[k] = std::move(*src[k]);
-      d.evalue = std::move(m_e);
-      d.load_offsets = std::move(dlo);
-      d.n = F;
-      d.n_loads = n_loads;
+    CLAST_CK(cudaMemcpyAsync(arena->p, res_dev.mem.p, need, cudaMemcpyDeviceToHost, st));
+    {
+      char* base = static_cast<char*>(arena->p);
+      auto host = [&](const void* dev) { return base + (static_cast<const char*>(dev) - res_dev.mem.p); };
+      int32_t** dst[10] = {&res.read, &res.strand, &res.t_load, &res.t_seq, &res.t_idx, &res.q_idx, &res.t_len,
+                           &res.q_len, &res.match, &res.score};
+      for (int k = 0; k < 10; ++k) *dst[k] = reinterpret_cast<int32_t*>(host(res_dev.f[k]));
+      res.evalue = reinterpret_cast<double*>(host(res_dev.evalue));
+      res.load_offsets = reinterpret_cast<int64_t*>(host(res_dev.load_offsets));
+      // the device copy stays with the arena for clast_format_tsv
+      arena->dev.slab = std::move(res_dev);
+      arena->dev.n = F;
+      arena->dev.n_loads = n_loads;
     }
     CLAST_CK(cudaEventRecord(ctx->ev2, st));
     CLAST_CK(cudaEventSynchronize(ctx->ev2));
@@ -1175,11 +1177,7 @@ int clast_ctx_trim(clast_ctx* ctx) {
     CLAST_CK(cudaSetDevice(ctx->device));
     CLAST_CK(cudaDeviceSynchronize());
     for (auto& a : ctx->arenas)
-      if (!a->in_use) {
-        for (auto& f : a->dev.f) f.release();
-        a->dev.evalue.release();
-        a->dev.load_offsets.release();
-      }
+      if (!a->in_use) a->dev.slab.mem.release();
     ctx->ws.release_all();
     for (auto& w : ctx->ws_build) w.release_all();
     CLAST_CK(cudaDeviceSynchronize());
@@ -1258,6 +1256,13 @@ size_t fixed_scratch_bytes(int64_t n, int64_t ns, int parts) {
          r(16 * s) + (64 << 10);
 }
 
+// Bytes of search_group's per-strand tables, as Workspace::get rounds them.
+size_t fixed_table_bytes(int64_t ns) {
+  auto r = [](size_t b) { return ((b ? b : 1) + 255) & ~size_t(255); };
+  const size_t s = (size_t)ns;
+  return r(8 * (s + 1)) + 2 * r(4 * s) + r(8 * (2 + 2 * (size_t)kSeedParts));
+}
+
 // Clears the busy flag of a device's scratch once the call's stream work has
 // ended (also when the call failed after launching work).
 struct ScratchClaim {
@@ -1296,8 +1301,7 @@ extern "C" int clast_search_noalloc(clast_ctx* ctx, const clast_index* ix, const
         throw std::invalid_argument("query sequence outside the base array");
     if (ctx->device < 0 || ctx->device >= kMaxScratchDevices)
       throw std::invalid_argument("device ordinal beyond the scratch table");
-    const int parts = seed_parts();
-    const size_t fixed = fixed_scratch_bytes(n_qbases, n_qseqs, parts);
+    const size_t fixed = fixed_scratch_bytes(n_qbases, n_qseqs, kSeedParts);
     if (fixed > kSearchScratchBytes)
       throw std::invalid_argument("query window of " + std::to_string(n_qbases) + " bases and " +
                                   std::to_string(n_qseqs) + " sequences needs " + std::to_string(fixed) +
@@ -1313,7 +1317,7 @@ extern "C" int clast_search_noalloc(clast_ctx* ctx, const clast_index* ix, const
     g_kernel_launches = 0;
     Workspace ws;
     ws.arena_begin(base, kSearchScratchBytes);
-    const int64_t ns = n_qseqs, nr = ns / 2, n = n_qbases;
+    const int64_t ns = n_qseqs, n = n_qbases;
     // the query window: padded bases, strand starts and lengths, 2-bit words
     char* qbases = ws.get<char>("q_bases", (size_t)n + 2 * kPad);
     CLAST_CK(cudaMemsetAsync(qbases, 'N', (size_t)n + 2 * kPad, st));
@@ -1341,8 +1345,6 @@ extern "C" int clast_search_noalloc(clast_ctx* ctx, const clast_index* ix, const
     q.start = qstart;
     q.len = qlen;
     q.nstrands = n_qseqs;
-    const IndexView iv = ix->view();
-    const TargetView tv = ix->tview();
     auto finish = [&](int64_t F) {
       CLAST_CK(cudaStreamSynchronize(st));
       ctx->last_launches = g_kernel_launches;
@@ -1350,45 +1352,6 @@ extern "C" int clast_search_noalloc(clast_ctx* ctx, const clast_index* ix, const
       return CLAST_OK;
     };
     if (ns == 0 || ix->n_keys == 0) return finish(0);
-    // createRawSeedList + deleteSeedsOnSequenceBoundary, one pass
-    int64_t* off = ws.get<int64_t>("s_off", ns + 1);
-    int32_t* len32 = ws.get<int32_t>("s_len32", ns);
-    int32_t* nvalid = ws.get<int32_t>("s_nvalid", ns);
-    unsigned long long* counters = ws.get<unsigned long long>("s_counters", 2 + 2 * parts);
-    // the seed partitions take at most half of the scratch still free
-    const size_t mark = ws.arena_used;
-    const int64_t fit = (int64_t)((ws.arena_cap - mark) / 2 / (12 * (size_t)parts)) - 256;
-    int64_t part_cap = std::max<int64_t>(ctx->seed_hint, n / 16 + (1 << 20)) / parts + 1;
-    part_cap = std::max<int64_t>(1, std::min(part_cap, fit));
-    int64_t S = 0;
-    uint64_t* skey = nullptr;
-    uint32_t* sq = nullptr;
-    for (int attempt = 0; attempt < 2; ++attempt) {
-      skey = ws.get<uint64_t>("s_key", (size_t)part_cap * parts);
-      sq = ws.get<uint32_t>("s_q", (size_t)part_cap * parts);
-      CLAST_CK(cudaMemsetAsync(counters, 0, (2 + 2 * parts) * sizeof(unsigned long long), st));
-      seed_fused(q, iv, tv, p->gap, p->local, counters + 2, counters + 2 + parts, off, len32, nvalid, skey, sq,
-                 part_cap, st);
-      unsigned long long cur[64];
-      CLAST_CK(cudaMemcpyAsync(cur, counters + 2, parts * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-      CLAST_CK(cudaStreamSynchronize(st));
-      S = 0;
-      int64_t most = 0;
-      for (int i = 0; i < parts; ++i) {
-        S += (int64_t)cur[i];
-        most = std::max<int64_t>(most, (int64_t)cur[i]);
-      }
-      if (most <= part_cap) break;
-      if (most > fit)  // the partitions this window needs do not fit the scratch
-        throw std::invalid_argument("query window needs seed partitions of " + std::to_string(most) +
-                                    " seeds; clast_search_noalloc's scratch holds " + std::to_string(fit) +
-                                    " (use clast_search)");
-      ws.arena_rewind(mark);  // strands past a full partition wrote nothing: run again, larger
-      part_cap = most;
-    }
-    if (S == 0) return finish(0);
-    // the stages after seeding are clast_search's, on the fixed scratch; the
-    // hits go to slots of the scratch, then to the caller's arrays
     int32_t lmin = INT32_MAX, lmax = 0;
     for (int32_t i = 0; i < n_qseqs; ++i) {
       lmin = std::min(lmin, q_lengths[i]);
@@ -1401,40 +1364,50 @@ extern "C" int clast_search_noalloc(clast_ctx* ctx, const clast_index* ix, const
     qr.nwin = 1;
     qr.min_len = lmin;
     qr.max_len = lmax;
-    SeedSet z;
-    z.ix = ix;
-    z.off = off;
-    z.len32 = len32;
-    z.nvalid = nvalid;
-    z.counters = counters;
-    z.skey = skey;
-    z.sq = sq;
-    z.part_cap = part_cap;
-    z.S = S;
+    // the search is clast_search's, on the fixed scratch; the seed partitions
+    // take at most half of what is free behind the seed tables (offsets,
+    // counts, counters); the hits go to slots of the scratch, then to the
+    // caller's arrays
+    Group g;
+    g.nw = 1;
+    g.ix[0] = ix;
+    const size_t tables = ws.arena_used + fixed_table_bytes(ns);
+    const size_t left = tables < ws.arena_cap ? ws.arena_cap - tables : 0;
+    g.part_fit = (int64_t)(left / 2 / (12 * (size_t)kSeedParts)) - 256;
+    g.part_cap = std::max<int64_t>(1, std::min(first_part_cap(ctx, n), g.part_fit));
     struct ArenaSink : HitSink {
       Workspace& ws;
       int64_t capacity;
       clast_hits* out;
-      FinalOut fo{};
+      OutView fo{};
+      int32_t q_first = 0;
       ArenaSink(Workspace& w, int64_t cap, clast_hits* o) : ws(w), capacity(cap), out(o) {}
-      FinalOut take(int64_t F, const int64_t*, int64_t, cudaStream_t) override {
+      OutView take(int64_t F, const int64_t*, int64_t, cudaStream_t) override {
         if (F > capacity) {
           out->n = F;
           throw std::invalid_argument("window has " + std::to_string(F) + " hits, capacity is " +
                                       std::to_string(capacity));
         }
-        fo = FinalOut{ws.get<int32_t>("o_tid", F), ws.get<int32_t>("o_tidx", F), ws.get<int32_t>("o_qid", F),
-                      ws.get<int32_t>("o_qidx", F), ws.get<int32_t>("o_tlen", F), ws.get<int32_t>("o_qlen", F),
-                      ws.get<int32_t>("o_match", F), ws.get<int32_t>("o_score", F), ws.get<double>("o_e", F)};
+        fo.t_seq = ws.get<int32_t>("o_tid", F);
+        fo.t_idx = ws.get<int32_t>("o_tidx", F);
+        fo.q_id = ws.get<int32_t>("o_qid", F);
+        fo.q_idx = ws.get<int32_t>("o_qidx", F);
+        fo.t_len = ws.get<int32_t>("o_tlen", F);
+        fo.q_len = ws.get<int32_t>("o_qlen", F);
+        fo.match = ws.get<int32_t>("o_match", F);
+        fo.score = ws.get<int32_t>("o_score", F);
+        fo.evalue = ws.get<double>("o_e", F);
+        fo.q_first = q_first;
         return fo;
       }
     } sink(ws, capacity, out);
-    const int64_t F = search_seeded(ctx, ws, p, qr, q_begin, z, sink);
+    sink.q_first = q_begin;
+    const int64_t F = search_group(ctx, ws, p, qr, g, sink);
     if (F == 0) return finish(0);
-    const FinalOut& fo = sink.fo;
+    const OutView& fo = sink.fo;
     int32_t* const dst[8] = {out->t_id, out->t_idx, out->q_id, out->q_idx, out->t_len, out->q_len, out->match,
                              out->score};
-    const int32_t* const src[8] = {fo.t_id, fo.t_idx, fo.q_id, fo.q_idx, fo.t_len, fo.q_len, fo.match, fo.score};
+    const int32_t* const src[8] = {fo.t_seq, fo.t_idx, fo.q_id, fo.q_idx, fo.t_len, fo.q_len, fo.match, fo.score};
     for (int k = 0; k < 8; ++k)
       CLAST_CK(cudaMemcpyAsync(dst[k], src[k], F * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     CLAST_CK(cudaMemcpyAsync(out->evalue, fo.evalue, F * sizeof(double), cudaMemcpyDeviceToHost, st));

@@ -144,23 +144,54 @@ struct StageTimer {
   }
 };
 
+// One search's results in one device allocation: per-load offsets, the ten
+// int32 fields read strand t_load t_seq t_idx q_idx t_len q_len match score,
+// and the E-values, each from a 256-byte boundary.
+struct ResultSlab {
+  DevArray<char> mem;
+  int64_t n = 0;
+  size_t bytes = 0;
+  int64_t* load_offsets = nullptr;
+  int32_t* f[10] = {};
+  double* evalue = nullptr;
+  void alloc(int64_t count, int32_t n_loads) {
+    auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
+    const size_t lo = al(((size_t)n_loads + 1) * sizeof(int64_t));
+    const size_t w = al((size_t)(count ? count : 1) * sizeof(int32_t));
+    n = count;
+    bytes = lo + 10 * w + al((size_t)(count ? count : 1) * sizeof(double));
+    mem.alloc(bytes);
+    load_offsets = reinterpret_cast<int64_t*>(mem.p);
+    for (int k = 0; k < 10; ++k) f[k] = reinterpret_cast<int32_t*>(mem.p + lo + k * w);
+    evalue = reinterpret_cast<double*>(mem.p + lo + 10 * w);
+  }
+  OutView view() const {
+    OutView v{};
+    v.read = f[0]; v.strand = f[1]; v.t_load = f[2]; v.t_seq = f[3]; v.t_idx = f[4];
+    v.q_idx = f[5]; v.t_len = f[6]; v.q_len = f[7]; v.match = f[8]; v.score = f[9];
+    v.evalue = evalue;
+    return v;
+  }
+};
+
 // Pinned host buffer that holds one clast_map result; reused once released.
 struct PinnedArena {
   void* p = nullptr;
   size_t bytes = 0;
   std::atomic<bool> in_use{false};  // released by the result's owner, possibly on another thread
-  // The result's arrays on the device, kept until the arena is reused (so the
-  // text of a result can be formatted on the GPU): read strand t_load t_seq
-  // t_idx q_idx t_len q_len match score, evalue, and the per-load offsets.
+  // The result on the device, kept until the arena is reused (so the text of a
+  // result can be formatted on the GPU).
   struct Device {
-    DevArray<int32_t> f[10];
-    DevArray<double> evalue;
-    DevArray<int64_t> load_offsets;
+    ResultSlab slab;
     int64_t n = 0;
     int32_t n_loads = 0;
   } dev;
 };
 
+// Reads of a batch up to which the host looks at every length itself.
+constexpr int64_t kHostLengths = 1 << 15;
+// Most bytes a context stages in its pinned buffer.
+constexpr size_t kStageMax = (size_t)16 << 20;
 constexpr int kBuildStreams = 2;  // target windows indexed at once by clast_targets_create
 
 }  // namespace clast
@@ -184,6 +215,34 @@ struct clast_ctx {
   clast_stats stats{};
   StageTimer timer;
   int64_t seed_hint = 0;  // seed buffer capacity that sufficed before
+  clast::GroupCtl* ctl = nullptr;  // pinned copy of a group's counters
+  // Pinned buffer for small tables on their way up and small results on their
+  // way down.  stage() waits for the copy made from it last (staged()).
+  char* staging = nullptr;
+  size_t staging_bytes = 0;
+  cudaEvent_t ev_stage = nullptr;
+  bool stage_pending = false;
+  char* stage(size_t bytes) {
+    if (stage_pending) CLAST_CK(cudaEventSynchronize(ev_stage));
+    stage_pending = false;
+    if (staging_bytes < bytes) {
+      if (staging) CLAST_CK(cudaFreeHost(staging));
+      staging = nullptr;
+      staging_bytes = 0;
+      const size_t want = bytes + bytes / 2 + (64 << 10);
+      if (cudaMallocHost(reinterpret_cast<void**>(&staging), want) != cudaSuccess) {
+        (void)cudaGetLastError();
+        staging = nullptr;
+        throw std::bad_alloc();
+      }
+      staging_bytes = want;
+    }
+    return staging;
+  }
+  void staged(cudaStream_t s) {
+    CLAST_CK(cudaEventRecord(ev_stage, s));
+    stage_pending = true;
+  }
   // the DP's one-hit-per-warp kernel runs on st_dp beside the one-per-thread
   // kernels on st (forked and joined by these events)
   cudaStream_t st_dp = nullptr;

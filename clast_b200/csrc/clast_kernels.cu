@@ -81,7 +81,8 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
 template <class Load>
 __global__ void __launch_bounds__(kScanThreads) k_scan_1pass(Load in, int64_t n_in, int64_t n_out,
                                                              int64_t* __restrict__ out,
-                                                             unsigned long long* __restrict__ state) {
+                                                             unsigned long long* __restrict__ state,
+                                                             long long* __restrict__ total) {
   __shared__ int64_t warp_tot[kScanThreads / 32];
   __shared__ int64_t s_prefix;
   __shared__ unsigned long long s_tile;
@@ -170,6 +171,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_1pass(Load in, int64_t n_
   for (int i = 0; i < kScanItems; ++i) {
     const int64_t idx = base + i;
     if (idx < n_out) out[idx] = run;
+    if (idx == n_in && total) *total = run;
     run += v[i];
   }
 }
@@ -180,7 +182,7 @@ void scan_1pass(Workspace& ws, Load in, int64_t n, int64_t* out, cudaStream_t st
   const int64_t tiles = (n_out + kScanTile - 1) / kScanTile;
   unsigned long long* state = ws.get<unsigned long long>("scan1_state", tiles + 1);
   CLAST_CK(cudaMemsetAsync(state, 0, (tiles + 1) * sizeof(unsigned long long), st));
-  k_scan_1pass<Load><<<(unsigned)tiles, kScanThreads, 0, st>>>(in, n, n_out, out, state);
+  k_scan_1pass<Load><<<(unsigned)tiles, kScanThreads, 0, st>>>(in, n, n_out, out, state, nullptr);
   CLAST_LAUNCHED();
 }
 
@@ -263,27 +265,26 @@ __device__ __forceinline__ char complement(char c) {
   }
 }
 
-__global__ void k_strand_meta(const int64_t* __restrict__ off, int64_t n_reads, int64_t* __restrict__ sstart,
-                              int32_t* __restrict__ slen) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n_reads) return;
-  const int64_t a = off[r], len = off[r + 1] - a;
-  sstart[2 * r] = 2 * a;
-  sstart[2 * r + 1] = 2 * a + len;
-  slen[2 * r] = (int32_t)len;
-  slen[2 * r + 1] = (int32_t)len;
-}
-
 // One warp per read: the '+' strand copy and the reverse complement are both
 // coalesced (the reversed writes of a warp still cover one contiguous run).
 // The read goes in chunks of 8 x 32 bytes whose loads are all issued before
-// the first store, so a short read waits for memory once.
+// the first store, so a short read waits for memory once.  The warp also
+// writes the two strands' starts and lengths; the first and last ones the
+// kPad 'N' bytes before and after the array.
 __global__ void k_strands(const char* __restrict__ reads, const int64_t* __restrict__ off, int64_t n_reads,
-                          char* __restrict__ out) {
+                          char* __restrict__ out, int64_t* __restrict__ sstart, int32_t* __restrict__ slen) {
   const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (r >= n_reads) return;
   const int64_t a = off[r], len = off[r + 1] - a;
+  if (lane < 2) {
+    sstart[2 * r + lane] = 2 * a + lane * len;
+    slen[2 * r + lane] = (int32_t)len;
+  }
+  if (r == 0)
+    for (int i = lane; i < kPad; i += 32) out[i - kPad] = 'N';
+  if (r == n_reads - 1)
+    for (int i = lane; i < kPad; i += 32) out[2 * (a + len) + i] = 'N';
   char* const fwd = out + 2 * a;
   char* const rev = out + 2 * a + 2 * len - 1;  // base j of the read -> rev[-j]
   for (int64_t j0 = 0; j0 < len; j0 += 8 * 32) {
@@ -301,6 +302,23 @@ __global__ void k_strands(const char* __restrict__ reads, const int64_t* __restr
         rev[-j] = complement(c[u]);
       }
     }
+  }
+}
+
+// Shortest and longest read.
+__global__ void k_read_lengths(const int64_t* __restrict__ off, int64_t n_reads, int* __restrict__ min_len,
+                               int* __restrict__ max_len) {
+  int lo = INT_MAX, hi = 0;
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_reads; r += (int64_t)gridDim.x * blockDim.x) {
+    const int len = (int)(off[r + 1] - off[r]);
+    lo = min(lo, len);
+    hi = max(hi, len);
+  }
+  lo = __reduce_min_sync(kFull, lo);
+  hi = __reduce_max_sync(kFull, hi);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMin(min_len, lo);
+    atomicMax(max_len, hi);
   }
 }
 
@@ -717,7 +735,6 @@ __global__ void k_maxscan_apply(int64_t* __restrict__ out, int64_t n, const int6
 // strand on one diagonal arrive already sorted.
 constexpr int kSeedPerLane = 5;
 constexpr int kSeedRound = 32 * kSeedPerLane;
-constexpr int kSeedParts = 32;
 
 // Both records of a home bucket: one 256-bit streaming load (sm_100), the
 // address 32-byte aligned (home records are even, the table 256-byte aligned).
@@ -1239,6 +1256,7 @@ __global__ void __launch_bounds__(kSeedFusedThreads, NW <= 2 ? 16 : 8) k_seed_mu
 #pragma unroll
   for (int w = 0; w < NW; ++w) tot[w] = (int)__reduce_add_sync(kFull, (unsigned)cnt[w]);
   const int part = (int)(s % kSeedParts);
+  const int64_t v0 = (s >> 1) * (2 * NW) + (s & 1);  // see strand_slot
   // the range reservations: lane w reserves window w's
   unsigned long long rel = 0;
   if (lane < NW) {
@@ -1255,14 +1273,14 @@ __global__ void __launch_bounds__(kSeedFusedThreads, NW <= 2 ? 16 : 8) k_seed_mu
 #pragma unroll
   for (int w = 0; w < NW; ++w) {
     const unsigned long long r = __shfl_sync(kFull, rel, w);
-    const int64_t base = (int64_t)part * W.w[w].part_cap + (int64_t)r;
+    const int64_t base = (int64_t)(w * kSeedParts + part) * W.part_cap + (int64_t)r;
     wpos[w] = base;
-    ok[w] = tot[w] > 0 && base + tot[w] <= (int64_t)(part + 1) * W.w[w].part_cap;
+    ok[w] = tot[w] > 0 && base + tot[w] <= (int64_t)(w * kSeedParts + part + 1) * W.part_cap;
     any |= ok[w];
     if (lane == 0) {
-      W.w[w].off[s] = base;
-      W.w[w].cnt[s] = tot[w];
-      if (!ok[w]) W.w[w].nvalid[s] = 0;
+      W.off[v0 + 2 * w] = base;
+      W.cnt[v0 + 2 * w] = tot[w];
+      if (!ok[w]) W.nvalid[v0 + 2 * w] = 0;
     }
   }
   if (!any) return;
@@ -1279,152 +1297,46 @@ __global__ void __launch_bounds__(kSeedFusedThreads, NW <= 2 ? 16 : 8) k_seed_mu
       uint64_t pl[P];
 #pragma unroll
       for (int i = 0; i < P; ++i) pl[i] = sm.pl[w][lane * P + i];
-      round_emit(W.w[w].ix, W.w[w].t, gap, local, qlen, r0, lane, pl, wpos[w], valid[w], W.w[w].skey, W.w[w].sq,
+      round_emit(W.w[w].ix, W.w[w].t, gap, local, qlen, r0, lane, pl, wpos[w], valid[w], W.skey, W.sq,
                  sm.u.stage.pl, sm.u.stage.qi);
     }
   }
 #pragma unroll
   for (int w = 0; w < NW; ++w) {
     const int v = (int)__reduce_add_sync(kFull, (unsigned)valid[w]);
-    if (lane == 0 && ok[w]) W.w[w].nvalid[s] = v;
+    if (lane == 0 && ok[w]) W.nvalid[v0 + 2 * w] = v;
   }
 }
 
-__global__ void k_window_first(const int32_t* __restrict__ nvalid, const int32_t* __restrict__ wstart, int nwin,
-                               int32_t* __restrict__ wfirst) {
-  const int w = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+// The first strand of every (target window, query window) with a valid seed:
+// its seed count is stored complemented (the isolate filter keeps the first
+// seed of a query window).
+__global__ void k_window_first(int32_t* __restrict__ nvalid, const int32_t* __restrict__ wstart, int nwin, int nw) {
+  const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
-  if (w >= nwin) return;
-  const int a = wstart[w], b = wstart[w + 1];
-  int first = -1;
-  for (int c = a; c < b && first < 0; c += 32) {
+  if (i >= nwin * nw) return;
+  const int w = i / nwin, qw = i % nwin;
+  const int a = wstart[qw], b = wstart[qw + 1];
+  for (int c = a; c < b; c += 32) {
     const int s = c + lane;
-    const unsigned m = __ballot_sync(kFull, s < b && nvalid[s] > 0);
-    if (m) first = c + __ffs(m) - 1;
+    const int64_t v = strand_slot(s, w, nw);
+    const int n = s < b ? nvalid[v] : 0;
+    const unsigned m = __ballot_sync(kFull, n > 0);
+    if (m) {
+      if (lane == __ffs(m) - 1) nvalid[v] = ~n;
+      return;
+    }
   }
-  if (lane == 0) wfirst[w] = first;
 }
 
-// ---- segmented sort (ascending compare-exchange network, safe with a ragged tail) ----
+// ---- sorting networks (ascending compare-exchange, safe with a ragged tail) ----
 template <class K2>
 __device__ __forceinline__ bool less2(uint64_t a1, K2 a2, uint64_t b1, K2 b2) {
   return a1 < b1 || (a1 == b1 && a2 < b2);
 }
 
-// Segments of 2..kThreadSegCap items are sorted one per thread (most reads
-// have one or two hits), up to 32 one per warp, up to 2048 per CTA, longer
-// in global memory.
-constexpr int kThreadSegCap = 8, kSegTiers = 4;
-
-template <class K2, bool PAY>
-__global__ void k_classify(const int32_t* __restrict__ len, int64_t nseg, int32_t* __restrict__ lists,
-                           int32_t* __restrict__ counts) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = (i < nseg) ? len[i] : 0;
-  const int tier = (n <= 1) ? -1 : (n <= kThreadSegCap ? 0 : ((n <= 32) ? 1 : (n <= 2048 ? 2 : 3)));
-  const int lane = threadIdx.x & 31;
-  // one atomic per warp and tier
-#pragma unroll
-  for (int t = 0; t < kSegTiers; ++t) {
-    const unsigned m = __ballot_sync(kFull, tier == t);
-    if (!m) continue;
-    int base = 0;
-    if (lane == __ffs(m) - 1) base = atomicAdd(&counts[t], __popc(m));
-    base = __shfl_sync(kFull, base, __ffs(m) - 1);
-    if (tier == t) lists[(int64_t)t * nseg + base + __popc(m & lanemask_lt())] = (int32_t)i;
-  }
-}
-
-// 2..kThreadSegCap items: one thread per segment, an odd-even transposition
-// network in registers over the segment's own items only (a compare-exchange
-// past its end is skipped, so nothing but its items moves).
-template <class K2, bool PAY>
-__global__ void k_sort_thread(uint64_t* __restrict__ k1, K2* __restrict__ k2, int32_t* __restrict__ pay,
-                              const int64_t* __restrict__ off, const int32_t* __restrict__ len,
-                              const int32_t* __restrict__ list, const int32_t* __restrict__ count) {
-  const int total = *count;
-  for (int64_t li = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; li < total;
-       li += (int64_t)gridDim.x * blockDim.x) {
-    const int seg = list[li];
-    const int64_t o = off[seg];
-    const int n = len[seg];
-    uint64_t a[kThreadSegCap];
-    K2 b[kThreadSegCap];
-    int32_t p[kThreadSegCap];
-#pragma unroll
-    for (int i = 0; i < kThreadSegCap; ++i) {
-      a[i] = i < n ? k1[o + i] : 0ull;
-      b[i] = i < n ? k2[o + i] : (K2)0;
-      p[i] = (PAY && i < n) ? pay[o + i] : 0;
-    }
-#pragma unroll
-    for (int pass = 0; pass < kThreadSegCap; ++pass)
-#pragma unroll
-      for (int i = pass & 1; i + 1 < kThreadSegCap; i += 2)
-        if (i + 1 < n && less2(a[i + 1], b[i + 1], a[i], b[i])) {
-          const uint64_t ta = a[i]; a[i] = a[i + 1]; a[i + 1] = ta;
-          const K2 tb = b[i]; b[i] = b[i + 1]; b[i + 1] = tb;
-          const int32_t tp = p[i]; p[i] = p[i + 1]; p[i + 1] = tp;
-        }
-#pragma unroll
-    for (int i = 0; i < kThreadSegCap; ++i)
-      if (i < n) {
-        k1[o + i] = a[i];
-        k2[o + i] = b[i];
-        if (PAY) pay[o + i] = p[i];
-      }
-  }
-}
-
-template <class K2, bool PAY>
-__global__ void k_sort_warp(uint64_t* __restrict__ k1, K2* __restrict__ k2, int32_t* __restrict__ pay,
-                            const int64_t* __restrict__ off, const int32_t* __restrict__ len,
-                            const int32_t* __restrict__ list, const int32_t* __restrict__ count) {
-  const int lane = threadIdx.x & 31;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int total = *count;
-  for (int64_t li = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; li < total; li += nwarps) {
-    const int seg = list[li];
-    const int64_t o = off[seg];
-    const int n = len[seg];
-    uint64_t a1 = ~0ull;
-    K2 a2 = (K2)~(K2)0;
-    int32_t ap = 0;
-    if (lane < n) {
-      a1 = k1[o + lane];
-      a2 = k2[o + lane];
-      if (PAY) ap = pay[o + lane];
-    }
-    for (int size = 2; size <= 32; size <<= 1) {
-      {
-        const int partner = lane ^ (size - 1);
-        const uint64_t b1 = __shfl_sync(kFull, a1, partner);
-        const K2 b2 = __shfl_sync(kFull, a2, partner);
-        const int32_t bp = __shfl_sync(kFull, ap, partner);
-        const bool lower = lane < partner;
-        const bool b_less = less2(b1, b2, a1, a2);
-        if (lower ? b_less : !b_less && (b1 != a1 || b2 != a2)) { a1 = b1; a2 = b2; ap = bp; }
-      }
-      for (int stride = size >> 2; stride > 0; stride >>= 1) {
-        const int partner = lane ^ stride;
-        const uint64_t b1 = __shfl_sync(kFull, a1, partner);
-        const K2 b2 = __shfl_sync(kFull, a2, partner);
-        const int32_t bp = __shfl_sync(kFull, ap, partner);
-        const bool lower = lane < partner;
-        const bool b_less = less2(b1, b2, a1, a2);
-        if (lower ? b_less : !b_less && (b1 != a1 || b2 != a2)) { a1 = b1; a2 = b2; ap = bp; }
-      }
-    }
-    if (lane < n) {
-      k1[o + lane] = a1;
-      k2[o + lane] = a2;
-      if (PAY) pay[o + lane] = ap;
-    }
-  }
-}
-
-template <class K2, bool PAY>
-__device__ __forceinline__ void cta_network(uint64_t* s1, K2* s2, int32_t* sp, int n) {
+template <class K2>
+__device__ __forceinline__ void cta_network(uint64_t* s1, K2* s2, int n) {
   int np = 1;
   while (np < n) np <<= 1;
   for (int size = 2; size <= np; size <<= 1) {
@@ -1434,7 +1346,6 @@ __device__ __forceinline__ void cta_network(uint64_t* s1, K2* s2, int32_t* sp, i
       if (b < n && less2(s1[b], s2[b], s1[a], s2[a])) {
         const uint64_t t1 = s1[a]; s1[a] = s1[b]; s1[b] = t1;
         const K2 t2 = s2[a]; s2[a] = s2[b]; s2[b] = t2;
-        if (PAY) { const int32_t tp = sp[a]; sp[a] = sp[b]; sp[b] = tp; }
       }
     }
     __syncthreads();
@@ -1445,7 +1356,6 @@ __device__ __forceinline__ void cta_network(uint64_t* s1, K2* s2, int32_t* sp, i
         if (b < n && less2(s1[b], s2[b], s1[a], s2[a])) {
           const uint64_t t1 = s1[a]; s1[a] = s1[b]; s1[b] = t1;
           const K2 t2 = s2[a]; s2[a] = s2[b]; s2[b] = t2;
-          if (PAY) { const int32_t tp = sp[a]; sp[a] = sp[b]; sp[b] = tp; }
         }
       }
       __syncthreads();
@@ -1453,75 +1363,27 @@ __device__ __forceinline__ void cta_network(uint64_t* s1, K2* s2, int32_t* sp, i
   }
 }
 
+// Compare-exchange of a network step held one element per lane: the lower
+// lane of the pair keeps the smaller element.
+template <class K2>
+__device__ __forceinline__ void warp_cx(uint64_t& a1, K2& a2, int lane, int partner) {
+  const uint64_t b1 = __shfl_sync(kFull, a1, partner);
+  const K2 b2 = __shfl_sync(kFull, a2, partner);
+  const bool b_less = less2(b1, b2, a1, a2);
+  if (lane < partner ? b_less : !b_less && (b1 != a1 || b2 != a2)) { a1 = b1; a2 = b2; }
+}
+// Sorts every group of N lanes (N a power of two up to 32).
+template <int N, class K2>
+__device__ __forceinline__ void lanes_sort(uint64_t& a1, K2& a2, int lane) {
+#pragma unroll
+  for (int size = 2; size <= N; size <<= 1) {
+    warp_cx(a1, a2, lane, lane ^ (size - 1));
+#pragma unroll
+    for (int stride = size >> 2; stride > 0; stride >>= 1) warp_cx(a1, a2, lane, lane ^ stride);
+  }
+}
+
 constexpr int kCtaSortCap = 2048;
-
-template <class K2, bool PAY>
-__global__ void __launch_bounds__(256) k_sort_cta(uint64_t* __restrict__ k1, K2* __restrict__ k2,
-                                                  int32_t* __restrict__ pay, const int64_t* __restrict__ off,
-                                                  const int32_t* __restrict__ len, const int32_t* __restrict__ list,
-                                                  const int32_t* __restrict__ count) {
-  __shared__ uint64_t s1[kCtaSortCap];
-  __shared__ K2 s2[kCtaSortCap];
-  __shared__ int32_t sp[PAY ? kCtaSortCap : 1];
-  const int total = *count;
-  for (int li = blockIdx.x; li < total; li += gridDim.x) {
-    const int seg = list[li];
-    const int64_t o = off[seg];
-    const int n = len[seg];
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      s1[i] = k1[o + i];
-      s2[i] = k2[o + i];
-      if (PAY) sp[i] = pay[o + i];
-    }
-    __syncthreads();
-    cta_network<K2, PAY>(s1, s2, sp, n);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      k1[o + i] = s1[i];
-      k2[o + i] = s2[i];
-      if (PAY) pay[o + i] = sp[i];
-    }
-    __syncthreads();
-  }
-}
-
-template <class K2, bool PAY>
-__global__ void __launch_bounds__(1024) k_sort_global(uint64_t* __restrict__ k1, K2* __restrict__ k2,
-                                                      int32_t* __restrict__ pay, const int64_t* __restrict__ off,
-                                                      const int32_t* __restrict__ len,
-                                                      const int32_t* __restrict__ list,
-                                                      const int32_t* __restrict__ count) {
-  const int total = *count;
-  for (int li = blockIdx.x; li < total; li += gridDim.x) {
-    const int seg = list[li];
-    const int64_t o = off[seg];
-    cta_network<K2, PAY>(k1 + o, k2 + o, PAY ? pay + o : pay, len[seg]);
-    __syncthreads();
-  }
-}
-
-template <class K2, bool PAY>
-void seg_sort(Workspace& ws, uint64_t* k1, K2* k2, int32_t* pay, const int64_t* off, const int32_t* len,
-              int64_t nseg, cudaStream_t st, int tag) {
-  if (nseg <= 0) return;
-  const std::string t = "segsort" + std::to_string(tag);
-  int32_t* lists = ws.get<int32_t>(t + "l", kSegTiers * nseg);
-  int32_t* counts = ws.get<int32_t>(t + "c", kSegTiers);
-  CLAST_CK(cudaMemsetAsync(counts, 0, kSegTiers * sizeof(int32_t), st));
-  k_classify<K2, PAY><<<blocks_for(nseg, 256), 256, 0, st>>>(len, nseg, lists, counts);
-  CLAST_LAUNCHED();
-  k_sort_thread<K2, PAY><<<grid_cap((nseg + 255) / 256), 256, 0, st>>>(k1, k2, pay, off, len, lists, counts);
-  CLAST_LAUNCHED();
-  k_sort_warp<K2, PAY><<<grid_cap((nseg * 32 + 255) / 256), 256, 0, st>>>(k1, k2, pay, off, len, lists + nseg,
-                                                                          counts + 1);
-  CLAST_LAUNCHED();
-  k_sort_cta<K2, PAY><<<grid_cap(nseg < 4096 ? nseg : 4096), 256, 0, st>>>(k1, k2, pay, off, len, lists + 2 * nseg,
-                                                                           counts + 2);
-  CLAST_LAUNCHED();
-  k_sort_global<K2, PAY><<<grid_cap(nseg < 1024 ? nseg : 1024), 1024, 0, st>>>(k1, k2, pay, off, len,
-                                                                                lists + 3 * nseg, counts + 3);
-  CLAST_LAUNCHED();
-}
-
 
 // is "s" near its predecessor "p" (hasNotNearPair / hasNearPair, same strand)
 __device__ __forceinline__ bool near_pred(int tid, int tidx, int diag, int ptid, int ptidx, int pdiag,
@@ -1531,26 +1393,15 @@ __device__ __forceinline__ bool near_pred(int tid, int tidx, int diag, int ptid,
 
 
 // ---- seed sort fused with the isolate / duplicate filters ----
+// Slots (strand, target window) of a group; nvalid as k_window_first leaves it.
 struct SeedFilterCtx {
   const int64_t* off;
   const int32_t* cnt;
   const int32_t* nvalid;
-  const int32_t* wstart;
-  int nwin;
-  const int32_t* wfirst;
   int width, gap;
   int32_t* hcnt;
 };
-
-__device__ __forceinline__ bool window_first_strand(int64_t s, const SeedFilterCtx& c) {
-  int lo = 0, hi = c.nwin;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (c.wstart[mid] <= s) lo = mid;
-    else hi = mid;
-  }
-  return c.wfirst[lo] == (int32_t)s;
-}
+__device__ __forceinline__ int valid_seeds(int nvalid) { return nvalid < 0 ? ~nvalid : nvalid; }
 
 // State carried from one 32-seed chunk of a strand to the next.
 struct FilterState {
@@ -1608,51 +1459,18 @@ __device__ __forceinline__ void filter_chunk(int c0, int n, uint64_t k, uint32_t
   }
 }
 
-// Seed-sort tiers by a strand's seed count: <= kThreadSortCap (one thread,
-// registers; most strands hold a few chance seeds), <= 32 (one warp,
-// registers), <= kWarpSmemCap (one warp, shared memory), <= kCtaSortCap (one
-// CTA, shared memory), longer (one CTA, global memory).  List entries are the
-// strand index with the window-first flag in bit 31.
-constexpr int kSortTiers = 5;
+// Seed-sort tiers by a slot's seed count: <= kThreadSortCap (one thread,
+// registers; most slots hold a few chance seeds), <= kWarpSmemCap (one warp:
+// up to 32 in registers, more in its slice of shared memory), longer (one CTA:
+// up to kCtaSortCap in shared memory, more in global memory).  The first tier
+// runs over all slots and lists the others' slots; so four launches do what
+// a classification and five tiers did, for every window of the group at once.
 constexpr int kThreadSortCap = 8;
 constexpr int kWarpSmemCap = 256;
-constexpr uint32_t kWinFirstBit = 0x80000000u;
 
-__global__ void k_seed_classify(SeedFilterCtx c, int64_t ns, int32_t* __restrict__ lists,
-                                int32_t* __restrict__ counts) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = (i < ns && c.nvalid[i] > 0) ? c.cnt[i] : 0;
-  const int tier = (n <= 0)                ? -1
-                 : (n <= kThreadSortCap) ? 0
-                 : (n <= 32)             ? 1
-                 : (n <= kWarpSmemCap)   ? 2
-                 : (n <= kCtaSortCap)    ? 3
-                                         : 4;
-  const int lane = threadIdx.x & 31;
-  const uint32_t entry = (uint32_t)i | ((tier >= 0 && window_first_strand(i, c)) ? kWinFirstBit : 0u);
-#pragma unroll
-  for (int t = 0; t < kSortTiers; ++t) {
-    const unsigned m = __ballot_sync(kFull, tier == t);
-    if (!m) continue;
-    int base = 0;
-    if (lane == __ffs(m) - 1) base = atomicAdd(&counts[t], __popc(m));
-    base = __shfl_sync(kFull, base, __ffs(m) - 1);
-    if (tier == t) lists[(int64_t)t * ns + base + __popc(m & lanemask_lt())] = (int32_t)entry;
-  }
-}
-
-// Compare-exchange of a warp-wide bitonic network step held one element per
-// lane: the lower lane of the pair keeps the smaller element.
-__device__ __forceinline__ void warp_cx(uint64_t& a1, uint32_t& a2, int lane, int partner) {
-  const uint64_t b1 = __shfl_sync(kFull, a1, partner);
-  const uint32_t b2 = __shfl_sync(kFull, a2, partner);
-  const bool b_less = less2(b1, b2, a1, a2);
-  if (lane < partner ? b_less : !b_less && (b1 != a1 || b2 != a2)) { a1 = b1; a2 = b2; }
-}
-
-// 1..kThreadSortCap seeds: one thread per strand.  The seeds (padded with
+// 1..kThreadSortCap seeds: one thread per slot.  The seeds (padded with
 // keys above every seed) go through an odd-even transposition network in
-// registers unless they already ascend; the strand's nvalid valid seeds then
+// registers unless they already ascend; the slot's valid seeds then
 // come first (seeds the boundary filters dropped hold kDroppedSeed, above
 // every valid key) and only they are filtered, in seed order, as
 // filter_chunk applies the filters to a warp's chunk:
@@ -1660,94 +1478,74 @@ __device__ __forceinline__ void warp_cx(uint64_t& a1, uint32_t& a2, int lane, in
 // strand's first seed only when the strand is its window's first), and the
 // duplicate filter then drops it when it is near the previous seed that
 // survived the isolate filter.
-__global__ void k_seed_sort_filter_thread(uint64_t* __restrict__ skey, uint32_t* __restrict__ sq, SeedFilterCtx c,
-                                          const int32_t* __restrict__ list, const int32_t* __restrict__ count) {
-  const int total = *count;
-  for (int64_t li = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; li < total;
-       li += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t e = (uint32_t)list[li];
-    const int s = (int)(e & ~kWinFirstBit);
-    const int64_t o = c.off[s];
-    const int n = c.cnt[s];
-    const int nv = c.nvalid[s];
-    uint64_t k[kThreadSortCap];
-    uint32_t q[kThreadSortCap];
-    bool sorted = true;
-#pragma unroll
-    for (int i = 0; i < kThreadSortCap; ++i) {
-      k[i] = i < n ? skey[o + i] : ~0ull;
-      q[i] = i < n ? sq[o + i] : ~0u;
-      if (i > 0 && less2(k[i], q[i], k[i - 1], q[i - 1])) sorted = false;
-    }
-    if (!sorted) {
-#pragma unroll
-      for (int pass = 0; pass < kThreadSortCap; ++pass)
-#pragma unroll
-        for (int i = pass & 1; i + 1 < kThreadSortCap; i += 2)
-          if (less2(k[i + 1], q[i + 1], k[i], q[i])) {
-            const uint64_t tk = k[i]; k[i] = k[i + 1]; k[i + 1] = tk;
-            const uint32_t tq = q[i]; q[i] = q[i + 1]; q[i + 1] = tq;
-          }
-    }
-    const bool wf = (e & kWinFirstBit) != 0;
-    int ptid = 0, ptidx = 0, pdiag = 0;  // previous seed
-    int stid = 0, stidx = 0, sdiag = 0;  // previous isolate-filter survivor
-    bool have = false;
-    int64_t out = o;
-#pragma unroll
-    for (int j = 0; j < kThreadSortCap; ++j) {
-      if (j < nv) {
-        const int tid = (int)(k[j] >> 32);
-        const int diag = (int)((uint32_t)k[j] ^ 0x80000000u);
-        const int tidx = diag + (int)q[j];
-        const bool k8 = (j == 0) ? wf : near_pred(tid, tidx, diag, ptid, ptidx, pdiag, c.width, c.gap);
-        const bool k9 = k8 && !(have && near_pred(tid, tidx, diag, stid, stidx, sdiag, c.width, c.gap));
-        if (k9) {
-          skey[out] = k[j];
-          sq[out] = q[j];
-          ++out;
-        }
-        if (k8) { stid = tid; stidx = tidx; sdiag = diag; have = true; }
-        ptid = tid; ptidx = tidx; pdiag = diag;
-      }
-    }
-    c.hcnt[s] = (int32_t)(out - o);
-  }
-}
-
-// <= 32 seeds: one warp sorts in registers (network sized to the count,
-// skipped when the seeds already ascend) and filters from registers.
-__global__ void k_seed_sort_filter_warp(uint64_t* __restrict__ skey, uint32_t* __restrict__ sq, SeedFilterCtx c,
-                                        const int32_t* __restrict__ list, const int32_t* __restrict__ count) {
+__global__ void k_seed_filter_small(uint64_t* __restrict__ skey, uint32_t* __restrict__ sq, SeedFilterCtx c, int64_t nv,
+                                    uint32_t* __restrict__ lists, GroupCtl* __restrict__ ctl) {
+  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int x = s < nv ? c.nvalid[s] : 0;
+  const int nvalid = valid_seeds(x);
+  const int n = nvalid > 0 ? c.cnt[s] : 0;
   const int lane = threadIdx.x & 31;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int total = *count;
-  for (int64_t li = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; li < total; li += nwarps) {
-    const uint32_t e = (uint32_t)list[li];
-    const int s = (int)(e & ~kWinFirstBit);
-    const int64_t o = c.off[s];
-    const int n = c.cnt[s];
-    uint64_t a1 = ~0ull;
-    uint32_t a2 = ~0u;
-    if (lane < n) {
-      a1 = skey[o + lane];
-      a2 = sq[o + lane];
-    }
-    const uint64_t n1 = __shfl_down_sync(kFull, a1, 1);
-    const uint32_t n2 = __shfl_down_sync(kFull, a2, 1);
-    if (__any_sync(kFull, lane + 1 < n && less2(n1, n2, a1, a2))) {
-      int np = 2;
-      while (np < n) np <<= 1;
-      for (int size = 2; size <= np; size <<= 1) {
-        warp_cx(a1, a2, lane, lane ^ (size - 1));
-        for (int stride = size >> 2; stride > 0; stride >>= 1) warp_cx(a1, a2, lane, lane ^ stride);
-      }
-    }
-    FilterState f;
-    f.out = o;
-    filter_chunk(0, c.nvalid[s], a1, a2, (e & kWinFirstBit) != 0, c.width, c.gap, f, skey, sq);
-    if (lane == 0) c.hcnt[s] = (int32_t)(f.out - o);
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    const bool in = t == 0   ? n > kThreadSortCap && n <= kWarpSmemCap
+                    : t == 1 ? n > kWarpSmemCap && n <= kCtaSortCap
+                             : n > kCtaSortCap;
+    const unsigned m = __ballot_sync(kFull, in);
+    if (!m) continue;
+    int base = 0;
+    if (lane == __ffs(m) - 1) base = atomicAdd(&ctl->n_seeds[t], __popc(m));
+    base = __shfl_sync(kFull, base, __ffs(m) - 1);
+    if (in) lists[t * nv + base + __popc(m & lanemask_lt())] = (uint32_t)s;
   }
+  if (s >= nv || n > kThreadSortCap) return;
+  if (n == 0) {
+    c.hcnt[s] = 0;
+    return;
+  }
+  const int64_t o = c.off[s];
+  const int nv_s = nvalid;
+  uint64_t k[kThreadSortCap];
+  uint32_t q[kThreadSortCap];
+  bool sorted = true;
+#pragma unroll
+  for (int i = 0; i < kThreadSortCap; ++i) {
+    k[i] = i < n ? skey[o + i] : ~0ull;
+    q[i] = i < n ? sq[o + i] : ~0u;
+    if (i > 0 && less2(k[i], q[i], k[i - 1], q[i - 1])) sorted = false;
+  }
+  if (!sorted) {
+#pragma unroll
+    for (int pass = 0; pass < kThreadSortCap; ++pass)
+#pragma unroll
+      for (int i = pass & 1; i + 1 < kThreadSortCap; i += 2)
+        if (less2(k[i + 1], q[i + 1], k[i], q[i])) {
+          const uint64_t tk = k[i]; k[i] = k[i + 1]; k[i + 1] = tk;
+          const uint32_t tq = q[i]; q[i] = q[i + 1]; q[i + 1] = tq;
+        }
+  }
+  const bool wf = x < 0;
+  int ptid = 0, ptidx = 0, pdiag = 0;  // previous seed
+  int stid = 0, stidx = 0, sdiag = 0;  // previous isolate-filter survivor
+  bool have = false;
+  int64_t out = o;
+#pragma unroll
+  for (int j = 0; j < kThreadSortCap; ++j) {
+    if (j < nv_s) {
+      const int tid = (int)(k[j] >> 32);
+      const int diag = (int)((uint32_t)k[j] ^ 0x80000000u);
+      const int tidx = diag + (int)q[j];
+      const bool k8 = (j == 0) ? wf : near_pred(tid, tidx, diag, ptid, ptidx, pdiag, c.width, c.gap);
+      const bool k9 = k8 && !(have && near_pred(tid, tidx, diag, stid, stidx, sdiag, c.width, c.gap));
+      if (k9) {
+        skey[out] = k[j];
+        sq[out] = q[j];
+        ++out;
+      }
+      if (k8) { stid = tid; stidx = tidx; sdiag = diag; have = true; }
+      ptid = tid; ptidx = tidx; pdiag = diag;
+    }
+  }
+  c.hcnt[s] = (int32_t)(out - o);
 }
 
 // Bitonic network over n <= np elements in shared memory, run by one warp.
@@ -1781,11 +1579,13 @@ __device__ __forceinline__ void warp_smem_network(uint64_t* s1, uint32_t* s2, in
 
 constexpr int kWarpSmemThreads = 128;
 
-// 33..kWarpSmemCap seeds: one warp sorts in its own slice of shared memory
-// (skipped when the seeds already ascend) and filters from there.
-__global__ void __launch_bounds__(kWarpSmemThreads) k_seed_sort_filter_warp_smem(
-    uint64_t* __restrict__ skey, uint32_t* __restrict__ sq, SeedFilterCtx c, const int32_t* __restrict__ list,
-    const int32_t* __restrict__ count) {
+// kThreadSortCap + 1 .. kWarpSmemCap seeds: one warp per slot, sorting in
+// registers up to 32 (a network sized to the count) and in its own slice of
+// shared memory above; skipped when the seeds already ascend.
+__global__ void __launch_bounds__(kWarpSmemThreads) k_seed_filter_mid(uint64_t* __restrict__ skey,
+                                                                      uint32_t* __restrict__ sq, SeedFilterCtx c,
+                                                                      const uint32_t* __restrict__ list,
+                                                                      const int* __restrict__ count) {
   __shared__ uint64_t sh1[kWarpSmemThreads / 32][kWarpSmemCap];
   __shared__ uint32_t sh2[kWarpSmemThreads / 32][kWarpSmemCap];
   const int lane = threadIdx.x & 31;
@@ -1794,79 +1594,76 @@ __global__ void __launch_bounds__(kWarpSmemThreads) k_seed_sort_filter_warp_smem
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int total = *count;
   for (int64_t li = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; li < total; li += nwarps) {
-    const uint32_t e = (uint32_t)list[li];
-    const int s = (int)(e & ~kWinFirstBit);
+    const int64_t s = list[li];
     const int64_t o = c.off[s];
     const int n = c.cnt[s];
-    for (int i = lane; i < n; i += 32) {
-      s1[i] = skey[o + i];
-      s2[i] = sq[o + i];
-    }
-    __syncwarp();
-    bool unsorted = false;
-    for (int i = lane; i + 1 < n; i += 32) unsorted |= less2(s1[i + 1], s2[i + 1], s1[i], s2[i]);
-    if (__any_sync(kFull, unsorted)) warp_smem_network(s1, s2, n);
-    const int nv = c.nvalid[s];
-    const bool wf = (e & kWinFirstBit) != 0;
+    const int x = c.nvalid[s];
+    const int nv = valid_seeds(x);
     FilterState f;
     f.out = o;
-    for (int c0 = 0; c0 < nv; c0 += 32) {
-      const int j = c0 + lane;
-      filter_chunk(c0, nv, j < nv ? s1[j] : 0ull, j < nv ? s2[j] : 0u, wf, c.width, c.gap, f, skey, sq);
+    if (n <= 32) {
+      uint64_t a1 = ~0ull;
+      uint32_t a2 = ~0u;
+      if (lane < n) {
+        a1 = skey[o + lane];
+        a2 = sq[o + lane];
+      }
+      const uint64_t n1 = __shfl_down_sync(kFull, a1, 1);
+      const uint32_t n2 = __shfl_down_sync(kFull, a2, 1);
+      if (__any_sync(kFull, lane + 1 < n && less2(n1, n2, a1, a2))) {
+        if (n <= 16) lanes_sort<16>(a1, a2, lane);
+        else lanes_sort<32>(a1, a2, lane);
+      }
+      filter_chunk(0, nv, a1, a2, x < 0, c.width, c.gap, f, skey, sq);
+    } else {
+      for (int i = lane; i < n; i += 32) {
+        s1[i] = skey[o + i];
+        s2[i] = sq[o + i];
+      }
+      __syncwarp();
+      bool unsorted = false;
+      for (int i = lane; i + 1 < n; i += 32) unsorted |= less2(s1[i + 1], s2[i + 1], s1[i], s2[i]);
+      if (__any_sync(kFull, unsorted)) warp_smem_network(s1, s2, n);
+      for (int c0 = 0; c0 < nv; c0 += 32) {
+        const int j = c0 + lane;
+        filter_chunk(c0, nv, j < nv ? s1[j] : 0ull, j < nv ? s2[j] : 0u, x < 0, c.width, c.gap, f, skey, sq);
+      }
+      __syncwarp();
     }
     if (lane == 0) c.hcnt[s] = (int32_t)(f.out - o);
-    __syncwarp();
   }
 }
 
-// <= kCtaSortCap seeds: one CTA sorts in shared memory, warp 0 filters from there.
-__global__ void __launch_bounds__(256) k_seed_sort_filter_cta(uint64_t* __restrict__ skey, uint32_t* __restrict__ sq,
-                                                              SeedFilterCtx c, const int32_t* __restrict__ list,
-                                                              const int32_t* __restrict__ count) {
-  __shared__ uint64_t s1[kCtaSortCap];
-  __shared__ uint32_t s2[kCtaSortCap];
+// Longer: one CTA per slot sorts and warp 0 filters from there.  Slots of up
+// to kCtaSortCap seeds are sorted in shared memory by 256 threads (1,024
+// threads, which the longer ones need, took 1.73 against 0.95 ms for the whole
+// stage on a repeat-rich genome), more in global memory by 1,024.
+template <bool SMEM>
+__global__ void __launch_bounds__(SMEM ? 256 : 1024) k_seed_filter_big(uint64_t* __restrict__ skey,
+                                                                       uint32_t* __restrict__ sq, SeedFilterCtx c,
+                                                                       const uint32_t* __restrict__ list,
+                                                                       const int* __restrict__ count) {
+  __shared__ uint64_t s1[SMEM ? kCtaSortCap : 1];
+  __shared__ uint32_t s2[SMEM ? kCtaSortCap : 1];
   const int total = *count;
   for (int li = blockIdx.x; li < total; li += gridDim.x) {
-    const uint32_t e = (uint32_t)list[li];
-    const int s = (int)(e & ~kWinFirstBit);
+    const int64_t s = list[li];
     const int64_t o = c.off[s];
     const int n = c.cnt[s];
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      s1[i] = skey[o + i];
-      s2[i] = sq[o + i];
-    }
-    __syncthreads();
-    cta_network<uint32_t, false>(s1, s2, nullptr, n);
-    if (threadIdx.x < 32) {
-      const int nv = c.nvalid[s];
-      const bool wf = (e & kWinFirstBit) != 0;
-      FilterState f;
-      f.out = o;
-      for (int c0 = 0; c0 < nv; c0 += 32) {
-        const int j = c0 + (int)threadIdx.x;
-        filter_chunk(c0, nv, j < nv ? s1[j] : 0ull, j < nv ? s2[j] : 0u, wf, c.width, c.gap, f, skey, sq);
+    if (SMEM) {
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        s1[i] = skey[o + i];
+        s2[i] = sq[o + i];
       }
-      if (threadIdx.x == 0) c.hcnt[s] = (int32_t)(f.out - o);
+      __syncthreads();
+      cta_network(s1, s2, n);
+    } else {
+      cta_network(skey + o, sq + o, n);
+      __syncthreads();
     }
-    __syncthreads();
-  }
-}
-
-// Longer: one CTA sorts in global memory, warp 0 filters in place.
-__global__ void __launch_bounds__(1024) k_seed_sort_filter_global(uint64_t* __restrict__ skey,
-                                                                  uint32_t* __restrict__ sq, SeedFilterCtx c,
-                                                                  const int32_t* __restrict__ list,
-                                                                  const int32_t* __restrict__ count) {
-  const int total = *count;
-  for (int li = blockIdx.x; li < total; li += gridDim.x) {
-    const uint32_t e = (uint32_t)list[li];
-    const int s = (int)(e & ~kWinFirstBit);
-    const int64_t o = c.off[s];
-    cta_network<uint32_t, false>(skey + o, sq + o, nullptr, c.cnt[s]);
-    __syncthreads();
     if (threadIdx.x < 32) {
-      const int nv = c.nvalid[s];
-      const bool wf = (e & kWinFirstBit) != 0;
+      const int x = c.nvalid[s];
+      const int nv = valid_seeds(x);
       FilterState f;
       f.out = o;
       for (int c0 = 0; c0 < nv; c0 += 32) {
@@ -1874,10 +1671,10 @@ __global__ void __launch_bounds__(1024) k_seed_sort_filter_global(uint64_t* __re
         uint64_t k = 0;
         uint32_t qv = 0;
         if (j < nv) {
-          k = skey[o + j];
-          qv = sq[o + j];
+          k = SMEM ? s1[j] : skey[o + j];
+          qv = SMEM ? s2[j] : sq[o + j];
         }
-        filter_chunk(c0, nv, k, qv, wf, c.width, c.gap, f, skey, sq);
+        filter_chunk(c0, nv, k, qv, x < 0, c.width, c.gap, f, skey, sq);
       }
       if (threadIdx.x == 0) c.hcnt[s] = (int32_t)(f.out - o);
     }
@@ -1887,22 +1684,23 @@ __global__ void __launch_bounds__(1024) k_seed_sort_filter_global(uint64_t* __re
 
 __global__ void k_gather_hits(const uint64_t* __restrict__ skey, const uint32_t* __restrict__ sq,
                               const int64_t* __restrict__ off, const int32_t* __restrict__ hcnt,
-                              const int64_t* __restrict__ hoff, int64_t nstrands, uint64_t* __restrict__ hk,
-                              int32_t* __restrict__ hq, int32_t* __restrict__ hs, const int32_t* __restrict__ qlen,
-                              int l, int band, unsigned long long* __restrict__ cells) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = (s < nstrands) ? hcnt[s] : 0;
+                              const int64_t* __restrict__ hoff, int64_t nv, int nw, uint64_t* __restrict__ hk,
+                              int32_t* __restrict__ hq, uint32_t* __restrict__ hs, const int32_t* __restrict__ qlen,
+                              int l, int band, GroupCtl* __restrict__ ctl) {
+  const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = (v < nv) ? hcnt[v] : 0;
   // every hit of the strand fills band * (qlen - l) cells: backward rows + forward rows
-  unsigned long long c = n ? (unsigned long long)n * (unsigned long long)band * (unsigned long long)(qlen[s] - l) : 0;
+  unsigned long long c =
+      n ? (unsigned long long)n * (unsigned long long)band * (unsigned long long)(qlen[slot_strand((uint32_t)v, nw)] - l) : 0;
 #pragma unroll
   for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
-  if ((threadIdx.x & 31) == 0 && c) atomicAdd(cells, c);
-  if (s >= nstrands) return;
-  const int64_t a = off[s], b = hoff[s];
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(&ctl->cells, c);
+  if (v >= nv) return;
+  const int64_t a = off[v], b = hoff[v];
   for (int i = 0; i < n; ++i) {
     hk[b + i] = skey[a + i];
     hq[b + i] = (int32_t)sq[a + i];
-    hs[b + i] = (int32_t)s;
+    hs[b + i] = (uint32_t)v;
   }
 }
 
@@ -2348,11 +2146,12 @@ __device__ __forceinline__ void banded_hit_warp(const DpTab<int2>& tab, const ch
 }
 
 struct DpKernelArgs {
-  TargetView t;
+  TargetView t[kMaxSeedWins];
+  int nw;
   QueryView q;
   const uint64_t* hk;
   const int32_t* hq;
-  const int32_t* hs;
+  const uint32_t* hs;
   const uint64_t* order;
   int64_t n;
   DpParams p;
@@ -2367,8 +2166,8 @@ struct DpKernelArgs {
 // A hit whose target sequence or strand lies outside the window cannot come
 // from the seeding stages; it is flagged and given empty outputs instead of
 // being read past the window.
-__device__ __forceinline__ bool dp_hit_outside(const DpKernelArgs& a, int tid, int s) {
-  return (unsigned)tid >= (unsigned)a.t.nseqs || (unsigned)s >= (unsigned)a.q.nstrands;
+__device__ __forceinline__ bool dp_hit_outside(const DpKernelArgs& a, const TargetView& t, int tid, int64_t s) {
+  return (unsigned)tid >= (unsigned)t.nseqs || s >= (int64_t)a.q.nstrands;
 }
 
 __device__ __forceinline__ int64_t dp_warp_hits(const DpKernelArgs& a) {
@@ -2406,21 +2205,22 @@ __device__ __forceinline__ void dp_one(const DpKernelArgs& a, const DpTab<float2
   const int64_t h = a.order ? (int64_t)(uint32_t)a.order[i] : i;
   const uint64_t k = a.hk[h];
   const int qidx = a.hq[h];
-  const int s = a.hs[h];
+  const int64_t s = slot_strand(a.hs[h], a.nw);
+  const TargetView& t = a.t[slot_window(a.hs[h], a.nw)];
   const int tid = (int)(k >> 32);
-  if (dp_hit_outside(a, tid, s)) {
+  if (dp_hit_outside(a, t, tid, s)) {
     dp_skip(a, h);
     return;
   }
   const int tidx = (int)((uint32_t)k ^ 0x80000000u) + qidx;
-  const int64_t tstart = a.t.gateway[tid];
-  const int tlen = a.t.lengths[tid];
+  const int64_t tstart = t.gateway[tid];
+  const int tlen = t.lengths[tid];
   const int64_t qstart = a.q.start[s];
   const int qlen = a.q.len[s];
   const int l = a.p.l;
   int t_hl = l, q_hl = l, match = l, score = l;  // CDeviceHitList.cu:283-286
   int o_tidx = tidx, o_qidx = qidx;
-  banded_hit<GAP, LOCAL>(tab, a.t.bases, tstart, tlen, a.q.bases, qstart, qlen, tidx, qidx, l, t_hl, q_hl, match,
+  banded_hit<GAP, LOCAL>(tab, t.bases, tstart, tlen, a.q.bases, qstart, qlen, tidx, qidx, l, t_hl, q_hl, match,
                          score, o_tidx, o_qidx);
   dp_store(a, h, qlen, o_tidx, o_qidx, t_hl, q_hl, match, score);
 }
@@ -2484,21 +2284,22 @@ __global__ void __launch_bounds__(128) k_banded_dp_warp(DpKernelArgs a) {
     const int64_t h = a.order ? (int64_t)(uint32_t)a.order[i] : i;
     const uint64_t k = a.hk[h];
     const int qidx = a.hq[h];
-    const int s = a.hs[h];
+    const int64_t s = slot_strand(a.hs[h], a.nw);
+    const TargetView& t = a.t[slot_window(a.hs[h], a.nw)];
     const int tid = (int)(k >> 32);
-    if (dp_hit_outside(a, tid, s)) {  // the same for every lane of the warp
+    if (dp_hit_outside(a, t, tid, s)) {  // the same for every lane of the warp
       if (lane == 0) dp_skip(a, h);
       continue;
     }
     const int tidx = (int)((uint32_t)k ^ 0x80000000u) + qidx;
-    const int64_t tstart = a.t.gateway[tid];
-    const int tlen = a.t.lengths[tid];
+    const int64_t tstart = t.gateway[tid];
+    const int tlen = t.lengths[tid];
     const int64_t qstart = a.q.start[s];
     const int qlen = a.q.len[s];
     const int l = a.p.l;
     int t_hl = l, q_hl = l, match = l, score = l;  // CDeviceHitList.cu:283-286
     int o_tidx = tidx, o_qidx = qidx;
-    banded_hit_warp<GAP, LOCAL>(tab, a.t.bases, tstart, tlen, a.q.bases, qstart, qlen, tidx, qidx, l, t_hl, q_hl,
+    banded_hit_warp<GAP, LOCAL>(tab, t.bases, tstart, tlen, a.q.bases, qstart, qlen, tidx, qidx, l, t_hl, q_hl,
                                 match, score, o_tidx, o_qidx);
     if (lane == 0) dp_store(a, h, qlen, o_tidx, o_qidx, t_hl, q_hl, match, score);
   }
@@ -2515,7 +2316,8 @@ __device__ __forceinline__ int dp_bucket(int rows) {
   return kDpBuckets - 1 - (16 * (e - 3) + sub);
 }
 
-__global__ void k_dp_bucket_count(const int32_t* __restrict__ hs, const int32_t* __restrict__ q_len, int64_t n, int l,
+__global__ void k_dp_bucket_count(const uint32_t* __restrict__ hs, int nw, const int32_t* __restrict__ q_len, int64_t n,
+                                  int l,
                                   unsigned int* __restrict__ count, unsigned long long* __restrict__ rows) {
   __shared__ unsigned int c[kDpBuckets];
   __shared__ unsigned long long sr[kDpBuckets];
@@ -2525,7 +2327,7 @@ __global__ void k_dp_bucket_count(const int32_t* __restrict__ hs, const int32_t*
   }
   __syncthreads();
   for (int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; h < n; h += (int64_t)gridDim.x * blockDim.x) {
-    const int r = max(0, q_len[hs[h]] - l);
+    const int r = max(0, q_len[slot_strand(hs[h], nw)] - l);
     const int b = dp_bucket(r);
     atomicAdd(&c[b], 1u);
     atomicAdd(&sr[b], (unsigned long long)r);
@@ -2688,90 +2490,183 @@ long long launch_dp_gap(const DpKernelArgs& a, bool local, const DpLaunch& m, cu
 // ------------------------------------------------------------------------
 // final per-read order
 // ------------------------------------------------------------------------
-__global__ void k_final_keys(const uint64_t* __restrict__ hk, const int32_t* __restrict__ hq,
-                             const int32_t* __restrict__ hs, DpOut o, int64_t n, uint64_t* __restrict__ k1,
-                             uint64_t* __restrict__ k2, int32_t* __restrict__ idx) {
-  const int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (h >= n) return;
-  if (!o.keep[h]) {  // filtered hits sort after every kept one
-    k1[h] = ~0ull;
-    k2[h] = ~0ull;
-    idx[h] = (int32_t)h;
+// A read's hits lie together, window after window.  Their order, (score desc,
+// window, seed qIdx desc, strand, target sequence, seed tIdx), is the one the
+// stable sorts of alignmentHits (by rows desc, then qIdx desc) and
+// resultSorting (qID/2 asc, score desc) leave a window's hits of one read in,
+// merged over the windows as fixResult's stable sort does.  The hits were
+// gathered by (window, strand, sequence, diagonal, qIdx), so the position in
+// the read's run decides what (score, window, qIdx) leave open.  Filtered hits
+// sort after every kept one.
+struct FinalCtx {
+  const uint64_t* hk;
+  const int32_t* hq;
+  const uint32_t* hs;
+  DpOut o;
+  const int64_t* hoff;  // per slot
+  int64_t n_reads;
+  int nw;
+  int32_t* fcnt;
+  int32_t* fsel;
+};
+__device__ __forceinline__ void final_key(const FinalCtx& c, int64_t a, int i, uint64_t& k1, uint64_t& k2) {
+  const int64_t h = a + i;
+  if (!c.o.keep[h]) {
+    k1 = k2 = ~0ull;
     return;
   }
-  const uint64_t k = hk[h];
-  const int qidx = hq[h];
-  const int tid = (int)(k >> 32);
-  const int tidx = (int)((uint32_t)k ^ 0x80000000u) + qidx;
-  // (score desc, seed qIdx desc, strand, target sequence, seed tIdx): the order the
-  // stable sorts of alignmentHits (by rows desc, then qIdx desc) and
-  // resultSorting (qID/2 asc, score desc) leave hits of one read in.
-  const uint32_t a1 = (uint32_t)((int64_t)INT_MAX - (int64_t)o.score[h]);
-  const uint32_t a2 = (uint32_t)((int64_t)INT_MAX - (int64_t)qidx);
-  k1[h] = ((uint64_t)a1 << 32) | a2;
-  k2[h] = ((uint64_t)(hs[h] & 1) << 62) | ((uint64_t)(uint32_t)tid << 31) | (uint64_t)(uint32_t)tidx;
-  idx[h] = (int32_t)h;
+  const uint32_t score = (uint32_t)((int64_t)INT_MAX - (int64_t)c.o.score[h]);
+  k1 = ((uint64_t)score << 32) | (uint32_t)slot_window(c.hs[h], c.nw);
+  k2 = ((uint64_t)(uint32_t)((int64_t)INT_MAX - (int64_t)c.hq[h]) << 32) | (uint32_t)i;
 }
-
-__global__ void k_read_ranges(const int64_t* __restrict__ hoff, int64_t n_reads, int64_t* __restrict__ roff,
-                              int32_t* __restrict__ rlen) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n_reads) return;
-  roff[r] = hoff[2 * r];
-  rlen[r] = (int32_t)(hoff[2 * r + 2] - hoff[2 * r]);
-}
-
-// Duplicate removal within one read (deleteHits_duplicateResult: a hit equal
-// in (tID, tIdx, qID, qIdx) to its predecessor in result order is dropped).
-__global__ void k_final_dedupe(const uint64_t* __restrict__ k1, const int32_t* __restrict__ idx,
-                               const uint64_t* __restrict__ hk, const int32_t* __restrict__ hs, DpOut o,
-                               const int64_t* __restrict__ roff, const int32_t* __restrict__ rlen,
-                               int64_t n_reads, int32_t* __restrict__ fcnt, int32_t* __restrict__ fsel) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n_reads) return;
-  const int64_t a = roff[r];
-  const int n = rlen[r];
-  int cnt = 0;
-  int ptid = 0, ptidx = 0, ps = 0, pqidx = 0;
-  for (int j = 0; j < n; ++j) {
-    if (k1[a + j] == ~0ull) break;  // the filtered hits
-    const int h = idx[a + j];
-    const int tid = (int)(hk[h] >> 32);
-    const int tidx = o.t_idx[h], qidx = o.q_idx[h], s = hs[h];
-    const bool dup = j > 0 && tid == ptid && tidx == ptidx && s == ps && qidx == pqidx;
-    if (!dup) fsel[a + cnt++] = h;
-    ptid = tid; ptidx = tidx; ps = s; pqidx = qidx;
+// What deleteHits_duplicateResult compares of a hit (tID, tIdx, qID, qIdx).
+struct FinalId {
+  int tid, tidx, qidx;
+  uint32_t slot;
+  __device__ __forceinline__ bool operator==(const FinalId& x) const {
+    return tid == x.tid && tidx == x.tidx && qidx == x.qidx && slot == x.slot;
   }
-  fcnt[r] = cnt;
+};
+__device__ __forceinline__ FinalId final_id(const FinalCtx& c, int64_t h) {
+  return FinalId{(int)(c.hk[h] >> 32), c.o.t_idx[h], c.o.q_idx[h], c.hs[h]};
 }
 
-__global__ void k_final_compact(const int32_t* __restrict__ fsel, const int64_t* __restrict__ roff,
-                                const int32_t* __restrict__ fcnt, const int64_t* __restrict__ foff,
-                                int64_t n_reads, const uint64_t* __restrict__ hk, const int32_t* __restrict__ hs,
-                                DpOut o, int32_t t_first, int32_t q_first, FinalOut out) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n_reads) return;
-  const int64_t a = roff[r], b = foff[r];
-  const int n = fcnt[r];
-  for (int j = 0; j < n; ++j) {
-    const int h = fsel[a + j];
-    const int64_t w = b + j;
-    out.t_id[w] = t_first + (int32_t)(hk[h] >> 32);
-    out.t_idx[w] = o.t_idx[h];
-    out.q_id[w] = q_first + hs[h];
-    out.q_idx[w] = o.q_idx[h];
-    out.t_len[w] = o.t_len[h];
-    out.q_len[w] = o.q_len[h];
-    out.match[w] = o.match[h];
-    out.score[w] = o.score[h];
-    out.evalue[w] = o.evalue[h];
+// Sorts the reads of the warp's groups of N lanes (n hits from a, one per
+// lane), drops every hit equal to its predecessor of the same window
+// (deleteHits_duplicateResult) and writes the kept ones.  Every lane of the
+// warp takes part; n = 0 for a group without a read.
+template <int N>
+__device__ __forceinline__ void final_lanes(const FinalCtx& c, int64_t r, int64_t a, int n) {
+  const int lane = threadIdx.x & 31, j = lane & (N - 1);
+  const unsigned group = N == 32 ? kFull : ((1u << (N & 31)) - 1) << (lane & ~(N - 1));
+  uint64_t k1 = ~0ull, k2 = ~0ull;
+  if (j < n) final_key(c, a, j, k1, k2);
+  if (__any_sync(kFull, n > 1)) lanes_sort<N>(k1, k2, lane);
+  const bool kept = k1 != ~0ull;
+  const int w = kept ? (int)(uint32_t)k1 : -1;
+  const int64_t h = a + (uint32_t)k2;
+  FinalId id{0, 0, 0, 0};
+  if (kept) id = final_id(c, h);
+  unsigned same = 0;  // the kept hits of this lane's window
+  for (int x = 0; x < c.nw; ++x) {
+    const unsigned m = __ballot_sync(kFull, w == x);
+    if (w == x) same = m;
+  }
+  const unsigned before = same & group & lanemask_lt();
+  const int src = before ? 31 - __clz(before) : lane;
+  FinalId pr;
+  pr.tid = __shfl_sync(kFull, id.tid, src);
+  pr.tidx = __shfl_sync(kFull, id.tidx, src);
+  pr.qidx = __shfl_sync(kFull, id.qidx, src);
+  pr.slot = __shfl_sync(kFull, id.slot, src);
+  const bool out = kept && !(before && id == pr);
+  const unsigned m = __ballot_sync(kFull, out) & group;
+  if (out) c.fsel[a + __popc(m & lanemask_lt())] = (int32_t)(uint32_t)k2;
+  if (j == 0 && r >= 0) c.fcnt[r] = __popc(m);
+}
+
+// Reads of up to 8 hits take 8 lanes (most have one or two), up to 32 the
+// whole warp; longer ones are listed for k_final_long.
+__global__ void k_final_small(FinalCtx c, uint32_t* __restrict__ list, GroupCtl* __restrict__ ctl) {
+  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const int lane = threadIdx.x & 31;
+  int64_t a = 0;
+  int n = 0;
+  const bool in = r < c.n_reads;
+  if (in) {
+    a = c.hoff[2 * (int64_t)c.nw * r];
+    n = (int)(c.hoff[2 * (int64_t)c.nw * (r + 1)] - a);
+  }
+  final_lanes<8>(c, in && n <= 8 ? r : -1, a, n <= 8 ? n : 0);
+  for (unsigned m = __ballot_sync(kFull, n > 8 && n <= 32 && (lane & 7) == 0); m; m &= m - 1) {
+    const int src = __ffs(m) - 1;
+    final_lanes<32>(c, __shfl_sync(kFull, r, src), __shfl_sync(kFull, a, src), __shfl_sync(kFull, n, src));
+  }
+  if (n > 32 && (lane & 7) == 0) list[atomicAdd(&ctl->n_long, 1)] = (uint32_t)r;
+}
+
+// More than 32 hits: one CTA per read, in shared memory up to kCtaSortCap,
+// else in global memory (g1, g2: one word per hit).
+constexpr int kFinalLongThreads = 256;
+__global__ void __launch_bounds__(kFinalLongThreads) k_final_long(FinalCtx c, uint64_t* __restrict__ g1,
+                                                                  uint64_t* __restrict__ g2,
+                                                                  const uint32_t* __restrict__ list,
+                                                                  const GroupCtl* __restrict__ ctl) {
+  __shared__ uint64_t s1[kCtaSortCap], s2[kCtaSortCap];
+  __shared__ int warp_n[kFinalLongThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int total = ctl->n_long;
+  for (int li = blockIdx.x; li < total; li += gridDim.x) {
+    const int64_t r = list[li];
+    const int64_t a = c.hoff[2 * (int64_t)c.nw * r];
+    const int n = (int)(c.hoff[2 * (int64_t)c.nw * (r + 1)] - a);
+    uint64_t* k1 = n <= kCtaSortCap ? s1 : g1 + a;
+    uint64_t* k2 = n <= kCtaSortCap ? s2 : g2 + a;
+    for (int i = threadIdx.x; i < n; i += kFinalLongThreads) final_key(c, a, i, k1[i], k2[i]);
+    __syncthreads();
+    cta_network(k1, k2, n);
+    __syncthreads();
+    int done = 0;
+    for (int c0 = 0; c0 < n; c0 += kFinalLongThreads) {
+      const int j = c0 + (int)threadIdx.x;
+      bool out = j < n && k1[j] != ~0ull;
+      if (out) {
+        const uint32_t w = (uint32_t)k1[j];
+        int p = j - 1;  // the predecessor of the same window
+        while (p >= 0 && (uint32_t)k1[p] != w) --p;
+        if (p >= 0) out = !(final_id(c, a + (uint32_t)k2[j]) == final_id(c, a + (uint32_t)k2[p]));
+      }
+      const unsigned m = __ballot_sync(kFull, out);
+      if (lane == 0) warp_n[warp] = __popc(m);
+      __syncthreads();
+      int at = done + __popc(m & lanemask_lt()), all = 0;
+      for (int x = 0; x < kFinalLongThreads / 32; ++x) {
+        if (x < warp) at += warp_n[x];
+        all += warp_n[x];
+      }
+      if (out) c.fsel[a + at] = (int32_t)(uint32_t)k2[j];
+      done += all;
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) c.fcnt[r] = done;
+    __syncthreads();
+  }
+}
+
+// The kept hits of every read, in order, 8 lanes per read.
+__global__ void k_final_write(FinalCtx c, const int64_t* __restrict__ foff, OutView out) {
+  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  if (r >= c.n_reads) return;
+  const int64_t a = c.hoff[2 * (int64_t)c.nw * r], b = foff[r];
+  const int n = c.fcnt[r];
+  for (int j = threadIdx.x & 7; j < n; j += 8) {
+    const int64_t h = a + c.fsel[a + j];
+    const int64_t x = b + j;
+    const uint32_t slot = c.hs[h];
+    const int w = slot_window(slot, c.nw);
+    const int strand = (int)(slot & 1u);
+    if (out.q_id) {
+      out.q_id[x] = out.q_first + (int32_t)(2 * r) + strand;
+    } else {
+      out.read[x] = (int32_t)r;
+      out.strand[x] = strand;
+      out.t_load[x] = out.load[w];
+    }
+    out.t_seq[x] = out.t_first[w] + (int32_t)(c.hk[h] >> 32);
+    out.t_idx[x] = c.o.t_idx[h];
+    out.q_idx[x] = c.o.q_idx[h];
+    out.t_len[x] = c.o.t_len[h];
+    out.q_len[x] = c.o.q_len[h];
+    out.match[x] = c.o.match[h];
+    out.score[x] = c.o.score[h];
+    out.evalue[x] = c.o.evalue[h];
   }
 }
 
 // ------------------------------------------------------------------------
-// merge of the per-window results in holder order (CHostResultHolder::fixResult)
+// merge of the groups' results in holder order (CHostResultHolder::fixResult)
 // ------------------------------------------------------------------------
-__global__ void k_merge_count(const WinHits* __restrict__ w, int nw, int64_t nreads, int32_t* __restrict__ cnt) {
+__global__ void k_merge_count(const GroupHits* __restrict__ w, int nw, int64_t nreads, int32_t* __restrict__ cnt) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= nreads) return;
   int64_t c = 0;
@@ -2779,45 +2674,44 @@ __global__ void k_merge_count(const WinHits* __restrict__ w, int nw, int64_t nre
   cnt[r] = (int32_t)c;
 }
 
-// Item j of window wi goes after every item of the same read from an earlier
-// window with score >= its score, and every item of a later window with a
+// Item j of group wi goes after every item of the same read from an earlier
+// group with score >= its score, and every item of a later group with a
 // strictly higher score: the stable sort by (read, score desc) of the
 // concatenation in window order.
-__global__ void k_merge_place(const WinHits* __restrict__ w, int nw, int64_t total, const int64_t* __restrict__ moff,
-                              MapOut out) {
+__global__ void k_merge_place(const GroupHits* __restrict__ w, int nw, int64_t total, const int64_t* __restrict__ moff,
+                              OutView out) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   int wi = 0;
   while (wi + 1 < nw && w[wi + 1].base <= i) ++wi;
-  const WinHits& a = w[wi];
+  const GroupHits& a = w[wi];
   const int64_t j = i - a.base;
-  const int qid = a.q_id[j];
-  const int64_t r = qid >> 1;
-  const int sc = a.score[j];
+  const int64_t r = a.f[0][j];
+  const int sc = a.f[9][j];
   int64_t pos = moff[r] + (j - a.foff[r]);
   for (int k = 0; k < nw; ++k) {
     if (k == wi) continue;
-    const WinHits& b = w[k];
+    const GroupHits& b = w[k];
     int64_t lo = b.foff[r], hi = b.foff[r + 1];
     const int64_t first = lo;
     // scores are non-increasing within a read: count the prefix that precedes sc
     while (lo < hi) {
       const int64_t mid = (lo + hi) >> 1;
-      const int v = b.score[mid];
+      const int v = b.f[9][mid];
       if (k < wi ? v >= sc : v > sc) lo = mid + 1;
       else hi = mid;
     }
     pos += lo - first;
   }
-  out.read[pos] = qid >> 1;
-  out.strand[pos] = qid & 1;
-  out.t_load[pos] = a.load;
-  out.t_seq[pos] = a.t_id[j];
-  out.t_idx[pos] = a.t_idx[j];
-  out.q_idx[pos] = a.q_idx[j];
-  out.t_len[pos] = a.t_len[j];
-  out.q_len[pos] = a.q_len[j];
-  out.match[pos] = a.match[j];
+  out.read[pos] = (int32_t)r;
+  out.strand[pos] = a.f[1][j];
+  out.t_load[pos] = a.f[2][j];
+  out.t_seq[pos] = a.f[3][j];
+  out.t_idx[pos] = a.f[4][j];
+  out.q_idx[pos] = a.f[5][j];
+  out.t_len[pos] = a.f[6][j];
+  out.q_len[pos] = a.f[7][j];
+  out.match[pos] = a.f[8][j];
   out.score[pos] = sc;
   out.evalue[pos] = a.evalue[j];
 }
@@ -2858,6 +2752,13 @@ __global__ void k_gather_i64(const int64_t* __restrict__ src, const int64_t* __r
 void scan_i32(Workspace& ws, const int32_t* in, int64_t n, int64_t* out, cudaStream_t st) {
   scan_1pass(ws, ArrayLoad<int32_t>{in}, n, out, st);
 }
+int64_t scan_state_words(int64_t n) { return (n + kScanTile) / kScanTile + 1; }
+void scan_i32_to(const int32_t* in, int64_t n, int64_t* out, unsigned long long* state, long long* total,
+                 cudaStream_t st) {
+  const int64_t tiles = scan_state_words(n) - 1;
+  k_scan_1pass<<<(unsigned)tiles, kScanThreads, 0, st>>>(ArrayLoad<int32_t>{in}, n, n + 1, out, state, total);
+  CLAST_LAUNCHED();
+}
 void scan_positive(Workspace& ws, const int32_t* in, int64_t n, int64_t* out, cudaStream_t st) {
   scan_1pass(ws, PositiveLoad{in}, n, out, st);
 }
@@ -2868,15 +2769,18 @@ void pack_bases(const char* bases, int64_t n, uint64_t* packed, uint64_t* nmask,
   CLAST_LAUNCHED();
 }
 
-void build_strands(const char* reads, const int64_t* offsets, int64_t n_reads, int64_t n_bases, char* strands,
-                   int64_t* strand_start, int32_t* strand_len, cudaStream_t st) {
+void build_strands(const char* reads, const int64_t* offsets, int64_t n_reads, char* strands, int64_t* strand_start,
+                   int32_t* strand_len, cudaStream_t st) {
   if (n_reads <= 0) return;
-  k_strand_meta<<<blocks_for(n_reads, 256), 256, 0, st>>>(offsets, n_reads, strand_start, strand_len);
+  k_strands<<<blocks_for(n_reads * 32, 256), 256, 0, st>>>(reads, offsets, n_reads, strands, strand_start, strand_len);
   CLAST_LAUNCHED();
-  if (n_bases > 0) {
-    k_strands<<<blocks_for(n_reads * 32, 256), 256, 0, st>>>(reads, offsets, n_reads, strands);
-    CLAST_LAUNCHED();
-  }
+}
+
+void read_lengths(const int64_t* offsets, int64_t n_reads, int* min_len, int* max_len, cudaStream_t st) {
+  if (n_reads <= 0) return;
+  k_read_lengths<<<(unsigned)std::min<int64_t>(148, blocks_for(n_reads, 256)), 256, 0, st>>>(offsets, n_reads, min_len,
+                                                                                           max_len);
+  CLAST_LAUNCHED();
 }
 
 void build_window(const char* src, const int64_t* src_off, const int32_t* gateway, const int32_t* lengths,
@@ -2968,8 +2872,6 @@ void index_buckets(const int64_t* ufirst, const int64_t* kpos, int64_t n, const 
 }
 
 
-int seed_parts() { return kSeedParts; }
-
 void seed_fused(const QueryView& q, const IndexView& ix, const TargetView& t, int gap, int local,
                 unsigned long long* cursors, unsigned long long* n_kmers, int64_t* off, int32_t* cnt, int32_t* nvalid,
                 uint64_t* skey, uint32_t* sq, int64_t part_cap, cudaStream_t st) {
@@ -3034,78 +2936,59 @@ void table_place(const uint64_t* ucode, const int32_t* ustart, const int32_t* uc
   CLAST_LAUNCHED();
 }
 
-void window_first(const int32_t* nvalid, const int32_t* win_start, int n_windows, int32_t* win_first,
-                  cudaStream_t st) {
-  if (n_windows <= 0) return;
-  k_window_first<<<blocks_for((int64_t)n_windows * 32, 256), 256, 0, st>>>(nvalid, win_start, n_windows,
-                                                                            win_first);
+void seed_filter(uint64_t* skey, uint32_t* sq, const int64_t* off, const int32_t* cnt, int32_t* nvalid,
+                 const int32_t* win_start, int n_windows, int nw, int width, int gap, int64_t nv, uint32_t* lists,
+                 int32_t* hcnt, GroupCtl* ctl, cudaStream_t st) {
+  if (nv <= 0) return;
+  if (n_windows > 0) {
+    k_window_first<<<blocks_for((int64_t)n_windows * nw * 32, 256), 256, 0, st>>>(nvalid, win_start, n_windows, nw);
+    CLAST_LAUNCHED();
+  }
+  SeedFilterCtx c{off, cnt, nvalid, width, gap, hcnt};
+  k_seed_filter_small<<<blocks_for(nv, 256), 256, 0, st>>>(skey, sq, c, nv, lists, ctl);
   CLAST_LAUNCHED();
-}
-void segmented_sort_u64(Workspace& ws, uint64_t* k1, uint64_t* k2, int32_t* payload, const int64_t* off,
-                        const int32_t* len, int64_t n_segments, cudaStream_t st, int tag) {
-  seg_sort<uint64_t, true>(ws, k1, k2, payload, off, len, n_segments, st, tag);
-}
-void seed_sort_filter(Workspace& ws, uint64_t* skey, uint32_t* sq, const int64_t* off, const int32_t* cnt,
-                      const int32_t* nvalid, const int32_t* win_start, int n_windows, const int32_t* win_first,
-                      int width, int gap, int64_t nstrands, int32_t* hcnt, cudaStream_t st) {
-  if (nstrands <= 0) return;
-  SeedFilterCtx c{off, cnt, nvalid, win_start, n_windows, win_first, width, gap, hcnt};
-  if (nstrands >= (int64_t)kWinFirstBit) throw std::invalid_argument("more than 2^31 strands in one batch");
-  int32_t* lists = ws.get<int32_t>("ssf_lists", kSortTiers * nstrands);
-  int32_t* counts = ws.get<int32_t>("ssf_counts", kSortTiers);
-  CLAST_CK(cudaMemsetAsync(counts, 0, kSortTiers * sizeof(int32_t), st));
-  CLAST_CK(cudaMemsetAsync(hcnt, 0, nstrands * sizeof(int32_t), st));
-  k_seed_classify<<<blocks_for(nstrands, 256), 256, 0, st>>>(c, nstrands, lists, counts);
+  k_seed_filter_mid<<<grid_cap(std::min<int64_t>((nv + 3) / 4, 148 * 64)), kWarpSmemThreads, 0, st>>>(
+      skey, sq, c, lists, &ctl->n_seeds[0]);
   CLAST_LAUNCHED();
-  k_seed_sort_filter_thread<<<grid_cap((nstrands + 255) / 256), 256, 0, st>>>(skey, sq, c, lists, counts);
+  k_seed_filter_big<true><<<grid_cap(nv < 4096 ? nv : 4096), 256, 0, st>>>(skey, sq, c, lists + nv, &ctl->n_seeds[1]);
   CLAST_LAUNCHED();
-  k_seed_sort_filter_warp<<<grid_cap((nstrands * 32 + 255) / 256), 256, 0, st>>>(skey, sq, c, lists + nstrands,
-                                                                                counts + 1);
-  CLAST_LAUNCHED();
-  k_seed_sort_filter_warp_smem<<<grid_cap(std::min<int64_t>(nstrands, 65536) * 32 / kWarpSmemThreads + 1),
-                                 kWarpSmemThreads, 0, st>>>(skey, sq, c, lists + 2 * nstrands, counts + 2);
-  CLAST_LAUNCHED();
-  k_seed_sort_filter_cta<<<grid_cap(nstrands < 4096 ? nstrands : 4096), 256, 0, st>>>(skey, sq, c,
-                                                                                     lists + 3 * nstrands, counts + 3);
-  CLAST_LAUNCHED();
-  k_seed_sort_filter_global<<<grid_cap(nstrands < 1024 ? nstrands : 1024), 1024, 0, st>>>(
-      skey, sq, c, lists + 4 * nstrands, counts + 4);
+  k_seed_filter_big<false><<<grid_cap(nv < 296 ? nv : 296), 1024, 0, st>>>(skey, sq, c, lists + 2 * nv,
+                                                                           &ctl->n_seeds[2]);
   CLAST_LAUNCHED();
 }
 
 void gather_hits(const uint64_t* skey, const uint32_t* sq, const int64_t* off, const int32_t* hcnt,
-                 const int64_t* hoff, int64_t nstrands, uint64_t* hk, int32_t* hq, int32_t* hs,
-                 const int32_t* qlen, int l, int band, unsigned long long* cells, cudaStream_t st) {
-  if (nstrands <= 0) return;
-  k_gather_hits<<<blocks_for(nstrands, 256), 256, 0, st>>>(skey, sq, off, hcnt, hoff, nstrands, hk, hq, hs, qlen, l,
-                                                           band, cells);
+                 const int64_t* hoff, int64_t nv, int nw, uint64_t* hk, int32_t* hq, uint32_t* hs,
+                 const int32_t* qlen, int l, int band, GroupCtl* ctl, cudaStream_t st) {
+  if (nv <= 0) return;
+  k_gather_hits<<<blocks_for(nv, 256), 256, 0, st>>>(skey, sq, off, hcnt, hoff, nv, nw, hk, hq, hs, qlen, l, band, ctl);
   CLAST_LAUNCHED();
 }
 
-__global__ void k_dp_order_keys(const int32_t* __restrict__ hs, const int32_t* __restrict__ q_len, int64_t n,
+__global__ void k_dp_order_keys(const uint32_t* __restrict__ hs, int nw, const int32_t* __restrict__ q_len, int64_t n,
                                 int l, int rows_max, uint64_t* __restrict__ keys) {
   const int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= n) return;
-  const int rows = max(0, min(rows_max, q_len[hs[h]] - l + 1));
+  const int rows = max(0, min(rows_max, q_len[slot_strand(hs[h], nw)] - l + 1));
   keys[h] = ((uint64_t)(rows_max - rows) << 32) | (uint32_t)h;
 }
 
-void dp_order_keys(const int32_t* hs, const int32_t* q_len, int64_t n_hits, int l, int rows_max, uint64_t* keys,
-                   cudaStream_t st) {
+void dp_order_keys(const uint32_t* hs, int nw, const int32_t* q_len, int64_t n_hits, int l, int rows_max,
+                   uint64_t* keys, cudaStream_t st) {
   if (n_hits <= 0) return;
-  k_dp_order_keys<<<blocks_for(n_hits, 256), 256, 0, st>>>(hs, q_len, n_hits, l, rows_max, keys);
+  k_dp_order_keys<<<blocks_for(n_hits, 256), 256, 0, st>>>(hs, nw, q_len, n_hits, l, rows_max, keys);
   CLAST_LAUNCHED();
 }
 
-DpBuckets dp_bucket_count(Workspace& ws, const int32_t* hs, const int32_t* q_len, int64_t n_hits, int l,
+DpBuckets dp_bucket_count(Workspace& ws, const uint32_t* hs, int nw, const int32_t* q_len, int64_t n_hits, int l,
                           cudaStream_t st) {
   unsigned int* count = ws.get<unsigned int>("dpb_count", kDpBuckets);
   unsigned long long* rows = ws.get<unsigned long long>("dpb_rows", kDpBuckets);
   CLAST_CK(cudaMemsetAsync(count, 0, kDpBuckets * sizeof(unsigned int), st));
   CLAST_CK(cudaMemsetAsync(rows, 0, kDpBuckets * sizeof(unsigned long long), st));
   if (n_hits > 0) {
-    k_dp_bucket_count<<<grid_cap(std::min<int64_t>(blocks_for(n_hits, 256), 1184)), 256, 0, st>>>(hs, q_len, n_hits,
-                                                                                                    l, count, rows);
+    k_dp_bucket_count<<<grid_cap(std::min<int64_t>(blocks_for(n_hits, 256), 1184)), 256, 0, st>>>(hs, nw, q_len,
+                                                                                                    n_hits, l, count, rows);
     CLAST_LAUNCHED();
   }
   DpBuckets b;
@@ -3122,11 +3005,22 @@ int dp_warp_mode_from_env(int fallback) {
   return fallback;
 }
 
-long long banded_dp(const TargetView& t, const QueryView& q, const uint64_t* hk, const int32_t* hq,
-                    const int32_t* hs, const uint64_t* order, int64_t n_hits, const DpParams& p, const DpOut& o,
+long long banded_dp(const TargetView* t, int nw, const QueryView& q, const uint64_t* hk, const int32_t* hq,
+                    const uint32_t* hs, const uint64_t* order, int64_t n_hits, const DpParams& p, const DpOut& o,
                     cudaStream_t st, const DpLaunch& m) {
   if (n_hits <= 0) return 0;
-  DpKernelArgs a{t, q, hk, hq, hs, order, n_hits, p, o, nullptr, 0, m.bad};
+  DpKernelArgs a{};
+  for (int w = 0; w < nw; ++w) a.t[w] = t[w];
+  a.nw = nw;
+  a.q = q;
+  a.hk = hk;
+  a.hq = hq;
+  a.hs = hs;
+  a.order = order;
+  a.n = n_hits;
+  a.p = p;
+  a.o = o;
+  a.bad = m.bad;
   const bool local = p.local != 0;
   switch (p.gap) {
     case 2: return launch_dp_gap<2>(a, local, m, st);
@@ -3148,14 +3042,14 @@ long long banded_dp(const TargetView& t, const QueryView& q, const uint64_t* hk,
   }
 }
 
-void merge_windows(const WinHits* wins, int nw, int64_t total, int64_t nreads, int32_t* cnt, int64_t* moff,
-                   const MapOut& out, Workspace& ws, cudaStream_t st) {
+void merge_groups(const GroupHits* groups, int n, int64_t total, int64_t nreads, int32_t* cnt, int64_t* moff,
+                  const OutView& out, Workspace& ws, cudaStream_t st) {
   if (nreads <= 0) return;
-  k_merge_count<<<blocks_for(nreads, 256), 256, 0, st>>>(wins, nw, nreads, cnt);
+  k_merge_count<<<blocks_for(nreads, 256), 256, 0, st>>>(groups, n, nreads, cnt);
   CLAST_LAUNCHED();
   scan_i32(ws, cnt, nreads, moff, st);
   if (total > 0) {
-    k_merge_place<<<blocks_for(total, 256), 256, 0, st>>>(wins, nw, total, moff, out);
+    k_merge_place<<<blocks_for(total, 256), 256, 0, st>>>(groups, n, total, moff, out);
     CLAST_LAUNCHED();
   }
 }
@@ -3189,30 +3083,21 @@ void gather_i64(const int64_t* src, const int64_t* idx, int n, int64_t* out, cud
   CLAST_LAUNCHED();
 }
 
-void final_keys(const uint64_t* hk, const int32_t* hq, const int32_t* hs, const DpOut& o, int64_t n_hits,
-                uint64_t* k1, uint64_t* k2, int32_t* idx, cudaStream_t st) {
-  if (n_hits <= 0) return;
-  k_final_keys<<<blocks_for(n_hits, 256), 256, 0, st>>>(hk, hq, hs, o, n_hits, k1, k2, idx);
+void final_order(const uint64_t* hk, const int32_t* hq, const uint32_t* hs, const DpOut& o, const int64_t* hoff,
+                 int64_t n_reads, int nw, uint64_t* g1, uint64_t* g2, uint32_t* list, int32_t* fcnt, int32_t* fsel,
+                 GroupCtl* ctl, cudaStream_t st) {
+  if (n_reads <= 0) return;
+  const FinalCtx c{hk, hq, hs, o, hoff, n_reads, nw, fcnt, fsel};
+  k_final_small<<<blocks_for(n_reads * 8, 256), 256, 0, st>>>(c, list, ctl);
+  CLAST_LAUNCHED();
+  k_final_long<<<grid_cap(n_reads < 2048 ? n_reads : 2048), kFinalLongThreads, 0, st>>>(c, g1, g2, list, ctl);
   CLAST_LAUNCHED();
 }
-void read_ranges(const int64_t* hoff, int64_t n_reads, int64_t* roff, int32_t* rlen, cudaStream_t st) {
+void final_write(const uint64_t* hk, const uint32_t* hs, const DpOut& o, const int64_t* hoff, int64_t n_reads, int nw,
+                 const int32_t* fcnt, const int32_t* fsel, const int64_t* foff, const OutView& out, cudaStream_t st) {
   if (n_reads <= 0) return;
-  k_read_ranges<<<blocks_for(n_reads, 256), 256, 0, st>>>(hoff, n_reads, roff, rlen);
-  CLAST_LAUNCHED();
-}
-void final_dedupe(const uint64_t* k1, const uint64_t* /*k2*/, const int32_t* idx, const uint64_t* hk,
-                  const int32_t* hs, const DpOut& o, const int64_t* roff, const int32_t* rlen, int64_t n_reads,
-                  int32_t* fcnt, int32_t* fsel, cudaStream_t st) {
-  if (n_reads <= 0) return;
-  k_final_dedupe<<<blocks_for(n_reads, 128), 128, 0, st>>>(k1, idx, hk, hs, o, roff, rlen, n_reads, fcnt, fsel);
-  CLAST_LAUNCHED();
-}
-void final_compact(const int32_t* fsel, const int64_t* roff, const int32_t* fcnt, const int64_t* foff,
-                   int64_t n_reads, const uint64_t* hk, const int32_t* hs, const DpOut& o, int32_t t_first,
-                   int32_t q_first, const FinalOut& out, cudaStream_t st) {
-  if (n_reads <= 0) return;
-  k_final_compact<<<blocks_for(n_reads, 128), 128, 0, st>>>(fsel, roff, fcnt, foff, n_reads, hk, hs, o, t_first,
-                                                             q_first, out);
+  const FinalCtx c{hk, nullptr, hs, o, hoff, n_reads, nw, const_cast<int32_t*>(fcnt), const_cast<int32_t*>(fsel)};
+  k_final_write<<<blocks_for(n_reads * 8, 256), 256, 0, st>>>(c, foff, out);
   CLAST_LAUNCHED();
 }
 

@@ -13,6 +13,11 @@ struct Workspace;  // device scratch pool (clast_engine.cu)
 
 // out[0..n] = exclusive prefix sums of in[0..n) (out[n] = total).
 void scan_i32(Workspace& ws, const int32_t* in, int64_t n, int64_t* out, cudaStream_t st);
+// The same with the caller's zeroed state of scan_state_words(n) words, the total
+// also in *total (device, may be null).
+int64_t scan_state_words(int64_t n);
+void scan_i32_to(const int32_t* in, int64_t n, int64_t* out, unsigned long long* state, long long* total,
+                 cudaStream_t st);
 // exclusive scan of (in[i] > 0)
 void scan_positive(Workspace& ws, const int32_t* in, int64_t n, int64_t* out, cudaStream_t st);
 
@@ -21,9 +26,14 @@ void scan_positive(Workspace& ws, const int32_t* in, int64_t n, int64_t* out, cu
 void pack_bases(const char* bases, int64_t n, uint64_t* packed, uint64_t* nmask, cudaStream_t st);
 
 // Query strands of n_reads one-strand reads: strand 2r = read r, strand 2r+1 its
-// reverse complement (utilReverseSeq.cpp:3-19), laid out back to back.
-void build_strands(const char* reads, const int64_t* offsets, int64_t n_reads, int64_t n_bases,
-                   char* strands, int64_t* strand_start, int32_t* strand_len, cudaStream_t st);
+// reverse complement (utilReverseSeq.cpp:3-19), laid out back to back, with kPad
+// 'N' bytes before and after them.
+void build_strands(const char* reads, const int64_t* offsets, int64_t n_reads, char* strands, int64_t* strand_start,
+                   int32_t* strand_len, cudaStream_t st);
+
+// Shortest and longest of the reads (*min_len preset to INT_MAX, *max_len to 0);
+// no read may be longer than INT_MAX.
+void read_lengths(const int64_t* offsets, int64_t n_reads, int* min_len, int* max_len, cudaStream_t st);
 
 // ---- index of one target window (CDeviceHashTable.cu:20-174) ----
 // Window base array (sequences with their joints) from a one-strand source set:
@@ -72,27 +82,54 @@ void table_place(const uint64_t* ucode, const int32_t* ustart, const int32_t* uc
                  uint32_t* filter, int fshift, unsigned long long* failed, cudaStream_t st);
 
 // ---- seeds (CDeviceHitList_createRawSeedList.cu, _deleteSeeds*.cu, _sortSeeds.cu) ----
-// One-pass seeding (lookups once): off/cnt/nvalid per strand, seeds in skey/sq,
-// which hold seed_parts() partitions of part_cap seeds.  Strand s reserves its
-// range in partition s % seed_parts() through cursors[partition]; a partition
-// whose cursor ends above part_cap was not fully written and the call must be
-// repeated with part_cap >= the largest cursor.  n_kmers holds seed_parts()
-// counters (valid l-mers of the strands of each partition; the caller sums
+// A group of up to kMaxSeedWins target windows is searched together.  Its slots
+// are the (strand, window) pairs, a read's slots side by side: slot (s, w) of
+// nw windows is (s / 2) * 2 nw + 2 w + (s & 1).
+constexpr int kMaxSeedWins = 4;
+constexpr int kSeedParts = 32;
+__host__ __device__ __forceinline__ int64_t strand_slot(int64_t s, int w, int nw) {
+  return (s >> 1) * (2 * nw) + 2 * w + (s & 1);
+}
+__host__ __device__ __forceinline__ int64_t slot_strand(uint32_t v, int nw) {
+  return nw == 1 ? (int64_t)v : 2 * (int64_t)(v / (uint32_t)(2 * nw)) + (v & 1u);
+}
+__host__ __device__ __forceinline__ int slot_window(uint32_t v, int nw) {
+  return nw == 1 ? 0 : (int)((v >> 1) % (uint32_t)nw);
+}
+
+// Counters of one group's search, zeroed before it.
+struct GroupCtl {
+  unsigned long long cursor[kMaxSeedWins][kSeedParts];  // seeds per window and partition
+  unsigned long long kmers[kMaxSeedWins][kSeedParts];   // valid l-mers of the partition's strands
+  unsigned long long cells;                             // DP cells
+  long long hits, results;
+  long long dp_warp;  // hits the DP's split sends to the one-per-warp kernel
+  int bad;            // see DpLaunch::bad
+  int n_seeds[3];     // slots listed for the seed filters' longer tiers
+  int n_long;         // reads listed for k_final_long
+};
+
+// One-pass seeding of one window (lookups once): off/cnt/nvalid per strand,
+// seeds in skey/sq, which hold kSeedParts partitions of part_cap seeds.  Strand
+// s reserves its range in partition s % kSeedParts through cursors[partition];
+// a partition whose cursor ends above part_cap was not fully written (its
+// strands have no valid seed then) and the call must be repeated with part_cap
+// >= the largest cursor.  n_kmers holds kSeedParts counters (the caller sums
 // them), so that no single address takes one atomic per strand.
-int seed_parts();
 void seed_fused(const QueryView& q, const IndexView& ix, const TargetView& t, int gap, int local,
                 unsigned long long* cursors, unsigned long long* n_kmers, int64_t* off, int32_t* cnt, int32_t* nvalid,
                 uint64_t* skey, uint32_t* sq, int64_t part_cap, cudaStream_t st);
-void window_first(const int32_t* nvalid, const int32_t* win_start, int n_windows, int32_t* win_first,
-                  cudaStream_t st);
-// The same outputs as seed_fused for up to kMaxSeedWins target windows in one
-// pass over the query (each window with its own cursors, counters and seed
-// partitions).  Every window must have been built with the same l.
+// The same for the nw windows of a group in one pass over the query: per slot
+// arrays, skey/sq hold nw x kSeedParts partitions.  Every window must have
+// been built with the same l.
 struct SeedWin {
   IndexView ix;
   TargetView t;
-  unsigned long long* cursor;   // seed_parts() cursors
-  unsigned long long* n_kmers;  // seed_parts() l-mer counters
+  unsigned long long* cursor;   // kSeedParts cursors
+  unsigned long long* n_kmers;  // kSeedParts l-mer counters
+};
+struct SeedWins {
+  SeedWin w[kMaxSeedWins];
   int64_t* off;
   int32_t* cnt;
   int32_t* nvalid;
@@ -100,28 +137,21 @@ struct SeedWin {
   uint32_t* sq;
   int64_t part_cap;
 };
-constexpr int kMaxSeedWins = 4;
-struct SeedWins {
-  SeedWin w[kMaxSeedWins];
-};
 void seed_multi(const QueryView& q, const SeedWins& W, int nw, int gap, int local, cudaStream_t st);
 
-// Sorts every segment [off[i], off[i]+len[i]) of (k1, k2[, payload]) ascending by
-// (k1, k2).  Segments of <= 32 are sorted by one warp in registers, <= 2048 by one
-// CTA in shared memory, longer ones by one CTA in global memory.
-void segmented_sort_u64(Workspace& ws, uint64_t* k1, uint64_t* k2, int32_t* payload, const int64_t* off,
-                        const int32_t* len, int64_t n_segments, cudaStream_t st, int tag);
-
-// sortSeeds + deletingIsolateSeeds + deleteDuplicateSeeds per strand: sorts the
-// cnt[s] seeds of strand s by (sequence, diagonal, qIdx) and writes the surviving
-// hits at off[s] onwards, hcnt[s] of them.
-void seed_sort_filter(Workspace& ws, uint64_t* skey, uint32_t* sq, const int64_t* off, const int32_t* cnt,
-                      const int32_t* nvalid, const int32_t* win_start, int n_windows, const int32_t* win_first,
-                      int width, int gap, int64_t nstrands, int32_t* hcnt, cudaStream_t st);
-// also adds band * (qlen - l) DP cells per hit to *cells
+// sortSeeds + deletingIsolateSeeds + deleteDuplicateSeeds per slot: sorts the
+// cnt[v] seeds of slot v by (sequence, diagonal, qIdx) and writes the surviving
+// hits at off[v] onwards, hcnt[v] of them.  lists: 3 nv words.  The first slot
+// of every (target window, query window) with a valid seed has its nvalid
+// complemented.
+void seed_filter(uint64_t* skey, uint32_t* sq, const int64_t* off, const int32_t* cnt, int32_t* nvalid,
+                 const int32_t* win_start, int n_windows, int nw, int width, int gap, int64_t nv, uint32_t* lists,
+                 int32_t* hcnt, GroupCtl* ctl, cudaStream_t st);
+// The hits of every slot back to back (hk: seed key, hq: qIdx, hs: slot); also
+// adds band * (qlen - l) DP cells per hit to ctl->cells.
 void gather_hits(const uint64_t* skey, const uint32_t* sq, const int64_t* off, const int32_t* hcnt,
-                 const int64_t* hoff, int64_t nstrands, uint64_t* hk, int32_t* hq, int32_t* hs,
-                 const int32_t* qlen, int l, int band, unsigned long long* cells, cudaStream_t st);
+                 const int64_t* hoff, int64_t nv, int nw, uint64_t* hk, int32_t* hq, uint32_t* hs,
+                 const int32_t* qlen, int l, int band, GroupCtl* ctl, cudaStream_t st);
 
 // ---- banded DP + E-value (krnlAlignment.cu, krnlCalculateEvalue.cu) ----
 struct DpOut {
@@ -171,53 +201,50 @@ struct DpLaunch {
 // whose low 32 bits are hit indices; outputs stay at the hit's own index.
 // Returns how many hits ran one per warp, or -1 when the split was made on the
 // device (the count is then in *m.warp_n).
-long long banded_dp(const TargetView& t, const QueryView& q, const uint64_t* hk, const int32_t* hq,
-               const int32_t* hs, const uint64_t* order, int64_t n_hits, const DpParams& p, const DpOut& o,
-               cudaStream_t st, const DpLaunch& m = DpLaunch());
+long long banded_dp(const TargetView* t, int nw, const QueryView& q, const uint64_t* hk, const int32_t* hq,
+                    const uint32_t* hs, const uint64_t* order, int64_t n_hits, const DpParams& p, const DpOut& o,
+                    cudaStream_t st, const DpLaunch& m = DpLaunch());
 // Hits per length bucket (16 per power of two of the row count, longest
 // first) and their row sums, in the workspace.
-DpBuckets dp_bucket_count(Workspace& ws, const int32_t* hs, const int32_t* q_len, int64_t n_hits, int l,
+DpBuckets dp_bucket_count(Workspace& ws, const uint32_t* hs, int nw, const int32_t* q_len, int64_t n_hits, int l,
                           cudaStream_t st);
 // CLAST_DP_WARP=off|all, else `fallback` (the environment overrides a
 // context's setting, for tests and measurements).
 int dp_warp_mode_from_env(int fallback);
 // keys[h] = (rows_max - rows of hit h) << 32 | h, rows = q_len[hs[h]] - l + 1:
 // ascending keys take the hits longest first.
-void dp_order_keys(const int32_t* hs, const int32_t* q_len, int64_t n_hits, int l, int rows_max, uint64_t* keys,
-                   cudaStream_t st);
+void dp_order_keys(const uint32_t* hs, int nw, const int32_t* q_len, int64_t n_hits, int l, int rows_max,
+                   uint64_t* keys, cudaStream_t st);
 
 // ---- per-read result order and duplicate removal (utilResultSorting.cuh, CDeviceHitList.cu:32-128) ----
-void final_keys(const uint64_t* hk, const int32_t* hq, const int32_t* hs, const DpOut& o, int64_t n_hits,
-                uint64_t* k1, uint64_t* k2, int32_t* idx, cudaStream_t st);
-void read_ranges(const int64_t* hoff, int64_t n_reads, int64_t* roff, int32_t* rlen, cudaStream_t st);
-void final_dedupe(const uint64_t* k1, const uint64_t* k2, const int32_t* idx, const uint64_t* hk,
-                  const int32_t* hs, const DpOut& o, const int64_t* roff, const int32_t* rlen,
-                  int64_t n_reads, int32_t* fcnt, int32_t* fsel, cudaStream_t st);
-struct FinalOut {
-  int32_t* t_id; int32_t* t_idx; int32_t* q_id; int32_t* q_idx; int32_t* t_len; int32_t* q_len;
-  int32_t* match; int32_t* score; double* evalue;
+// fcnt[r] kept hits of read r, fsel[hoff of the read + j] the j-th of them (its
+// position in the read's run).  g1, g2: one word per hit; list: one per read.
+void final_order(const uint64_t* hk, const int32_t* hq, const uint32_t* hs, const DpOut& o, const int64_t* hoff,
+                 int64_t n_reads, int nw, uint64_t* g1, uint64_t* g2, uint32_t* list, int32_t* fcnt, int32_t* fsel,
+                 GroupCtl* ctl, cudaStream_t st);
+// Where result items go: q_id (q_first + strand) when given, else read, strand
+// and t_load.
+struct OutView {
+  int32_t *read, *strand, *t_load, *t_seq, *t_idx, *q_idx, *t_len, *q_len, *match, *score;
+  double* evalue;
+  int32_t* q_id;
+  int32_t q_first;
+  int32_t t_first[kMaxSeedWins], load[kMaxSeedWins];  // per window of the group
 };
-void final_compact(const int32_t* fsel, const int64_t* roff, const int32_t* fcnt, const int64_t* foff,
-                   int64_t n_reads, const uint64_t* hk, const int32_t* hs, const DpOut& o, int32_t t_first,
-                   int32_t q_first, const FinalOut& out, cudaStream_t st);
+void final_write(const uint64_t* hk, const uint32_t* hs, const DpOut& o, const int64_t* hoff, int64_t n_reads, int nw,
+                 const int32_t* fcnt, const int32_t* fsel, const int64_t* foff, const OutView& out, cudaStream_t st);
 
-// ---- merge of target windows in holder order (CHostResultHolder::fixResult) ----
-struct WinHits {  // one target window's final hits (reads ascending)
-  const int32_t* t_id; const int32_t* t_idx; const int32_t* q_id; const int32_t* q_idx;
-  const int32_t* t_len; const int32_t* q_len; const int32_t* match; const int32_t* score;
+// ---- merge of the groups in holder order (CHostResultHolder::fixResult) ----
+struct GroupHits {  // one group's results (reads ascending), fields in OutView's order
+  const int32_t* f[10];
   const double* evalue;
   const int64_t* foff;  // per read offsets, n_reads + 1
-  int64_t base;         // position of its first item in the concatenation of all windows
-  int32_t load;         // target RAM load of the window
+  int64_t base;         // position of its first item in the concatenation of all groups
 };
-struct MapOut {
-  int32_t* read; int32_t* strand; int32_t* t_load; int32_t* t_seq; int32_t* t_idx; int32_t* q_idx;
-  int32_t* t_len; int32_t* q_len; int32_t* match; int32_t* score; double* evalue;
-};
-// wins: device array of nw windows; total = items of all windows; moff (nreads+1)
+// groups: device array of n; total = items of all groups; moff (nreads+1)
 // receives per-read offsets of the merged result.
-void merge_windows(const WinHits* wins, int nw, int64_t total, int64_t nreads, int32_t* cnt, int64_t* moff,
-                   const MapOut& out, Workspace& ws, cudaStream_t st);
+void merge_groups(const GroupHits* groups, int n, int64_t total, int64_t nreads, int32_t* cnt, int64_t* moff,
+                  const OutView& out, Workspace& ws, cudaStream_t st);
 void gather_i64(const int64_t* src, const int64_t* idx, int n, int64_t* out, cudaStream_t st);
 // Measured INT32 throughput of this GPU in tera-ops/s (add, max, logic mix).
 double int32_probe(cudaStream_t st, int* sink);

@@ -464,17 +464,17 @@ extern "C" int clast_format_tsv(clast_ctx* ctx, const clast_targets* T, const cl
     const int64_t F = r->n;
     TsvArgs a{};
     a.n = F;
-    a.read = ra->dev.f[0].p;
-    a.strand = ra->dev.f[1].p;
-    a.t_load = ra->dev.f[2].p;
-    a.t_seq = ra->dev.f[3].p;
-    a.t_idx = ra->dev.f[4].p;
-    a.q_idx = ra->dev.f[5].p;
-    a.t_len = ra->dev.f[6].p;
-    a.q_len = ra->dev.f[7].p;
-    a.match = ra->dev.f[8].p;
-    a.score = ra->dev.f[9].p;
-    a.evalue = ra->dev.evalue.p;
+    a.read = ra->dev.slab.f[0];
+    a.strand = ra->dev.slab.f[1];
+    a.t_load = ra->dev.slab.f[2];
+    a.t_seq = ra->dev.slab.f[3];
+    a.t_idx = ra->dev.slab.f[4];
+    a.q_idx = ra->dev.slab.f[5];
+    a.t_len = ra->dev.slab.f[6];
+    a.q_len = ra->dev.slab.f[7];
+    a.match = ra->dev.slab.f[8];
+    a.score = ra->dev.slab.f[9];
+    a.evalue = ra->dev.slab.evalue;
     const int64_t qc = reads->n ? reads->offsets[reads->n] : 0, tc = targets->n ? targets->offsets[targets->n] : 0;
     a.q_chars = upload(ws, "tsv_qchars", reads->chars, (size_t)qc, st);
     a.q_off = upload(ws, "tsv_qoff", reads->offsets, (size_t)reads->n + 1, st);
@@ -498,7 +498,7 @@ extern "C" int clast_format_tsv(clast_ctx* ctx, const clast_targets* T, const cl
     int64_t* off = ws.get<int64_t>("tsv_off", (size_t)F + 1);
     const unsigned blocks = (unsigned)((F + 255) / 256);
     if (F > 0) {
-      k_tsv_heads<<<blocks, 256, 0, st>>>(a, ra->dev.load_offsets.p, n_loads, head, cnt);
+      k_tsv_heads<<<blocks, 256, 0, st>>>(a, ra->dev.slab.load_offsets, n_loads, head, cnt);
       CLAST_LAUNCHED();
       k_tsv_select<<<blocks, 256, 0, st>>>(a, head, cnt, len, cnt + 1, host_idx, kHostCap);
       CLAST_LAUNCHED();
@@ -519,7 +519,7 @@ extern "C" int clast_format_tsv(clast_ctx* ctx, const clast_targets* T, const cl
     }
     int64_t* lo_dev = ws.get<int64_t>("tsv_loadoff", (size_t)n_loads + 1);
     int64_t* pos_dev = ws.get<int64_t>("tsv_hostpos", (size_t)std::max(1, h.c[1]));
-    gather_i64(off, ra->dev.load_offsets.p, n_loads + 1, lo_dev, st);
+    gather_i64(off, ra->dev.slab.load_offsets, n_loads + 1, lo_dev, st);
     if (h.c[1] > 0) {
       k_tsv_gather<<<(unsigned)((h.c[1] + 255) / 256), 256, 0, st>>>(off, host_idx, h.c[1], pos_dev);
       CLAST_LAUNCHED();
