@@ -78,55 +78,16 @@ void build_index_device(Workspace& ws, cudaStream_t st, const clast_params* p, c
   int32_t* pos2 = pbits ? nullptr : ws.get<int32_t>("ix_pos2", ns);
   sample_keys(packed, nmask, ns, p->stride, l, pbits, items, pos, st);
   const int in_alt = radix_sort_u64(ws, items, pos, items2, pos2, ns, pbits, pbits + 2 * l + 1, st);
-  // key heads (first sample of every valid code) come with the split
-  const uint64_t bound = 1ull << (2 * l);  // the code of l-mers with a non-ACGT base
-  uint64_t* keys;
-  int32_t* vals;
-  int32_t* head = ws.get<int32_t>("ix_head", ns);
-  if (pbits) {
-    keys = ws.get<uint64_t>("ix_keys", ns);
-    vals = ws.get<int32_t>("ix_vals", ns);
-    split_items(in_alt ? items2 : items, ns, pbits, bound, keys, vals, head, st);
-  } else {
-    keys = in_alt ? items2 : items;
-    vals = in_alt ? pos2 : pos;
-    index_heads(keys, ns, bound, head, st);
-  }
-  // From here on no host synchronisation: every array is sized for the ns
-  // samples (an upper bound of the valid samples nv, the unique keys nu and
-  // the entries); nv = *nv_dev and nu = hpos[ns] stay on the device.
-  int64_t* nv_dev = ws.get<int64_t>("ix_nv", 1);
-  if (ns > 0) count_below(keys, ns, bound, nv_dev, st);
-  else CLAST_CK(cudaMemsetAsync(nv_dev, 0, sizeof(int64_t), st));
-  int64_t* hpos = ws.get<int64_t>("ix_hpos", ns + 1);
-  scan_i32(ws, head, ns, hpos, st);
-  const int64_t* nu_dev = hpos + ns;
-  uint64_t* ukeys = ws.get<uint64_t>("ix_ukeys", ns);
-  int64_t* ufirst = ws.get<int64_t>("ix_ufirst", ns + 1);
-  index_unique(keys, head, hpos, ns, nv_dev, ukeys, ufirst, st);
-  int32_t* keep = ws.get<int32_t>("ix_keep", ns);
-  int2* resolved = ws.get<int2>("ix_resolved", ns);
-  int64_t* kpos = ws.get<int64_t>("ix_kpos", ns + 1);
-  index_keep(vals, hpos, ufirst, ns, nv_dev, p->stride, l, p->cut_repeat, ix->gateway.p, ix->lengths.p, ix->nseqs,
-             keep, resolved, st);
-  scan_i32(ws, keep, ns, kpos, st);
-  ix->entries.alloc(ns);
-  index_entries(keep, kpos, resolved, ns, ix->entries.p, st);
-  int32_t* ustart = ws.get<int32_t>("ix_ustart", ns);
-  int32_t* ucnt = ws.get<int32_t>("ix_ucnt", ns);
-  index_buckets(ufirst, kpos, ns, nu_dev, ustart, ucnt, st);
+  // From here on every array is sized for the ns samples (an upper bound of
+  // the valid ones and of the kept ones), with no host synchronisation.
   // Hash table: buckets of two records, one bucket per sample, so at most half
   // of the records are used (84 % of the keys then sit in their home bucket),
   // plus a tail for the probe run past the last bucket
   const int64_t nb = std::max<int64_t>(1, ns);
   if (nb >= (int64_t)UINT32_MAX) throw std::invalid_argument("window has too many sampled l-mers");
   ix->nbuckets = (uint32_t)nb;
-  int64_t* rank = ws.get<int64_t>("ix_rank", ns + 1);
-  scan_positive(ws, ucnt, ns, rank, st);
+  ix->entries.alloc(ns);
   ix->kept.alloc(1);
-  CLAST_CK(cudaMemcpyAsync(ix->kept.p, rank + ns, sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
-  int64_t* run_max = ws.get<int64_t>("ix_runmax", ns);
-  table_runmax(ws, ukeys, ucnt, rank, ns, l, ix->nbuckets, run_max, st);
   ix->n_records = 2 * nb + (1 << 16);
   ix->table.alloc((size_t)ix->n_records);
   CLAST_CK(cudaMemsetAsync(ix->table.p, 0xff, (size_t)ix->n_records * sizeof(ulonglong2), st));
@@ -141,8 +102,13 @@ void build_index_device(Workspace& ws, cudaStream_t st, const clast_params* p, c
   ix->fshift = 64 - (bits - 5);
   ix->filter.alloc((size_t)1 << (bits - 5));
   CLAST_CK(cudaMemsetAsync(ix->filter.p, 0, ((size_t)1 << (bits - 5)) * sizeof(uint32_t), st));
-  table_place(ukeys, ustart, ucnt, ix->entries.p, rank, run_max, ns, ix->table.p, ix->n_records, ix->filter.p,
-              ix->fshift, failed, st);
+  CLAST_CK(cudaMemsetAsync(ix->kept.p, 0, sizeof(int64_t), st));
+  const size_t words = (size_t)index_state_words(ns);
+  unsigned long long* state = ws.get<unsigned long long>("ix_state", words);
+  CLAST_CK(cudaMemsetAsync(state, 0, words * sizeof(unsigned long long), st));
+  index_place(in_alt ? items2 : items, in_alt ? pos2 : pos, ns, pbits, p->stride, l, p->cut_repeat, ix->gateway.p,
+              ix->lengths.p, ix->nseqs, ix->nbuckets, ix->entries.p, ix->table.p, ix->n_records, ix->filter.p,
+              ix->fshift, state, reinterpret_cast<unsigned long long*>(ix->kept.p), failed, st);
   ix->n_keys = ns;
 }
 

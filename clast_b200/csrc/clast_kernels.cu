@@ -47,15 +47,11 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 // ------------------------------------------------------------------------
 constexpr int kScanThreads = 256, kScanItems = 8, kScanTile = kScanThreads * kScanItems;
 
-// Element loaders of the scans: an array, or a flag computed from one.
+// Element loader of the scans.
 template <class T>
 struct ArrayLoad {
   const T* __restrict__ p;
   __device__ __forceinline__ int64_t operator()(int64_t i) const { return (int64_t)p[i]; }
-};
-struct PositiveLoad {  // 1 where p[i] > 0
-  const int32_t* __restrict__ p;
-  __device__ __forceinline__ int64_t operator()(int64_t i) const { return p[i] > 0 ? 1 : 0; }
 };
 
 // ---- single-pass exclusive scan (decoupled look-back) ----
@@ -400,19 +396,6 @@ __global__ void k_sample_keys(const uint64_t* __restrict__ packed, const uint64_
   }
 }
 
-// keys / vals of the sorted words, and head[i] = whether key i is valid
-// (< bound) and differs from key i - 1.
-__global__ void k_split_items(const uint64_t* __restrict__ items, int64_t n, int pbits, uint64_t bound,
-                              uint64_t* __restrict__ keys, int32_t* __restrict__ vals, int32_t* __restrict__ head) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint64_t v = items[i];
-  const uint64_t k = v >> pbits;
-  keys[i] = k;
-  vals[i] = (int32_t)(v & ((1ull << pbits) - 1));
-  head[i] = (k < bound && (i == 0 || (items[i - 1] >> pbits) != k)) ? 1 : 0;
-}
-
 // ---- LSD radix sort of 64-bit words by a bit range, 8 bits per pass ----
 // A block takes a tile of kRsTile consecutive words; warp w owns words
 // [w * kRsWarpItems, (w + 1) * kRsWarpItems) of it.  Each pass: per-block digit
@@ -544,54 +527,38 @@ __global__ void __launch_bounds__(kRsThreads, 3) k_rs_scatter(const uint64_t* __
   }
 }
 
-__global__ void k_count_below(const uint64_t* __restrict__ keys, int64_t n, uint64_t bound,
-                              int64_t* __restrict__ out) {
-  int64_t lo = 0, hi = n;  // first key >= bound in a sorted array
-  while (lo < hi) {
-    const int64_t mid = (lo + hi) >> 1;
-    if (keys[mid] < bound) lo = mid + 1;
-    else hi = mid;
-  }
-  *out = lo;
-}
+// ---- the index from the sorted samples, in one pass ----
+// A tile of kIxTile sorted samples is one block's.  Equal codes form runs; a
+// run belongs to the tile that holds its first sample, and the repeat cut
+// counts all of its samples.  The kept samples of a run (not cut, not on a
+// joint) go to `entries` from the run's first index on, so that no count of
+// the kept ones before it is needed.  Every run that keeps a sample is a
+// record of the hash table.  The codes arrive ascending, so their home records
+// do too, and linear probing puts record u at max(home_u, pos_{u-1} + 1): for a
+// tile that starts after the free position x, at u + max(max_{j <= u} (home_j -
+// j), x) with u counted within the tile.  A tile that holds C records and ends
+// at A for x = 0 therefore maps x to max(A, x + C); x comes from a decoupled
+// look-back over those pairs, one word each (flag, C, A).  Tiles take their
+// number from a counter in launch order, so a tile waits only for tiles that
+// have started, and at most kScanSpinLimit polls per step: past that it counts
+// into *failed, which the host reports.
+//
+// Bound by memory: 8 bytes read and about 24 written per sample, and one
+// random atomic per code for the filter.  The fourteen kernels this replaced
+// (heads, two scans, unique codes, kept samples, entries, bucket bounds, a scan
+// of the kept codes, a two-level running maximum, placement) wrote and read
+// some 120 bytes per sample in between.
+constexpr int kIxThreads = 256, kIxRounds = 4, kIxTile = kIxThreads * kIxRounds;
+constexpr int kIxWarps = kIxThreads / 32, kIxWarpItems = 32 * kIxRounds;
 
-// The index build runs without host synchronisation: kernels cover the n
-// samples (an upper bound) and read the counts that matter from the device
-// (*nv valid samples; *nu = hpos[n] unique keys, as the scans end with the
-// total and every flag past the valid range is 0).
-__global__ void k_index_heads(const uint64_t* __restrict__ k, int64_t n, uint64_t bound,
-                              int32_t* __restrict__ head) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) head[i] = (k[i] < bound && (i == 0 || k[i] != k[i - 1])) ? 1 : 0;
+template <bool PAIR>
+__device__ __forceinline__ uint64_t ix_code(const uint64_t* __restrict__ items, int pbits, int64_t i) {
+  return PAIR ? items[i] : items[i] >> pbits;
 }
-
-__global__ void k_index_unique(const uint64_t* __restrict__ k, const int32_t* __restrict__ head,
-                               const int64_t* __restrict__ hpos, int64_t n, const int64_t* __restrict__ nv_dev,
-                               uint64_t* __restrict__ ukeys, int64_t* __restrict__ ufirst) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nv = *nv_dev;
-  if (i < n && head[i]) {
-    ukeys[hpos[i]] = k[i];
-    ufirst[hpos[i]] = i;
-  }
-  if (i == 0) ufirst[hpos[nv]] = nv;
-}
-
-__global__ void k_index_keep(const int32_t* __restrict__ vals, const int64_t* __restrict__ hpos,
-                             const int64_t* __restrict__ ufirst, int64_t n, const int64_t* __restrict__ nv_dev,
-                             int stride, int l, int cut, const int32_t* __restrict__ gw,
-                             const int32_t* __restrict__ len, int nseqs, int32_t* __restrict__ keep,
-                             int2* __restrict__ resolved) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (i >= *nv_dev) {
-    keep[i] = 0;
-    return;
-  }
-  const int64_t u = hpos[i + 1] - 1;
-  const int64_t cnt = ufirst[u + 1] - ufirst[u];
-  const bool pass = (cut == -1) || (cnt < (int64_t)cut);  // removeRepeatedSequence
-  const int64_t pos = (int64_t)vals[i] * stride;
+// Sequence and index of the sample at window position pos (onTargetBoundary: a
+// sample that reaches into the joint is none, x = -1).
+__device__ __forceinline__ int2 ix_resolve(int64_t pos, int l, const int32_t* __restrict__ gw,
+                                           const int32_t* __restrict__ len, int nseqs) {
   int lo = 0, hi = nseqs;  // last sequence starting at or before pos
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -599,122 +566,304 @@ __global__ void k_index_keep(const int32_t* __restrict__ vals, const int64_t* __
     else hi = mid;
   }
   const int tidx = (int)(pos - gw[lo]);
-  const bool joint = (int64_t)tidx + l > (int64_t)len[lo];  // onTargetBoundary
-  keep[i] = (pass && !joint) ? 1 : 0;
-  resolved[i] = make_int2(lo, tidx);
+  return (int64_t)tidx + l > (int64_t)len[lo] ? make_int2(-1, 0) : make_int2(lo, tidx);
 }
 
-__global__ void k_index_entries(const int32_t* __restrict__ keep, const int64_t* __restrict__ kpos,
-                                const int2* __restrict__ resolved, int64_t n, int2* __restrict__ entries) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && keep[i]) entries[kpos[i]] = resolved[i];
-}
-
-__global__ void k_index_buckets(const int64_t* __restrict__ ufirst, const int64_t* __restrict__ kpos,
-                                int64_t n, const int64_t* __restrict__ nu_dev, int32_t* __restrict__ ustart,
-                                int32_t* __restrict__ ucnt) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  if (k >= *nu_dev) {
-    ucnt[k] = 0;
-    return;
+// Exclusive prefix over the block's warps of v (one value per warp); *total = their sum.
+__device__ __forceinline__ int ix_warp_prefix(int v, int* __restrict__ buf, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) buf[warp] = v;
+  __syncthreads();
+  int before = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < kIxWarps; ++w) {
+    const int x = buf[w];
+    if (w < warp) before += x;
+    all += x;
   }
-  const int64_t a = kpos[ufirst[k]], b = kpos[ufirst[k + 1]];
-  ustart[k] = (int32_t)a;
-  ucnt[k] = (int32_t)(b - a);
+  __syncthreads();
+  *total = all;
+  return before;
 }
 
-// ---- hash table of the index, placed without atomics ----
-// The unique codes arrive ascending, so their home records do too; with
-// r = rank among the kept codes, linear probing puts code r at
-// max(home_r, pos_{r-1} + 1) = r + max_{j <= r}(home_j - j).
-
-// The running maximum is taken over the unique codes k (not over the ranks):
-// for kept code k it equals max over kept j <= k of home_j - rank_j.  Codes
-// without entries (repeat cut, joints only, past the keys: ucnt 0) count as
-// INT64_MIN.
-struct SlackLoad {
-  const uint64_t* __restrict__ ucode;
-  const int32_t* __restrict__ ucnt;
-  const int64_t* __restrict__ rank;
-  int l;
+struct IndexBuild {
+  const uint64_t* items;  // sorted: code << pbits | sample, or codes with the samples in vals (pbits 0)
+  const int32_t* vals;
+  int64_t ns;
+  int pbits;
+  uint64_t bound;  // codes from here on are l-mers with a non-ACGT base
+  int stride, l, cut;
+  const int32_t* gw;
+  const int32_t* len;
+  int nseqs;
   uint32_t nbuckets;
-  __device__ __forceinline__ int64_t operator()(int64_t k) const {
-    return ucnt[k] > 0 ? record_home(ucode[k], l, nbuckets) - rank[k] : INT64_MIN;
-  }
+  int2* entries;
+  ulonglong2* table;
+  int64_t n_records;
+  uint32_t* filter;
+  int fshift;
+  unsigned long long* state;  // [0] tile counter, then one word per tile
+  unsigned long long* kept;   // records placed
+  unsigned long long* failed;
 };
 
-__global__ void k_table_place(const uint64_t* __restrict__ ucode, const int32_t* __restrict__ ustart,
-                              const int32_t* __restrict__ ucnt, const int2* __restrict__ entries,
-                              const int64_t* __restrict__ rank, const int64_t* __restrict__ run_max, int64_t nu,
-                              ulonglong2* __restrict__ table, int64_t n_records, uint32_t* __restrict__ filter,
-                              int fshift, unsigned long long* __restrict__ failed) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nu) return;
-  const int c = ucnt[k];
-  if (c <= 0) return;
-  const uint64_t code = ucode[k];
-  const uint64_t h = key_hash(code);
-  atomicOr(filter + filter_word(h, fshift), filter_mask(h));
-  uint64_t payload;
-  if (c == 1) {
-    const int2 e = entries[ustart[k]];
-    payload = ((uint64_t)(uint32_t)e.x << 32) | (uint32_t)e.y;
-  } else {
-    payload = kMulti | ((uint64_t)(uint32_t)ustart[k] << 32) | (uint32_t)c;
-  }
-  const int64_t pos = rank[k] + run_max[k];
-  if (pos >= 0 && pos < n_records) table[pos] = make_ulonglong2(code, payload);
-  else atomicAdd(failed, 1ull);  // unreachable: positions rise to the last one, which the table holds
-}
-
-// ---- inclusive running maximum (int64) ----
-template <class Load>
-__global__ void __launch_bounds__(kScanThreads) k_maxscan_tiles(Load in, int64_t n, int64_t* __restrict__ out,
-                                                                int64_t* __restrict__ tile_max) {
-  __shared__ int64_t warp_max[kScanThreads / 32];
-  const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
-  int64_t v[kScanItems];
-  int64_t m = INT64_MIN;
-#pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    const int64_t idx = base + i;
-    v[i] = (idx < n) ? in(idx) : INT64_MIN;
-    m = v[i] > m ? v[i] : m;
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int64_t incl = m;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int64_t y = __shfl_up_sync(kFull, incl, o);
-    if (lane >= o && y > incl) incl = y;
-  }
-  if (lane == 31) warp_max[warp] = incl;
+template <bool PAIR>
+__global__ void __launch_bounds__(kIxThreads) k_index_place(IndexBuild b) {
+  __shared__ uint64_t code[kIxTile + 1];
+  __shared__ int2 res[kIxTile];
+  __shared__ uint16_t start[kIxTile + 1];  // first sample of every run of the tile
+  __shared__ uint16_t kpre[kIxTile + 1];   // kept samples before sample k
+  __shared__ uint16_t first[kIxTile];      // first kept sample of the run that starts at k
+  __shared__ int wbuf[kIxWarps];
+  __shared__ int64_t wmax[kIxWarps];
+  __shared__ uint64_t s_prev;
+  __shared__ unsigned long long s_tile;
+  __shared__ int64_t s_x;
+  __shared__ int2 s_cross;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned lt = lanemask_lt();
+  unsigned long long* status = b.state + 1;
+  if (tid == 0) s_tile = atomicAdd(b.state, 1ull);
   __syncthreads();
-  int64_t wpre = INT64_MIN, tot = INT64_MIN;
+  const int64_t t = (int64_t)s_tile, i0 = t * kIxTile;
+  const int nt = (int)min((int64_t)kIxTile, b.ns - i0);
+  const uint64_t pmask = PAIR ? 0 : (1ull << b.pbits) - 1;
+  int pos[kIxRounds];
 #pragma unroll
-  for (int w = 0; w < kScanThreads / 32; ++w) {
-    const int64_t t = warp_max[w];
-    if (w < warp && t > wpre) wpre = t;
-    if (t > tot) tot = t;
+  for (int j = 0; j < kIxRounds; ++j) {
+    const int k = warp * kIxWarpItems + j * 32 + lane;
+    uint64_t c = ~0ull;
+    pos[j] = 0;
+    if (k < nt) {
+      const uint64_t w = b.items[i0 + k];
+      c = PAIR ? w : w >> b.pbits;
+      pos[j] = PAIR ? b.vals[i0 + k] : (int)(w & pmask);
+    }
+    code[k] = c;
   }
-  int64_t run = __shfl_up_sync(kFull, incl, 1);
-  if (lane == 0) run = INT64_MIN;
-  if (wpre > run) run = wpre;
+  if (tid == 0) {
+    code[kIxTile] = i0 + kIxTile < b.ns ? ix_code<PAIR>(b.items, b.pbits, i0 + kIxTile) : ~0ull;
+    s_prev = i0 > 0 ? ix_code<PAIR>(b.items, b.pbits, i0 - 1) : ~0ull;
+  }
+  __syncthreads();
+  // runs: rid[j] = the run of this thread's sample within the tile (-1: it began before the tile)
+  int rid[kIxRounds];
+  unsigned started = 0;
+  int n_runs;
+  {
+    unsigned m[kIxRounds];
+    int n = 0;
 #pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    const int64_t idx = base + i;
-    if (v[i] > run) run = v[i];
-    if (idx < n) out[idx] = run;
+    for (int j = 0; j < kIxRounds; ++j) {
+      const int k = warp * kIxWarpItems + j * 32 + lane;
+      const bool st = k < nt && (k == 0 ? s_prev : code[k - 1]) != code[k];
+      m[j] = __ballot_sync(kFull, st);
+      rid[j] = n + __popc(m[j] & lt) + (st ? 1 : 0) - 1;
+      started |= (st ? 1u : 0u) << j;
+      n += __popc(m[j]);
+    }
+    const int before = ix_warp_prefix(n, wbuf, &n_runs);
+#pragma unroll
+    for (int j = 0; j < kIxRounds; ++j) {
+      rid[j] += before;
+      if ((started >> j) & 1u) start[rid[j]] = (uint16_t)(warp * kIxWarpItems + j * 32 + lane);
+    }
+    if (tid == 0) start[n_runs] = (uint16_t)nt;
   }
-  if (threadIdx.x == 0) tile_max[blockIdx.x] = tot;
-}
-
-__global__ void k_maxscan_apply(int64_t* __restrict__ out, int64_t n, const int64_t* __restrict__ tile_run) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int64_t t = i / kScanTile;
-  if (t > 0 && tile_run[t - 1] > out[i]) out[i] = tile_run[t - 1];
+  __syncthreads();
+  // the last run may go on past the tile
+  const uint64_t last_code = n_runs > 0 ? code[start[n_runs - 1]] : ~0ull;
+  const bool cross = n_runs > 0 && nt == kIxTile && last_code < b.bound && code[kIxTile] == last_code;
+  // kept samples
+  unsigned kept = 0;
+  {
+    unsigned m[kIxRounds];
+    int n = 0;
+#pragma unroll
+    for (int j = 0; j < kIxRounds; ++j) {
+      const int k = warp * kIxWarpItems + j * 32 + lane;
+      bool keep = false;
+      if (k < nt && code[k] < b.bound && rid[j] >= 0 && !(cross && rid[j] == n_runs - 1)) {
+        const int cnt = start[rid[j] + 1] - start[rid[j]];
+        if (b.cut == -1 || cnt < b.cut) {  // removeRepeatedSequence
+          const int2 r = ix_resolve((int64_t)pos[j] * b.stride, b.l, b.gw, b.len, b.nseqs);
+          keep = r.x >= 0;
+          res[k] = r;
+        }
+      }
+      m[j] = __ballot_sync(kFull, keep);
+      kept |= (keep ? 1u : 0u) << j;
+      n += __popc(m[j]);
+    }
+    int total;
+    int at = ix_warp_prefix(n, wbuf, &total);
+#pragma unroll
+    for (int j = 0; j < kIxRounds; ++j) {
+      kpre[warp * kIxWarpItems + j * 32 + lane] = (uint16_t)(at + __popc(m[j] & lt));
+      at += __popc(m[j]);
+    }
+    if (tid == 0) kpre[kIxTile] = (uint16_t)total;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kIxRounds; ++j)
+    if ((kept >> j) & 1u) {
+      const int k = warp * kIxWarpItems + j * 32 + lane, h = start[rid[j]];
+      const int rank = kpre[k] - kpre[h];
+      b.entries[i0 + h + rank] = res[k];
+      if (rank == 0) first[h] = (uint16_t)k;
+    }
+  // a run that goes on past the tile: the whole block walks it
+  int cross_kept = 0;
+  if (cross) {
+    const int64_t h = i0 + start[n_runs - 1];
+    bool pass = true;
+    if (b.cut != -1) {
+      int64_t cnt = 0;
+      for (int64_t base = h;; base += kIxThreads) {
+        const int64_t i = base + tid;
+        const int in = __syncthreads_count(i < b.ns && ix_code<PAIR>(b.items, b.pbits, i) == last_code);
+        cnt += in;
+        if (in < kIxThreads || cnt >= b.cut) break;
+      }
+      pass = cnt < b.cut;
+    }
+    for (int64_t base = h; pass; base += kIxThreads) {
+      const int64_t i = base + tid;
+      int2 r = make_int2(-1, 0);
+      bool in = false;
+      if (i < b.ns) {
+        const uint64_t w = b.items[i];
+        in = (PAIR ? w : w >> b.pbits) == last_code;
+        if (in)
+          r = ix_resolve((int64_t)(PAIR ? b.vals[i] : (int)(w & pmask)) * b.stride, b.l, b.gw, b.len, b.nseqs);
+      }
+      const unsigned m = __ballot_sync(kFull, r.x >= 0);
+      int total;
+      const int at = cross_kept + ix_warp_prefix(__popc(m), wbuf, &total) + __popc(m & lt);
+      if (r.x >= 0) {
+        b.entries[h + at] = r;
+        if (at == 0) s_cross = r;
+      }
+      cross_kept += total;
+      if (__syncthreads_count(in) < kIxThreads) break;
+    }
+  }
+  __syncthreads();
+  // records: u = rank within the tile, slack = home - u, its running maximum
+  unsigned rec = 0;
+  int u[kIxRounds], kc[kIxRounds];
+  int64_t run[kIxRounds], home[kIxRounds];
+  int n_rec;
+  int64_t tile_max = INT64_MIN;
+  {
+    unsigned m[kIxRounds];
+    int n = 0;
+#pragma unroll
+    for (int j = 0; j < kIxRounds; ++j) {
+      const int k = warp * kIxWarpItems + j * 32 + lane;
+      kc[j] = 0;
+      home[j] = 0;
+      if ((started >> j) & 1u) {
+        const bool c = cross && rid[j] == n_runs - 1;
+        kc[j] = c ? cross_kept : kpre[start[rid[j] + 1]] - kpre[k];
+        if (kc[j] > 0) home[j] = record_home(code[k], b.l, b.nbuckets);
+      }
+      m[j] = __ballot_sync(kFull, kc[j] > 0);
+      u[j] = n + __popc(m[j] & lt);
+      rec |= (kc[j] > 0 ? 1u : 0u) << j;
+      n += __popc(m[j]);
+    }
+    const int before = ix_warp_prefix(n, wbuf, &n_rec);
+    int64_t carry = INT64_MIN;
+#pragma unroll
+    for (int j = 0; j < kIxRounds; ++j) {
+      u[j] += before;
+      int64_t v = (rec >> j) & 1u ? home[j] - u[j] : INT64_MIN;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int64_t y = __shfl_up_sync(kFull, v, o);
+        if (lane >= o && y > v) v = y;
+      }
+      run[j] = v > carry ? v : carry;
+      carry = __shfl_sync(kFull, run[j], 31);
+    }
+    if (lane == 0) wmax[warp] = carry;
+    __syncthreads();
+    int64_t pre = INT64_MIN;
+#pragma unroll
+    for (int w = 0; w < kIxWarps; ++w) {
+      const int64_t x = wmax[w];
+      if (w < warp && x > pre) pre = x;
+      if (x > tile_max) tile_max = x;
+    }
+#pragma unroll
+    for (int j = 0; j < kIxRounds; ++j) run[j] = run[j] > pre ? run[j] : pre;
+  }
+  // x: the position after the records of all earlier tiles
+  if (warp == 0) {
+    const int64_t A = n_rec > 0 ? n_rec + tile_max : 0;
+    int64_t x = 0;
+    if (t > 0) {
+      if (lane == 0) st_relaxed_u64(status + t, kScanAgg | ((unsigned long long)n_rec << 50) | (unsigned long long)A);
+      int64_t after = 0;  // records of the tiles walked over
+      for (int64_t j = t - 1;; j -= 32) {
+        const int64_t jj = j - lane;
+        unsigned long long w = jj >= 0 ? ld_relaxed_u64(status + jj) : kScanInc;
+        for (int spin = 0; __any_sync(kFull, (w >> 62) == 0) && spin < kScanSpinLimit; ++spin)
+          if ((w >> 62) == 0) w = ld_relaxed_u64(status + jj);
+        if (__any_sync(kFull, (w >> 62) == 0)) {
+          if (lane == 0) atomicAdd(b.failed, 1ull);
+          break;
+        }
+        const unsigned inc = __ballot_sync(kFull, (w & kScanInc) != 0);
+        const int last = inc ? __ffs(inc) - 1 : 31;
+        const bool whole = (w & kScanInc) != 0;  // an inclusive position, else a pair
+        const int64_t C = lane <= last && !whole ? (int64_t)((w >> 50) & 0xfff) : 0;
+        int64_t incl = C;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int64_t y = __shfl_up_sync(kFull, incl, o);
+          if (lane >= o) incl += y;
+        }
+        int64_t v = lane <= last ? (int64_t)(whole ? w & kScanValue : w & ((1ull << 50) - 1)) + after + incl - C : 0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const int64_t y = __shfl_xor_sync(kFull, v, o);
+          v = y > v ? y : v;
+        }
+        x = v > x ? v : x;
+        after += __shfl_sync(kFull, incl, 31);
+        if (inc) break;
+      }
+    }
+    if (lane == 0) {
+      const int64_t end = A > x + n_rec ? A : x + n_rec;
+      st_relaxed_u64(status + t, kScanInc | (unsigned long long)end);
+      s_x = x;
+      if (n_rec) atomicAdd(b.kept, (unsigned long long)n_rec);
+    }
+  }
+  __syncthreads();
+  const int64_t x = s_x;
+#pragma unroll
+  for (int j = 0; j < kIxRounds; ++j) {
+    if (!((rec >> j) & 1u)) continue;
+    const int k = warp * kIxWarpItems + j * 32 + lane;
+    const uint64_t c = code[k];
+    const uint64_t h = key_hash(c);
+    atomicOr(b.filter + filter_word(h, b.fshift), filter_mask(h));
+    uint64_t payload;
+    if (kc[j] == 1) {
+      const int2 e = cross && rid[j] == n_runs - 1 ? s_cross : res[first[k]];
+      payload = ((uint64_t)(uint32_t)e.x << 32) | (uint32_t)e.y;
+    } else {
+      payload = kMulti | ((uint64_t)(i0 + k) << 32) | (uint32_t)kc[j];
+    }
+    const int64_t at = u[j] + (run[j] > x ? run[j] : x);
+    if (at >= 0 && at < b.n_records) b.table[at] = make_ulonglong2(c, payload);
+    else atomicAdd(b.failed, 1ull);  // unreachable: positions rise to the last one, which the table holds
+  }
 }
 
 // ------------------------------------------------------------------------
@@ -2759,9 +2908,6 @@ void scan_i32_to(const int32_t* in, int64_t n, int64_t* out, unsigned long long*
   k_scan_1pass<<<(unsigned)tiles, kScanThreads, 0, st>>>(ArrayLoad<int32_t>{in}, n, n + 1, out, state, total);
   CLAST_LAUNCHED();
 }
-void scan_positive(Workspace& ws, const int32_t* in, int64_t n, int64_t* out, cudaStream_t st) {
-  scan_1pass(ws, PositiveLoad{in}, n, out, st);
-}
 
 void pack_bases(const char* bases, int64_t n, uint64_t* packed, uint64_t* nmask, cudaStream_t st) {
   const int64_t nwords = (n + 63) / 64 + 1;  // one extra word so kmer_at may read w+1
@@ -2798,13 +2944,6 @@ void sample_keys(const uint64_t* packed, const uint64_t* nmask, int64_t n_sample
   CLAST_LAUNCHED();
 }
 
-void split_items(const uint64_t* items, int64_t n, int pbits, uint64_t bound, uint64_t* keys, int32_t* vals,
-                 int32_t* head, cudaStream_t st) {
-  if (n <= 0) return;
-  k_split_items<<<blocks_for(n, 256), 256, 0, st>>>(items, n, pbits, bound, keys, vals, head);
-  CLAST_LAUNCHED();
-}
-
 int radix_sort_u64(Workspace& ws, uint64_t* keys, int32_t* vals, uint64_t* keys_alt, int32_t* vals_alt, int64_t n,
                    int lo_bit, int hi_bit, cudaStream_t st) {
   if (n <= 1) return 0;
@@ -2835,42 +2974,20 @@ int radix_sort_u64(Workspace& ws, uint64_t* keys, int32_t* vals, uint64_t* keys_
   return which;
 }
 
-void count_below(const uint64_t* keys, int64_t n, uint64_t bound, int64_t* out, cudaStream_t st) {
-  k_count_below<<<1, 1, 0, st>>>(keys, n, bound, out);
-  CLAST_LAUNCHED();
-}
+int64_t index_state_words(int64_t n_samples) { return (n_samples + kIxTile - 1) / kIxTile + 1; }
 
-void index_heads(const uint64_t* keys, int64_t n, uint64_t bound, int32_t* head, cudaStream_t st) {
-  if (n <= 0) return;
-  k_index_heads<<<blocks_for(n, 256), 256, 0, st>>>(keys, n, bound, head);
+void index_place(const uint64_t* items, const int32_t* vals, int64_t n_samples, int pbits, int stride, int l, int cut,
+                 const int32_t* gateway, const int32_t* lengths, int nseqs, uint32_t nbuckets, int2* entries,
+                 ulonglong2* table, int64_t n_records, uint32_t* filter, int fshift, unsigned long long* state,
+                 unsigned long long* kept, unsigned long long* failed, cudaStream_t st) {
+  if (n_samples <= 0) return;
+  const IndexBuild b{items, vals, n_samples, pbits, 1ull << (2 * l), stride, l, cut, gateway, lengths, nseqs, nbuckets,
+                     entries, table, n_records, filter, fshift, state, kept, failed};
+  const unsigned tiles = (unsigned)(index_state_words(n_samples) - 1);
+  if (pbits > 0) k_index_place<false><<<tiles, kIxThreads, 0, st>>>(b);
+  else k_index_place<true><<<tiles, kIxThreads, 0, st>>>(b);
   CLAST_LAUNCHED();
 }
-void index_unique(const uint64_t* keys, const int32_t* head, const int64_t* hpos, int64_t n, const int64_t* nv_dev,
-                  uint64_t* ukeys, int64_t* ufirst, cudaStream_t st) {
-  k_index_unique<<<blocks_for(n > 0 ? n : 1, 256), 256, 0, st>>>(keys, head, hpos, n, nv_dev, ukeys, ufirst);
-  CLAST_LAUNCHED();
-}
-void index_keep(const int32_t* vals, const int64_t* hpos, const int64_t* ufirst, int64_t n, const int64_t* nv_dev,
-                int stride, int l, int cut, const int32_t* gateway, const int32_t* lengths, int nseqs, int32_t* keep,
-                int2* resolved, cudaStream_t st) {
-  if (n <= 0) return;
-  k_index_keep<<<blocks_for(n, 256), 256, 0, st>>>(vals, hpos, ufirst, n, nv_dev, stride, l, cut, gateway, lengths,
-                                                   nseqs, keep, resolved);
-  CLAST_LAUNCHED();
-}
-void index_entries(const int32_t* keep, const int64_t* kpos, const int2* resolved, int64_t nv, int2* entries,
-                   cudaStream_t st) {
-  if (nv <= 0) return;
-  k_index_entries<<<blocks_for(nv, 256), 256, 0, st>>>(keep, kpos, resolved, nv, entries);
-  CLAST_LAUNCHED();
-}
-void index_buckets(const int64_t* ufirst, const int64_t* kpos, int64_t n, const int64_t* nu_dev, int32_t* ustart,
-                   int32_t* ucnt, cudaStream_t st) {
-  if (n <= 0) return;
-  k_index_buckets<<<blocks_for(n, 256), 256, 0, st>>>(ufirst, kpos, n, nu_dev, ustart, ucnt);
-  CLAST_LAUNCHED();
-}
-
 
 void seed_fused(const QueryView& q, const IndexView& ix, const TargetView& t, int gap, int local,
                 unsigned long long* cursors, unsigned long long* n_kmers, int64_t* off, int32_t* cnt, int32_t* nvalid,
@@ -2904,36 +3021,6 @@ void seed_multi(const QueryView& q, const SeedWins& W, int nw, int gap, int loca
     case 4: launch_seed_multi<4>(q, W, gap, local, st); break;
     default: throw std::invalid_argument("seed_multi: 1 to 4 windows per pass");
   }
-}
-
-template <class Load>
-void maxscan_impl(Workspace& ws, Load in, int64_t n, int64_t* out, cudaStream_t st, int level) {
-  if (n <= 0) return;
-  const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-  const std::string tag = "maxscan" + std::to_string(level);
-  int64_t* tmax = ws.get<int64_t>(tag + "m", tiles);
-  k_maxscan_tiles<Load><<<(unsigned)tiles, kScanThreads, 0, st>>>(in, n, out, tmax);
-  CLAST_LAUNCHED();
-  if (tiles > 1) {
-    int64_t* trun = ws.get<int64_t>(tag + "r", tiles);
-    maxscan_impl(ws, ArrayLoad<int64_t>{tmax}, tiles, trun, st, level + 1);
-    k_maxscan_apply<<<blocks_for(n, 256), 256, 0, st>>>(out, n, trun);
-    CLAST_LAUNCHED();
-  }
-}
-
-void table_runmax(Workspace& ws, const uint64_t* ucode, const int32_t* ucnt, const int64_t* rank, int64_t n_unique,
-                  int l, uint32_t nbuckets, int64_t* run_max, cudaStream_t st) {
-  maxscan_impl(ws, SlackLoad{ucode, ucnt, rank, l, nbuckets}, n_unique, run_max, st, 0);
-}
-
-void table_place(const uint64_t* ucode, const int32_t* ustart, const int32_t* ucnt, const int2* entries,
-                 const int64_t* rank, const int64_t* run_max, int64_t n_unique, ulonglong2* table, int64_t n_records,
-                 uint32_t* filter, int fshift, unsigned long long* failed, cudaStream_t st) {
-  if (n_unique <= 0) return;
-  k_table_place<<<blocks_for(n_unique, 256), 256, 0, st>>>(ucode, ustart, ucnt, entries, rank, run_max, n_unique,
-                                                            table, n_records, filter, fshift, failed);
-  CLAST_LAUNCHED();
 }
 
 void seed_filter(uint64_t* skey, uint32_t* sq, const int64_t* off, const int32_t* cnt, int32_t* nvalid,

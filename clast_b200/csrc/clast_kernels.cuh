@@ -18,9 +18,6 @@ void scan_i32(Workspace& ws, const int32_t* in, int64_t n, int64_t* out, cudaStr
 int64_t scan_state_words(int64_t n);
 void scan_i32_to(const int32_t* in, int64_t n, int64_t* out, unsigned long long* state, long long* total,
                  cudaStream_t st);
-// exclusive scan of (in[i] > 0)
-void scan_positive(Workspace& ws, const int32_t* in, int64_t n, int64_t* out, cudaStream_t st);
-
 // 2-bit codes (32 bases per word) and non-ACGT mask (64 per word) of bases[0..n);
 // positions >= n count as 'N'.  packed needs ceil(n/32)+2 words, nmask ceil(n/64)+2.
 void pack_bases(const char* bases, int64_t n, uint64_t* packed, uint64_t* nmask, cudaStream_t st);
@@ -45,41 +42,22 @@ void build_window(const char* src, const int64_t* src_off, const int32_t* gatewa
 // items[j] = code, vals[j] = j.
 void sample_keys(const uint64_t* packed, const uint64_t* nmask, int64_t n_samples, int stride, int l, int pbits,
                  uint64_t* items, int32_t* vals, cudaStream_t st);
-// keys[i] = items[i] >> pbits, vals[i] = the low pbits bits, head[i] =
-// whether keys[i] < bound and differs from keys[i - 1].
-void split_items(const uint64_t* items, int64_t n, int pbits, uint64_t bound, uint64_t* keys, int32_t* vals,
-                 int32_t* head, cudaStream_t st);
 // Stable LSD radix sort of 64-bit words by bits [lo_bit, hi_bit), carrying
 // vals along unless vals is null.  Returns 0 when the result is in (keys,
 // vals), 1 when it is in (keys_alt, vals_alt).
 int radix_sort_u64(Workspace& ws, uint64_t* keys, int32_t* vals, uint64_t* keys_alt, int32_t* vals_alt, int64_t n,
                    int lo_bit, int hi_bit, cudaStream_t st);
-// *out = number of keys < bound in the sorted array keys[0..n)
-void count_below(const uint64_t* keys, int64_t n, uint64_t bound, int64_t* out, cudaStream_t st);
-// Index build over n samples with the valid count *nv_dev and the unique
-// count *nu_dev on the device (no host synchronisation).  head[i] = whether
-// keys[i] < bound and differs from keys[i - 1].
-void index_heads(const uint64_t* keys, int64_t n, uint64_t bound, int32_t* head, cudaStream_t st);
-void index_unique(const uint64_t* keys, const int32_t* head, const int64_t* hpos, int64_t n, const int64_t* nv_dev,
-                  uint64_t* ukeys, int64_t* ufirst, cudaStream_t st);
-void index_keep(const int32_t* vals, const int64_t* hpos, const int64_t* ufirst, int64_t n, const int64_t* nv_dev,
-                int stride, int l, int cut, const int32_t* gateway, const int32_t* lengths, int nseqs, int32_t* keep,
-                int2* resolved, cudaStream_t st);
-void index_entries(const int32_t* keep, const int64_t* kpos, const int2* resolved, int64_t nv,
-                   int2* entries, cudaStream_t st);
-void index_buckets(const int64_t* ufirst, const int64_t* kpos, int64_t n, const int64_t* nu_dev, int32_t* ustart,
-                   int32_t* ucnt, cudaStream_t st);
-// Hash table of the index without atomics (layout: IndexView).  rank =
-// exclusive scan of (ucnt > 0), the codes that keep entries; table_runmax:
-// run_max[k] = max over kept j <= k of home_j - rank_j; table_place writes
-// every kept code's record at rank[k] + run_max[k] and sets its filter bits
-// (filter zeroed, table records set to ~0 by the caller); *failed counts
-// records that would fall outside the table (none).
-void table_runmax(Workspace& ws, const uint64_t* ucode, const int32_t* ucnt, const int64_t* rank, int64_t n_unique,
-                  int l, uint32_t nbuckets, int64_t* run_max, cudaStream_t st);
-void table_place(const uint64_t* ucode, const int32_t* ustart, const int32_t* ucnt, const int2* entries,
-                 const int64_t* rank, const int64_t* run_max, int64_t n_unique, ulonglong2* table, int64_t n_records,
-                 uint32_t* filter, int fshift, unsigned long long* failed, cudaStream_t st);
+// The index from the sorted samples (as sample_keys lays them out): entries of
+// the kept ones (n_samples long, runs of equal codes apart), the hash table
+// without atomics (layout: IndexView; records set to ~0 by the caller) and the
+// filter (zeroed by the caller).  state: index_state_words(n_samples) zeroed
+// words; *kept is raised by the records placed, *failed by records outside the
+// table and by waits that gave up (neither happens).
+int64_t index_state_words(int64_t n_samples);
+void index_place(const uint64_t* items, const int32_t* vals, int64_t n_samples, int pbits, int stride, int l, int cut,
+                 const int32_t* gateway, const int32_t* lengths, int nseqs, uint32_t nbuckets, int2* entries,
+                 ulonglong2* table, int64_t n_records, uint32_t* filter, int fshift, unsigned long long* state,
+                 unsigned long long* kept, unsigned long long* failed, cudaStream_t st);
 
 // ---- seeds (CDeviceHitList_createRawSeedList.cu, _deleteSeeds*.cu, _sortSeeds.cu) ----
 // A group of up to kMaxSeedWins target windows is searched together.  Its slots

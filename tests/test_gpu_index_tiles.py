@@ -1,0 +1,50 @@
+"""The index build at the edges of its tiles (1,024 sorted samples): sample
+counts around a tile, runs of one l-mer that end at, cross or span tiles, with
+and without the repeat cut, codes in one word with their position and in two."""
+import numpy as np
+import pytest
+
+import oracle as O
+from clast_b200 import api, synth
+from _cases import compare
+
+pytestmark = pytest.mark.gpu
+
+
+def case(seed, samples, stride, lmer, poly):
+    """A target of about `samples` samples with runs of poly-A, poly-AC and N,
+    and reads from it and from the runs."""
+    rng = np.random.Generator(np.random.PCG64(seed))
+    n = samples * stride
+    parts = np.array_split(synth.ACGT[rng.integers(0, 4, size=n)], 3)
+    seqs = [bytearray(p.tobytes()) for p in parts]
+    if poly:
+        at = len(seqs[1]) // 3
+        seqs[1][at:at + poly] = b"A" * poly
+        seqs[2][10:10 + poly // 2] = b"AC" * (poly // 4)
+        seqs[0][-40:] = b"A" * 40  # up to the joint
+        seqs[2][-30:-20] = b"N" * 10
+    t = [bytes(x) for x in seqs]
+    reads = []
+    for s in t:
+        for p in rng.integers(0, max(1, len(s) - 120), size=8):
+            reads.append(s[p:p + 120])
+    if poly:
+        reads += [b"A" * 60 + t[0][50:90], b"AC" * 30, t[1][len(t[1]) // 3 - 50:len(t[1]) // 3 + 50]]
+    return t, [r for r in reads if len(r) >= lmer]
+
+
+@pytest.mark.parametrize("lmer,cut", [(8, -1), (8, 20), (15, 20), (15, 3), (15, 5000), (15, -1), (24, 20), (31, -1)])
+@pytest.mark.parametrize("samples,poly", [(60, 0), (1023, 0), (1024, 0), (1025, 0), (1600, 900), (4096, 7000), (9000, 1000)])
+def test_index_tiles_equal_oracle(engine, samples, poly, lmer, cut):
+    stride = 3 if lmer < 24 else 2
+    t, reads = case(samples + lmer, samples, stride, lmer, poly)
+    s = api.Setting(lmer=lmer, stride=stride, cut_repeat=cut, total_db=float(sum(map(len, t))))
+    tl = api.SeqList(s.lmer).add_targets(t)
+    ql = api.SeqList(s.lmer).add_queries(reads)
+    tb, tg, tn = tl.window(0, len(t))
+    qb, qg, qn = ql.window(0, len(ql.lengths))
+    want = O.window_search(s, tb, tg, tn, 0, qb, qg, qn, 0)
+    ix = engine.hash_table(s, tl, 0, len(t))
+    compare(engine.hit_list(s, ix, ql, 0, len(reads)), want)
+    ix.close()
