@@ -26,10 +26,14 @@ constexpr uint64_t kDroppedSeed = ~0ull;
 // (sequence within window << 32 | index within sequence) or, for keys with
 // several entries, kMulti | start << 32 | count into `entries`.  A blocked
 // Bloom filter (3 bits in one 32-bit word per key) answers most absent keys
-// from L2.
+// from L2.  An l-mer and its reverse complement share their word (see
+// filter_hash), so a read's two strands are looked up with one load; and the
+// words of two windows that are searched together lie side by side, so that
+// load serves both.
 struct IndexView {
   int l;
-  int fshift;                // filter word = key_hash(code) >> fshift (fshift >= 32)
+  int fshift;                // filter word = filter_hash >> fshift (fshift >= 32)
+  int fstride;               // words from one filter word to the next: 2 when two windows' words alternate
   const uint32_t* filter;
   const ulonglong2* table;   // n_records records; payload ~0 = free
   uint32_t nbuckets;         // home records are 2 * [0, nbuckets)
@@ -111,22 +115,49 @@ __device__ __forceinline__ int64_t record_home(uint64_t code, int l, uint32_t nb
 __device__ __forceinline__ int64_t record_home16(uint32_t code, int l, uint32_t nbuckets) {
   return 2 * (int64_t)__umulhi(code << (32 - 2 * l), nbuckets);
 }
-// Filter hash of a code: an xorshift then a multiply by an odd constant
-// (Fibonacci hashing).  The top bits select the 32-bit filter word, bits
-// 16..30 the three filter bits.  (Filter words taken from the code's own top
-// bits, which would let the sorted codes fill the filter without atomics,
-// measured slower at lookup time.)
-__host__ __device__ __forceinline__ uint64_t key_hash(uint64_t code) {
-  return (code ^ (code >> 31)) * 0x9E3779B97F4A7C15ull;
+// Key of a code (order_code's inverse).
+__host__ __device__ __forceinline__ uint64_t key_of_code(uint64_t code, int l) {
+  return (code * 0xCFEE444D8B59A89Bull) & ((1ull << (2 * l)) - 1);
+}
+// Reverse complement of a 2l-bit key.
+__device__ __forceinline__ uint64_t key_revcomp(uint64_t key, int l) {
+  uint64_t y = (uint64_t)__brevll((long long)(~key << (64 - 2 * l)));
+  y = ((y >> 1) & 0x5555555555555555ull) | ((y & 0x5555555555555555ull) << 1);
+  return y & ((1ull << (2 * l)) - 1);
+}
+// Filter hash of an l-mer: of the smaller of its key and its reverse
+// complement's.  The top bits select the 32-bit filter word; the low bits hold
+// the three filter bits of the smaller key (bits 0..14) and of the larger one
+// (bits 15..29).  Keys of up to 32 bits take a 32-bit form, a third of the
+// instructions.
+__host__ __device__ __forceinline__ uint64_t filter_hash16(uint32_t smaller) {
+  const uint64_t p = (uint64_t)smaller * 0x9E3779B1u;
+  const uint32_t lo = (uint32_t)p, hi = (uint32_t)(p >> 32);
+  return ((uint64_t)lo << 32) | (((lo ^ hi) * 0x85EBCA6Bu) >> 2);
+}
+__host__ __device__ __forceinline__ uint64_t filter_hash(uint64_t smaller, int l) {
+  if (l <= 16) return filter_hash16((uint32_t)smaller);
+  uint64_t h = smaller * 0x9E3779B97F4A7C15ull;
+  h ^= h >> 32;
+  return h * 0xD6E8FEB86659FD93ull;
 }
 // fshift >= 32: filter word = (h >> 32) >> (fshift - 32)
 __host__ __device__ __forceinline__ uint32_t filter_word(uint64_t h, int fshift) {
   return (uint32_t)(h >> 32) >> (fshift - 32);
 }
-__host__ __device__ __forceinline__ uint32_t filter_mask(uint64_t h) {
-  const uint32_t v = (uint32_t)(h >> 16);
+__host__ __device__ __forceinline__ uint32_t filter_bits3(uint32_t v) {
   return (1u << (v & 31)) | (1u << ((v >> 5) & 31)) | (1u << ((v >> 10) & 31));
 }
+__host__ __device__ __forceinline__ uint32_t filter_mask(uint64_t h, bool larger) {
+  return filter_bits3((uint32_t)h >> (larger ? 15 : 0));
+}
+// The filter that index files hold (one word per code, not shared with the
+// reverse complement): an xorshift then a multiply by an odd constant; the top
+// bits select the word, bits 16..30 the three filter bits.
+__host__ __device__ __forceinline__ uint64_t file_filter_hash(uint64_t code) {
+  return (code ^ (code >> 31)) * 0x9E3779B97F4A7C15ull;
+}
+__host__ __device__ __forceinline__ uint32_t file_filter_mask(uint64_t h) { return filter_bits3((uint32_t)(h >> 16)); }
 // Entries of a payload (0 for none).
 __host__ __device__ __forceinline__ int payload_count(uint64_t p) {
   return p == kNoPayload ? 0 : ((p & kMulti) ? (int)(uint32_t)p : 1);

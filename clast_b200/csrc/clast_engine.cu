@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <climits>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -91,32 +92,26 @@ void build_index_device(Workspace& ws, cudaStream_t st, const clast_params* p, c
   ix->n_records = 2 * nb + (1 << 16);
   ix->table.alloc((size_t)ix->n_records);
   CLAST_CK(cudaMemsetAsync(ix->table.p, 0xff, (size_t)ix->n_records * sizeof(ulonglong2), st));
-  // Bloom filter: about 24 bits per sample, between 2^12 and 2^F bits; F = 27
-  // (16 MB: the filters of the two windows a seeding pass reads stay in L2
-  // beside the streams that pass through it) unless CLAST_FILTER_BITS says
-  // otherwise (16..32)
-  int fbits = 27;
-  if (const char* e = std::getenv("CLAST_FILTER_BITS")) fbits = std::max(16, std::min(32, std::atoi(e)));
-  int bits = 12;
-  while (bits < fbits && (1ll << bits) < ns * 24) ++bits;
-  ix->fshift = 64 - (bits - 5);
-  ix->filter.alloc((size_t)1 << (bits - 5));
-  CLAST_CK(cudaMemsetAsync(ix->filter.p, 0, ((size_t)1 << (bits - 5)) * sizeof(uint32_t), st));
+  if (!ix->filter_mem) {
+    clast_index* one[1] = {ix};
+    alloc_filters(one, 1, filter_shift(ns), st);
+  }
   CLAST_CK(cudaMemsetAsync(ix->kept.p, 0, sizeof(int64_t), st));
   const size_t words = (size_t)index_state_words(ns);
   unsigned long long* state = ws.get<unsigned long long>("ix_state", words);
   CLAST_CK(cudaMemsetAsync(state, 0, words * sizeof(unsigned long long), st));
   index_place(in_alt ? items2 : items, in_alt ? pos2 : pos, ns, pbits, p->stride, l, p->cut_repeat, ix->gateway.p,
-              ix->lengths.p, ix->nseqs, ix->nbuckets, ix->entries.p, ix->table.p, ix->n_records, ix->filter.p,
-              ix->fshift, state, reinterpret_cast<unsigned long long*>(ix->kept.p), failed, st);
+              ix->lengths.p, ix->nseqs, ix->nbuckets, ix->entries.p, ix->table.p, ix->n_records, ix->filter,
+              ix->fshift, ix->fstride, state, reinterpret_cast<unsigned long long*>(ix->kept.p), failed, st);
   ix->n_keys = ns;
 }
 
-// Index of a window whose padded base array is already on the device.
+// Index of a window whose padded base array is already on the device (its
+// filter memory set already, or none).
 clast_index* make_index_resident(Workspace& ws, cudaStream_t st, const clast_params* p, DevArray<char>&& padded,
                                  int64_t n_bases, DevArray<int32_t>&& gateway, DevArray<int32_t>&& lengths,
-                                 int32_t n_seqs, int32_t t_begin, unsigned long long* failed) {
-  std::unique_ptr<clast_index> ix(new clast_index());
+                                 int32_t n_seqs, int32_t t_begin, unsigned long long* failed,
+                                 std::unique_ptr<clast_index> ix = std::unique_ptr<clast_index>(new clast_index())) {
   ix->l = p->lmer;
   ix->stride = p->stride;
   ix->cut = p->cut_repeat;
@@ -244,6 +239,7 @@ struct HitSink {
 // partitions.
 struct Group {
   int nw = 0;
+  bool reads = false;             // the strands are reads and their reverse complements, pair by pair
   const clast_index* ix[kMaxSeedWins] = {};
   int32_t load[kMaxSeedWins] = {};
   int64_t part_cap = 0;           // seeds per partition to begin with
@@ -281,6 +277,7 @@ int64_t search_group(clast_ctx* c, Workspace& ws, const clast_params* p, const Q
   int32_t *cnt = nullptr, *nvalid = nullptr, *hcnt = nullptr;
   uint64_t* skey = nullptr;
   uint32_t* sq = nullptr;
+  FirstSeeds first{};
   int64_t H = 0;
   for (int attempt = 0;; ++attempt) {
     off = ws.get<int64_t>("s_off", nv);
@@ -295,47 +292,64 @@ int64_t search_group(clast_ctx* c, Workspace& ws, const clast_params* p, const Q
     hcnt = ws.get<int32_t>("s_hcnt", nv);
     hoff = ws.get<int64_t>("s_hoff", nv + 1);
     uint32_t* lists = ws.get<uint32_t>("s_lists", 3 * nv);
+    uint64_t* first_key = nullptr;
+    uint32_t* first_q = nullptr;
     CLAST_CK(cudaMemsetAsync(zero, 0, zero_bytes, st));
     tm.begin(st);
-    static const bool force_multi = std::getenv("CLAST_SEED_MULTI_ONLY") != nullptr;
-    if (nw == 1 && !force_multi) {  // the single-window kernel (round 0 staged while its range is reserved)
-      seed_fused(q, g.ix[0]->view(), g.ix[0]->tview(), p->gap, p->local, ctl->cursor[0], ctl->kmers[0], off, cnt,
-                 nvalid, skey, sq, g.part_cap, st);
+    if (!g.reads) {  // any strands, one window
+      seed_fused(q, g.ix[0]->view(), g.ix[0]->tview(), p->gap, p->local, ctl->cursor, ctl->kmers[0], off, cnt, nvalid,
+                 skey, sq, g.part_cap, st);
     } else {
+      first_key = ws.get<uint64_t>("s_first", nv);
+      first_q = ws.get<uint32_t>("s_firstq", nv);
       SeedWins W{};
-      for (int w = 0; w < nw; ++w)
-        W.w[w] = SeedWin{g.ix[w]->view(), g.ix[w]->tview(), ctl->cursor[w], ctl->kmers[w]};
+      for (int w = 0; w < nw; ++w) {
+        W.w[w] = SeedWin{g.ix[w]->view(), g.ix[w]->tview(), ctl->kmers[w], ctl->seeds[w], 0};
+        W.w[w].paired = w % 2 == 1 && g.ix[w]->filter_mem == g.ix[w - 1]->filter_mem &&
+                        g.ix[w]->filter == g.ix[w - 1]->filter + 1;
+      }
+      W.cursor = ctl->cursor;
       W.off = off;
       W.cnt = cnt;
       W.nvalid = nvalid;
+      W.hcnt = hcnt;
+      W.first_key = first_key;
+      W.first_q = first_q;
+      W.lists = lists;
+      W.n_listed = ctl->n_seeds;
+      W.long_reads = ws.get<uint32_t>("s_long", nr);
+      W.n_long = ctl->n_stored;
+      W.words = 1;
+      for (int w = 0; w < nw; ++w)
+        if (g.ix[w]->nseqs >= (1 << 20)) W.words = 0;
       W.skey = skey;
       W.sq = sq;
       W.part_cap = g.part_cap;
-      seed_multi(q, W, nw, p->gap, p->local, st);
+      seed_reads(q, W, nw, p->width, p->gap, p->local, qb.lens ? INT_MAX : qb.max_len, st);
     }
+    first = FirstSeeds{first_key, first_q, nvalid, cnt};
     tm.end(StageTimer::SEED, st);
     // sortSeeds, deletingIsolateSeeds, deleteDuplicateSeeds
     tm.begin(st);
-    seed_filter(skey, sq, off, cnt, nvalid, qb.wstart, qb.nwin, nw, p->width, p->gap, nv, lists, hcnt, ctl, st);
+    seed_filter(skey, sq, off, cnt, nvalid, first_q, qb.wstart, qb.nwin, nw, p->width, p->gap, nv, lists, hcnt, ctl, st);
     tm.end(StageTimer::SORT, st, 4);
     scan_i32_to(hcnt, nv, hoff, state1, &ctl->hits, st);
     const GroupCtl& h = read_ctl(c, ctl, st);
     tm.flush();
-    int64_t most = 0, kmers = 0, S = 0, most_win = 0;
-    for (int w = 0; w < nw; ++w) {
-      int64_t sw = 0;
-      for (int i = 0; i < kSeedParts; ++i) {
-        sw += (int64_t)h.cursor[w][i];
-        most = std::max<int64_t>(most, (int64_t)h.cursor[w][i]);
+    int64_t most = 0, kmers = 0, S = 0, stored = 0;
+    for (int i = 0; i < kSeedParts; ++i) {
+      most = std::max<int64_t>(most, (int64_t)h.cursor[i]);
+      stored += (int64_t)h.cursor[i];
+      for (int w = 0; w < nw; ++w) {
         kmers += (int64_t)h.kmers[w][i];
+        S += (int64_t)h.seeds[w][i];
       }
-      S += sw;
-      most_win = std::max(most_win, sw);
     }
-    if (most <= g.part_cap) {
+    if (!g.reads) S = stored;
+    if (most <= g.part_cap * nw) {
       c->stats.query_kmers += kmers;
       c->stats.seeds += S;
-      c->seed_hint = std::max<int64_t>(c->seed_hint, most_win + most_win / 4);
+      c->seed_hint = std::max<int64_t>(c->seed_hint, (stored + stored / 4) / nw);
       H = h.hits;
       break;
     }
@@ -345,7 +359,7 @@ int64_t search_group(clast_ctx* c, Workspace& ws, const clast_params* p, const Q
                                   " seeds; clast_search_noalloc's scratch holds " + std::to_string(g.part_fit) +
                                   " (use clast_search)");
     if (ws.arena) ws.arena_rewind(mark);
-    g.part_cap = most;  // strands past a full partition wrote nothing: run again
+    g.part_cap = (most + nw - 1) / nw;  // strands past a full partition wrote nothing: run again
   }
   if (H >= ((int64_t)1 << 32)) throw std::invalid_argument("more than 2^32 hits in one window");  // DP order words
   c->stats.hits += H;
@@ -353,7 +367,7 @@ int64_t search_group(clast_ctx* c, Workspace& ws, const clast_params* p, const Q
   uint64_t* hk = ws.get<uint64_t>("h_key", H);
   int32_t* hq = ws.get<int32_t>("h_q", H);
   uint32_t* hs = ws.get<uint32_t>("h_s", H);
-  gather_hits(skey, sq, off, hcnt, hoff, nv, nw, hk, hq, hs, q.len, p->lmer, 2 * p->gap + 1, ctl, st);
+  gather_hits(skey, sq, off, hcnt, hoff, nv, nw, hk, hq, hs, q.len, p->lmer, 2 * p->gap + 1, first, ctl, st);
   // alignmentHits + calculateEvalue + deleteHits_lowEValue / _tooShort
   DpOut o;
   o.t_idx = ws.get<int32_t>("d_tidx", H);
@@ -467,6 +481,27 @@ struct SlabSink : HitSink {
 // ----------------------------------------------------------------------------
 
 namespace clast {
+
+int filter_shift(int64_t ns) {
+  int fbits = 27;
+  if (const char* e = std::getenv("CLAST_FILTER_BITS")) fbits = std::max(16, std::min(32, std::atoi(e)));
+  int bits = 12;
+  while (bits < fbits && (1ll << bits) < ns * 24) ++bits;
+  return 64 - (bits - 5);
+}
+
+void alloc_filters(clast_index* const* ix, int n, int fshift, cudaStream_t st) {
+  auto mem = std::make_shared<DevArray<uint32_t>>();
+  const size_t words = (size_t)n << (64 - fshift);
+  mem->alloc(words);
+  CLAST_CK(cudaMemsetAsync(mem->p, 0, words * sizeof(uint32_t), st));
+  for (int k = 0; k < n; ++k) {
+    ix[k]->filter_mem = mem;
+    ix[k]->filter = mem->p + k;
+    ix[k]->fstride = n;
+    ix[k]->fshift = fshift;
+  }
+}
 
 // Waits for the index builds of clast_targets_create (once), records their
 // time in the context's stats and reports a table overflow.
@@ -814,6 +849,16 @@ int clast_targets_create(clast_ctx* ctx, const clast_params* p, int32_t t_vram, 
     // its own scratch, so that two builds run at once (a build is a chain of
     // small, latency-bound kernels); every build stream starts after the plan's
     // upload above and the compute stream waits for all of them at the end.
+    // Windows searched together (2k and 2k + 1) share their filter memory.
+    std::vector<std::unique_ptr<clast_index>> shells;
+    for (size_t wi = 0; wi < plan.size(); ++wi) shells.emplace_back(new clast_index());
+    for (size_t wi = 0; wi < plan.size(); wi += 2) {
+      const int n = wi + 1 < plan.size() ? 2 : 1;
+      clast_index* two[2] = {shells[wi].get(), n > 1 ? shells[wi + 1].get() : nullptr};
+      int fshift = 63;
+      for (int k = 0; k < n; ++k) fshift = std::min(fshift, filter_shift(plan[wi + k].n / p->stride));
+      alloc_filters(two, n, fshift, st);
+    }
     cudaEvent_t planned = ctx->timer.take();
     win_ev.push_back(planned);
     CLAST_CK(cudaEventRecord(planned, st));
@@ -847,11 +892,11 @@ int clast_targets_create(clast_ctx* ctx, const clast_params* p, int32_t t_vram, 
       win.load = w.load;
       win.first = w.first;
       win.ix.reset(make_index_resident(ctx->ws_build[b], bs, p, std::move(padded), w.n, std::move(dgw),
-                                       std::move(dln), w.nseqs, w.first, failed));
+                                       std::move(dln), w.nseqs, w.first, failed, std::move(shells[wi])));
       g_alloc_stream = st;
       // the index is used and finally freed in the compute stream's order
       clast_index& ix = *win.ix;
-      ix.bases.st = ix.gateway.st = ix.lengths.st = ix.filter.st = ix.table.st = ix.entries.st = ix.kept.st = st;
+      ix.bases.st = ix.gateway.st = ix.lengths.st = ix.table.st = ix.entries.st = ix.kept.st = st;
       T->wins.push_back(std::move(win));
     }
     // the builds end on build stream 0 (which waits for the others): ev_done
@@ -1020,6 +1065,7 @@ static int map_impl(clast_ctx* ctx, const clast_targets* T, const clast_params* 
     std::vector<Group> groups;
     for (size_t g0 = 0; g0 < T->wins.size() && qr.q.nstrands > 0; g0 += (size_t)group) {
       Group g;
+      g.reads = true;
       for (size_t w = g0; w < std::min(T->wins.size(), g0 + (size_t)group); ++w) {
         if (T->wins[w].ix->n_keys == 0) continue;
         g.load[g.nw] = T->wins[w].load;

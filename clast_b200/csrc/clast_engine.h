@@ -260,7 +260,11 @@ struct clast_index {
   int32_t nseqs = 0;
   clast::DevArray<char> bases;  // padded
   clast::DevArray<int32_t> gateway, lengths;
-  clast::DevArray<uint32_t> filter;     // blocked Bloom filter, 2^(64 - fshift) words
+  // blocked Bloom filter, 2^(64 - fshift) words of stride fstride from `filter`;
+  // windows that are searched together share the memory, their words alternating
+  std::shared_ptr<clast::DevArray<uint32_t>> filter_mem;
+  uint32_t* filter = nullptr;
+  int fstride = 1;
   clast::DevArray<ulonglong2> table;    // 2 * nbuckets records {key, payload}
   clast::DevArray<int2> entries;
   int64_t n_unique = 0, n_keys = 0, n_entries = 0;
@@ -273,7 +277,8 @@ struct clast_index {
     clast::IndexView v;
     v.l = l;
     v.fshift = fshift;
-    v.filter = filter.p;
+    v.fstride = fstride;
+    v.filter = filter;
     v.table = table.p;
     v.nbuckets = nbuckets;
     v.n_records = n_records;
@@ -291,6 +296,18 @@ struct clast_index {
     return t;
   }
 };
+
+namespace clast {
+
+// Words of the filter of a window of ns samples: about 24 bits per sample,
+// between 2^12 and 2^F bits; F = 27 (16 MB: the filters of the two windows a
+// group searches stay in L2 beside the streams that pass through it) unless
+// CLAST_FILTER_BITS says otherwise (16..32).  Returns fshift.
+int filter_shift(int64_t ns);
+// Zeroed filter memory for n windows (1 or 2, the words of two alternating).
+void alloc_filters(clast_index* const* ix, int n, int fshift, cudaStream_t st);
+
+}  // namespace clast
 
 struct clast_targets {
   clast_ctx* ctx = nullptr;

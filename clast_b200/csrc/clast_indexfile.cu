@@ -201,9 +201,14 @@ extern "C" int clast_targets_save(clast_ctx* ctx, const clast_targets* T, const 
       put<int32_t>(f, ix.nseqs);
       put<int64_t>(f, ix.n);
       put<uint32_t>(f, ix.nbuckets);
-      put<int32_t>(f, ix.fshift);
+      // the file's filter has one word per code, which older readers of the
+      // layout search; it is made from the table here and from the table again
+      // when the file is loaded
+      const int fshift = filter_shift(ix.n / ix.stride);
+      const int64_t n_filter = (int64_t)1 << (64 - fshift);
+      put<int32_t>(f, fshift);
       put<int64_t>(f, ix.n_records);
-      put<int64_t>(f, (int64_t)ix.filter.n);
+      put<int64_t>(f, n_filter);
       put<int64_t>(f, (int64_t)ix.entries.n);
       put<int64_t>(f, ix.n_keys);
       put_array(f, ix.bases.p, ix.n + 2 * kPad, buf, st);
@@ -211,7 +216,12 @@ extern "C" int clast_targets_save(clast_ctx* ctx, const clast_targets* T, const 
       put_array(f, ix.lengths.p, ix.nseqs, buf, st);
       put_array(f, ix.entries.p, (int64_t)ix.entries.n, buf, st);
       put_array(f, ix.table.p, ix.n_records, buf, st);
-      put_array(f, ix.filter.p, (int64_t)ix.filter.n, buf, st);
+      g_alloc_stream = st;
+      DevArray<uint32_t> filter;
+      filter.alloc((size_t)n_filter);
+      CLAST_CK(cudaMemsetAsync(filter.p, 0, (size_t)n_filter * sizeof(uint32_t), st));
+      filter_from_table(ix.table.p, ix.n_records, ix.l, filter.p, fshift, 1, true, st);
+      put_array(f, filter.p, n_filter, buf, st);
     }
     if (std::fflush(f) != 0) throw std::runtime_error("index file write failed");
     return CLAST_OK;
@@ -275,7 +285,6 @@ extern "C" int clast_targets_load(clast_ctx* ctx, const clast_params* p, const c
       ix->nseqs = w.nseqs;
       ix->n = w.n;
       ix->nbuckets = w.nbuckets;
-      ix->fshift = w.fshift;
       ix->n_records = w.n_records;
       ix->n_keys = w.n_keys;
       auto up = [&](auto& dev, const auto& host) {
@@ -288,12 +297,21 @@ extern "C" int clast_targets_load(clast_ctx* ctx, const clast_params* p, const c
       up(ix->lengths, w.lengths);
       up(ix->entries, w.entries);
       up(ix->table, w.table);
-      up(ix->filter, w.filter);
       CLAST_CK(cudaStreamSynchronize(st));  // the host window is reused
       win.ix = std::move(ix);
       T->wins.push_back(std::move(win));
     }
     if (std::fgetc(f) != EOF) throw std::invalid_argument("index file has bytes past its last window");
+    // the filters, those of two windows that are searched together side by side
+    for (size_t k = 0; k < T->wins.size(); k += 2) {
+      const int n = k + 1 < T->wins.size() ? 2 : 1;
+      clast_index* two[2] = {T->wins[k].ix.get(), n > 1 ? T->wins[k + 1].ix.get() : nullptr};
+      int fshift = 63;
+      for (int j = 0; j < n; ++j) fshift = std::min(fshift, filter_shift(two[j]->n / two[j]->stride));
+      alloc_filters(two, n, fshift, st);
+      for (int j = 0; j < n; ++j)
+        filter_from_table(two[j]->table.p, two[j]->n_records, two[j]->l, two[j]->filter, fshift, n, false, st);
+    }
     // records per load: every record of a load lies in one of its windows
     std::vector<int64_t> per_load((size_t)h.n_loads, 0);
     for (const auto& x : T->wins)

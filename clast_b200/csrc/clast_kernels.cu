@@ -543,11 +543,13 @@ __global__ void __launch_bounds__(kRsThreads, 3) k_rs_scatter(const uint64_t* __
 // have started, and at most kScanSpinLimit polls per step: past that it counts
 // into *failed, which the host reports.
 //
-// Bound by memory: 8 bytes read and about 24 written per sample, and one
-// random atomic per code for the filter.  The fourteen kernels this replaced
-// (heads, two scans, unique codes, kept samples, entries, bucket bounds, a scan
-// of the kept codes, a two-level running maximum, placement) wrote and read
-// some 120 bytes per sample in between.
+// 8 bytes read and about 24 written per sample, and one random atomic per code
+// for the filter; bound by the waits at its barriers and by instructions (443
+// per sample), at a fifth of the memory rate.  The fourteen kernels this
+// replaced (heads, two scans, unique codes, kept samples, entries, bucket
+// bounds, a scan of the kept codes, a two-level running maximum, placement)
+// wrote and read some 120 bytes per sample in between: index of a 250 Mbp
+// window (50 M samples) 6.28 to 3.76 ms, of which this kernel takes 1.18.
 constexpr int kIxThreads = 256, kIxRounds = 4, kIxTile = kIxThreads * kIxRounds;
 constexpr int kIxWarps = kIxThreads / 32, kIxWarpItems = 32 * kIxRounds;
 
@@ -586,6 +588,29 @@ __device__ __forceinline__ int ix_warp_prefix(int v, int* __restrict__ buf, int*
   return before;
 }
 
+// Sets the filter bits of the l-mer of code c.
+__device__ __forceinline__ void filter_set(uint32_t* __restrict__ filter, int fshift, int fstride, uint64_t c, int l) {
+  const uint64_t key = key_of_code(c, l), rc = key_revcomp(key, l);
+  const uint64_t h = filter_hash(key < rc ? key : rc, l);
+  atomicOr(filter + (size_t)filter_word(h, fshift) * fstride, filter_mask(h, key > rc));
+}
+
+// The filter of a table's keys: as searched, or (FILE) as index files hold it.
+template <bool FILE>
+__global__ void k_filter_from_table(const ulonglong2* __restrict__ table, int64_t n_records, int l,
+                                    uint32_t* __restrict__ filter, int fshift, int fstride) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_records) return;
+  const ulonglong2 r = table[i];
+  if (r.y == kNoPayload) return;
+  if (FILE) {
+    const uint64_t h = file_filter_hash(r.x);
+    atomicOr(filter + filter_word(h, fshift), file_filter_mask(h));
+  } else {
+    filter_set(filter, fshift, fstride, r.x, l);
+  }
+}
+
 struct IndexBuild {
   const uint64_t* items;  // sorted: code << pbits | sample, or codes with the samples in vals (pbits 0)
   const int32_t* vals;
@@ -601,7 +626,7 @@ struct IndexBuild {
   ulonglong2* table;
   int64_t n_records;
   uint32_t* filter;
-  int fshift;
+  int fshift, fstride;
   unsigned long long* state;  // [0] tile counter, then one word per tile
   unsigned long long* kept;   // records placed
   unsigned long long* failed;
@@ -851,8 +876,7 @@ __global__ void __launch_bounds__(kIxThreads) k_index_place(IndexBuild b) {
     if (!((rec >> j) & 1u)) continue;
     const int k = warp * kIxWarpItems + j * 32 + lane;
     const uint64_t c = code[k];
-    const uint64_t h = key_hash(c);
-    atomicOr(b.filter + filter_word(h, b.fshift), filter_mask(h));
+    filter_set(b.filter, b.fshift, b.fstride, c, b.l);
     uint64_t payload;
     if (kc[j] == 1) {
       const int2 e = cross && rid[j] == n_runs - 1 ? s_cross : res[first[k]];
@@ -953,9 +977,10 @@ __device__ __forceinline__ int round_lookup(const QueryView& q, const IndexView&
   uint32_t fw[P], fm[P];
 #pragma unroll
   for (int i = 0; i < P; ++i) {
-    const uint64_t h = key_hash(code[i]);
-    fm[i] = filter_mask(h);
-    fw[i] = ((vmask >> i) & 1u) ? __ldg(ix.filter + filter_word(h, ix.fshift)) : 0u;
+    const uint64_t key = key_of_code(code[i], ix.l), rc = key_revcomp(key, ix.l);
+    const uint64_t h = filter_hash(key < rc ? key : rc, ix.l);
+    fm[i] = filter_mask(h, key > rc);
+    fw[i] = ((vmask >> i) & 1u) ? __ldg(ix.filter + (size_t)filter_word(h, ix.fshift) * ix.fstride) : 0u;
   }
   // The home bucket (records home and home + 1, one aligned 32-byte sector)
   // in one load; only keys displaced past it probe further.
@@ -1197,287 +1222,6 @@ __global__ void __launch_bounds__(kSeedFusedThreads, SMALL ? 16 : 12) k_seed_fus
   if (lane == 0) nvalid[s] = valid;
 }
 
-// ------------------------------------------------------------------------
-// Seeding of several target windows in one pass over the query
-// ------------------------------------------------------------------------
-// One warp per strand as in k_seed_fused, but every round's l-mers are looked
-// up in NW target windows at once: the 2-bit words and N flags are read once
-// for all windows, the NW filter words of every l-mer are loaded together, and
-// the l-mers that pass a filter are listed in the warp's shared memory (code,
-// window, l-mer) so that the 32 lanes share the bucket reads evenly (about one
-// per lane and window in a round of 160 l-mers) instead of each lane reading
-// the buckets of its own l-mers.  Payloads land in shared memory, one slot per
-// (window, l-mer); the emission of each window's seeds is round_emit's.
-// A strand reserves its range in every window with one atomic per window,
-// issued by lanes 0..NW-1 together.
-template <int NW>
-struct SeedSmem {
-  uint64_t pl[NW][kSeedRound];  // payload of (window, l-mer) of the current round
-  union {
-    struct {
-      uint64_t code[NW * kSeedRound];
-      uint16_t tag[NW * kSeedRound];  // window << 8 | l-mer within the round
-    } list;                           // the l-mers that passed a window's filter
-    struct {
-      uint64_t pl[kSeedRound];
-      int32_t qi[kSeedRound];
-    } stage;  // round_emit's staging
-  } u;
-};
-
-// Payload of the key of code c in the table of one window (home bucket in one
-// 32-byte read, then linear probing).
-template <bool SMALL>
-__device__ __forceinline__ uint64_t bucket_payload(const IndexView& ix, uint64_t c) {
-  const int64_t home = SMALL ? record_home16((uint32_t)c, ix.l, ix.nbuckets) : record_home(c, ix.l, ix.nbuckets);
-  uint64_t c0, p0, c1, p1;
-  ld_bucket(ix.table + home, c0, p0, c1, p1);
-  if (c0 == c || p0 == kNoPayload) return p0;
-  if (c1 == c || p1 == kNoPayload) return p1;
-  return table_probe(ix, c, home + 2);
-}
-
-// Looks up the l-mers r0 + lane * P + i (i < P) of a strand in the NW windows.
-// When `keep`, their payloads go to sm.pl (kNoPayload for invalid or absent
-// l-mers); cnt[w] adds the entries of the l-mers this lane resolved in window
-// w.  Returns the number of valid l-mers of this lane.
-template <bool SMALL, int NW>
-__device__ __forceinline__ int round_lookup_multi(const QueryView& q, const SeedWins& W, int64_t st, int nk, int r0,
-                                                  int lane, SeedSmem<NW>& sm, bool keep, int (&cnt)[NW]) {
-  constexpr int P = kSeedPerLane;
-  const int l = W.w[0].ix.l;
-  const int q0 = r0 + lane * P;
-  const int nv = max(0, min(P, nk - q0));
-  uint64_t code[P];
-  uint32_t vmask = 0;
-#pragma unroll
-  for (int i = 0; i < P; ++i) code[i] = 0;
-  if (nv > 0) {
-    const int64_t f = st + q0;
-    vmask = (1u << nv) - 1;
-    if (SMALL) {
-      const uint32_t* p32 = reinterpret_cast<const uint32_t*>(q.packed);
-      const uint32_t* n32 = reinterpret_cast<const uint32_t*>(q.nmask);
-      const int64_t j0 = f >> 4, k0 = f >> 5;
-      const uint32_t u0 = __ldcs(p32 + (j0 ^ 1)), u1 = __ldcs(p32 + ((j0 + 1) ^ 1)),
-                     u2 = __ldcs(p32 + ((j0 + 2) ^ 1));
-      const uint32_t m0 = __ldcs(n32 + (k0 ^ 1)), m1 = __ldcs(n32 + ((k0 + 1) ^ 1));
-      const uint32_t nflag = __funnelshift_l(m1, m0, (int)(f & 31));
-      const int o = 2 * (int)(f & 15);
-      const uint32_t mask = (2 * l == 32) ? ~0u : ((1u << (2 * l)) - 1);
-#pragma unroll
-      for (int i = 0; i < P; ++i) {
-        const int bo = o + 2 * i;
-        const uint32_t x = bo < 32 ? __funnelshift_l(u1, u0, bo) : __funnelshift_l(u2, u1, bo - 32);
-        const uint32_t key = x >> (32 - 2 * l);
-        code[i] = (uint32_t)(key * (uint32_t)0x6659FD93u) & mask;  // order_code for l <= 16
-        if ((nflag << i) >> (32 - l)) vmask &= ~(1u << i);
-      }
-    } else {
-      const int64_t w0 = f >> 5, k0 = f >> 6;
-      const uint64_t u0 = ld_stream(q.packed + w0), u1 = ld_stream(q.packed + w0 + 1),
-                     u2 = ld_stream(q.packed + w0 + 2);
-      const uint64_t nflag = funnel64(ld_stream(q.nmask + k0), ld_stream(q.nmask + k0 + 1), (int)(f & 63));
-      const int o = 2 * (int)(f & 31);
-#pragma unroll
-      for (int i = 0; i < P; ++i) {
-        const int bo = o + 2 * i;
-        const uint64_t x = bo < 64 ? funnel64(u0, u1, bo) : funnel64(u1, u2, bo - 64);
-        code[i] = order_code(x >> (64 - 2 * l), l);
-        if ((nflag << i) >> (64 - l)) vmask &= ~(1u << i);
-      }
-    }
-  }
-  // the filter words of every window, all in flight together
-  uint32_t pass = 0;  // bit w * P + i
-  {
-    uint32_t fm[P], fw[NW][P];
-#pragma unroll
-    for (int i = 0; i < P; ++i) {
-      const uint64_t h = key_hash(code[i]);
-      fm[i] = filter_mask(h);
-#pragma unroll
-      for (int w = 0; w < NW; ++w)
-        fw[w][i] = ((vmask >> i) & 1u) ? __ldg(W.w[w].ix.filter + filter_word(h, W.w[w].ix.fshift)) : 0u;
-    }
-#pragma unroll
-    for (int w = 0; w < NW; ++w)
-#pragma unroll
-      for (int i = 0; i < P; ++i)
-        if (((vmask >> i) & 1u) && (fw[w][i] & fm[i]) == fm[i]) pass |= 1u << (w * P + i);
-  }
-  if (keep) {
-#pragma unroll
-    for (int w = 0; w < NW; ++w)
-#pragma unroll
-      for (int i = 0; i < P; ++i) sm.pl[w][lane * P + i] = kNoPayload;
-  }
-  int total;
-  int k = warp_excl_scan(__popc(pass), lane, &total);
-#pragma unroll
-  for (int w = 0; w < NW; ++w)
-#pragma unroll
-    for (int i = 0; i < P; ++i)
-      if ((pass >> (w * P + i)) & 1u) {
-        sm.u.list.code[k] = code[i];
-        sm.u.list.tag[k] = (uint16_t)((w << 8) | (lane * P + i));
-        ++k;
-      }
-  __syncwarp();
-  // the bucket reads, shared by the lanes: two in flight per lane
-  for (int j = lane; j < total; j += 64) {
-    const bool two = j + 32 < total;
-    const uint64_t ca = sm.u.list.code[j];
-    const int ta = sm.u.list.tag[j];
-    const uint64_t cb = two ? sm.u.list.code[j + 32] : 0ull;
-    const int tb = two ? sm.u.list.tag[j + 32] : 0;
-    const int wa = ta >> 8, wb = tb >> 8;
-    const IndexView& ia = W.w[wa].ix;
-    const int64_t ha = SMALL ? record_home16((uint32_t)ca, l, ia.nbuckets) : record_home(ca, l, ia.nbuckets);
-    uint64_t a0, a1, a2, a3, b0 = 0, b1 = kNoPayload, b2 = 0, b3 = kNoPayload;
-    ld_bucket(ia.table + ha, a0, a1, a2, a3);
-    int64_t hb = 0;
-    if (two) {
-      const IndexView& ib = W.w[wb].ix;
-      hb = SMALL ? record_home16((uint32_t)cb, l, ib.nbuckets) : record_home(cb, l, ib.nbuckets);
-      ld_bucket(ib.table + hb, b0, b1, b2, b3);
-    }
-    uint64_t pa;
-    if (a0 == ca || a1 == kNoPayload) pa = a1;
-    else if (a2 == ca || a3 == kNoPayload) pa = a3;
-    else pa = table_probe(ia, ca, ha + 2);
-    if (keep) sm.pl[wa][ta & 0xff] = pa;
-    const int na = payload_count(pa);
-#pragma unroll
-    for (int w = 0; w < NW; ++w) cnt[w] += (w == wa) ? na : 0;
-    if (two) {
-      uint64_t pb;
-      if (b0 == cb || b1 == kNoPayload) pb = b1;
-      else if (b2 == cb || b3 == kNoPayload) pb = b3;
-      else pb = table_probe(W.w[wb].ix, cb, hb + 2);
-      if (keep) sm.pl[wb][tb & 0xff] = pb;
-      const int nb = payload_count(pb);
-#pragma unroll
-      for (int w = 0; w < NW; ++w) cnt[w] += (w == wb) ? nb : 0;
-    }
-  }
-  __syncwarp();
-  return __popc(vmask);
-}
-
-template <bool SMALL, int NW>
-__global__ void __launch_bounds__(kSeedFusedThreads, NW <= 2 ? 16 : 8) k_seed_multi(QueryView q, SeedWins W, int gap,
-                                                                                    int local) {
-  constexpr int P = kSeedPerLane;
-  __shared__ SeedSmem<NW> smem[kSeedFusedThreads / 32];
-  const int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int wib = threadIdx.x >> 5;
-  if (s >= q.nstrands) return;
-  SeedSmem<NW>& sm = smem[wib];
-  const int64_t st = q.start[s];
-  const int qlen = q.len[s];
-  const int nk = qlen - W.w[0].ix.l + 1;
-  // L2 prefetch for the block kSeedPrefetchBlocks later (as in k_seed_fused);
-  // every address stays inside its array
-  if (wib == 0 && lane < 5) {
-    const int64_t sp = ((int64_t)blockIdx.x + kSeedPrefetchBlocks) * (kSeedFusedThreads / 32);
-    if (sp < q.nstrands && q.n > 0) {
-      const int64_t f = min(q.n - 1, st + (sp - s) * (q.n / q.nstrands));
-      const void* a = lane == 0 ? (const void*)(q.start + sp)
-                    : lane == 1 ? (const void*)(q.len + sp)
-                    : lane == 4 ? (const void*)(q.nmask + (f >> 6))
-                                : (const void*)(q.packed + min((f >> 5) + 16 * (lane - 2), q.n / 32 + 3));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
-    }
-  }
-  // pass 1: counts of every window; round 0's payloads stay in shared memory
-  int cnt[NW];
-#pragma unroll
-  for (int w = 0; w < NW; ++w) cnt[w] = 0;
-  int valid_kmers = 0;
-  if (nk > 0) {
-    for (int r0 = 0; r0 < nk; r0 += kSeedRound)
-      valid_kmers += round_lookup_multi<SMALL, NW>(q, W, st, nk, r0, lane, sm, r0 == 0, cnt);
-  }
-  valid_kmers = (int)__reduce_add_sync(kFull, (unsigned)valid_kmers);
-  int tot[NW];
-#pragma unroll
-  for (int w = 0; w < NW; ++w) tot[w] = (int)__reduce_add_sync(kFull, (unsigned)cnt[w]);
-  const int part = (int)(s % kSeedParts);
-  const int64_t v0 = (s >> 1) * (2 * NW) + (s & 1);  // see strand_slot
-  // the range reservations: lane w reserves window w's
-  unsigned long long rel = 0;
-  if (lane < NW) {
-    int my = 0;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) my = (w == lane) ? tot[w] : my;
-    const SeedWin& sw = W.w[lane];
-    if (valid_kmers) atomicAdd(sw.n_kmers + part, (unsigned long long)valid_kmers);
-    rel = my ? atomicAdd(&sw.cursor[part], (unsigned long long)my) : 0ull;
-  }
-  int64_t wpos[NW];
-  bool ok[NW];
-  bool any = false;
-#pragma unroll
-  for (int w = 0; w < NW; ++w) {
-    const unsigned long long r = __shfl_sync(kFull, rel, w);
-    const int64_t base = (int64_t)(w * kSeedParts + part) * W.part_cap + (int64_t)r;
-    wpos[w] = base;
-    ok[w] = tot[w] > 0 && base + tot[w] <= (int64_t)(w * kSeedParts + part + 1) * W.part_cap;
-    any |= ok[w];
-    if (lane == 0) {
-      W.off[v0 + 2 * w] = base;
-      W.cnt[v0 + 2 * w] = tot[w];
-      if (!ok[w]) W.nvalid[v0 + 2 * w] = 0;
-    }
-  }
-  if (!any) return;
-  // pass 2: the seeds of every window, round by round
-  int valid[NW];
-  int dummy[NW];
-#pragma unroll
-  for (int w = 0; w < NW; ++w) valid[w] = dummy[w] = 0;
-  for (int r0 = 0; r0 < nk; r0 += kSeedRound) {
-    if (r0 > 0) round_lookup_multi<SMALL, NW>(q, W, st, nk, r0, lane, sm, true, dummy);
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      if (!ok[w]) continue;
-      uint64_t pl[P];
-#pragma unroll
-      for (int i = 0; i < P; ++i) pl[i] = sm.pl[w][lane * P + i];
-      round_emit(W.w[w].ix, W.w[w].t, gap, local, qlen, r0, lane, pl, wpos[w], valid[w], W.skey, W.sq,
-                 sm.u.stage.pl, sm.u.stage.qi);
-    }
-  }
-#pragma unroll
-  for (int w = 0; w < NW; ++w) {
-    const int v = (int)__reduce_add_sync(kFull, (unsigned)valid[w]);
-    if (lane == 0 && ok[w]) W.nvalid[v0 + 2 * w] = v;
-  }
-}
-
-// The first strand of every (target window, query window) with a valid seed:
-// its seed count is stored complemented (the isolate filter keeps the first
-// seed of a query window).
-__global__ void k_window_first(int32_t* __restrict__ nvalid, const int32_t* __restrict__ wstart, int nwin, int nw) {
-  const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (i >= nwin * nw) return;
-  const int w = i / nwin, qw = i % nwin;
-  const int a = wstart[qw], b = wstart[qw + 1];
-  for (int c = a; c < b; c += 32) {
-    const int s = c + lane;
-    const int64_t v = strand_slot(s, w, nw);
-    const int n = s < b ? nvalid[v] : 0;
-    const unsigned m = __ballot_sync(kFull, n > 0);
-    if (m) {
-      if (lane == __ffs(m) - 1) nvalid[v] = ~n;
-      return;
-    }
-  }
-}
-
 // ---- sorting networks (ascending compare-exchange, safe with a ragged tail) ----
 template <class K2>
 __device__ __forceinline__ bool less2(uint64_t a1, K2 a2, uint64_t b1, K2 b2) {
@@ -1540,6 +1284,711 @@ __device__ __forceinline__ bool near_pred(int tid, int tidx, int diag, int ptid,
   return tid == ptid && width >= tidx - ptidx && width >= ptidx - tidx && gap >= pdiag - diag;
 }
 
+
+constexpr int kWarpSmemCap = 256;
+
+// ------------------------------------------------------------------------
+// Seeding of whole reads in a group of target windows
+// ------------------------------------------------------------------------
+// One warp per read looks the l-mers of both its strands up in all NW windows:
+// the l-mer at position i of the '+' strand and its reverse complement, at
+// position len - l - i of the '-' strand, come from the same words of the '+'
+// strand and share their filter word, and the words of two windows lie side by
+// side, so one 8-byte load answers four look-ups.  The (l-mer, strand, window)
+// that pass a filter are listed in the warp's shared memory, and the lanes
+// share the bucket reads, two in flight each.  Seeds gather by slot (strand,
+// window) in shared memory; with at most kSlotSeeds per slot, which most reads
+// stay under, the warp sorts and filters them there (four slots of up to eight
+// seeds at once), so that only the hits reach memory.  A read of more than
+// kFastRounds rounds of kSeedRound l-mers, or with a fuller slot, is left to
+// k_seed_reads_long, which writes its seeds for the tiers of the seed filter.
+//
+// Bound by issue (0.66 per cycle and scheduler, some 1,900 warp instructions per
+// read of 150 bp) with the latency of the filter and bucket reads.  One warp per
+// strand with a load per strand, l-mer and window, and every seed through
+// memory into the filters, took on a million reads against two windows 4.17 ms
+// for the seeds and 1.00 ms for the filters, against 3.05 and 0.46 ms now; on
+// 10,000 reads of 100 - 5,000 bp 0.85 against 0.56 ms, on 300 bp reads 0.50
+// against 0.36 ms.  (The same with the long reads in this kernel ran out of the
+// instruction cache: 5.45 ms.)
+constexpr int kSlotSeeds = 32;
+constexpr int kFastRounds = 3;  // reads of up to 480 l-mers may stay in shared memory
+
+template <bool SMALL>
+struct SeedKey {
+  typedef uint64_t K;
+};
+template <>
+struct SeedKey<true> {
+  typedef uint32_t K;
+};
+
+template <bool SMALL, int NW>
+struct ListSmem {
+  static constexpr int kList = 2 * NW * kSeedRound;
+  typename SeedKey<SMALL>::K code[kList];
+  uint16_t tag[kList];  // l-mer within the round << 3 | slot
+};
+
+// Keys of the lane's l-mers q0 .. q0 + P - 1 (from strand position st + q0) and
+// of their reverse complements; bit i of the result: l-mer i has bases A/C/G/T
+// only.
+template <bool SMALL>
+__device__ __forceinline__ uint32_t lane_keys(const QueryView& q, int64_t f, int nv, int l,
+                                              typename SeedKey<SMALL>::K (&kf)[kSeedPerLane],
+                                              typename SeedKey<SMALL>::K (&kr)[kSeedPerLane]) {
+  constexpr int P = kSeedPerLane;
+  uint32_t vmask = (1u << nv) - 1;
+  if constexpr (SMALL) {
+    // 16-base units j0 .. j0 + 2 of the codes, 32-base units k0, k0 + 1 of
+    // the flags (unit j = 32-bit element j ^ 1)
+    const uint32_t* p32 = reinterpret_cast<const uint32_t*>(q.packed);
+    const uint32_t* n32 = reinterpret_cast<const uint32_t*>(q.nmask);
+    const int64_t j0 = f >> 4, k0 = f >> 5;
+    const uint32_t u0 = __ldcs(p32 + (j0 ^ 1)), u1 = __ldcs(p32 + ((j0 + 1) ^ 1)), u2 = __ldcs(p32 + ((j0 + 2) ^ 1));
+    const uint32_t m0 = __ldcs(n32 + (k0 ^ 1)), m1 = __ldcs(n32 + ((k0 + 1) ^ 1));
+    const uint32_t nflag = __funnelshift_l(m1, m0, (int)(f & 31));  // base f in the top bit
+    const int o = 2 * (int)(f & 15);
+    const uint32_t mask = l == 16 ? ~0u : (1u << (2 * l)) - 1;
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      const int bo = o + 2 * i;
+      const uint32_t x = bo < 32 ? __funnelshift_l(u1, u0, bo) : __funnelshift_l(u2, u1, bo - 32);
+      const uint32_t y = __brev(~x);
+      kf[i] = x >> (32 - 2 * l);
+      kr[i] = (((y >> 1) & 0x55555555u) | ((y & 0x55555555u) << 1)) & mask;
+      if ((nflag << i) >> (32 - l)) vmask &= ~(1u << i);
+    }
+  } else {
+    // 32-base words w0 .. w0 + 2 of the codes, 64-base words k0, k0 + 1 of the flags
+    const int64_t w0 = f >> 5, k0 = f >> 6;
+    const uint64_t u0 = ld_stream(q.packed + w0), u1 = ld_stream(q.packed + w0 + 1), u2 = ld_stream(q.packed + w0 + 2);
+    const uint64_t nflag = funnel64(ld_stream(q.nmask + k0), ld_stream(q.nmask + k0 + 1), (int)(f & 63));
+    const int o = 2 * (int)(f & 31);
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      const int bo = o + 2 * i;  // < 2 * (31 + P)
+      const uint64_t x = bo < 64 ? funnel64(u0, u1, bo) : funnel64(u1, u2, bo - 64);
+      kf[i] = x >> (64 - 2 * l);
+      kr[i] = key_revcomp(kf[i], l);
+      if ((nflag << i) >> (64 - l)) vmask &= ~(1u << i);
+    }
+  }
+  return vmask;
+}
+
+// Lists the (l-mer, slot) of a round that pass the windows' filters, in l-mer
+// order; returns their number.  *valid is raised by the lane's valid l-mers.
+template <bool SMALL, int NW>
+__device__ __forceinline__ int round_list(const QueryView& q, const SeedWins& W, int64_t st, int nk, int r0, int lane,
+                                          ListSmem<SMALL, NW>& sm, int& valid) {
+  typedef typename SeedKey<SMALL>::K K;
+  constexpr int P = kSeedPerLane, NS = 2 * NW;
+  const int l = W.w[0].ix.l;
+  const int q0 = r0 + lane * P;
+  const int nv = max(0, min(P, nk - q0));
+  K kf[P], kr[P];
+  uint32_t vmask = 0;
+#pragma unroll
+  for (int i = 0; i < P; ++i) kf[i] = kr[i] = 0;
+  if (nv > 0) vmask = lane_keys<SMALL>(q, st + q0, nv, l, kf, kr);
+  valid += __popc(vmask);
+  // the filter words of every window, all in flight together
+  uint32_t fw[P][NW], low[P];
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    const K smaller = kf[i] < kr[i] ? kf[i] : kr[i];
+    const uint64_t h = SMALL ? filter_hash16((uint32_t)smaller) : filter_hash((uint64_t)smaller, l);
+    low[i] = (uint32_t)h;
+    const bool on = (vmask >> i) & 1u;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) fw[i][w] = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      const IndexView& ix = W.w[w].ix;
+      if (w % 2 == 1 && W.w[w].paired) continue;
+      const uint32_t* a = ix.filter + (size_t)filter_word(h, ix.fshift) * ix.fstride;
+      if (w + 1 < NW && W.w[w + 1 < NW ? w + 1 : w].paired) {
+        if (on) {
+          const uint2 x = __ldg(reinterpret_cast<const uint2*>(a));
+          fw[i][w] = x.x;
+          fw[i][w + 1 < NW ? w + 1 : w] = x.y;
+        }
+      } else if (on) {
+        fw[i][w] = __ldg(a);
+      }
+    }
+  }
+  typedef std::conditional_t<(P * NS <= 32), uint32_t, uint64_t> Mask;
+  Mask pass = 0;  // bit i * NS + slot
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    if (!((vmask >> i) & 1u)) continue;
+    const uint32_t ms = filter_bits3(low[i]), ml = filter_bits3(low[i] >> 15);
+    const uint32_t mf = kf[i] > kr[i] ? ml : ms, mr = kr[i] > kf[i] ? ml : ms;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      if ((fw[i][w] & mf) == mf) pass |= (Mask)1 << (i * NS + 2 * w);
+      if ((fw[i][w] & mr) == mr) pass |= (Mask)1 << (i * NS + 2 * w + 1);
+    }
+  }
+  int total;
+  int k = warp_excl_scan(__popcll(pass), lane, &total);
+  const K mult = SMALL ? (K)0x6659FD93u : (K)0xD6E8FEB86659FD93ull;  // order_code
+  const K mask = 2 * l == 8 * (int)sizeof(K) ? ~(K)0 : ((K)1 << (2 * l)) - 1;
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    uint32_t m = (uint32_t)(pass >> (i * NS)) & ((1u << NS) - 1);
+    while (m) {
+      const int x = __ffs(m) - 1;
+      m &= m - 1;
+      sm.code[k] = ((x & 1 ? kr[i] : kf[i]) * mult) & mask;
+      sm.tag[k] = (uint16_t)((lane * P + i) << 3 | x);
+      ++k;
+    }
+  }
+  __syncwarp();
+  return total;
+}
+
+// The home buckets of list entries j (kNoPayload past the list) and their tags:
+// two per lane in flight.
+template <bool SMALL, int NW>
+__device__ __forceinline__ void list_payloads(const SeedWins& W, const ListSmem<SMALL, NW>& sm, int c0, int lane,
+                                              int total, uint64_t (&pl)[2], int (&tag)[2]) {
+  const int l = W.w[0].ix.l;
+  uint64_t b0[2], b1[2], b2[2], b3[2];
+  int64_t home[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int j = c0 + 32 * u + lane;
+    const bool in = j < total;
+    tag[u] = in ? sm.tag[j] : 0;
+    b0[u] = b2[u] = 0;
+    b1[u] = b3[u] = kNoPayload;
+    home[u] = 0;
+    if (in) {
+      const IndexView& ix = W.w[(tag[u] & 7) >> 1].ix;
+      home[u] = SMALL ? record_home16((uint32_t)sm.code[j], l, ix.nbuckets) : record_home(sm.code[j], l, ix.nbuckets);
+      ld_bucket(ix.table + home[u], b0[u], b1[u], b2[u], b3[u]);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int j = c0 + 32 * u + lane;
+    pl[u] = kNoPayload;
+    if (j < total) {
+      const uint64_t c = sm.code[j];
+      if (b0[u] == c || b1[u] == kNoPayload) pl[u] = b1[u];
+      else if (b2[u] == c || b3[u] == kNoPayload) pl[u] = b3[u];
+      else pl[u] = table_probe(W.w[(tag[u] & 7) >> 1].ix, c, home[u] + 2);
+    }
+  }
+}
+
+// Index of the l-mer of `tag` within its strand.
+__device__ __forceinline__ int tag_qidx(int tag, int r0, int nk) {
+  const int i = r0 + (tag >> 3);
+  return tag & 1 ? nk - 1 - i : i;
+}
+// The seed of entry e of l-mer qi: its key, kDroppedSeed for is_onCorner.
+__device__ __forceinline__ uint64_t seed_key(const SeedWins& W, int slot, int2 e, int qi, int gap, int local, int qlen) {
+  const int s0 = e.y - qi;  // tHitStartIdx
+  if (!local && ((s0 + gap < 0) || (s0 + qlen - gap > W.w[slot >> 1].t.lengths[e.x]))) return kDroppedSeed;
+  return ((uint64_t)(uint32_t)e.x << 32) | ((uint32_t)s0 ^ 0x80000000u);
+}
+// Entry i of payload pl.
+__device__ __forceinline__ int2 payload_entry(const SeedWins& W, int slot, uint64_t pl, int i) {
+  if (pl & kMulti) return __ldcs(W.w[slot >> 1].ix.entries + ((int)(pl >> 32) & 0x7fffffff) + i);
+  return make_int2((int)(pl >> 32), (int)(uint32_t)pl);
+}
+// The lane whose items (the warp's, lane after lane; lane L's first is number
+// first_L) hold item t.
+__device__ __forceinline__ int item_lane(int first, int t) {
+  int src = 0;
+#pragma unroll
+  for (int step = 16; step > 0; step >>= 1)
+    if (__shfl_sync(kFull, first, src + step) <= t) src += step;
+  return src;
+}
+
+// A seed as one sortable word, (sequence, diagonal, l-mer), for sequences below
+// 2^20 and l-mers below 2^12.
+constexpr int kWordQBits = 12;
+__device__ __forceinline__ uint64_t seed_word(uint64_t key, int qi) {
+  return ((key >> 32) << (32 + kWordQBits)) | ((uint64_t)(uint32_t)key << kWordQBits) | (uint32_t)qi;
+}
+__device__ __forceinline__ int word_seq(uint64_t k) { return (int)(k >> (32 + kWordQBits)); }
+__device__ __forceinline__ uint32_t word_diag(uint64_t k) { return (uint32_t)(k >> kWordQBits); }
+__device__ __forceinline__ int word_q(uint64_t k) { return (int)(k & ((1u << kWordQBits) - 1)); }
+__device__ __forceinline__ uint64_t word_key(uint64_t k) { return ((uint64_t)word_seq(k) << 32) | word_diag(k); }
+
+// One slot's seed words, one per lane of a group of G lanes (a power of two; n
+// of them, the j-th in lane j): sorts them and applies the isolate and
+// duplicate filters as filter_chunk does, the slot not being its query window's
+// first.  Returns whether this lane's seed is a hit; near = whether the group's
+// first seed that survives the isolate filter is near the slot's first seed
+// (k_window_first).
+__device__ __forceinline__ bool slot_filter(uint64_t& k, int n, int G, unsigned group, int width, int gap, bool& near) {
+  const int lane = threadIdx.x & 31, j = lane & (G - 1);
+  const uint64_t n1 = __shfl_down_sync(kFull, k, 1);
+  if (__any_sync(kFull, j + 1 < n && n1 < k)) {
+#pragma unroll 1
+    for (int size = 2; size <= G; size <<= 1)
+#pragma unroll 1
+      for (int m = size - 1; m > 0; m = m == size - 1 ? size >> 2 : m >> 1) {
+        const uint64_t o = __shfl_xor_sync(kFull, k, m);
+        if ((lane & m) < ((lane ^ m) & m) ? o < k : o > k) k = o;
+      }
+  }
+  const int tid = word_seq(k), diag = (int)(word_diag(k) ^ 0x80000000u), tidx = diag + word_q(k);
+  const int ptid = __shfl_up_sync(kFull, tid, 1), ptidx = __shfl_up_sync(kFull, tidx, 1);
+  const int pdiag = __shfl_up_sync(kFull, diag, 1);
+  const bool keep8 = j > 0 && j < n && near_pred(tid, tidx, diag, ptid, ptidx, pdiag, width, gap);
+  const unsigned kept = __ballot_sync(kFull, keep8);
+  near = false;
+  if (kept == 0) return false;
+  const unsigned below = kept & group & lanemask_lt();
+  // the previous survivor, or for the first one the slot's first seed
+  const int src = below ? 31 - __clz(below) : lane & ~(G - 1);
+  const int stid = __shfl_sync(kFull, tid, src), stidx = __shfl_sync(kFull, tidx, src);
+  const int sdiag = __shfl_sync(kFull, diag, src);
+  const bool dup = keep8 && near_pred(tid, tidx, diag, stid, stidx, sdiag, width, gap);
+  near = (__ballot_sync(kFull, dup && !below) & group) != 0;
+  return keep8 && !(dup && below);
+}
+
+template <bool SMALL, int NW>
+struct ReadSmem {
+  uint64_t word[2 * NW][kSlotSeeds];  // valid seeds per slot, then hits
+  int n[2 * NW];                      // their counts
+  ListSmem<SMALL, NW> list;
+};
+
+template <bool SMALL, int NW>
+__global__ void __launch_bounds__(kSeedFusedThreads, NW <= 2 ? 18 : 8) k_seed_reads(QueryView q, SeedWins W, int width,
+                                                                                  int gap, int local) {
+  constexpr int NS = 2 * NW;                           // the read's slots
+  constexpr int kG = NW == 1 ? 16 : NW == 2 ? 8 : 4;   // lanes per slot when all are filtered at once
+  __shared__ ReadSmem<SMALL, NW> smem[kSeedFusedThreads / 32];
+  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int64_t n_reads = q.nstrands / 2;
+  if (r >= n_reads) return;
+  ReadSmem<SMALL, NW>& sm = smem[wib];
+  const int64_t st = q.start[2 * r];
+  const int qlen = q.len[2 * r];
+  const int nk = qlen - W.w[0].ix.l + 1;
+  const int64_t v0 = r * NS;
+  const unsigned lt = lanemask_lt();
+  // L2 prefetch for the block kSeedPrefetchBlocks later: its strand table
+  // entries and, estimated from this read's start and the mean strand length,
+  // its 2-bit words and N flags.  Every address stays inside its array.
+  if (wib == 0 && lane < 4) {
+    const int64_t rp = ((int64_t)blockIdx.x + kSeedPrefetchBlocks) * (kSeedFusedThreads / 32);
+    if (rp < n_reads && q.n > 0) {
+      const int64_t f = min(q.n - 1, st + (rp - r) * 2 * (q.n / q.nstrands));
+      const void* a = lane == 0 ? (const void*)(q.start + 2 * rp)
+                    : lane == 1 ? (const void*)(q.len + 2 * rp)
+                    : lane == 2 ? (const void*)(q.nmask + (f >> 6))
+                                : (const void*)(q.packed + min(f >> 5, q.n / 32 + 3));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
+    }
+  }
+  if (nk <= 0) {
+    if (lane < NS) W.nvalid[v0 + lane] = W.cnt[v0 + lane] = W.hcnt[v0 + lane] = 0;
+    return;
+  }
+  bool fast = nk <= kFastRounds * kSeedRound && W.words;
+  int valid_kmers = 0;
+  int seeds[NW];  // entries found per window, the ones on a corner among them
+#pragma unroll
+  for (int w = 0; w < NW; ++w) seeds[w] = 0;
+  if (lane < NS) sm.n[lane] = 0;
+#pragma unroll 1
+  for (int r0 = 0; r0 < nk && fast; r0 += kSeedRound) {
+    __syncwarp();
+    const int total = round_list<SMALL, NW>(q, W, st, nk, r0, lane, sm.list, valid_kmers);
+#pragma unroll 1
+    for (int c0 = 0; c0 < total && fast; c0 += 64) {
+      uint64_t pl2[2];
+      int tag2[2];
+      list_payloads(W, sm.list, c0, lane, total, pl2, tag2);
+#pragma unroll 1
+      for (int u = 0; u < 2; ++u) {
+        const uint64_t pl = u ? pl2[1] : pl2[0];
+        const int tag = u ? tag2[1] : tag2[0];
+        const int c = payload_count(pl);
+        const unsigned found = __ballot_sync(kFull, c > 0);
+        if (!found) continue;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) seeds[w] += ((tag & 7) >> 1) == w ? c : 0;
+        const unsigned multi = __ballot_sync(kFull, c > 1);
+        int all, first = 0;
+        if (multi) {
+          first = warp_excl_scan(c, lane, &all);
+          if (all > NS * kSlotSeeds) {  // too many for the slots
+            fast = false;
+            break;
+          }
+        } else {
+          all = 32;  // an entry per lane, as they lie
+        }
+#pragma unroll 1
+        for (int t0 = 0; t0 < all; t0 += 32) {
+          int tg = tag, i = 0;
+          uint64_t p = pl;
+          bool in = c > 0;
+          if (multi) {
+            const int t = t0 + lane, src = item_lane(first, t);
+            in = t < all;
+            p = __shfl_sync(kFull, pl, src);
+            tg = __shfl_sync(kFull, tag, src);
+            i = t - __shfl_sync(kFull, first, src);
+          }
+          const int slot = tg & 7, qi = tag_qidx(tg, r0, nk);
+          uint64_t key = kDroppedSeed;
+          if (in) key = seed_key(W, slot, payload_entry(W, slot, p, i), qi, gap, local, qlen);
+          const bool ok = key != kDroppedSeed;
+          const unsigned peers = __match_any_sync(kFull, ok ? slot : 8);
+          const int leader = __ffs(peers) - 1;
+          int at = 0;
+          if (ok && lane == leader) at = atomicAdd(&sm.n[slot], __popc(peers));
+          at = __shfl_sync(kFull, at, leader) + __popc(peers & lt);
+          if (ok && at < kSlotSeeds) sm.word[slot][at] = seed_word(key, qi);
+        }
+      }
+      __syncwarp();
+      if (__any_sync(kFull, sm.n[lane < NS ? lane : 0] > kSlotSeeds)) fast = false;
+    }
+  }
+  if (!fast) {  // k_seed_reads_long's: reads of one round from the list's start, longer ones from its end
+    if (lane == 0) {
+      if (nk <= kSeedRound) W.long_reads[atomicAdd(W.n_long, 1)] = (uint32_t)r;
+      else W.long_reads[n_reads - 1 - atomicAdd(W.n_long + 1, 1)] = (uint32_t)r;
+    }
+    return;
+  }
+  const int part = (int)(r % kSeedParts);
+  const int64_t cap = W.part_cap * NW;  // the group's windows share a partition
+  valid_kmers = (int)__reduce_add_sync(kFull, (unsigned)valid_kmers);
+#pragma unroll
+  for (int w = 0; w < NW; ++w) {
+    const int n = (int)__reduce_add_sync(kFull, (unsigned)seeds[w]);
+    if (lane == w) {
+      if (valid_kmers) atomicAdd(W.w[w].n_kmers + part, 2ull * (unsigned long long)valid_kmers);
+      if (n) atomicAdd(W.w[w].n_seeds + part, (unsigned long long)n);
+    }
+  }
+  const int n_slot = lane < NS ? sm.n[lane < NS ? lane : 0] : 0;  // lane x < NS: valid seeds of slot x
+  if (lane < NS) {
+    W.nvalid[v0 + lane] = n_slot;
+    W.cnt[v0 + lane] = 0;  // nothing left to filter
+  }
+  if (!__any_sync(kFull, n_slot > 0)) {
+    if (lane < NS) W.hcnt[v0 + lane] = 0;
+    return;
+  }
+  // every slot of up to kG seeds at once, a group of lanes each; then each fuller one with the whole warp
+  unsigned todo = __ballot_sync(kFull, n_slot > kG);
+  int h_slot = 0;  // lane x < NS: hits of slot x
+  int x = lane / kG, G = kG;
+  unsigned group = ((1u << kG) - 1) << (lane & ~(kG - 1));
+  int n = __shfl_sync(kFull, n_slot, x < NS ? x : 0);
+  if (x >= NS || n > kG) n = 0;
+#pragma unroll 1
+  for (bool groups = true;; groups = false) {
+    if (!groups) {
+      if (!todo) break;
+      x = __ffs(todo) - 1;
+      todo &= todo - 1;
+      G = 32;
+      group = kFull;
+      n = __shfl_sync(kFull, n_slot, x);
+    }
+    const int j = lane & (G - 1);
+    uint64_t k = j < n ? sm.word[x][j] : ~0ull;
+    bool near;
+    const bool hit = slot_filter(k, n, G, group, width, gap, near);
+    if (j == 0 && n > 0) {  // the slot's hit if it is its query window's first
+      W.first_key[v0 + x] = word_key(k);
+      W.first_q[v0 + x] = (uint32_t)word_q(k) | (near ? 0x80000000u : 0u);
+    }
+    const unsigned m = __ballot_sync(kFull, hit);
+    if (hit) sm.word[x][__popc(m & group & lt)] = k;  // the slot's hits, in order, wait for their place
+    if (groups) {
+      if (lane < NS) h_slot = __popc(m & (((1u << kG) - 1) << (lane * kG)));
+    } else if (lane == x) {
+      h_slot = __popc(m);
+    }
+    __syncwarp();
+  }
+  int all;
+  const int before = warp_excl_scan(h_slot, lane, &all);
+  unsigned long long rel = 0;
+  if (all > 0) {
+    if (lane == 0) rel = atomicAdd(W.cursor + part, (unsigned long long)all);
+    rel = __shfl_sync(kFull, rel, 0);
+    if ((int64_t)rel + all > cap) {  // the partition is full: the search runs again with larger ones
+      if (lane < NS) W.hcnt[v0 + lane] = W.nvalid[v0 + lane] = 0;
+      return;
+    }
+  }
+  const int64_t base = part * cap + (int64_t)rel;
+  if (lane < NS) {
+    W.off[v0 + lane] = base + before;
+    W.hcnt[v0 + lane] = h_slot;
+  }
+  for (unsigned m = __ballot_sync(kFull, h_slot > 0); m; m &= m - 1) {
+    const int y = __ffs(m) - 1;
+    const int ny = __shfl_sync(kFull, h_slot, y), by = __shfl_sync(kFull, before, y);
+    if (lane < ny) {
+      const uint64_t k = sm.word[y][lane];
+      W.skey[base + by + lane] = word_key(k);
+      W.sq[base + by + lane] = (uint32_t)word_q(k);
+    }
+  }
+}
+
+// The reads k_seed_reads leaves: their seeds go to memory.  Counts of every
+// slot, then a range for the read, then the seeds, the entries of a chunk of
+// l-mers shared by the lanes.  TEAM warps take a read, the rounds of it in
+// equal runs: one for reads of one round, which keep their payloads in shared
+// memory in between, a block of four (two for three or four windows) for longer ones, which are looked up
+// again.  Teams take reads from a counter, as they finish.  The '-' strand's
+// l-mers come from its end to its start, so its slots are filled from their
+// end: all slots are in l-mer order.
+template <bool SMALL, int NW, int TEAM>
+struct LongSmem {
+  ListSmem<SMALL, NW> list;
+  uint64_t pl[TEAM == 1 ? ListSmem<SMALL, NW>::kList : 1];
+};
+template <int NW>
+constexpr int kLongTeam = NW <= 2 ? 4 : 2;
+template <bool SMALL, int NW, int TEAM>
+__global__ void __launch_bounds__(TEAM == 1 ? kSeedFusedThreads : 32 * TEAM)
+    k_seed_reads_long(QueryView q, SeedWins W, int gap, int local) {
+  constexpr int NS = 2 * NW;
+  constexpr int kWarps = TEAM == 1 ? kSeedFusedThreads / 32 : TEAM;
+  __shared__ LongSmem<SMALL, NW, TEAM> smem[kWarps];
+  __shared__ int team_n[TEAM][NS];    // entries per warp and slot
+  __shared__ int team_valid[NS];      // valid seeds per slot
+  __shared__ int team_kmers, team_li;
+  __shared__ unsigned long long team_rel;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  LongSmem<SMALL, NW, TEAM>& sm = smem[warp];
+  const int n_long = W.n_long[TEAM == 1 ? 0 : 1];
+  int* const next = W.n_long + (TEAM == 1 ? 2 : 3);
+  const int64_t n_reads = q.nstrands / 2;
+  for (;;) {
+    int li = 0;
+    if (TEAM == 1) {
+      if (lane == 0) li = atomicAdd(next, 1);
+      li = __shfl_sync(kFull, li, 0);
+    } else {
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        team_li = atomicAdd(next, 1);
+        team_kmers = 0;
+      }
+      if (threadIdx.x < NS) team_valid[threadIdx.x] = 0;
+      __syncthreads();
+      li = team_li;
+    }
+    if (li >= n_long) break;
+    const int64_t r = W.long_reads[TEAM == 1 ? (int64_t)li : n_reads - 1 - li];
+    const int64_t st = q.start[2 * r];
+    const int qlen = q.len[2 * r];
+    const int nk = qlen - W.w[0].ix.l + 1;
+    const int64_t v0 = r * NS;
+    const int part = (int)(r % kSeedParts);
+    const int64_t cap = W.part_cap * NW;
+    const bool one_round = TEAM == 1;
+    // this warp's rounds
+    const int rounds = (nk + kSeedRound - 1) / kSeedRound;
+    const int r_from = TEAM == 1 ? 0 : (int)((int64_t)rounds * warp / TEAM) * kSeedRound;
+    const int r_to = TEAM == 1 ? nk : (int)((int64_t)rounds * (warp + 1) / TEAM) * kSeedRound;
+    int n_all = 0;  // lane x < NS: entries of slot x
+    int valid_kmers = 0, total = 0;
+    for (int r0 = r_from; r0 < r_to; r0 += kSeedRound) {
+      total = round_list<SMALL, NW>(q, W, st, nk, r0, lane, sm.list, valid_kmers);
+#pragma unroll 1
+      for (int c0 = 0; c0 < total; c0 += 64) {
+        uint64_t pl[2];
+        int tag[2];
+        list_payloads(W, sm.list, c0, lane, total, pl, tag);
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (one_round && c0 + 32 * u + lane < total) sm.pl[c0 + 32 * u + lane] = pl[u];
+        const int ca = payload_count(pl[0]), cb = payload_count(pl[1]);
+#pragma unroll
+        for (int x = 0; x < NS; ++x) {
+          const int n = (int)__reduce_add_sync(kFull, (unsigned)(((tag[0] & 7) == x ? ca : 0) + ((tag[1] & 7) == x ? cb : 0)));
+          if (lane == x) n_all += n;
+        }
+      }
+      __syncwarp();
+    }
+    valid_kmers = (int)__reduce_add_sync(kFull, (unsigned)valid_kmers);
+    int done = 0;  // lane x < NS: entries of slot x written, or before this warp's
+    if (TEAM > 1) {
+      if (lane < NS) team_n[warp][lane] = n_all;
+      if (lane == 0) atomicAdd(&team_kmers, valid_kmers);
+      __syncthreads();
+      n_all = 0;
+      if (lane < NS)
+#pragma unroll
+        for (int w = 0; w < TEAM; ++w) {
+          if (w == warp) done = n_all;
+          n_all += team_n[w][lane];
+        }
+      valid_kmers = team_kmers;
+    }
+    int64_t all = 0, before = 0;
+#pragma unroll
+    for (int x = 0; x < NS; ++x) {
+      const int n = __shfl_sync(kFull, n_all, x);
+      if (x < lane) before += n;
+      all += n;
+    }
+    unsigned long long rel = 0;
+    if (TEAM == 1 || warp == 0) {
+      if (lane == 0 && all > 0) rel = atomicAdd(W.cursor + part, (unsigned long long)all);
+      rel = __shfl_sync(kFull, rel, 0);
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        const int n = __shfl_sync(kFull, n_all, 2 * w) + __shfl_sync(kFull, n_all, 2 * w + 1);
+        if (lane == w) {
+          if (valid_kmers) atomicAdd(W.w[w].n_kmers + part, 2ull * (unsigned long long)valid_kmers);
+          if (n) atomicAdd(W.w[w].n_seeds + part, (unsigned long long)n);
+        }
+      }
+    }
+    if (TEAM > 1) {
+      if (threadIdx.x == 0) team_rel = rel;
+      __syncthreads();
+      rel = team_rel;
+    }
+    if (all == 0 || (int64_t)rel + all > cap) {
+      if ((TEAM == 1 || warp == 0) && lane < NS) W.nvalid[v0 + lane] = W.cnt[v0 + lane] = W.hcnt[v0 + lane] = 0;
+      continue;
+    }
+    const int64_t base = part * cap + (int64_t)rel + before;  // lane x < NS: of slot x
+    int valid[NS];  // this lane's valid seeds per slot
+#pragma unroll
+    for (int x = 0; x < NS; ++x) valid[x] = 0;
+    for (int r0 = r_from; r0 < r_to; r0 += kSeedRound) {
+      int dummy = 0;
+      if (!one_round) total = round_list<SMALL, NW>(q, W, st, nk, r0, lane, sm.list, dummy);
+#pragma unroll 1
+      for (int c0 = 0; c0 < total; c0 += 64) {
+        uint64_t pl2[2];
+        int tag2[2];
+        if (one_round) {
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int j = c0 + 32 * u + lane;
+            tag2[u] = j < total ? sm.list.tag[j] : 0;
+            pl2[u] = j < total ? sm.pl[j] : kNoPayload;
+          }
+        } else {
+          list_payloads(W, sm.list, c0, lane, total, pl2, tag2);
+        }
+#pragma unroll 1
+        for (int u = 0; u < 2; ++u) {
+          const uint64_t pl = u ? pl2[1] : pl2[0];
+          const int tag = u ? tag2[1] : tag2[0];
+          const int c = payload_count(pl);
+          // this lane's first entry among its slot's, and among the chunk's
+          int64_t at = 0;
+          int first = 0, chunk = 0;
+#pragma unroll
+          for (int x = 0; x < NS; ++x) {
+            int n;
+            const int mine = warp_excl_scan((tag & 7) == x ? c : 0, lane, &n);
+            const int d = __shfl_sync(kFull, done, x), size = __shfl_sync(kFull, n_all, x);
+            const int64_t b = __shfl_sync(kFull, base, x);
+            if ((tag & 7) == x) at = x & 1 ? b + size - (d + mine) - c : b + d + mine;
+            if (lane == x) done += n;
+            chunk += n;
+          }
+          int sum;
+          first = warp_excl_scan(c, lane, &sum);
+#pragma unroll 1
+          for (int t0 = 0; t0 < chunk; t0 += 32) {
+            const int t = t0 + lane, src = item_lane(first, t);
+            const uint64_t p = __shfl_sync(kFull, pl, src);
+            const int tg = __shfl_sync(kFull, tag, src), i = t - __shfl_sync(kFull, first, src);
+            const int64_t to = __shfl_sync(kFull, at, src) + i;
+            const int slot = tg & 7, qi = tag_qidx(tg, r0, nk);
+            bool ok = false;
+            if (t < chunk) {
+              const uint64_t key = seed_key(W, slot, payload_entry(W, slot, p, i), qi, gap, local, qlen);
+              __stcs(reinterpret_cast<unsigned long long*>(W.skey + to), key);
+              __stcs(W.sq + to, (uint32_t)qi);
+              ok = key != kDroppedSeed;
+            }
+#pragma unroll
+            for (int x = 0; x < NS; ++x) valid[x] += ok && slot == x;
+          }
+        }
+      }
+      __syncwarp();
+    }
+    int n_slot = 0;
+#pragma unroll
+    for (int x = 0; x < NS; ++x) {
+      const int n = (int)__reduce_add_sync(kFull, (unsigned)valid[x]);
+      if (lane == x) n_slot = n;
+    }
+    if (TEAM > 1) {
+      if (lane < NS && n_slot) atomicAdd(&team_valid[lane], n_slot);
+      __syncthreads();
+      if (warp == 0 && lane < NS) n_slot = team_valid[lane];
+    }
+    if ((TEAM == 1 || warp == 0) && lane < NS) {
+      const int64_t v = v0 + lane;
+      W.off[v] = base;
+      W.cnt[v] = n_all;
+      W.nvalid[v] = n_slot;
+      if (n_slot > 0) {
+        const int t = n_all <= kWarpSmemCap ? 0 : n_all <= kCtaSortCap ? 1 : 2;
+        W.lists[t * (int64_t)NW * q.nstrands + atomicAdd(W.n_listed + t, 1)] = (uint32_t)v;
+      } else {
+        W.hcnt[v] = 0;
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// The first strand of every (target window, query window) with a valid seed:
+// its seed count is stored complemented, for the isolate filter keeps the first
+// seed of a query window.  Where the seeding kernel filtered the slot itself
+// (cnt 0), as one that is not first, that seed is a hit more, and the slot's
+// first other hit is none if it lies near that seed (first_q's top bit).
+__global__ void k_window_first(int32_t* __restrict__ nvalid, const int32_t* __restrict__ wstart, int nwin, int nw,
+                               const int32_t* __restrict__ cnt, const uint32_t* __restrict__ first_q,
+                               int32_t* __restrict__ hcnt) {
+  const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  if (i >= nwin * nw) return;
+  const int w = i / nwin, qw = i % nwin;
+  const int a = wstart[qw], b = wstart[qw + 1];
+  for (int c = a; c < b; c += 32) {
+    const int s = c + lane;
+    const int64_t v = strand_slot(s, w, nw);
+    const int n = s < b ? nvalid[v] : 0;
+    const unsigned m = __ballot_sync(kFull, n > 0);
+    if (m) {
+      if (lane == __ffs(m) - 1) {
+        nvalid[v] = ~n;
+        if (first_q && cnt[v] == 0) hcnt[v] += 1 - (int)(first_q[v] >> 31);
+      }
+      return;
+    }
+  }
+}
 
 // ---- seed sort fused with the isolate / duplicate filters ----
 // Slots (strand, target window) of a group; nvalid as k_window_first leaves it.
@@ -1615,7 +2064,6 @@ __device__ __forceinline__ void filter_chunk(int c0, int n, uint64_t k, uint32_t
 // runs over all slots and lists the others' slots; so four launches do what
 // a classification and five tiers did, for every window of the group at once.
 constexpr int kThreadSortCap = 8;
-constexpr int kWarpSmemCap = 256;
 
 // 1..kThreadSortCap seeds: one thread per slot.  The seeds (padded with
 // keys above every seed) go through an odd-even transposition network in
@@ -1835,7 +2283,7 @@ __global__ void k_gather_hits(const uint64_t* __restrict__ skey, const uint32_t*
                               const int64_t* __restrict__ off, const int32_t* __restrict__ hcnt,
                               const int64_t* __restrict__ hoff, int64_t nv, int nw, uint64_t* __restrict__ hk,
                               int32_t* __restrict__ hq, uint32_t* __restrict__ hs, const int32_t* __restrict__ qlen,
-                              int l, int band, GroupCtl* __restrict__ ctl) {
+                              int l, int band, FirstSeeds first, GroupCtl* __restrict__ ctl) {
   const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int n = (v < nv) ? hcnt[v] : 0;
   // every hit of the strand fills band * (qlen - l) cells: backward rows + forward rows
@@ -1845,8 +2293,18 @@ __global__ void k_gather_hits(const uint64_t* __restrict__ skey, const uint32_t*
   for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(&ctl->cells, c);
   if (v >= nv) return;
-  const int64_t a = off[v], b = hoff[v];
-  for (int i = 0; i < n; ++i) {
+  if (n == 0) return;
+  int64_t a = off[v], b = hoff[v];
+  int i = 0;
+  if (first.key && first.nvalid[v] < 0 && first.cnt[v] == 0) {  // see k_window_first
+    const uint32_t q0 = first.q[v];
+    hk[b] = first.key[v];
+    hq[b] = (int32_t)(q0 & 0x7fffffffu);
+    hs[b] = (uint32_t)v;
+    a += (int)(q0 >> 31) - 1;
+    i = 1;
+  }
+  for (; i < n; ++i) {
     hk[b + i] = skey[a + i];
     hq[b + i] = (int32_t)sq[a + i];
     hs[b + i] = (uint32_t)v;
@@ -2978,14 +3436,23 @@ int64_t index_state_words(int64_t n_samples) { return (n_samples + kIxTile - 1) 
 
 void index_place(const uint64_t* items, const int32_t* vals, int64_t n_samples, int pbits, int stride, int l, int cut,
                  const int32_t* gateway, const int32_t* lengths, int nseqs, uint32_t nbuckets, int2* entries,
-                 ulonglong2* table, int64_t n_records, uint32_t* filter, int fshift, unsigned long long* state,
-                 unsigned long long* kept, unsigned long long* failed, cudaStream_t st) {
+                 ulonglong2* table, int64_t n_records, uint32_t* filter, int fshift, int fstride,
+                 unsigned long long* state, unsigned long long* kept, unsigned long long* failed, cudaStream_t st) {
   if (n_samples <= 0) return;
   const IndexBuild b{items, vals, n_samples, pbits, 1ull << (2 * l), stride, l, cut, gateway, lengths, nseqs, nbuckets,
-                     entries, table, n_records, filter, fshift, state, kept, failed};
+                     entries, table, n_records, filter, fshift, fstride, state, kept, failed};
   const unsigned tiles = (unsigned)(index_state_words(n_samples) - 1);
   if (pbits > 0) k_index_place<false><<<tiles, kIxThreads, 0, st>>>(b);
   else k_index_place<true><<<tiles, kIxThreads, 0, st>>>(b);
+  CLAST_LAUNCHED();
+}
+
+void filter_from_table(const ulonglong2* table, int64_t n_records, int l, uint32_t* filter, int fshift, int fstride,
+                       bool file, cudaStream_t st) {
+  if (n_records <= 0) return;
+  const unsigned grid = (unsigned)((n_records + 255) / 256);
+  if (file) k_filter_from_table<true><<<grid, 256, 0, st>>>(table, n_records, l, filter, fshift, fstride);
+  else k_filter_from_table<false><<<grid, 256, 0, st>>>(table, n_records, l, filter, fshift, fstride);
   CLAST_LAUNCHED();
 }
 
@@ -3005,35 +3472,55 @@ void seed_fused(const QueryView& q, const IndexView& ix, const TargetView& t, in
 }
 
 template <int NW>
-void launch_seed_multi(const QueryView& q, const SeedWins& W, int gap, int local, cudaStream_t st) {
-  const unsigned grid = blocks_for((int64_t)q.nstrands * 32, kSeedFusedThreads);
-  if (W.w[0].ix.l <= 16) k_seed_multi<true, NW><<<grid, kSeedFusedThreads, 0, st>>>(q, W, gap, local);
-  else k_seed_multi<false, NW><<<grid, kSeedFusedThreads, 0, st>>>(q, W, gap, local);
+void launch_seed_reads(const QueryView& q, const SeedWins& W, int width, int gap, int local, int max_len,
+                       cudaStream_t st) {
+  const unsigned grid = blocks_for((int64_t)q.nstrands / 2 * 32, kSeedFusedThreads);
+  const unsigned few = std::min<unsigned>(grid, 148 * 12);  // blocks that share the listed reads
+  const unsigned teams = (unsigned)std::min<int64_t>(q.nstrands / 2, 148 * 8);
+  if (W.w[0].ix.l <= 16) {
+    k_seed_reads<true, NW><<<grid, kSeedFusedThreads, 0, st>>>(q, W, width, gap, local);
+    CLAST_LAUNCHED();
+    k_seed_reads_long<true, NW, 1><<<few, kSeedFusedThreads, 0, st>>>(q, W, gap, local);
+    CLAST_LAUNCHED();
+    if (max_len - W.w[0].ix.l < kSeedRound) return;
+    k_seed_reads_long<true, NW, kLongTeam<NW>><<<teams, 32 * kLongTeam<NW>, 0, st>>>(q, W, gap, local);
+  } else {
+    k_seed_reads<false, NW><<<grid, kSeedFusedThreads, 0, st>>>(q, W, width, gap, local);
+    CLAST_LAUNCHED();
+    k_seed_reads_long<false, NW, 1><<<few, kSeedFusedThreads, 0, st>>>(q, W, gap, local);
+    CLAST_LAUNCHED();
+    if (max_len - W.w[0].ix.l < kSeedRound) return;
+    k_seed_reads_long<false, NW, kLongTeam<NW>><<<teams, 32 * kLongTeam<NW>, 0, st>>>(q, W, gap, local);
+  }
   CLAST_LAUNCHED();
 }
 
-void seed_multi(const QueryView& q, const SeedWins& W, int nw, int gap, int local, cudaStream_t st) {
+void seed_reads(const QueryView& q, const SeedWins& W, int nw, int width, int gap, int local, int max_len,
+                cudaStream_t st) {
   if (q.nstrands <= 0 || nw <= 0) return;
   switch (nw) {
-    case 1: launch_seed_multi<1>(q, W, gap, local, st); break;
-    case 2: launch_seed_multi<2>(q, W, gap, local, st); break;
-    case 3: launch_seed_multi<3>(q, W, gap, local, st); break;
-    case 4: launch_seed_multi<4>(q, W, gap, local, st); break;
-    default: throw std::invalid_argument("seed_multi: 1 to 4 windows per pass");
+    case 1: launch_seed_reads<1>(q, W, width, gap, local, max_len, st); break;
+    case 2: launch_seed_reads<2>(q, W, width, gap, local, max_len, st); break;
+    case 3: launch_seed_reads<3>(q, W, width, gap, local, max_len, st); break;
+    case 4: launch_seed_reads<4>(q, W, width, gap, local, max_len, st); break;
+    default: throw std::invalid_argument("seed_reads: 1 to 4 windows per group");
   }
 }
 
 void seed_filter(uint64_t* skey, uint32_t* sq, const int64_t* off, const int32_t* cnt, int32_t* nvalid,
-                 const int32_t* win_start, int n_windows, int nw, int width, int gap, int64_t nv, uint32_t* lists,
-                 int32_t* hcnt, GroupCtl* ctl, cudaStream_t st) {
+                 const uint32_t* first_q, const int32_t* win_start, int n_windows, int nw, int width, int gap,
+                 int64_t nv, uint32_t* lists, int32_t* hcnt, GroupCtl* ctl, cudaStream_t st) {
   if (nv <= 0) return;
   if (n_windows > 0) {
-    k_window_first<<<blocks_for((int64_t)n_windows * nw * 32, 256), 256, 0, st>>>(nvalid, win_start, n_windows, nw);
+    k_window_first<<<blocks_for((int64_t)n_windows * nw * 32, 256), 256, 0, st>>>(nvalid, win_start, n_windows, nw, cnt,
+                                                                                 first_q, hcnt);
     CLAST_LAUNCHED();
   }
   SeedFilterCtx c{off, cnt, nvalid, width, gap, hcnt};
-  k_seed_filter_small<<<blocks_for(nv, 256), 256, 0, st>>>(skey, sq, c, nv, lists, ctl);
-  CLAST_LAUNCHED();
+  if (!first_q) {
+    k_seed_filter_small<<<blocks_for(nv, 256), 256, 0, st>>>(skey, sq, c, nv, lists, ctl);
+    CLAST_LAUNCHED();
+  }
   k_seed_filter_mid<<<grid_cap(std::min<int64_t>((nv + 3) / 4, 148 * 64)), kWarpSmemThreads, 0, st>>>(
       skey, sq, c, lists, &ctl->n_seeds[0]);
   CLAST_LAUNCHED();
@@ -3046,9 +3533,10 @@ void seed_filter(uint64_t* skey, uint32_t* sq, const int64_t* off, const int32_t
 
 void gather_hits(const uint64_t* skey, const uint32_t* sq, const int64_t* off, const int32_t* hcnt,
                  const int64_t* hoff, int64_t nv, int nw, uint64_t* hk, int32_t* hq, uint32_t* hs,
-                 const int32_t* qlen, int l, int band, GroupCtl* ctl, cudaStream_t st) {
+                 const int32_t* qlen, int l, int band, const FirstSeeds& first, GroupCtl* ctl, cudaStream_t st) {
   if (nv <= 0) return;
-  k_gather_hits<<<blocks_for(nv, 256), 256, 0, st>>>(skey, sq, off, hcnt, hoff, nv, nw, hk, hq, hs, qlen, l, band, ctl);
+  k_gather_hits<<<blocks_for(nv, 256), 256, 0, st>>>(skey, sq, off, hcnt, hoff, nv, nw, hk, hq, hs, qlen, l, band, first,
+                                                     ctl);
   CLAST_LAUNCHED();
 }
 

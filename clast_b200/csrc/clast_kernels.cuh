@@ -56,8 +56,12 @@ int radix_sort_u64(Workspace& ws, uint64_t* keys, int32_t* vals, uint64_t* keys_
 int64_t index_state_words(int64_t n_samples);
 void index_place(const uint64_t* items, const int32_t* vals, int64_t n_samples, int pbits, int stride, int l, int cut,
                  const int32_t* gateway, const int32_t* lengths, int nseqs, uint32_t nbuckets, int2* entries,
-                 ulonglong2* table, int64_t n_records, uint32_t* filter, int fshift, unsigned long long* state,
-                 unsigned long long* kept, unsigned long long* failed, cudaStream_t st);
+                 ulonglong2* table, int64_t n_records, uint32_t* filter, int fshift, int fstride,
+                 unsigned long long* state, unsigned long long* kept, unsigned long long* failed, cudaStream_t st);
+// The filter (zeroed by the caller) of a table's keys: as it is searched, or
+// with `file` as index files hold it (fstride 1).
+void filter_from_table(const ulonglong2* table, int64_t n_records, int l, uint32_t* filter, int fshift, int fstride,
+                       bool file, cudaStream_t st);
 
 // ---- seeds (CDeviceHitList_createRawSeedList.cu, _deleteSeeds*.cu, _sortSeeds.cu) ----
 // A group of up to kMaxSeedWins target windows is searched together.  Its slots
@@ -77,13 +81,15 @@ __host__ __device__ __forceinline__ int slot_window(uint32_t v, int nw) {
 
 // Counters of one group's search, zeroed before it.
 struct GroupCtl {
-  unsigned long long cursor[kMaxSeedWins][kSeedParts];  // seeds per window and partition
+  unsigned long long cursor[kSeedParts];                // seeds and hits stored per partition
   unsigned long long kmers[kMaxSeedWins][kSeedParts];   // valid l-mers of the partition's strands
+  unsigned long long seeds[kMaxSeedWins][kSeedParts];   // their seeds (seed_reads)
   unsigned long long cells;                             // DP cells
   long long hits, results;
   long long dp_warp;  // hits the DP's split sends to the one-per-warp kernel
   int bad;            // see DpLaunch::bad
   int n_seeds[3];     // slots listed for the seed filters' longer tiers
+  int n_stored[4];    // reads whose seeds are stored: of one round, longer, and how many of each are taken
   int n_long;         // reads listed for k_final_long
 };
 
@@ -97,39 +103,65 @@ struct GroupCtl {
 void seed_fused(const QueryView& q, const IndexView& ix, const TargetView& t, int gap, int local,
                 unsigned long long* cursors, unsigned long long* n_kmers, int64_t* off, int32_t* cnt, int32_t* nvalid,
                 uint64_t* skey, uint32_t* sq, int64_t part_cap, cudaStream_t st);
-// The same for the nw windows of a group in one pass over the query: per slot
-// arrays, skey/sq hold nw x kSeedParts partitions.  Every window must have
-// been built with the same l.
+// Seeding of whole reads (strand 2r + 1 the reverse complement of strand 2r) in
+// the nw windows of a group, in one pass.  Slots of up to 32 seeds of reads of
+// up to 160 l-mers are filtered at once: hcnt hits at off, cnt 0, nvalid valid
+// seeds, and the first of them in first_key / first_q (see k_window_first).
+// The others' seeds are stored (off, cnt, nvalid) and the slots listed for
+// seed_filter (lists: three of nw * nstrands words, n_listed: their counts).
+// Seeds and hits share kSeedParts partitions of nw * part_cap of skey/sq, read
+// r's in partition r % kSeedParts, reserved through cursor as in seed_fused.
+// Every window must have been built with the same l.  max_len: no strand is
+// longer (INT_MAX when that is not known).
 struct SeedWin {
   IndexView ix;
   TargetView t;
-  unsigned long long* cursor;   // kSeedParts cursors
   unsigned long long* n_kmers;  // kSeedParts l-mer counters
+  unsigned long long* n_seeds;  // kSeedParts seed counters
+  int paired;                   // an odd window whose filter words follow those of the window before it
 };
 struct SeedWins {
   SeedWin w[kMaxSeedWins];
+  unsigned long long* cursor;
   int64_t* off;
   int32_t* cnt;
   int32_t* nvalid;
+  int32_t* hcnt;
+  uint64_t* first_key;
+  uint32_t* first_q;
+  uint32_t* lists;
+  int* n_listed;
+  uint32_t* long_reads;  // the reads whose seeds are stored, one word per read
+  int* n_long;           // GroupCtl::n_stored
+  int words;             // every window has less than 2^20 sequences (seed_word)
   uint64_t* skey;
   uint32_t* sq;
   int64_t part_cap;
 };
-void seed_multi(const QueryView& q, const SeedWins& W, int nw, int gap, int local, cudaStream_t st);
+void seed_reads(const QueryView& q, const SeedWins& W, int nw, int width, int gap, int local, int max_len,
+                cudaStream_t st);
 
 // sortSeeds + deletingIsolateSeeds + deleteDuplicateSeeds per slot: sorts the
 // cnt[v] seeds of slot v by (sequence, diagonal, qIdx) and writes the surviving
-// hits at off[v] onwards, hcnt[v] of them.  lists: 3 nv words.  The first slot
+// hits at off[v] onwards, hcnt[v] of them.  lists: 3 nv words.  With first_q
+// (seed_reads) only the listed slots are left to filter.  The first slot
 // of every (target window, query window) with a valid seed has its nvalid
 // complemented.
 void seed_filter(uint64_t* skey, uint32_t* sq, const int64_t* off, const int32_t* cnt, int32_t* nvalid,
-                 const int32_t* win_start, int n_windows, int nw, int width, int gap, int64_t nv, uint32_t* lists,
-                 int32_t* hcnt, GroupCtl* ctl, cudaStream_t st);
+                 const uint32_t* first_q, const int32_t* win_start, int n_windows, int nw, int width, int gap,
+                 int64_t nv, uint32_t* lists, int32_t* hcnt, GroupCtl* ctl, cudaStream_t st);
+// First seeds of the slots that seed_reads filtered (key null: none).
+struct FirstSeeds {
+  const uint64_t* key;
+  const uint32_t* q;
+  const int32_t* nvalid;
+  const int32_t* cnt;
+};
 // The hits of every slot back to back (hk: seed key, hq: qIdx, hs: slot); also
 // adds band * (qlen - l) DP cells per hit to ctl->cells.
 void gather_hits(const uint64_t* skey, const uint32_t* sq, const int64_t* off, const int32_t* hcnt,
                  const int64_t* hoff, int64_t nv, int nw, uint64_t* hk, int32_t* hq, uint32_t* hs,
-                 const int32_t* qlen, int l, int band, GroupCtl* ctl, cudaStream_t st);
+                 const int32_t* qlen, int l, int band, const FirstSeeds& first, GroupCtl* ctl, cudaStream_t st);
 
 // ---- banded DP + E-value (krnlAlignment.cu, krnlCalculateEvalue.cu) ----
 struct DpOut {
