@@ -2424,13 +2424,15 @@ __device__ __forceinline__ float max3_f32(float a, float b, float c) {
 // their additions run on the FMA pipe instead, at twice the rate, and a cell's
 // ALU work is one three-way and two two-way maxima, two compares and two
 // selects.  The columns' letters are packed four to a word, one dp4a makes a
-// table address of them, and each pair is looked up a row ahead of its use
-// (without that, a lone hit waits 2.1 against 1.1 ms on 5 kbp).  Measured
+// table address of them, and each pair is looked up well ahead of its use
+// (without that, a lone hit waits 2.1 against 0.96 ms on 5 kbp).  Measured
 // against the integer form with a spread table that this replaced: 1,172 to
-// 1,980 GCUPS on uneven reads of 50 bp - 10 kbp (28.7 to 17.0 ms), 1,185 to
-// 1,590 on a million reads of 150 bp (4.55 to 3.39 ms), 599 to 1,200 at gap 16.
-// (Tried: packed f32x2 additions, arithmetic selects by saturated differences
-// on the FMA pipe, the row in two loops; all slower or within the noise.)
+// 2,045 GCUPS on uneven reads of 50 bp - 10 kbp (28.7 to 16.4 ms), 1,185 to
+// 1,740 on a million reads of 150 bp (4.55 to 3.09 ms), 599 to 1,200 at gap 16.
+// FMA: the second select is a saturated difference times the two values'
+// difference (whole numbers, so exact), on the FMA pipe; faster only where
+// four blocks share an SM (see kDpBlocksFull).  (Tried: packed f32x2
+// additions, both selects so; slower.)
 template <int GAP>
 struct Band {
   static constexpr int W = 2 * GAP + 1;
@@ -2473,7 +2475,7 @@ struct Band {
   }
 };
 
-template <int GAP, bool LOCAL>
+template <int GAP, bool LOCAL, bool FMA>
 __device__ __forceinline__ void banded_hit(const DpTab<float2>& tab, const char* __restrict__ tb, int64_t tstart,
                                            int tlen, const char* __restrict__ qb, int64_t qstart, int qlen, int tidx,
                                            int qidx, int l, int& t_hl, int& q_hl, int& match, int& score,
@@ -2492,16 +2494,26 @@ __device__ __forceinline__ void banded_hit(const DpTab<float2>& tab, const char*
   const char* __restrict__ tp = tb + tstart + tidx + l + GAP + 1;
   const char* __restrict__ qp = qb + qstart + qidx + l;
   int t_end = tlen - (tidx + l + GAP + 1), q_end = rows_b;
-  float2 w[W];  // the row's letter pairs, looked up one row ahead
+  // The row's letter pairs come in K parts through two buffers: a part is
+  // looked up before the cells of the part ahead of it run, the first one
+  // during the row before.  (With one buffer of W pairs, each reloaded right
+  // after its use, the compiler copies nearly every pair into another register
+  // first.  At gap 2 the five pairs stay in place all the same: K = 1.)
+  constexpr int K = GAP <= 2 ? 1 : GAP >= 10 && GAP <= 14 ? 4 : 2, CH = (W + K - 1) / K;
+  float2 w[K == 1 ? 1 : 2][CH];
   uint32_t qo = 0;   // the row's query letter
   char t_n, q_n;     // letters of the next row
+  auto pair = [&](int c) { return dp_pair(tab, __dp4a(bd.tw[c / 4], 1u << (8 * (c % 4)), qo)); };
+  auto look_up = [&](int k) {
+#pragma unroll
+    for (int c = k * CH; c < W && c < (k + 1) * CH; ++c) w[k & 1][c - k * CH] = pair(c);
+  };
   // r0: the pass's first row
   auto enter = [&](int r0) {
     const char q0 = r0 < q_end ? *qp : 'N';
     qp += step;
     qo = dp_q_off(tab, q0);
-#pragma unroll
-    for (int c = 0; c < W; ++c) w[c] = dp_pair(tab, __dp4a(bd.tw[c / 4], 1u << (8 * (c % 4)), qo));
+    look_up(0);
     t_n = r0 < t_end ? *tp : 'X';
     q_n = r0 + 1 < q_end ? *qp : 'N';
     tp += step;
@@ -2549,26 +2561,37 @@ __device__ __forceinline__ void banded_hit(const DpTab<float2>& tab, const char*
     const char t_nn = r < t_end ? *tp : 'X', q_nn = r < q_end ? *qp : 'N';
     tp += step;
     qp += step;
-    bd.shift_in(dp_t_off(tab, t_n));  // 'X' is the bad-area letter itself
-    qo = dp_q_off(tab, q_n);
     float h = lift + (float)(kDpLeftH<GAP> - kStepRow), mh = kMarginScore;  // row 0 of the band (left margin)
     float top = -3e38f;                                                     // highest score of the row + lift (local)
     const float vbot = lift + (float)(kDpBottomV<GAP> - kStepRow);
-#pragma unroll
-    for (int c = 0; c < W; ++c) {
+    auto cell = [&](int c, float2 w) {
       const float v = (c + 1 < W) ? bd.u[(c + 1) % W] : vbot;
       const float vm = (c + 1 < W) ? bd.sm[(c + 1) % W].y : 0.0f;
-      const float2 d = make_float2(bd.sm[c].x + w[c].x, bd.sm[c].y + w[c].y);
-      w[c] = dp_pair(tab, __dp4a(bd.tw[c / 4], 1u << (8 * (c % 4)), qo));
+      const float2 d = make_float2(bd.sm[c].x + w.x, bd.sm[c].y + w.y);
       const float S = max3_f32(d.x, v, h);
       const float open = S + kOpen;
-      const float Q = S == v ? vm : d.y;
+      const float Q = FMA ? fmaf(__saturatef(S - v), d.y - vm, vm) : S == v ? vm : d.y;
       const float M = S == h ? mh : Q;
       bd.sm[c] = make_float2(S, M);
       bd.u[c] = fmaxf(open, v);
       h = fmaxf(open, h);
       mh = M;
       if (LOCAL) top = fmaxf(S - (float)(kStepCol * c), top);
+    };
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      if (k + 1 < K) {
+        look_up(k + 1);
+      } else {
+        bd.shift_in(dp_t_off(tab, t_n));  // 'X' is the bad-area letter itself
+        qo = dp_q_off(tab, q_n);
+        if (K > 1) look_up(0);
+      }
+#pragma unroll
+      for (int c = k * CH; c < W && c < (k + 1) * CH; ++c) {
+        cell(c, w[k & 1][c - k * CH]);
+        if (K == 1) w[0][c] = pair(c);
+      }
     }
     if (LOCAL && top - lift > (float)bs) {  // the first column with the row's highest score
       bs = (int)(top - lift);
@@ -2807,7 +2830,7 @@ __device__ __forceinline__ void dp_skip(const DpKernelArgs& a, int64_t h) {
 
 // Extension of the hit at position i of the order (alignmentHits +
 // calculateEvalue + the two hit filters of deleteBadHits).
-template <int GAP, bool LOCAL>
+template <int GAP, bool LOCAL, bool FMA>
 __device__ __forceinline__ void dp_one(const DpKernelArgs& a, const DpTab<float2>& tab, int64_t i) {
   const int64_t h = a.order ? (int64_t)(uint32_t)a.order[i] : i;
   const uint64_t k = a.hk[h];
@@ -2827,7 +2850,7 @@ __device__ __forceinline__ void dp_one(const DpKernelArgs& a, const DpTab<float2
   const int l = a.p.l;
   int t_hl = l, q_hl = l, match = l, score = l;  // CDeviceHitList.cu:283-286
   int o_tidx = tidx, o_qidx = qidx;
-  banded_hit<GAP, LOCAL>(tab, t.bases, tstart, tlen, a.q.bases, qstart, qlen, tidx, qidx, l, t_hl, q_hl, match,
+  banded_hit<GAP, LOCAL, FMA>(tab, t.bases, tstart, tlen, a.q.bases, qstart, qlen, tidx, qidx, l, t_hl, q_hl, match,
                          score, o_tidx, o_qidx);
   dp_store(a, h, qlen, o_tidx, o_qidx, t_hl, q_hl, match, score);
 }
@@ -2839,15 +2862,22 @@ __device__ __forceinline__ void dp_one(const DpKernelArgs& a, const DpTab<float2
 // is some 350 instructions that every lane leaving at a row of its own would
 // run alone (3.63 to 3.44 ms on a million reads of 150 bp).
 constexpr int kDpThreads = 128, kDpMaxRounds = 4;
-// Blocks per SM by the registers the band takes (natural: 96 at gap 2, 194 at
-// gap 8, 254 at gap 16).  At gap 8, three blocks of up to 168 registers run
-// the uneven reads in 16.1 ms against 17.2 for four of 128: what the fourth
-// block hides, its register moves cost again.
+// Blocks per SM by the registers the band takes (natural: 90 at gap 2, 145 at
+// gap 8, 227 at gap 16).  Where the reads are long and uneven, three blocks of
+// up to 168 registers are the better ones at gap 8: 2.69 ms against 2.93 for
+// four of 128 on 10,000 reads of 100 - 5,000 bp, the same on 30,000.  At gaps
+// 10 - 14 three blocks (with the letter pairs in four parts) take 9.4 ms
+// against 10.4 for the two that the whole row's pairs left room for.
+// kDpBlocksFull: hits of equal length, more of them than those blocks hold, run
+// four to an SM at gaps 5 - 8 (a million reads of 150 bp at gap 8: 3.25 to 3.09
+// ms; 60,000 local ones: 1.05 to 0.89).
 template <int GAP>
-constexpr int kDpBlocksPerSm = GAP <= 4 ? 4 : (GAP <= 9 ? 3 : 2);
+constexpr int kDpBlocksPerSm = GAP <= 4 ? 4 : GAP <= 14 ? 3 : 2;
+template <int GAP>
+constexpr int kDpBlocksFull = GAP >= 5 && GAP <= 8 ? 4 : kDpBlocksPerSm<GAP>;
 
-template <int GAP, bool LOCAL>
-__global__ void __launch_bounds__(kDpThreads, kDpBlocksPerSm<GAP>)
+template <int GAP, bool LOCAL, int BLOCKS>
+__global__ void __launch_bounds__(kDpThreads, BLOCKS)
     k_banded_dp(DpKernelArgs a, int rounds, int by_rows) {
   __shared__ DpTab<float2> tab;
   __shared__ uint32_t key[kDpThreads * kDpMaxRounds];  // forward rows << 16 | hit within the block
@@ -2873,7 +2903,7 @@ __global__ void __launch_bounds__(kDpThreads, kDpBlocksPerSm<GAP>)
   __syncthreads();
   for (int i = threadIdx.x; i < n; i += kDpThreads) {
     const int64_t at = base + (by_rows ? (int64_t)(key[i] & 0xffffu) : (int64_t)i);
-    if (at < a.n && !(by_rows && key[i] == ~0u)) dp_one<GAP, LOCAL>(a, tab, at);
+    if (at < a.n && !(by_rows && key[i] == ~0u)) dp_one<GAP, LOCAL, !LOCAL && (BLOCKS > kDpBlocksPerSm<GAP>)>(a, tab, at);
   }
 }
 
@@ -3034,7 +3064,7 @@ long long launch_dp_mode(DpKernelArgs a, const DpLaunch& m, cudaStream_t st) {
     int dev = 0;
     CLAST_CK(cudaGetDevice(&dev));
     CLAST_CK(cudaDeviceGetAttribute(&o.sms, cudaDevAttrMultiProcessorCount, dev));
-    CLAST_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.per_sm, k_banded_dp<GAP, LOCAL>, kDpThreads, 0));
+    CLAST_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.per_sm, k_banded_dp<GAP, LOCAL, kDpBlocksPerSm<GAP>>, kDpThreads, 0));
     CLAST_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.warp_per_sm, k_banded_dp_warp<GAP, LOCAL>, kDpThreads, 0));
     o.per_sm = std::max(1, o.per_sm);
     o.warp_per_sm = std::max(1, o.warp_per_sm);
@@ -3080,10 +3110,15 @@ long long launch_dp_mode(DpKernelArgs a, const DpLaunch& m, cudaStream_t st) {
   if (rest <= 0) return warp_hits;
   // blocks of several rounds sort more hits together; short batches need the blocks
   const bool by_rows = m.uniform_rows >= 0;
-  const int64_t waves = rest / ((int64_t)sms * per_sm * threads);
+  // the variant of more blocks only where they all have hits to run
+  const bool full = kDpBlocksFull<GAP> > kDpBlocksPerSm<GAP> && by_rows && rest > (int64_t)sms * per_sm * threads;
+  const int64_t waves = rest / ((int64_t)sms * (full ? kDpBlocksFull<GAP> : per_sm) * threads);
   const int rounds = !by_rows ? 1 : waves >= 8 ? kDpMaxRounds : waves >= 4 ? 2 : 1;
   const unsigned grid = (unsigned)((rest + threads * rounds - 1) / (threads * rounds));
-  k_banded_dp<GAP, LOCAL><<<grid, threads, 0, st>>>(a, rounds, by_rows);
+  if (full)
+    k_banded_dp<GAP, LOCAL, kDpBlocksFull<GAP>><<<grid, threads, 0, st>>>(a, rounds, by_rows);
+  else
+    k_banded_dp<GAP, LOCAL, kDpBlocksPerSm<GAP>><<<grid, threads, 0, st>>>(a, rounds, by_rows);
   CLAST_LAUNCHED();
   if (joined) CLAST_CK(cudaStreamWaitEvent(st, m.ev_join, 0));
   return warp_hits;

@@ -74,3 +74,30 @@ def test_longest_reads_equal_oracle(engine, length):
     want = O.window_search(s, tbases, tgw, tln, 0, qbases, qgw, qln, 0)
     assert len(want["t_id"]) > 0 and want["score"].max() > length // 2
     compare(hits(engine, s, tl, ql, "off"), want)
+
+
+@pytest.mark.parametrize("gap,local", [(4, 0), (5, 0), (5, 1), (6, 0), (7, 1), (8, 0), (8, 1), (10, 1), (14, 0), (15, 0)])
+def test_bands_of_a_full_grid_match_one_hit_per_warp(engine, gap, local):
+    """More equally long hits than three blocks per SM hold (bands of 5 - 8 run
+    four to an SM then), and the bands next to those that take the row's letter
+    pairs in another number of parts."""
+    rng = np.random.Generator(np.random.PCG64(gap + 100 * local))
+    t = synth.make_target(rng, 1_000_000, n_contigs=2, median=400_000)
+    q = synth.make_reads_fixed(rng, t, 130_000, length=61, sub=0.04, indel=0.02)
+    s = api.Setting(gap=gap, local=local, total_db=float(t.offsets[-1]))
+    _, t_loads = api.ram_loads(np.diff(t.offsets), 64_000_000)
+    _, q_loads = api.ram_loads(np.diff(q.offsets), 32_000_000)
+    T = engine.targets(s, t.bases, t.offsets, t_loads, 64_000_000)
+    out = {}
+    for mode in ("off", "all"):
+        os.environ["CLAST_DP_WARP"] = mode
+        try:
+            r = engine.map(s, T, q.bases, q.offsets, q_loads, 2_000_000)
+        finally:
+            os.environ.pop("CLAST_DP_WARP", None)
+        out[mode] = {f: np.array(r[f]) for f in api.MAP_FIELDS}
+        del r
+    T.close()
+    assert len(out["off"]["score"]) > 60_000
+    for f in api.MAP_FIELDS:
+        assert np.array_equal(out["off"][f], out["all"][f]), f
