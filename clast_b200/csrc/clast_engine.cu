@@ -91,13 +91,12 @@ void build_index_device(Workspace& ws, cudaStream_t st, const clast_params* p, c
   ix->kept.alloc(1);
   ix->n_records = 2 * nb + (1 << 16);
   ix->table.alloc((size_t)ix->n_records);
-  CLAST_CK(cudaMemsetAsync(ix->table.p, 0xff, (size_t)ix->n_records * sizeof(ulonglong2), st));
   if (!ix->filter_mem) {
     clast_index* one[1] = {ix};
     alloc_filters(one, 1, filter_shift(ns), st);
   }
   CLAST_CK(cudaMemsetAsync(ix->kept.p, 0, sizeof(int64_t), st));
-  const size_t words = (size_t)index_state_words(ns);
+  const size_t words = (size_t)index_state_words(ns, ix->n_records);
   unsigned long long* state = ws.get<unsigned long long>("ix_state", words);
   CLAST_CK(cudaMemsetAsync(state, 0, words * sizeof(unsigned long long), st));
   index_place(in_alt ? items2 : items, in_alt ? pos2 : pos, ns, pbits, p->stride, l, p->cut_repeat, ix->gateway.p,

@@ -543,13 +543,16 @@ __global__ void __launch_bounds__(kRsThreads, 3) k_rs_scatter(const uint64_t* __
 // have started, and at most kScanSpinLimit polls per step: past that it counts
 // into *failed, which the host reports.
 //
-// 8 bytes read and about 24 written per sample, and one random atomic per code
-// for the filter; bound by the waits at its barriers and by instructions (443
-// per sample), at a fifth of the memory rate.  The fourteen kernels this
-// replaced (heads, two scans, unique codes, kept samples, entries, bucket
-// bounds, a scan of the kept codes, a two-level running maximum, placement)
-// wrote and read some 120 bytes per sample in between: index of a 250 Mbp
-// window (50 M samples) 6.28 to 3.76 ms, of which this kernel takes 1.18.
+// 8 bytes read and 40 written per sample (the table's free half included), and
+// one random atomic per code for the filter; bound by instructions (506 per
+// sample, half of the issue slots) and the waits at its barriers (38 % of the
+// stalls), at a quarter of the memory rate.  The fourteen kernels this replaced
+// (heads, two scans, unique codes, kept samples, entries, bucket bounds, a scan
+// of the kept codes, a two-level running maximum, placement) wrote and read
+// some 120 bytes per sample in between: index of a 250 Mbp window (50 M samples)
+// 6.28 to 3.80 ms; with the free records written here too, instead of the whole
+// table before, and five blocks per SM (48 registers, 92 bytes spilled; four:
+// 3.70) 3.63.
 constexpr int kIxThreads = 256, kIxRounds = 4, kIxTile = kIxThreads * kIxRounds;
 constexpr int kIxWarps = kIxThreads / 32, kIxWarpItems = 32 * kIxRounds;
 
@@ -611,6 +614,36 @@ __global__ void k_filter_from_table(const ulonglong2* __restrict__ table, int64_
   }
 }
 
+// Free records.  Most lie between two records of a tile and are written with
+// them, so that a sector of the table is written whole and once.  What a long
+// free stretch covers of the table's chunks of kIxChunk records is only marked
+// here and filled by k_index_free, which has the whole GPU for it (a window of
+// N's is one such stretch).
+constexpr int kIxChunkLog = 12, kIxChunk = 1 << kIxChunkLog, kIxOwnFree = 32;
+
+// [from, to) of the table; every lane of the warp takes part.
+__device__ __forceinline__ void ix_free(ulonglong2* __restrict__ table, unsigned char* __restrict__ chunk_free,
+                                        int64_t from, int64_t to) {
+  const int lane = threadIdx.x & 31;
+  const ulonglong2 free_rec = make_ulonglong2(~0ull, kNoPayload);
+  const int64_t a = (from + kIxChunk - 1) >> kIxChunkLog, z = to >> kIxChunkLog;
+  const int64_t head = z > a ? a << kIxChunkLog : to;
+  for (int64_t i = from + lane; i < head; i += 32) table[i] = free_rec;
+  if (z > a) {
+    for (int64_t c = a + lane; c < z; c += 32) chunk_free[c] = 1;
+    for (int64_t i = (z << kIxChunkLog) + lane; i < to; i += 32) table[i] = free_rec;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_index_free(ulonglong2* __restrict__ table,
+                                                    const unsigned char* __restrict__ chunk_free, int64_t chunks) {
+  for (int64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
+    if (!chunk_free[c]) continue;  // the same for the whole block
+    for (int i = threadIdx.x; i < kIxChunk; i += 256)
+      table[(c << kIxChunkLog) + i] = make_ulonglong2(~0ull, kNoPayload);
+  }
+}
+
 struct IndexBuild {
   const uint64_t* items;  // sorted: code << pbits | sample, or codes with the samples in vals (pbits 0)
   const int32_t* vals;
@@ -628,12 +661,13 @@ struct IndexBuild {
   uint32_t* filter;
   int fshift, fstride;
   unsigned long long* state;  // [0] tile counter, then one word per tile
+  unsigned char* chunk_free;  // per whole chunk of the table: no record lies in it
   unsigned long long* kept;   // records placed
   unsigned long long* failed;
 };
 
 template <bool PAIR>
-__global__ void __launch_bounds__(kIxThreads) k_index_place(IndexBuild b) {
+__global__ void __launch_bounds__(kIxThreads, 5) k_index_place(IndexBuild b) {
   __shared__ uint64_t code[kIxTile + 1];
   __shared__ int2 res[kIxTile];
   __shared__ uint16_t start[kIxTile + 1];  // first sample of every run of the tile
@@ -775,7 +809,7 @@ __global__ void __launch_bounds__(kIxThreads) k_index_place(IndexBuild b) {
     }
   }
   __syncthreads();
-  // records: u = rank within the tile, slack = home - u, its running maximum
+  // records: u = rank within the tile, slack = home - u, the maximum of the records before
   unsigned rec = 0;
   int u[kIxRounds], kc[kIxRounds];
   int64_t run[kIxRounds], home[kIxRounds];
@@ -810,8 +844,11 @@ __global__ void __launch_bounds__(kIxThreads) k_index_place(IndexBuild b) {
         const int64_t y = __shfl_up_sync(kFull, v, o);
         if (lane >= o && y > v) v = y;
       }
-      run[j] = v > carry ? v : carry;
-      carry = __shfl_sync(kFull, run[j], 31);
+      int64_t y = __shfl_up_sync(kFull, v, 1);
+      if (lane == 0) y = INT64_MIN;
+      run[j] = y > carry ? y : carry;
+      y = __shfl_sync(kFull, v, 31);
+      if (y > carry) carry = y;
     }
     if (lane == 0) wmax[warp] = carry;
     __syncthreads();
@@ -868,25 +905,40 @@ __global__ void __launch_bounds__(kIxThreads) k_index_place(IndexBuild b) {
       s_x = x;
       if (n_rec) atomicAdd(b.kept, (unsigned long long)n_rec);
     }
+    if (t == (int64_t)gridDim.x - 1) ix_free(b.table, b.chunk_free, A > x + n_rec ? A : x + n_rec, b.n_records);
   }
   __syncthreads();
   const int64_t x = s_x;
 #pragma unroll
   for (int j = 0; j < kIxRounds; ++j) {
-    if (!((rec >> j) & 1u)) continue;
-    const int k = warp * kIxWarpItems + j * 32 + lane;
-    const uint64_t c = code[k];
-    filter_set(b.filter, b.fshift, b.fstride, c, b.l);
-    uint64_t payload;
-    if (kc[j] == 1) {
-      const int2 e = cross && rid[j] == n_runs - 1 ? s_cross : res[first[k]];
-      payload = ((uint64_t)(uint32_t)e.x << 32) | (uint32_t)e.y;
-    } else {
-      payload = kMulti | ((uint64_t)(i0 + k) << 32) | (uint32_t)kc[j];
+    // the free records between the record before this one and this one: [from, at)
+    const int64_t from = u[j] + (run[j] > x ? run[j] : x);
+    int64_t at = from;
+    if ((rec >> j) & 1u) {
+      const int k = warp * kIxWarpItems + j * 32 + lane;
+      const uint64_t c = code[k];
+      filter_set(b.filter, b.fshift, b.fstride, c, b.l);
+      uint64_t payload;
+      if (kc[j] == 1) {
+        const int2 e = cross && rid[j] == n_runs - 1 ? s_cross : res[first[k]];
+        payload = ((uint64_t)(uint32_t)e.x << 32) | (uint32_t)e.y;
+      } else {
+        payload = kMulti | ((uint64_t)(i0 + k) << 32) | (uint32_t)kc[j];
+      }
+      if (home[j] > from) at = home[j];
+      if (from >= 0 && at < b.n_records) {
+        if (at - from <= kIxOwnFree)
+          for (int64_t i = from; i < at; ++i) b.table[i] = make_ulonglong2(~0ull, kNoPayload);
+        b.table[at] = make_ulonglong2(c, payload);
+      } else {  // unreachable: positions rise to the last one, which the table holds
+        atomicAdd(b.failed, 1ull);
+        at = from;
+      }
     }
-    const int64_t at = u[j] + (run[j] > x ? run[j] : x);
-    if (at >= 0 && at < b.n_records) b.table[at] = make_ulonglong2(c, payload);
-    else atomicAdd(b.failed, 1ull);  // unreachable: positions rise to the last one, which the table holds
+    for (unsigned far = __ballot_sync(kFull, at - from > kIxOwnFree); far; far &= far - 1) {
+      const int src = __ffs(far) - 1;
+      ix_free(b.table, b.chunk_free, __shfl_sync(kFull, from, src), __shfl_sync(kFull, at, src));
+    }
   }
 }
 
@@ -3467,19 +3519,30 @@ int radix_sort_u64(Workspace& ws, uint64_t* keys, int32_t* vals, uint64_t* keys_
   return which;
 }
 
-int64_t index_state_words(int64_t n_samples) { return (n_samples + kIxTile - 1) / kIxTile + 1; }
+int64_t index_state_words(int64_t n_samples, int64_t n_records) {
+  return (n_samples + kIxTile - 1) / kIxTile + 1 + ((n_records >> kIxChunkLog) + 7) / 8;
+}
 
 void index_place(const uint64_t* items, const int32_t* vals, int64_t n_samples, int pbits, int stride, int l, int cut,
                  const int32_t* gateway, const int32_t* lengths, int nseqs, uint32_t nbuckets, int2* entries,
                  ulonglong2* table, int64_t n_records, uint32_t* filter, int fshift, int fstride,
                  unsigned long long* state, unsigned long long* kept, unsigned long long* failed, cudaStream_t st) {
-  if (n_samples <= 0) return;
+  if (n_samples <= 0) {  // no tile: all records are free
+    CLAST_CK(cudaMemsetAsync(table, 0xff, (size_t)n_records * sizeof(ulonglong2), st));
+    return;
+  }
+  const int64_t tiles = (n_samples + kIxTile - 1) / kIxTile;
+  unsigned char* chunk_free = reinterpret_cast<unsigned char*>(state + tiles + 1);
   const IndexBuild b{items, vals, n_samples, pbits, 1ull << (2 * l), stride, l, cut, gateway, lengths, nseqs, nbuckets,
-                     entries, table, n_records, filter, fshift, fstride, state, kept, failed};
-  const unsigned tiles = (unsigned)(index_state_words(n_samples) - 1);
-  if (pbits > 0) k_index_place<false><<<tiles, kIxThreads, 0, st>>>(b);
-  else k_index_place<true><<<tiles, kIxThreads, 0, st>>>(b);
+                     entries, table, n_records, filter, fshift, fstride, state, chunk_free, kept, failed};
+  if (pbits > 0) k_index_place<false><<<(unsigned)tiles, kIxThreads, 0, st>>>(b);
+  else k_index_place<true><<<(unsigned)tiles, kIxThreads, 0, st>>>(b);
   CLAST_LAUNCHED();
+  const int64_t chunks = n_records >> kIxChunkLog;
+  if (chunks > 0) {
+    k_index_free<<<(unsigned)std::min<int64_t>(chunks, 148 * 8), 256, 0, st>>>(table, chunk_free, chunks);
+    CLAST_LAUNCHED();
+  }
 }
 
 void filter_from_table(const ulonglong2* table, int64_t n_records, int l, uint32_t* filter, int fshift, int fstride,

@@ -48,3 +48,42 @@ def test_index_tiles_equal_oracle(engine, samples, poly, lmer, cut):
     ix = engine.hash_table(s, tl, 0, len(t))
     compare(engine.hit_list(s, ix, ql, 0, len(reads)), want)
     ix.close()
+
+
+@pytest.mark.parametrize("real", [0, 20, 150, 900, 30_000])
+@pytest.mark.parametrize("cut", [-1, 3])
+def test_free_records_between_few_keys(engine, real, cut):
+    """A window of N's with `real` bases in it: free stretches within a tile,
+    of one record to many whole chunks of 4,096, and a table without a record.
+    The full index built before it leaves its records in the memory that the
+    new table is given."""
+    rng = np.random.Generator(np.random.PCG64(real + 10 + cut))
+    n = 240_000
+    t = synth.ACGT[rng.integers(0, 4, size=n)]
+    s = api.Setting(lmer=12, stride=2, cut_repeat=cut, total_db=float(n))
+    full = api.SeqList(s.lmer).add_targets([t.tobytes()])
+    sparse_seq = np.full(n, ord("N"), np.uint8)
+    at = n // 3
+    sparse_seq[at:at + real] = t[at:at + real]
+    sparse = api.SeqList(s.lmer).add_targets([sparse_seq.tobytes()])
+    reads = [t[p:p + 100].tobytes() for p in list(rng.integers(0, n - 100, size=200)) + [at, at + max(0, real - 100)]]
+    ql = api.SeqList(s.lmer).add_queries(reads)
+    qb, qg, qn = ql.window(0, len(ql.lengths))
+    for tl in (full, sparse, full):
+        tb, tg, tn = tl.window(0, 1)
+        want = O.window_search(s, tb, tg, tn, 0, qb, qg, qn, 0)
+        ix = engine.hash_table(s, tl, 0, 1)
+        compare(engine.hit_list(s, ix, ql, 0, len(reads)), want)
+        ix.close()
+
+
+def test_window_without_a_sample_equals_oracle(engine):
+    s = api.Setting(lmer=8, stride=90, total_db=20.0)
+    tl = api.SeqList(s.lmer).add_targets([b"ACGTTGCAACGGTCATTGCA"])
+    ql = api.SeqList(s.lmer).add_queries([b"ACGTTGCAACGGTCATTGCA"])
+    tb, tg, tn = tl.window(0, 1)
+    qb, qg, qn = ql.window(0, len(ql.lengths))
+    want = O.window_search(s, tb, tg, tn, 0, qb, qg, qn, 0)
+    ix = engine.hash_table(s, tl, 0, 1)
+    compare(engine.hit_list(s, ix, ql, 0, 1), want)
+    ix.close()
