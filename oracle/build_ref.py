@@ -93,6 +93,9 @@ def main():
             out = os.path.join(SRC, os.path.splitext(name)[0] + ".cpp")
             open(out, "w", encoding="latin-1").write(rewrite(text))
             units.append(out)
+    if not units:
+        print("no reference sources in %s; nothing built" % ref)
+        return 0
     flags = ["-std=c++17", "-O2", "-fopenmp", "-w",
              "-DTHRUST_DEVICE_SYSTEM=THRUST_DEVICE_SYSTEM_CPP",
              "-DTHRUST_HOST_SYSTEM=THRUST_HOST_SYSTEM_CPP",
