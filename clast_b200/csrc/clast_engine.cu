@@ -96,7 +96,7 @@ void build_index_device(Workspace& ws, cudaStream_t st, const clast_params* p, c
     alloc_filters(one, 1, filter_shift(ns), st);
   }
   CLAST_CK(cudaMemsetAsync(ix->kept.p, 0, sizeof(int64_t), st));
-  const size_t words = (size_t)index_state_words(ns, ix->n_records);
+  const size_t words = (size_t)index_state_words(ns, ix->n_records, p->cut_repeat);
   unsigned long long* state = ws.get<unsigned long long>("ix_state", words);
   CLAST_CK(cudaMemsetAsync(state, 0, words * sizeof(unsigned long long), st));
   index_place(in_alt ? items2 : items, in_alt ? pos2 : pos, ns, pbits, p->stride, l, p->cut_repeat, ix->gateway.p,

@@ -644,6 +644,14 @@ __global__ void __launch_bounds__(256) k_index_free(ulonglong2* __restrict__ tab
   }
 }
 
+// A run of equal codes of which k_index_place has placed the record.
+struct IndexLong {
+  int64_t record, first, next;  // the record; the run's first sample; the first one not looked at yet
+  int64_t kept;                 // samples kept before that one
+};
+// Runs of up to this many samples are never left to k_index_long.
+constexpr int kIxLongRun = kIxThreads;
+
 struct IndexBuild {
   const uint64_t* items;  // sorted: code << pbits | sample, or codes with the samples in vals (pbits 0)
   const int32_t* vals;
@@ -662,6 +670,7 @@ struct IndexBuild {
   int fshift, fstride;
   unsigned long long* state;  // [0] tile counter, then one word per tile
   unsigned char* chunk_free;  // per whole chunk of the table: no record lies in it
+  IndexLong* longs;           // per tile: its run that k_index_long ends (kept 0: none)
   unsigned long long* kept;   // records placed
   unsigned long long* failed;
 };
@@ -772,21 +781,18 @@ __global__ void __launch_bounds__(kIxThreads, 5) k_index_place(IndexBuild b) {
       b.entries[i0 + h + rank] = res[k];
       if (rank == 0) first[h] = (uint16_t)k;
     }
-  // a run that goes on past the tile: the whole block walks it
+  // A run that goes on past the tile: the whole block walks it as far as it
+  // takes to know that the run has a record, nearly always one step.  What is
+  // then left of the run is k_index_long's, so that later tiles, which wait for
+  // this one's records, do not wait for a walk of millions of samples.
   int cross_kept = 0;
+  int64_t cross_next = 0;  // the walk goes on here
   if (cross) {
     const int64_t h = i0 + start[n_runs - 1];
-    bool pass = true;
-    if (b.cut != -1) {
-      int64_t cnt = 0;
-      for (int64_t base = h;; base += kIxThreads) {
-        const int64_t i = base + tid;
-        const int in = __syncthreads_count(i < b.ns && ix_code<PAIR>(b.items, b.pbits, i) == last_code);
-        cnt += in;
-        if (in < kIxThreads || cnt >= b.cut) break;
-      }
-      pass = cnt < b.cut;
-    }
+    // codes ascend: the run has `cut` samples if the one cut - 1 on is still its own
+    const int64_t at_cut = h + b.cut - 1;
+    const bool pass = b.cut == -1 || (b.cut > 0 && !(at_cut < b.ns &&
+                                                     ix_code<PAIR>(b.items, b.pbits, at_cut) == last_code));
     for (int64_t base = h; pass; base += kIxThreads) {
       const int64_t i = base + tid;
       int2 r = make_int2(-1, 0);
@@ -798,14 +804,16 @@ __global__ void __launch_bounds__(kIxThreads, 5) k_index_place(IndexBuild b) {
           r = ix_resolve((int64_t)(PAIR ? b.vals[i] : (int)(w & pmask)) * b.stride, b.l, b.gw, b.len, b.nseqs);
       }
       const unsigned m = __ballot_sync(kFull, r.x >= 0);
-      int total;
-      const int at = cross_kept + ix_warp_prefix(__popc(m), wbuf, &total) + __popc(m & lt);
+      const int at = ix_warp_prefix(__popc(m), wbuf, &cross_kept) + __popc(m & lt);
       if (r.x >= 0) {
         b.entries[h + at] = r;
         if (at == 0) s_cross = r;
       }
-      cross_kept += total;
       if (__syncthreads_count(in) < kIxThreads) break;
+      if (cross_kept > 0) {
+        cross_next = base + kIxThreads;
+        break;
+      }
     }
   }
   __syncthreads();
@@ -930,6 +938,8 @@ __global__ void __launch_bounds__(kIxThreads, 5) k_index_place(IndexBuild b) {
         if (at - from <= kIxOwnFree)
           for (int64_t i = from; i < at; ++i) b.table[i] = make_ulonglong2(~0ull, kNoPayload);
         b.table[at] = make_ulonglong2(c, payload);
+        if (cross_next > 0 && rid[j] == n_runs - 1)
+          b.longs[t] = IndexLong{at, i0 + k, cross_next, kc[j]};
       } else {  // unreachable: positions rise to the last one, which the table holds
         atomicAdd(b.failed, 1ull);
         at = from;
@@ -939,6 +949,62 @@ __global__ void __launch_bounds__(kIxThreads, 5) k_index_place(IndexBuild b) {
       const int src = __ffs(far) - 1;
       ix_free(b.table, b.chunk_free, __shfl_sync(kFull, from, src), __shfl_sync(kFull, at, src));
     }
+  }
+}
+
+// The rest of the runs that k_index_place left, a block per run: entries of the
+// kept samples and the record's payload.  Runs this long need the repeat cut
+// off, or above kIxLongRun, and low-complexity sequence; a block of 1,024 threads
+// takes 4,096 samples of one per step, and is bound by the step's latency.
+constexpr int kIxLongThreads = 1024, kIxLongRounds = 4;
+
+template <bool PAIR>
+__global__ void __launch_bounds__(kIxLongThreads) k_index_long(IndexBuild b, int64_t tiles) {
+  __shared__ int wbuf[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned lt = lanemask_lt();
+  const uint64_t pmask = PAIR ? 0 : (1ull << b.pbits) - 1;
+  for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const IndexLong run = b.longs[t];
+    if (run.kept == 0) continue;  // the same for the whole block
+    const uint64_t c = b.table[run.record].x;
+    int64_t kept = run.kept;
+    for (int64_t base = run.next;; base += kIxLongThreads * kIxLongRounds) {
+      int2 r[kIxLongRounds];
+      unsigned m[kIxLongRounds];
+      int n = 0;
+      bool in = false;  // of the last sample
+#pragma unroll
+      for (int j = 0; j < kIxLongRounds; ++j) {
+        const int64_t i = base + warp * (32 * kIxLongRounds) + j * 32 + lane;
+        r[j] = make_int2(-1, 0);
+        in = false;
+        if (i < b.ns) {
+          const uint64_t w = b.items[i];
+          in = (PAIR ? w : w >> b.pbits) == c;
+          if (in)
+            r[j] = ix_resolve((int64_t)(PAIR ? b.vals[i] : (int)(w & pmask)) * b.stride, b.l, b.gw, b.len, b.nseqs);
+        }
+        m[j] = __ballot_sync(kFull, r[j].x >= 0);
+        n += __popc(m[j]);
+      }
+      if (lane == 0) wbuf[warp] = n;
+      const bool more = __syncthreads_and(lane < 31 || in) != 0;  // codes ascend: every warp's last sample is in
+      int total = wbuf[lane], before = lane < warp ? total : 0;
+      total = __reduce_add_sync(kFull, total);
+      before = __reduce_add_sync(kFull, before);
+      int64_t at = run.first + kept + before;
+#pragma unroll
+      for (int j = 0; j < kIxLongRounds; ++j) {
+        if (r[j].x >= 0) b.entries[at + __popc(m[j] & lt)] = r[j];
+        at += __popc(m[j]);
+      }
+      kept += total;
+      __syncthreads();
+      if (!more) break;
+    }
+    if (tid == 0 && kept > run.kept)
+      b.table[run.record].y = kMulti | ((uint64_t)run.first << 32) | (uint32_t)kept;
   }
 }
 
@@ -3519,8 +3585,13 @@ int radix_sort_u64(Workspace& ws, uint64_t* keys, int32_t* vals, uint64_t* keys_
   return which;
 }
 
-int64_t index_state_words(int64_t n_samples, int64_t n_records) {
-  return (n_samples + kIxTile - 1) / kIxTile + 1 + ((n_records >> kIxChunkLog) + 7) / 8;
+// Runs can be longer than what k_index_place looks at of them.
+static bool index_long_runs(int cut) { return cut == -1 || cut > kIxLongRun; }
+
+int64_t index_state_words(int64_t n_samples, int64_t n_records, int cut) {
+  const int64_t tiles = (n_samples + kIxTile - 1) / kIxTile;
+  return tiles + 1 + ((n_records >> kIxChunkLog) + 7) / 8 +
+         (index_long_runs(cut) ? tiles * (int64_t)(sizeof(IndexLong) / sizeof(unsigned long long)) : 0);
 }
 
 void index_place(const uint64_t* items, const int32_t* vals, int64_t n_samples, int pbits, int stride, int l, int cut,
@@ -3532,13 +3603,20 @@ void index_place(const uint64_t* items, const int32_t* vals, int64_t n_samples, 
     return;
   }
   const int64_t tiles = (n_samples + kIxTile - 1) / kIxTile;
+  const int64_t chunks = n_records >> kIxChunkLog;
   unsigned char* chunk_free = reinterpret_cast<unsigned char*>(state + tiles + 1);
+  IndexLong* longs = reinterpret_cast<IndexLong*>(state + tiles + 1 + (chunks + 7) / 8);
   const IndexBuild b{items, vals, n_samples, pbits, 1ull << (2 * l), stride, l, cut, gateway, lengths, nseqs, nbuckets,
-                     entries, table, n_records, filter, fshift, fstride, state, chunk_free, kept, failed};
+                     entries, table, n_records, filter, fshift, fstride, state, chunk_free, longs, kept, failed};
   if (pbits > 0) k_index_place<false><<<(unsigned)tiles, kIxThreads, 0, st>>>(b);
   else k_index_place<true><<<(unsigned)tiles, kIxThreads, 0, st>>>(b);
   CLAST_LAUNCHED();
-  const int64_t chunks = n_records >> kIxChunkLog;
+  if (index_long_runs(cut)) {
+    const unsigned grid = (unsigned)std::min<int64_t>(tiles, 148 * 2);
+    if (pbits > 0) k_index_long<false><<<grid, kIxLongThreads, 0, st>>>(b, tiles);
+    else k_index_long<true><<<grid, kIxLongThreads, 0, st>>>(b, tiles);
+    CLAST_LAUNCHED();
+  }
   if (chunks > 0) {
     k_index_free<<<(unsigned)std::min<int64_t>(chunks, 148 * 8), 256, 0, st>>>(table, chunk_free, chunks);
     CLAST_LAUNCHED();

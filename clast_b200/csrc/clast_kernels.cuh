@@ -51,10 +51,10 @@ int radix_sort_u64(Workspace& ws, uint64_t* keys, int32_t* vals, uint64_t* keys_
 // the kept ones (n_samples long, runs of equal codes apart), the hash table
 // without atomics (layout: IndexView; every record of it is written, free ones
 // as ~0) and the filter (zeroed by the caller).  state:
-// index_state_words(n_samples, n_records) zeroed words; *kept is raised by the
+// index_state_words(n_samples, n_records, cut) zeroed words; *kept is raised by the
 // records placed, *failed by records outside the table and by waits that gave
 // up (neither happens).
-int64_t index_state_words(int64_t n_samples, int64_t n_records);
+int64_t index_state_words(int64_t n_samples, int64_t n_records, int cut);
 void index_place(const uint64_t* items, const int32_t* vals, int64_t n_samples, int pbits, int stride, int l, int cut,
                  const int32_t* gateway, const int32_t* lengths, int nseqs, uint32_t nbuckets, int2* entries,
                  ulonglong2* table, int64_t n_records, uint32_t* filter, int fshift, int fstride,

@@ -87,3 +87,27 @@ def test_window_without_a_sample_equals_oracle(engine):
     ix = engine.hash_table(s, tl, 0, 1)
     compare(engine.hit_list(s, ix, ql, 0, 1), want)
     ix.close()
+
+
+# k_index_place looks at 256 samples of a run that leaves its tile, the kernel
+# after it at 4,096 a step; the last size takes many thousand steps of a block
+@pytest.mark.parametrize("cut", [-1, 257, 5000, 5_000_000])
+@pytest.mark.parametrize("run", [255, 256, 257, 258, 256 + 4096, 256 + 4097, 30_000, 3_000_000])
+def test_long_runs_equal_oracle(engine, run, cut):
+    lmer, rng = 13, np.random.Generator(np.random.PCG64(run + cut))
+    flank = [synth.ACGT[rng.integers(1, 4, size=m)].tobytes() for m in (1500, 700, 900)]  # no A beside the run
+    poly = min(run, 1000)  # of `run` samples of poly-A, so many in a second sequence, up to its end
+    rest = run - poly
+    t = [flank[0] + (b"A" * (rest + lmer - 1) if rest else b"") + flank[1], flank[2] + b"A" * (poly + lmer - 1)]
+    s = api.Setting(lmer=lmer, stride=1, cut_repeat=cut, total_db=float(sum(map(len, t))))
+    reads = [x[p:p + 90] for x in flank for p in range(0, len(x) - 90, 61)]
+    if run < 1_000_000:  # one l-mer of the run in each: as many seeds as the run has samples
+        reads += [flank[2][-60:] + b"A" * lmer, b"A" * lmer + flank[1][:60]]
+    tl = api.SeqList(s.lmer).add_targets(t)
+    ql = api.SeqList(s.lmer).add_queries(reads)
+    tb, tg, tn = tl.window(0, len(t))
+    qb, qg, qn = ql.window(0, len(ql.lengths))
+    want = O.window_search(s, tb, tg, tn, 0, qb, qg, qn, 0)
+    ix = engine.hash_table(s, tl, 0, len(t))
+    compare(engine.hit_list(s, ix, ql, 0, len(reads)), want)
+    ix.close()
