@@ -435,10 +435,8 @@ def served_leg(eng, s, t, t_loads, args):
 # ---------------------------------------------------------------------------
 def uneven_leg(eng, s, t, t_loads, reads, args):
     """The batched uneven-read shape: the medium target and reads of 50 bp -
-    10 kbp (per-read error 1-12 %), mapped in one clast_map per step with the
-    DP's order and launch chosen by the context's autotuner; beside it the
-    same job with the autotuner off (exact sort, one thread per hit over a
-    full grid).  Mbp/s with inputs in HBM, CUDA events."""
+    10 kbp (per-read error 1-12 %), mapped in one clast_map per step.  Mbp/s
+    with inputs in HBM, CUDA events."""
     import torch
     qb, ql = reads
     q_off = np.concatenate([[0], np.cumsum(ql)]).astype(np.int64)
@@ -472,20 +470,10 @@ def uneven_leg(eng, s, t, t_loads, reads, args):
                     "dp_ms": round(st["dp_ms"], 2), "dp_order_ms": round(st["dp_order_ms"], 2),
                     "dp_gcups": round(st["dp_cells"] / (st["dp_ms"] / 1e3) / 1e9, 1) if st["dp_ms"] > 0 else None,
                     "dp_frac_int32": round(dp_frac, 4) if dp_frac else None,
-                    "dp_order": {0: "none", 1: "sorted by rows", 2: "length buckets"}[st["dp_order_kind"]],
-                    "dp_launch": ("persistent queue, %d x 32 hits per take" % st["dp_queue_chunk"])
-                    if st["dp_queue_chunk"] else "one thread per hit, full grid",
+                    "dp_order": {0: "none", 1: "sorted by rows"}[st["dp_order_kind"]],
                     "dp_warp_hits": st["dp_warp_hits"]}
 
-    run(eng, "tuned")
-    os.environ["CLAST_DP_NO_TUNE"] = "1"
-    plain = api.Engine(torch.cuda.current_device())
-    try:
-        run(plain, "untuned")
-    finally:
-        plain.close()
-        del os.environ["CLAST_DP_NO_TUNE"]
-    out["tuned_over_untuned"] = round(out["tuned"]["value"] / out["untuned"]["value"], 3)
+    run(eng, "map")
     return out
 
 
@@ -716,8 +704,8 @@ def run_ours(args):
     ix_bytes = st["index_bases"] / 4 + 12 * st["index_bases"] / s.stride + 16 * st["index_keys"]
     filt_bytes = 16 * st["seeds"] + 16 * st["hits"]
     roofline = {
-        "kernel": "seeding (k_seed_multi: l-mer keys, filter + table lookups of two target windows per pass, "
-                  "seed writes)",
+        "kernel": "seeding (k_seed_reads: l-mer keys, filter + table lookups of both strands in two target windows "
+                  "per pass, seed filters of reads with few seeds)",
         "bound": "hbm", "achieved": round(seed_gbs, 1), "peak": hbm_peak, "unit": "GB/s",
         "frac": round(seed_gbs / hbm_peak, 4),
         "peak_source": peak_src,
