@@ -2464,6 +2464,12 @@ __device__ __forceinline__ int2 cell_score(int t, int q) {
 // diagonal); otherwise V wins iff V >= diagonal.
 constexpr int kStepRow = 4, kStepCol = 2;
 constexpr int kOpenPot = kGapOpen + kGapExtend + kStepCol;  // -5
+// The integer kernel takes kStepRow * kDpRebaseRows out of its potentials every
+// kDpRebaseRows rows, and starts that much below zero, so that they stay below
+// S + 200 whatever the number of rows: without it a matching read's potentials
+// rise by 5 per row and pass 2^31 at row 429,496,729.  Half a dozen subtractions
+// per 4,096 rows; short enough that reads of some kbp go through several.
+constexpr int kDpRebaseRows = 4096;
 
 // Shared memory of a DP block: the letter-pair table (POINT + 4, match
 // increment) by class, and the classes' byte offsets into it by letter byte
@@ -2774,6 +2780,17 @@ __device__ __forceinline__ void banded_hit_warp(const DpTab<int2>& tab, const ch
     dp_init_col<GAP>(ce, se, ue, me);
     dp_init_col<GAP>(co, so, uo, mo);
     int ho = 0;
+    int lift = kStepRow * (1 - lane);  // of the lane's row: kStepRow * (row + 1), less what rebase() took out
+    auto rebase = [&]() {
+      constexpr int d = kStepRow * kDpRebaseRows;
+      se -= d;
+      ue -= d;
+      so -= d;
+      uo -= d;
+      ho -= d;
+      lift -= d;
+    };
+    rebase();
     int bs = 0, bm = 0, calc = -1, ep = GAP;
     // Row r of this lane uses the target bases r + 2j (even column; the odd
     // column's base of row r - 1) and r + 2j + 1, and query base r.  Bytes are
@@ -2791,7 +2808,6 @@ __device__ __forceinline__ void banded_hit_warp(const DpTab<int2>& tab, const ch
     char t4 = t_byte(ib0 + step * (r + 4 + co));
     char q2 = q_byte(r + 2), q3 = q_byte(r + 3), q4 = q_byte(r + 4);
     int tk = ib0 + step * (r + 5 + co);
-    int lift = kStepRow * (r + 1);
     // One row.  EDGE: some lanes may be outside the pass's rows and keep their state.
     auto row = [&](auto edge) {
       constexpr bool EDGE = decltype(edge)::value;
@@ -2851,8 +2867,12 @@ __device__ __forceinline__ void banded_hit_warp(const DpTab<int2>& tab, const ch
     // lane GAP starts GAP rows after lane 0 and ends GAP rows after it
     const int n_ramp = min(GAP, rows_p);
     for (int it = 0; it < n_ramp; ++it) row(std::true_type());
+    for (int it = n_ramp; it < rows_p;) {
+      const int stop = rows_p - it > kDpRebaseRows ? it + kDpRebaseRows : rows_p;
 #pragma unroll 2
-    for (int it = n_ramp; it < rows_p; ++it) row(std::false_type());
+      for (; it < stop; ++it) row(std::false_type());
+      rebase();  // every lane at once, whatever row it is in: the lanes' states stay comparable
+    }
     for (int it = 0; it < GAP; ++it) row(std::true_type());
     int best, best_m, e, move;
     if (LOCAL) {  // first maximum in row-major order: (score desc, row asc, column asc)
@@ -2868,8 +2888,9 @@ __device__ __forceinline__ void banded_hit_warp(const DpTab<int2>& tab, const ch
       move = calc + 1;
     } else {  // end node: the first column of the last row with the highest score above the margin
       int sc = INT_MIN, c = W, m = 0;
-      if (has_e) { sc = se - kStepRow * rows_p - kStepCol * ce; c = ce; m = me; }
-      const int sco = so - kStepRow * rows_p - kStepCol * co;
+      const int top = lift - kStepRow * (GAP - lane + 1);  // the last row's lift: lane j ended GAP - j rows ago
+      if (has_e) { sc = se - top - kStepCol * ce; c = ce; m = me; }
+      const int sco = so - top - kStepCol * co;
       if (has_o && sco > sc) { sc = sco; c = co; m = mo; }
 #pragma unroll
       for (int off = 16; off; off >>= 1) {
