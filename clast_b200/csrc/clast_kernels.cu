@@ -45,6 +45,18 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 // ------------------------------------------------------------------------
 // exclusive scan
 // ------------------------------------------------------------------------
+// Exclusive prefix sum over the warp; *total = the warp's sum.
+__device__ __forceinline__ int warp_excl_scan(int v, int lane, int* total) {
+  int incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(kFull, incl, o);
+    if (lane >= o) incl += y;
+  }
+  *total = __shfl_sync(kFull, incl, 31);
+  return incl - v;
+}
+
 constexpr int kScanThreads = 256, kScanItems = 8, kScanTile = kScanThreads * kScanItems;
 
 // Element loader of the scans.
@@ -644,12 +656,24 @@ __global__ void __launch_bounds__(256) k_index_free(ulonglong2* __restrict__ tab
   }
 }
 
-// A run of equal codes of which k_index_place has placed the record.
-struct IndexLong {
-  int64_t record, first, next;  // the record; the run's first sample; the first one not looked at yet
-  int64_t kept;                 // samples kept before that one
+// The samples at the start of a tile that belong to a run begun in an earlier
+// tile.  With the repeat cut off, or above kIxLongRun, such a run can span any
+// number of tiles, and whether it has a record at all (samples on joints are
+// none) may only show in its last one.  So k_index_leads looks at all tiles'
+// before the placement, the tile that holds a run's first sample adds them up,
+// a word per tile, and k_index_lead_entries writes their entries after it: no
+// tile waits for another one's walk over samples.  Stride 1 without a cut, index
+// of a 60 Mbp window of poly-A 4.3 ms, of one with 100 runs of 100 kbp 4.15, of
+// 400,000 records of 14 A's 8.7; with one block walking each such run 54.6, 14.7
+// and no index (the later tiles' waits ran out).  Windows without such runs pay
+// two launches: 1.00 against 0.97 ms for 12 M samples.
+struct IndexLead {
+  int32_t kept;   // samples of them that no joint holds
+  int32_t whole;  // the run goes on past the tile
+  int2 first;     // the first kept one
+  int64_t to;     // where the kept ones go in the entries; -1: the run is cut
 };
-// Runs of up to this many samples are never left to k_index_long.
+// Runs that pass a repeat cut of up to this are seen whole by one step of a block.
 constexpr int kIxLongRun = kIxThreads;
 
 struct IndexBuild {
@@ -670,12 +694,53 @@ struct IndexBuild {
   int fshift, fstride;
   unsigned long long* state;  // [0] tile counter, then one word per tile
   unsigned char* chunk_free;  // per whole chunk of the table: no record lies in it
-  IndexLong* longs;           // per tile: its run that k_index_long ends (kept 0: none)
+  IndexLead* leads;           // per tile, with the cut off or above kIxLongRun
   unsigned long long* kept;   // records placed
   unsigned long long* failed;
 };
 
 template <bool PAIR>
+__global__ void __launch_bounds__(kIxThreads) k_index_leads(IndexBuild b) {
+  __shared__ int s_first;
+  const int64_t t = blockIdx.x, i0 = t * kIxTile;
+  const uint64_t c = ix_code<PAIR>(b.items, b.pbits, i0);
+  IndexLead* const lead = b.leads + t;
+  if (t == 0 || c >= b.bound || ix_code<PAIR>(b.items, b.pbits, i0 - 1) != c) {  // the same for the whole block
+    if (threadIdx.x == 0) *lead = IndexLead{0, 0, make_int2(-1, 0), -1};
+    return;
+  }
+  if (threadIdx.x == 0) s_first = kIxTile;
+  __syncthreads();
+  const uint64_t pmask = PAIR ? 0 : (1ull << b.pbits) - 1;
+  int kept = 0, mine = kIxTile;
+  int2 r_mine = make_int2(-1, 0);
+#pragma unroll
+  for (int j = kIxRounds - 1; j >= 0; --j) {
+    const int k = j * kIxThreads + (int)threadIdx.x;
+    bool keep = false;
+    if (i0 + k < b.ns) {
+      const uint64_t w = b.items[i0 + k];
+      if ((PAIR ? w : w >> b.pbits) == c) {
+        const int2 r = ix_resolve((int64_t)(PAIR ? b.vals[i0 + k] : (int)(w & pmask)) * b.stride, b.l, b.gw, b.len, b.nseqs);
+        keep = r.x >= 0;
+        if (keep) {
+          mine = k;
+          r_mine = r;
+        }
+      }
+    }
+    kept += __syncthreads_count(keep);
+  }
+  if (mine < kIxTile) atomicMin(&s_first, mine);
+  __syncthreads();
+  if (kept ? mine == s_first : threadIdx.x == 0) {
+    const int64_t next = i0 + kIxTile;
+    *lead = IndexLead{kept, next < b.ns && ix_code<PAIR>(b.items, b.pbits, next) == c, r_mine, -1};
+  }
+}
+
+// LONG: the cut is off or above kIxLongRun (see IndexLead).
+template <bool PAIR, bool LONG>
 __global__ void __launch_bounds__(kIxThreads, 5) k_index_place(IndexBuild b) {
   __shared__ uint64_t code[kIxTile + 1];
   __shared__ int2 res[kIxTile];
@@ -742,6 +807,12 @@ __global__ void __launch_bounds__(kIxThreads, 5) k_index_place(IndexBuild b) {
   // the last run may go on past the tile
   const uint64_t last_code = n_runs > 0 ? code[start[n_runs - 1]] : ~0ull;
   const bool cross = n_runs > 0 && nt == kIxTile && last_code < b.bound && code[kIxTile] == last_code;
+  bool cross_pass = false;  // it passes the cut: codes ascend, so it has `cut` samples if the one cut - 1 on is its own
+  if (cross) {
+    const int64_t at_cut = i0 + start[n_runs - 1] + b.cut - 1;
+    cross_pass = b.cut == -1 ||
+                 (b.cut > 0 && !(at_cut < b.ns && ix_code<PAIR>(b.items, b.pbits, at_cut) == last_code));
+  }
   // kept samples
   unsigned kept = 0;
   {
@@ -751,9 +822,10 @@ __global__ void __launch_bounds__(kIxThreads, 5) k_index_place(IndexBuild b) {
     for (int j = 0; j < kIxRounds; ++j) {
       const int k = warp * kIxWarpItems + j * 32 + lane;
       bool keep = false;
-      if (k < nt && code[k] < b.bound && rid[j] >= 0 && !(cross && rid[j] == n_runs - 1)) {
+      const bool last = cross && rid[j] == n_runs - 1;
+      if (k < nt && code[k] < b.bound && rid[j] >= 0 && (LONG || !last)) {
         const int cnt = start[rid[j] + 1] - start[rid[j]];
-        if (b.cut == -1 || cnt < b.cut) {  // removeRepeatedSequence
+        if (LONG && last ? cross_pass : b.cut == -1 || cnt < b.cut) {  // removeRepeatedSequence
           const int2 r = ix_resolve((int64_t)pos[j] * b.stride, b.l, b.gw, b.len, b.nseqs);
           keep = r.x >= 0;
           res[k] = r;
@@ -781,40 +853,54 @@ __global__ void __launch_bounds__(kIxThreads, 5) k_index_place(IndexBuild b) {
       b.entries[i0 + h + rank] = res[k];
       if (rank == 0) first[h] = (uint16_t)k;
     }
-  // A run that goes on past the tile: the whole block walks it as far as it
-  // takes to know that the run has a record, nearly always one step.  What is
-  // then left of the run is k_index_long's, so that later tiles, which wait for
-  // this one's records, do not wait for a walk of millions of samples.
+  // A run that goes on past the tile: its samples from there on that are kept.
+  // A run that passes a cut of up to kIxLongRun ends within one step of the block.
   int cross_kept = 0;
-  int64_t cross_next = 0;  // the walk goes on here
-  if (cross) {
-    const int64_t h = i0 + start[n_runs - 1];
-    // codes ascend: the run has `cut` samples if the one cut - 1 on is still its own
-    const int64_t at_cut = h + b.cut - 1;
-    const bool pass = b.cut == -1 || (b.cut > 0 && !(at_cut < b.ns &&
-                                                     ix_code<PAIR>(b.items, b.pbits, at_cut) == last_code));
-    for (int64_t base = h; pass; base += kIxThreads) {
-      const int64_t i = base + tid;
-      int2 r = make_int2(-1, 0);
-      bool in = false;
-      if (i < b.ns) {
-        const uint64_t w = b.items[i];
-        in = (PAIR ? w : w >> b.pbits) == last_code;
-        if (in)
-          r = ix_resolve((int64_t)(PAIR ? b.vals[i] : (int)(w & pmask)) * b.stride, b.l, b.gw, b.len, b.nseqs);
-      }
-      const unsigned m = __ballot_sync(kFull, r.x >= 0);
-      const int at = ix_warp_prefix(__popc(m), wbuf, &cross_kept) + __popc(m & lt);
-      if (r.x >= 0) {
-        b.entries[h + at] = r;
-        if (at == 0) s_cross = r;
-      }
-      if (__syncthreads_count(in) < kIxThreads) break;
-      if (cross_kept > 0) {
-        cross_next = base + kIxThreads;
-        break;
-      }
+  if (cross_pass && !LONG) {
+    const int64_t h = i0 + start[n_runs - 1], i = h + tid;
+    int2 r = make_int2(-1, 0);
+    if (i < b.ns) {
+      const uint64_t w = b.items[i];
+      if ((PAIR ? w : w >> b.pbits) == last_code)
+        r = ix_resolve((int64_t)(PAIR ? b.vals[i] : (int)(w & pmask)) * b.stride, b.l, b.gw, b.len, b.nseqs);
     }
+    const unsigned m = __ballot_sync(kFull, r.x >= 0);
+    const int at = ix_warp_prefix(__popc(m), wbuf, &cross_kept) + __popc(m & lt);
+    if (r.x >= 0) {
+      b.entries[h + at] = r;
+      if (at == 0) s_cross = r;
+    }
+  }
+  int own = 0;  // kept samples of that run within the tile
+  if (cross_pass && LONG) {
+    own = kpre[kIxTile] - kpre[start[n_runs - 1]];
+    const int64_t h = i0 + start[n_runs - 1] + own;
+    for (int64_t u = t + 1;; u += kIxThreads) {
+      IndexLead* const lead = b.leads + u + tid;
+      const bool in = u + tid < (int64_t)gridDim.x;
+      const int k0 = in ? lead->kept : 0;
+      const unsigned ends = __ballot_sync(kFull, !in || !lead->whole);
+      if (lane == 0) wbuf[warp] = ends ? 1 : 0;
+      __syncthreads();
+      bool part = !(ends & lt), done = false;  // the run's tiles: up to the first one that it does not fill
+#pragma unroll
+      for (int w = 0; w < kIxWarps; ++w) {
+        if (w < warp && wbuf[w]) part = false;
+        if (wbuf[w]) done = true;
+      }
+      __syncthreads();
+      int all;
+      const int k = part ? k0 : 0, before = warp_excl_scan(k, lane, &all);
+      const int at = ix_warp_prefix(all, wbuf, &all) + before;
+      if (k > 0) {
+        lead->to = h + cross_kept + at;
+        if (own == 0 && cross_kept + at == 0) s_cross = lead->first;
+      }
+      cross_kept += all;
+      if (done) break;
+    }
+    if (own > 0 && tid == 0) s_cross = res[first[start[n_runs - 1]]];
+    cross_kept += own;
   }
   __syncthreads();
   // records: u = rank within the tile, slack = home - u, the maximum of the records before
@@ -938,8 +1024,6 @@ __global__ void __launch_bounds__(kIxThreads, 5) k_index_place(IndexBuild b) {
         if (at - from <= kIxOwnFree)
           for (int64_t i = from; i < at; ++i) b.table[i] = make_ulonglong2(~0ull, kNoPayload);
         b.table[at] = make_ulonglong2(c, payload);
-        if (cross_next > 0 && rid[j] == n_runs - 1)
-          b.longs[t] = IndexLong{at, i0 + k, cross_next, kc[j]};
       } else {  // unreachable: positions rise to the last one, which the table holds
         atomicAdd(b.failed, 1ull);
         at = from;
@@ -952,59 +1036,31 @@ __global__ void __launch_bounds__(kIxThreads, 5) k_index_place(IndexBuild b) {
   }
 }
 
-// The rest of the runs that k_index_place left, a block per run: entries of the
-// kept samples and the record's payload.  Runs this long need the repeat cut
-// off, or above kIxLongRun, and low-complexity sequence; a block of 1,024 threads
-// takes 4,096 samples of one per step, and is bound by the step's latency.
-constexpr int kIxLongThreads = 1024, kIxLongRounds = 4;
-
+// The entries of the leads (see IndexLead) whose run has a record.
 template <bool PAIR>
-__global__ void __launch_bounds__(kIxLongThreads) k_index_long(IndexBuild b, int64_t tiles) {
-  __shared__ int wbuf[32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const unsigned lt = lanemask_lt();
+__global__ void __launch_bounds__(kIxThreads) k_index_lead_entries(IndexBuild b, int64_t tiles) {
+  __shared__ int wbuf[kIxWarps];
+  const int tid = threadIdx.x, lane = tid & 31;
   const uint64_t pmask = PAIR ? 0 : (1ull << b.pbits) - 1;
   for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-    const IndexLong run = b.longs[t];
-    if (run.kept == 0) continue;  // the same for the whole block
-    const uint64_t c = b.table[run.record].x;
-    int64_t kept = run.kept;
-    for (int64_t base = run.next;; base += kIxLongThreads * kIxLongRounds) {
-      int2 r[kIxLongRounds];
-      unsigned m[kIxLongRounds];
-      int n = 0;
-      bool in = false;  // of the last sample
-#pragma unroll
-      for (int j = 0; j < kIxLongRounds; ++j) {
-        const int64_t i = base + warp * (32 * kIxLongRounds) + j * 32 + lane;
-        r[j] = make_int2(-1, 0);
-        in = false;
-        if (i < b.ns) {
-          const uint64_t w = b.items[i];
-          in = (PAIR ? w : w >> b.pbits) == c;
-          if (in)
-            r[j] = ix_resolve((int64_t)(PAIR ? b.vals[i] : (int)(w & pmask)) * b.stride, b.l, b.gw, b.len, b.nseqs);
-        }
-        m[j] = __ballot_sync(kFull, r[j].x >= 0);
-        n += __popc(m[j]);
+    const int64_t i0 = t * kIxTile;
+    int64_t to = b.leads[t].to;
+    if (b.leads[t].kept == 0 || to < 0) continue;  // the same for the whole block
+    const uint64_t c = ix_code<PAIR>(b.items, b.pbits, i0);
+    for (int j = 0; j < kIxRounds; ++j) {
+      const int64_t i = i0 + j * kIxThreads + tid;
+      int2 r = make_int2(-1, 0);
+      if (i < b.ns) {
+        const uint64_t w = b.items[i];
+        if ((PAIR ? w : w >> b.pbits) == c)
+          r = ix_resolve((int64_t)(PAIR ? b.vals[i] : (int)(w & pmask)) * b.stride, b.l, b.gw, b.len, b.nseqs);
       }
-      if (lane == 0) wbuf[warp] = n;
-      const bool more = __syncthreads_and(lane < 31 || in) != 0;  // codes ascend: every warp's last sample is in
-      int total = wbuf[lane], before = lane < warp ? total : 0;
-      total = __reduce_add_sync(kFull, total);
-      before = __reduce_add_sync(kFull, before);
-      int64_t at = run.first + kept + before;
-#pragma unroll
-      for (int j = 0; j < kIxLongRounds; ++j) {
-        if (r[j].x >= 0) b.entries[at + __popc(m[j] & lt)] = r[j];
-        at += __popc(m[j]);
-      }
-      kept += total;
-      __syncthreads();
-      if (!more) break;
+      const unsigned m = __ballot_sync(kFull, r.x >= 0);
+      int all;
+      const int at = ix_warp_prefix(__popc(m), wbuf, &all) + __popc(m & lanemask_lt());
+      if (r.x >= 0) b.entries[to + at] = r;
+      to += all;
     }
-    if (tid == 0 && kept > run.kept)
-      b.table[run.record].y = kMulti | ((uint64_t)run.first << 32) | (uint32_t)kept;
   }
 }
 
@@ -1148,18 +1204,6 @@ __device__ __forceinline__ void seed_put(const IndexView& ix, const TargetView& 
     const int2 e = multi ? __ldcs(ix.entries + us + i) : make_int2((int)(pl >> 32), (int)(uint32_t)pl);
     seed_store(e, qi, local ? 0 : t.lengths[e.x], gap, local, qlen, w + i, valid, skey, sq);
   }
-}
-
-// Exclusive prefix sum over the warp; *total = the warp's sum.
-__device__ __forceinline__ int warp_excl_scan(int v, int lane, int* total) {
-  int incl = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(kFull, incl, o);
-    if (lane >= o) incl += y;
-  }
-  *total = __shfl_sync(kFull, incl, 31);
-  return incl - v;
 }
 
 // Writes a round's seeds (lane L's l-mers r0 + L*P .. in order, lanes in
@@ -3606,13 +3650,13 @@ int radix_sort_u64(Workspace& ws, uint64_t* keys, int32_t* vals, uint64_t* keys_
   return which;
 }
 
-// Runs can be longer than what k_index_place looks at of them.
+// Runs that pass the cut can span more than a tile and the next (see IndexLead).
 static bool index_long_runs(int cut) { return cut == -1 || cut > kIxLongRun; }
 
 int64_t index_state_words(int64_t n_samples, int64_t n_records, int cut) {
   const int64_t tiles = (n_samples + kIxTile - 1) / kIxTile;
   return tiles + 1 + ((n_records >> kIxChunkLog) + 7) / 8 +
-         (index_long_runs(cut) ? tiles * (int64_t)(sizeof(IndexLong) / sizeof(unsigned long long)) : 0);
+         (index_long_runs(cut) ? tiles * (int64_t)(sizeof(IndexLead) / sizeof(unsigned long long)) : 0);
 }
 
 void index_place(const uint64_t* items, const int32_t* vals, int64_t n_samples, int pbits, int stride, int l, int cut,
@@ -3626,18 +3670,24 @@ void index_place(const uint64_t* items, const int32_t* vals, int64_t n_samples, 
   const int64_t tiles = (n_samples + kIxTile - 1) / kIxTile;
   const int64_t chunks = n_records >> kIxChunkLog;
   unsigned char* chunk_free = reinterpret_cast<unsigned char*>(state + tiles + 1);
-  IndexLong* longs = reinterpret_cast<IndexLong*>(state + tiles + 1 + (chunks + 7) / 8);
+  IndexLead* leads = reinterpret_cast<IndexLead*>(state + tiles + 1 + (chunks + 7) / 8);
   const IndexBuild b{items, vals, n_samples, pbits, 1ull << (2 * l), stride, l, cut, gateway, lengths, nseqs, nbuckets,
-                     entries, table, n_records, filter, fshift, fstride, state, chunk_free, longs, kept, failed};
-  if (pbits > 0) k_index_place<false><<<(unsigned)tiles, kIxThreads, 0, st>>>(b);
-  else k_index_place<true><<<(unsigned)tiles, kIxThreads, 0, st>>>(b);
-  CLAST_LAUNCHED();
+                     entries, table, n_records, filter, fshift, fstride, state, chunk_free, leads, kept, failed};
+  const unsigned grid = (unsigned)tiles, some = (unsigned)std::min<int64_t>(tiles, 148 * 8);
   if (index_long_runs(cut)) {
-    const unsigned grid = (unsigned)std::min<int64_t>(tiles, 148 * 2);
-    if (pbits > 0) k_index_long<false><<<grid, kIxLongThreads, 0, st>>>(b, tiles);
-    else k_index_long<true><<<grid, kIxLongThreads, 0, st>>>(b, tiles);
+    if (pbits > 0) k_index_leads<false><<<grid, kIxThreads, 0, st>>>(b);
+    else k_index_leads<true><<<grid, kIxThreads, 0, st>>>(b);
     CLAST_LAUNCHED();
+    if (pbits > 0) k_index_place<false, true><<<grid, kIxThreads, 0, st>>>(b);
+    else k_index_place<true, true><<<grid, kIxThreads, 0, st>>>(b);
+    CLAST_LAUNCHED();
+    if (pbits > 0) k_index_lead_entries<false><<<some, kIxThreads, 0, st>>>(b, tiles);
+    else k_index_lead_entries<true><<<some, kIxThreads, 0, st>>>(b, tiles);
+  } else {
+    if (pbits > 0) k_index_place<false, false><<<grid, kIxThreads, 0, st>>>(b);
+    else k_index_place<true, false><<<grid, kIxThreads, 0, st>>>(b);
   }
+  CLAST_LAUNCHED();
   if (chunks > 0) {
     k_index_free<<<(unsigned)std::min<int64_t>(chunks, 148 * 8), 256, 0, st>>>(table, chunk_free, chunks);
     CLAST_LAUNCHED();
