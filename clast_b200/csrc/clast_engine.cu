@@ -389,7 +389,8 @@ int64_t search_group(clast_ctx* c, Workspace& ws, const clast_params* p, const Q
   // from the length buckets, or for equal lengths from the row count).
   const int min_len = qb.lens ? qb.lens[0] : qb.min_len, max_len = qb.lens ? qb.lens[1] : qb.max_len;
   const bool uneven = max_len != min_len && H > 1;
-  const int warp_mode = max_len > kDpMaxThreadLen ? kDpWarpAll : dp_warp_mode_from_env(c->dp_warp);
+  const int warp_mode = dp_warp_mode_from_env(c->dp_warp);
+  const bool long_hits = uneven && max_len - p->lmer >= kDpMaxThreadRows;
   c->stats.dp_order_kind = uneven ? 1 : 0;
   c->stats.dp_queue_chunk = 0;
   DpBuckets buckets;
@@ -403,12 +404,13 @@ int64_t search_group(clast_ctx* c, Workspace& ws, const clast_params* p, const Q
     uint64_t* ok2 = ws.get<uint64_t>("h_order2", H);
     dp_order_keys(hs, nw, q.len, H, p->lmer, rows_max, ok, st);
     order = radix_sort_u64(ws, ok, nullptr, ok2, nullptr, H, 32, 32 + bits, st) ? ok2 : ok;
-    if (warp_mode == kDpWarpAuto) buckets = dp_bucket_count(ws, hs, nw, q.len, H, p->lmer, st);
+    if (warp_mode == kDpWarpAuto || long_hits) buckets = dp_bucket_count(ws, hs, nw, q.len, H, p->lmer, st);
     tm.end(StageTimer::DPORDER, st);
   }
   tm.begin(st);
   DpLaunch dl;
   dl.warp = warp_mode;
+  dl.long_hits = long_hits;
   dl.buckets = buckets;
   dl.warp_n = &ctl->dp_warp;
   dl.aux = c->st_dp;

@@ -2588,7 +2588,7 @@ __device__ __forceinline__ float max3_f32(float a, float b, float c) {
 //
 // Bound by the ALU pipe (79 % busy on 2 kbp reads), where a warp instruction
 // takes two cycles and where maxima, compares and selects run whatever their
-// type.  So the whole numbers are held in floats (exact: see kDpMaxThreadLen):
+// type.  So the whole numbers are held in floats (exact: see kDpMaxThreadRows):
 // their additions run on the FMA pipe instead, at twice the rate, and a cell's
 // ALU work is one three-way and two two-way maxima, two compares and two
 // selects.  The columns' letters are packed four to a word, one dp4a makes a
@@ -3203,35 +3203,35 @@ __host__ __device__ __forceinline__ double dp_split_cycles(int W, long long s, d
   return fmax(lat + 0.5 * issue, issue) + (s > 0 ? kDpLaunchCycles : 0.0);
 }
 
-// The split on the device: every bucket boundary (longest first) is a
-// candidate; the earliest estimated end wins.  One thread; ~500 buckets.
+// The split on the device: the hits of kDpMaxThreadRows rows or more one per
+// warp; then, with `split`, every bucket boundary (longest first) is a candidate,
+// and the earliest estimated end wins.  One thread; ~500 buckets.
 __global__ void k_dp_warp_split(const unsigned int* __restrict__ count, const unsigned long long* __restrict__ rows,
-                                int W, long long cap, long long* __restrict__ warp_n) {
+                                int W, long long cap, bool split, long long* __restrict__ warp_n) {
   if (threadIdx.x != 0) return;
   double total = 0;
   for (int b = 0; b < kDpBuckets; ++b) total += (double)rows[b];
   long long s = 0, best_s = 0;
   double sw = 0, r1 = -1, best = 0;
-  bool all_taken = true;
+  bool all_taken = true, any = false;  // any: `best` holds a candidate's time
   for (int b = 0; b < kDpBuckets; ++b) {
     if (!count[b]) continue;
     const double rn = (double)dp_bucket_hi(b);
-    // candidate: the buckets before b one per warp, b and the rest one per thread
-    if (r1 < 0) {
-      r1 = rn;
-      best = dp_split_cycles(W, 0, 0, 0, rn, total);
-    } else {
-      const double t = dp_split_cycles(W, s, r1, sw, rn, total - sw);
-      if (t < best) { best = t; best_s = s; }
-    }
-    if (dp_bucket_lo(b) < kDpWarpMinRows || s + count[b] > cap) {
-      all_taken = false;
-      break;
+    if (r1 < 0) r1 = rn;
+    if (dp_bucket_lo(b) < kDpMaxThreadRows) {
+      // candidate: the buckets before b one per warp, b and the rest one per thread
+      const double t = dp_split_cycles(W, s, s > 0 ? r1 : 0, sw, rn, total - sw);
+      if (!any || t < best) { best = t; best_s = s; }
+      any = true;
+      if (!split || dp_bucket_lo(b) < kDpWarpMinRows || s + count[b] > cap) {
+        all_taken = false;
+        break;
+      }
     }
     s += count[b];
     sw += (double)rows[b];
   }
-  if (all_taken && s > 0 && dp_split_cycles(W, s, r1, sw, 0, 0) < best) best_s = s;  // every hit one per warp
+  if (all_taken && s > 0 && (!any || dp_split_cycles(W, s, r1, sw, 0, 0) < best)) best_s = s;  // every hit one per warp
   *warp_n = best_s;
 }
 
@@ -3259,17 +3259,15 @@ long long launch_dp_mode(DpKernelArgs a, const DpLaunch& m, cudaStream_t st) {
   const long long cap = (long long)sms * warp_per_sm * (threads / 32);
   a.warp_n = nullptr;
   a.warp_fixed = 0;
-  if (m.warp == kDpWarpAll) {
+  if (m.warp == kDpWarpAll || m.uniform_rows >= kDpMaxThreadRows) {
     a.warp_fixed = a.n;
-  } else if (m.warp == kDpWarpAuto) {
-    if (m.buckets.count && m.warp_n) {
-      k_dp_warp_split<<<1, 32, 0, st>>>(m.buckets.count, m.buckets.rows, W, cap, m.warp_n);
-      CLAST_LAUNCHED();
-      a.warp_n = m.warp_n;
-    } else if (m.uniform_rows >= kDpWarpMinRows && a.n <= cap) {
-      const double r = (double)m.uniform_rows, rows = r * (double)a.n;
-      if (dp_split_cycles(W, a.n, r, rows, 0, 0) < dp_split_cycles(W, 0, 0, 0, r, rows)) a.warp_fixed = a.n;
-    }
+  } else if (m.buckets.count && m.warp_n && (m.warp == kDpWarpAuto || m.long_hits)) {
+    k_dp_warp_split<<<1, 32, 0, st>>>(m.buckets.count, m.buckets.rows, W, cap, m.warp == kDpWarpAuto, m.warp_n);
+    CLAST_LAUNCHED();
+    a.warp_n = m.warp_n;
+  } else if (m.warp == kDpWarpAuto && m.uniform_rows >= kDpWarpMinRows && a.n <= cap) {
+    const double r = (double)m.uniform_rows, rows = r * (double)a.n;
+    if (dp_split_cycles(W, a.n, r, rows, 0, 0) < dp_split_cycles(W, 0, 0, 0, r, rows)) a.warp_fixed = a.n;
   }
   const int64_t rest = a.n - (a.warp_n ? 0 : a.warp_fixed);  // hits left for the one-per-thread kernels (at most)
   bool joined = false;

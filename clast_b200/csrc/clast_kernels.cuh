@@ -186,11 +186,15 @@ struct DpParams {
 // none on the host; kDpWarpOff runs every hit one per thread, kDpWarpAll one
 // per warp.  Results are the same either way.
 constexpr int kDpWarpAuto = 0, kDpWarpOff = 1, kDpWarpAll = 2;
-// Longest read the one-per-thread kernel takes: it holds whole numbers in
-// floats, which are exact below 2^24, and a pass of r rows stays within
-// 5 r + 34,000 of zero (potentials rise by up to 5 per row from margins of
-// -30,000).  Longer reads run one hit per warp, in 32-bit integers.
-constexpr int kDpMaxThreadLen = 1 << 20;
+// Rows from which a hit runs one per warp, in 32-bit integers, whatever the
+// launch asks for: the one-per-thread kernel holds whole numbers in floats,
+// which are exact below 2^24.  In a pass of r rows its potentials stay within
+// 5 r + 34,000 of zero (they rise by up to 5 per row, and a score is never below
+// what the left margin of -30,000 and a gap along the row give), and its match
+// counts between -30,100 and r (a step adds at least as much to them as to the
+// score).  A bound of the length buckets; such hits are the first of the order,
+// so the others of their batch are split as in any other.
+constexpr int kDpMaxThreadRows = 1 << 20;
 struct DpBuckets {
   const unsigned int* count = nullptr;      // hits per length bucket (longest first)
   const unsigned long long* rows = nullptr;  // their rows, summed
@@ -200,6 +204,7 @@ struct DpLaunch {
   DpBuckets buckets;
   long long* warp_n = nullptr;  // device word for the split (with buckets)
   int uniform_rows = -1;
+  bool long_hits = false;  // some hit may have kDpMaxThreadRows rows or more (needs buckets and warp_n)
   // with aux, the one-per-warp kernel runs there, beside the others (forked
   // from and joined back into the launch stream by the two events)
   cudaStream_t aux = nullptr;
