@@ -247,7 +247,6 @@ struct Group {
 
 // Host copy of the group's counters: waits for the stream.
 const GroupCtl& read_ctl(clast_ctx* c, const GroupCtl* dev, cudaStream_t st) {
-  if (!c->ctl) CLAST_CK(cudaMallocHost(reinterpret_cast<void**>(&c->ctl), sizeof(GroupCtl)));
   CLAST_CK(cudaMemcpyAsync(c->ctl, dev, sizeof(GroupCtl), cudaMemcpyDeviceToHost, st));
   CLAST_CK(cudaStreamSynchronize(st));
   return *c->ctl;
@@ -579,6 +578,12 @@ int clast_ctx_create(int device, clast_ctx** out) {
     return CLAST_ERR_CUDA;
   for (int b = 0; b < kBuildStreams; ++b)
     if (cudaStreamCreateWithFlags(&c->st_build[b], cudaStreamNonBlocking) != cudaSuccess) return CLAST_ERR_CUDA;
+  // here and not with the first search, which may be one that must not allocate
+  if (cudaMallocHost(reinterpret_cast<void**>(&c->ctl), sizeof(GroupCtl)) != cudaSuccess) {
+    (void)cudaGetLastError();
+    c->ctl = nullptr;
+    return CLAST_ERR_NOMEM;
+  }
   {  // keep freed pool memory for reuse by later calls of this process
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
