@@ -245,6 +245,11 @@ struct Group {
   int64_t part_fit = INT64_MAX;   // most the scratch holds (arena mode)
 };
 
+// A group's hits do not fit the 32-bit words of the DP's order.
+struct TooManyHits : std::invalid_argument {
+  using std::invalid_argument::invalid_argument;
+};
+
 // Host copy of the group's counters: waits for the stream.
 const GroupCtl& read_ctl(clast_ctx* c, const GroupCtl* dev, cudaStream_t st) {
   CLAST_CK(cudaMemcpyAsync(c->ctl, dev, sizeof(GroupCtl), cudaMemcpyDeviceToHost, st));
@@ -359,7 +364,7 @@ int64_t search_group(clast_ctx* c, Workspace& ws, const clast_params* p, const Q
     if (ws.arena) ws.arena_rewind(mark);
     g.part_cap = (most + nw - 1) / nw;  // strands past a full partition wrote nothing: run again
   }
-  if (H >= ((int64_t)1 << 32)) throw std::invalid_argument("more than 2^32 hits in one window");  // DP order words
+  if (H >= ((int64_t)1 << 32)) throw TooManyHits("more than 2^32 hits in one window");
   c->stats.hits += H;
   if (H == 0) return 0;
   uint64_t* hk = ws.get<uint64_t>("h_key", H);
@@ -1081,10 +1086,40 @@ static int map_impl(clast_ctx* ctx, const clast_targets* T, const clast_params* 
     }
     std::vector<std::unique_ptr<SlabSink>> found;
     int64_t F = 0;
-    for (Group& g : groups) {
+    for (size_t k = 0; k < groups.size(); ++k) {
+      Group g = groups[k];
       std::unique_ptr<SlabSink> sink(new SlabSink(n_loads, groups.size() > 1));
       g.part_cap = first_part_cap(ctx, qr.n);
-      const int64_t f = search_group(ctx, ctx->ws, p, qr, g, *sink);
+      const clast_stats before = S;
+      int64_t f = 0;
+      bool split = false;
+      try {
+        f = search_group(ctx, ctx->ws, p, qr, g, *sink);
+      } catch (const std::bad_alloc&) {
+        if (g.nw == 1) throw;
+        split = true;
+      } catch (const TooManyHits&) {
+        if (g.nw == 1) throw;
+        split = true;
+      }
+      if (split) {  // the hits of all its windows at once are too many: its windows one by one
+        sink.reset();
+        S = before;
+        CLAST_CK(cudaStreamSynchronize(st));
+        ctx->timer.flush();
+        ctx->ws.release_all();  // buffers that grew for the whole group
+        groups.erase(groups.begin() + k);
+        for (int w = 0; w < g.nw; ++w) {
+          Group one;
+          one.reads = g.reads;
+          one.nw = 1;
+          one.ix[0] = g.ix[w];
+          one.load[0] = g.load[w];
+          groups.insert(groups.begin() + k + w, one);
+        }
+        --k;
+        continue;
+      }
       if (f == 0) continue;
       F += f;
       found.push_back(std::move(sink));

@@ -1,0 +1,96 @@
+"""Maps that run short of device memory: a group of windows is searched at once
+when its hits fit, else window by window."""
+import os
+
+import numpy as np
+import pytest
+
+from clast_b200 import api, synth
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+class Hold:
+    """Device memory taken until a given amount is free."""
+
+    def __init__(self):
+        import torch
+        self.torch, self.blocks = torch, []
+
+    def leave(self, free):
+        self.blocks = []
+        self.torch.cuda.empty_cache()
+        self.torch.cuda.synchronize()
+        for unit in (1 << 30, 64 * MB, 2 * MB):
+            while self.torch.cuda.mem_get_info()[0] - unit >= free:
+                self.blocks.append(self.torch.empty(unit, dtype=self.torch.uint8, device="cuda"))
+
+    def close(self):
+        self.blocks = []
+        self.torch.cuda.empty_cache()
+
+
+def repeats(n_reads):
+    """Two contigs of 1 Mbp holding 20 copies each of one 20 kbp stretch, and reads from it."""
+    rng = np.random.Generator(np.random.PCG64(77))
+    element = synth.ACGT[rng.integers(0, 4, size=20_000)]
+    ctg = []
+    for _ in range(2):
+        c = synth.ACGT[rng.integers(0, 4, size=1_000_000)].copy()
+        for k in range(20):
+            c[k * 50_000 + 100:k * 50_000 + 20_100] = element
+        ctg.append(c)
+    at = rng.integers(0, 20_000 - 100, size=n_reads)
+    reads = element[at[:, None] + np.arange(100)]
+    return np.concatenate(ctg), np.array([0, 1_000_000, 2_000_000], np.int64), np.ascontiguousarray(reads).reshape(-1), \
+        np.arange(n_reads + 1, dtype=np.int64) * 100
+
+
+def test_group_that_does_not_fit_is_searched_window_by_window():
+    t, toff, q, qoff = repeats(60_000)
+    n = len(qoff) - 1
+    s = api.Setting(cut_repeat=-1, total_db=float(len(t)))
+    eng, hold = api.Engine(0), Hold()
+    T = eng.targets(s, t, toff, [2], 1_000_100)  # a window per contig
+
+    def run(group=None):
+        eng.trim()
+        if group:
+            os.environ["CLAST_SEED_WINDOWS"] = group
+        try:
+            r = eng.map(s, T, q, qoff, [n], 2_000_000)
+        finally:
+            os.environ.pop("CLAST_SEED_WINDOWS", None)
+        out = {f: np.array(r[f]) for f in api.MAP_FIELDS}
+        del r
+        return out, eng.stats()
+
+    try:
+        want, ample = run()
+        assert ample["hits"] > 2_000_000  # some 85 bytes each, with the windows' together
+        free = 128 * MB
+        while True:  # what one window at a time needs
+            eng.trim()
+            hold.leave(free)
+            try:
+                run("1")
+                break
+            except api.ClastError as e:
+                assert e.code == -3, str(e)
+                free += 32 * MB
+                assert free < 4096 * MB
+        eng.trim()
+        hold.leave(free + 48 * MB)
+        got, short = run()
+        for f in api.MAP_FIELDS:
+            np.testing.assert_array_equal(got[f], want[f], err_msg=f)
+        # it did not fit at once, and what it counted before that is not counted twice
+        assert short["map_launches"] > ample["map_launches"]
+        for k in ("seeds", "hits", "dp_cells", "query_kmers"):
+            assert short[k] == ample[k], k
+    finally:
+        hold.close()
+        T.close()
+        eng.close()
