@@ -454,6 +454,21 @@ int64_t search_group(clast_ctx* c, Workspace& ws, const clast_params* p, const Q
   return F;
 }
 
+// Tables on their way up: in the context's pinned staging buffer, or, larger than
+// that may be, in pageable memory (a copy from there returns once it has been read).
+struct HostTables {
+  clast_ctx* c;
+  std::vector<char> own;
+  char* p;
+  HostTables(clast_ctx* ctx, size_t bytes) : c(ctx), own(bytes <= kStageMax ? 0 : bytes) {
+    p = own.empty() ? c->stage(bytes) : own.data();
+  }
+  void upload(void* dev, size_t bytes, cudaStream_t st) {
+    CLAST_CK(cudaMemcpyAsync(dev, p, bytes, cudaMemcpyHostToDevice, st));
+    if (own.empty()) c->staged(st);
+  }
+};
+
 // Seeds per partition that a group begins with.
 int64_t first_part_cap(const clast_ctx* c, int64_t n_bases) {
   return std::max<int64_t>(c->seed_hint, n_bases / 16 + (1 << 20)) / kSeedParts + 1;
@@ -584,11 +599,12 @@ int clast_ctx_create(int device, clast_ctx** out) {
   for (int b = 0; b < kBuildStreams; ++b)
     if (cudaStreamCreateWithFlags(&c->st_build[b], cudaStreamNonBlocking) != cudaSuccess) return CLAST_ERR_CUDA;
   // here and not with the first search, which may be one that must not allocate
-  if (cudaMallocHost(reinterpret_cast<void**>(&c->ctl), sizeof(GroupCtl)) != cudaSuccess) {
+  if (cudaMallocHost(reinterpret_cast<void**>(&c->ctl), sizeof(GroupCtl) + 2 * sizeof(int32_t)) != cudaSuccess) {
     (void)cudaGetLastError();
     c->ctl = nullptr;
     return CLAST_ERR_NOMEM;
   }
+  c->lens = reinterpret_cast<int32_t*>(c->ctl + 1);
   {  // keep freed pool memory for reuse by later calls of this process
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
@@ -688,7 +704,8 @@ int clast_search(clast_ctx* ctx, const clast_index* ix, const clast_params* p, c
     const size_t len_at = QueryBatch::al((size_t)n_qseqs * sizeof(int64_t));
     const size_t win_at = len_at + QueryBatch::al((size_t)n_qseqs * sizeof(int32_t));
     const size_t table_bytes = win_at + 2 * sizeof(int32_t);
-    char* host_tables = ctx->stage(table_bytes);
+    HostTables tables(ctx, table_bytes);
+    char* host_tables = tables.p;
     int64_t* start = reinterpret_cast<int64_t*>(host_tables);
     for (int32_t i = 0; i < n_qseqs; ++i) {
       start[i] = q_gateway[i];
@@ -706,8 +723,7 @@ int clast_search(clast_ctx* ctx, const clast_index* ix, const clast_params* p, c
     qb.max_len = max_len;
     qb.nwin = 1;
     qb.wstart = reinterpret_cast<const int32_t*>(qb.meta);
-    CLAST_CK(cudaMemcpyAsync(qb.start, host_tables, table_bytes, cudaMemcpyHostToDevice, st));
-    ctx->staged(st);
+    tables.upload(qb.start, table_bytes, st);
     CLAST_CK(cudaMemsetAsync(qb.bases, 'N', kPad, st));
     CLAST_CK(cudaMemsetAsync(qb.bases + kPad + n_qbases, 'N', kPad, st));
     if (n_qbases > 0)
@@ -1018,8 +1034,8 @@ static int map_impl(clast_ctx* ctx, const clast_targets* T, const clast_params* 
     }
     // The tables of the batch behind its strands: first reads of the loads,
     // strands where the query windows start, read offsets relative to the first
-    // read.  They are staged in pinned memory and go up in one copy; the
-    // offsets of a large batch come straight from the caller's array.
+    // read.  They go up in one copy; the offsets of a large batch come straight
+    // from the caller's array.
     const size_t win_at = QueryBatch::al(((size_t)n_loads + 1) * sizeof(int64_t));
     const size_t len_at = win_at + QueryBatch::al(wfirst.size() * sizeof(int32_t));
     const size_t off_at = len_at + QueryBatch::al(2 * sizeof(int32_t));  // shortest, longest read
@@ -1036,7 +1052,9 @@ static int map_impl(clast_ctx* ctx, const clast_targets* T, const clast_params* 
     qb.wstart = reinterpret_cast<const int32_t*>(qb.meta + win_at);
     const int64_t* dlf = reinterpret_cast<const int64_t*>(qb.meta);
     const int64_t* doff = reinterpret_cast<const int64_t*>(qb.meta + off_at);
-    char* tables = ctx->stage(off_at + (offs_staged ? off_bytes : 0));
+    const size_t table_bytes = off_at + (offs_staged ? off_bytes : 0);
+    HostTables host_tables(ctx, table_bytes);
+    char* tables = host_tables.p;
     std::memcpy(tables, load_first.data(), load_first.size() * sizeof(int64_t));
     int32_t* wstart = reinterpret_cast<int32_t*>(tables + win_at);
     for (size_t i = 0; i < wfirst.size(); ++i) wstart[i] = (int32_t)(2 * wfirst[i]);
@@ -1047,8 +1065,7 @@ static int map_impl(clast_ctx* ctx, const clast_targets* T, const clast_params* 
       for (int64_t i = 0; i <= nreads; ++i) o[i] = reads->offsets[i] - reads->offsets[0];
     }
     S.map_prep_ms = wall_ms() - w0;
-    CLAST_CK(cudaMemcpyAsync(qb.meta, tables, off_at + (offs_staged ? off_bytes : 0), cudaMemcpyHostToDevice, cs));
-    ctx->staged(cs);
+    host_tables.upload(qb.meta, table_bytes, cs);
     if (!offs_staged)
       CLAST_CK(cudaMemcpyAsync(qb.meta + off_at, reads->offsets, off_bytes, cudaMemcpyHostToDevice, cs));
     CLAST_CK(cudaEventRecord(ctx->ev3, cs));
@@ -1059,14 +1076,14 @@ static int map_impl(clast_ctx* ctx, const clast_targets* T, const clast_params* 
     int32_t* dlen = reinterpret_cast<int32_t*>(qb.meta + len_at);
     if (dev_lengths) {
       read_lengths(doff, nreads, dlen, dlen + 1, st);
-      CLAST_CK(cudaMemcpyAsync(tables + len_at, dlen, sizeof(lens), cudaMemcpyDeviceToHost, st));
+      CLAST_CK(cudaMemcpyAsync(ctx->lens, dlen, sizeof(lens), cudaMemcpyDeviceToHost, st));
     }
     S.query_bases = qb.n;
     // the index builds of clast_targets_create end before the first search
     settle_targets(ctx, T);
     CLAST_CK(cudaStreamWaitEvent(st, T->ev_done, 0));
     QueryRef qr = qb.ref();
-    if (dev_lengths) qr.lens = reinterpret_cast<const int32_t*>(tables + len_at);
+    if (dev_lengths) qr.lens = ctx->lens;
     // windows searched per group (CLAST_SEED_WINDOWS, 1..4), as long as the
     // group's slots have 32-bit numbers
     int group = 2;
@@ -1232,6 +1249,7 @@ int clast_ctx_trim(clast_ctx* ctx) {
     for (auto& a : ctx->arenas)
       if (!a->in_use) a->dev.slab.mem.release();
     ctx->ws.release_all();
+    ctx->release_staging();
     for (auto& w : ctx->ws_build) w.release_all();
     CLAST_CK(cudaDeviceSynchronize());
     cudaMemPool_t pool;

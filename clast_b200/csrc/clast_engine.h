@@ -190,7 +190,7 @@ struct PinnedArena {
 
 // Reads of a batch up to which the host looks at every length itself.
 constexpr int64_t kHostLengths = 1 << 15;
-// Most bytes a context stages in its pinned buffer.
+// Largest pinned staging buffer of a context.
 constexpr size_t kStageMax = (size_t)16 << 20;
 constexpr int kBuildStreams = 2;  // target windows indexed at once by clast_targets_create
 
@@ -216,8 +216,10 @@ struct clast_ctx {
   StageTimer timer;
   int64_t seed_hint = 0;  // seed buffer capacity that sufficed before
   clast::GroupCtl* ctl = nullptr;  // pinned copy of a group's counters
-  // Pinned buffer for small tables on their way up and small results on their
-  // way down.  stage() waits for the copy made from it last (staged()).
+  int32_t* lens = nullptr;         // pinned, behind it: shortest and longest read, when the device looks at them
+  // Pinned buffer of up to kStageMax bytes for small tables on their way up and
+  // small results on their way down.  stage() waits for the copy made from it
+  // last (staged()).
   char* staging = nullptr;
   size_t staging_bytes = 0;
   cudaEvent_t ev_stage = nullptr;
@@ -229,7 +231,7 @@ struct clast_ctx {
       if (staging) CLAST_CK(cudaFreeHost(staging));
       staging = nullptr;
       staging_bytes = 0;
-      const size_t want = bytes + bytes / 2 + (64 << 10);
+      const size_t want = std::max(bytes, std::min(bytes + bytes / 2 + (64 << 10), clast::kStageMax));
       if (cudaMallocHost(reinterpret_cast<void**>(&staging), want) != cudaSuccess) {
         (void)cudaGetLastError();
         staging = nullptr;
@@ -242,6 +244,13 @@ struct clast_ctx {
   void staged(cudaStream_t s) {
     CLAST_CK(cudaEventRecord(ev_stage, s));
     stage_pending = true;
+  }
+  void release_staging() {
+    if (stage_pending) CLAST_CK(cudaEventSynchronize(ev_stage));
+    stage_pending = false;
+    if (staging) CLAST_CK(cudaFreeHost(staging));
+    staging = nullptr;
+    staging_bytes = 0;
   }
   // the DP's one-hit-per-warp kernel runs on st_dp beside the one-per-thread
   // kernels on st (forked and joined by these events)

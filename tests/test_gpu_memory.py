@@ -1,5 +1,5 @@
 """Maps that run short of device memory: a group of windows is searched at once
-when its hits fit, else window by window."""
+when its hits fit, else window by window.  And the pinned memory that calls keep."""
 import os
 
 import numpy as np
@@ -92,5 +92,47 @@ def test_group_that_does_not_fit_is_searched_window_by_window():
             assert short[k] == ample[k], k
     finally:
         hold.close()
+        T.close()
+        eng.close()
+
+
+def pinned():
+    """Bytes of pinned host memory of this process (the runtime maps it from /dev/zero)."""
+    total = 0
+    for line in open("/proc/self/maps"):
+        x = line.split()
+        if len(x) > 5 and x[5] == "/dev/zero":
+            a, b = x[0].split("-")
+            total += int(b, 16) - int(a, 16)
+    return total
+
+
+def test_pinned_staging_is_bounded_and_trimmed():
+    """Offsets that do not start at 0 are made relative on the host: 32 MB of them
+    must not stay pinned (16 MB may, until clast_ctx_trim)."""
+    n = 4_000_000
+    rng = np.random.Generator(np.random.PCG64(5))
+    t = synth.make_target(rng, 200_000, n_contigs=2, median=90_000)
+    q = synth.ACGT[rng.integers(0, 4, size=20 * (n + 1))]
+    qoff = np.arange(n + 2, dtype=np.int64) * 20
+    s = api.Setting(total_db=float(t.offsets[-1]))
+    eng = api.Engine(0)
+    T = eng.targets(s, t.bases, t.offsets, [2], 64_000_000)
+    try:
+        for off in (qoff[:-1], qoff[:-1], qoff[1:]):  # the same sizes everywhere else: only the last one shifts
+            before = pinned()
+            r = eng.map(s, T, q, off, [n], 2_000_000)
+            del r
+            grown = pinned() - before
+        assert before > 0
+        assert grown < 20 * MB, grown
+        eng.trim()
+        kept = pinned()
+        r = eng.map(s, T, q, qoff[1:1_500_002], [1_500_000], 2_000_000)  # 12 MB: staged
+        del r
+        assert pinned() - kept >= 12 * MB
+        eng.trim()
+        assert pinned() == kept
+    finally:
         T.close()
         eng.close()
