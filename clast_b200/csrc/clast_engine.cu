@@ -245,6 +245,19 @@ struct Group {
   int64_t part_fit = INT64_MAX;   // most the scratch holds (arena mode)
 };
 
+// Waits for streams when the scope that holds it is left by an exception: what
+// it holds may still be read or written by work queued there.
+struct UnwindSync {
+  std::vector<cudaStream_t> streams;
+  int pending = std::uncaught_exceptions();
+  UnwindSync(std::initializer_list<cudaStream_t> s) : streams(s) {}
+  ~UnwindSync() {
+    if (std::uncaught_exceptions() == pending) return;
+    for (cudaStream_t s : streams) cudaStreamSynchronize(s);
+    (void)cudaGetLastError();
+  }
+};
+
 // A group's hits do not fit the 32-bit words of the DP's order.
 struct TooManyHits : std::invalid_argument {
   using std::invalid_argument::invalid_argument;
@@ -816,6 +829,9 @@ int clast_targets_create(clast_ctx* ctx, const clast_params* p, int32_t t_vram, 
     const bool host_src = !targets->bases_on_device;
     const char* hsrc = targets->bases + (nt ? targets->offsets[0] : 0);
     DevArray<char> traw;
+    DevArray<int32_t> all_gw, all_ln;
+    DevArray<int64_t> all_so;
+    std::vector<std::unique_ptr<clast_index>> shells;
     cudaStream_t cs = host_src ? ctx->st_copy : st;
     if (host_src) {
       g_alloc_stream = ctx->st_copy;
@@ -828,6 +844,11 @@ int clast_targets_create(clast_ctx* ctx, const clast_params* p, int32_t t_vram, 
     if (!host_src) CLAST_CK(cudaEventRecord(T->ev_up, cs));  // nothing to upload
     int64_t copied = 0;  // source bytes already queued for upload
     std::vector<cudaEvent_t> win_ev;
+    // a call that fails part-way frees its blocks on the compute stream, which
+    // does not wait for the builds and copies that still use them (declared
+    // after what it guards)
+    UnwindSync unwind{ctx->st_copy, ctx->st_build[0], ctx->st_build[1], st};
+    static_assert(kBuildStreams == 2, "the streams that unwind waits for");
     // the windows are indexed back to back on the stream with no host
     // synchronisation; the table-overflow count is read by the first clast_map
     unsigned long long* failed = T->failed.p;
@@ -862,8 +883,6 @@ int clast_targets_create(clast_ctx* ctx, const clast_params* p, int32_t t_vram, 
         }
       }
     }
-    DevArray<int32_t> all_gw, all_ln;
-    DevArray<int64_t> all_so;
     all_gw.alloc(gw.size());
     all_ln.alloc(ln.size());
     all_so.alloc(so.size());
@@ -877,7 +896,6 @@ int clast_targets_create(clast_ctx* ctx, const clast_params* p, int32_t t_vram, 
     // small, latency-bound kernels); every build stream starts after the plan's
     // upload above and the compute stream waits for all of them at the end.
     // Windows searched together (2k and 2k + 1) share their filter memory.
-    std::vector<std::unique_ptr<clast_index>> shells;
     for (size_t wi = 0; wi < plan.size(); ++wi) shells.emplace_back(new clast_index());
     for (size_t wi = 0; wi < plan.size(); wi += 2) {
       const int n = wi + 1 < plan.size() ? 2 : 1;

@@ -23,7 +23,7 @@ class Hold:
         self.blocks = []
         self.torch.cuda.empty_cache()
         self.torch.cuda.synchronize()
-        for unit in (1 << 30, 64 * MB, 2 * MB):
+        for unit in (16 << 30, 1 << 30, 64 * MB, 2 * MB):
             while self.torch.cuda.mem_get_info()[0] - unit >= free:
                 self.blocks.append(self.torch.empty(unit, dtype=self.torch.uint8, device="cuda"))
 
@@ -135,4 +135,47 @@ def test_pinned_staging_is_bounded_and_trimmed():
         assert pinned() == kept
     finally:
         T.close()
+        eng.close()
+
+
+def test_failed_builds_leave_the_context_usable():
+    """Targets whose later windows find no memory while the earlier ones are being
+    indexed: the call fails, and the next ones are not disturbed by what was queued."""
+    rng = np.random.Generator(np.random.PCG64(6))
+    t = synth.make_target(rng, 32_000_000, n_contigs=8, median=4_000_000)
+    q = synth.make_reads_fixed(rng, t, 3000, length=120)
+    small = synth.make_target(rng, 1_000_000, n_contigs=2, median=400_000)
+    qs = synth.make_reads_fixed(rng, small, 2000, length=120)
+    s = api.Setting(total_db=float(t.offsets[-1]))
+    eng, hold = api.Engine(0), Hold()
+
+    def mapped(target, reads, t_vram):
+        T = eng.targets(s, target.bases, target.offsets, [len(target)], t_vram)
+        r = eng.map(s, T, reads.bases, reads.offsets, [len(reads)], 2_000_000)
+        out = {f: np.array(r[f]) for f in api.MAP_FIELDS}
+        del r
+        T.close()
+        return out
+
+    try:
+        want, want_small = mapped(t, q, 4_500_000), mapped(small, qs, 64_000_000)
+        failed = 0
+        for free in (256 * MB, 320 * MB, 384 * MB):
+            eng.trim()
+            hold.leave(free)
+            try:
+                mapped(t, q, 4_500_000)
+            except api.ClastError as e:
+                assert e.code == -3, str(e)
+                failed += 1
+            got = mapped(small, qs, 64_000_000)  # at once, in what the failed call gave back
+            for f in api.MAP_FIELDS:
+                np.testing.assert_array_equal(got[f], want_small[f], err_msg=f)
+        assert failed > 0
+        hold.close()
+        got = mapped(t, q, 4_500_000)
+        for f in api.MAP_FIELDS:
+            np.testing.assert_array_equal(got[f], want[f], err_msg=f)
+    finally:
+        hold.close()
         eng.close()
