@@ -179,8 +179,8 @@ struct PinnedArena {
   void* p = nullptr;
   size_t bytes = 0;
   std::atomic<bool> in_use{false};  // released by the result's owner, possibly on another thread
-  // The result on the device, kept until the arena is reused (so the text of a
-  // result can be formatted on the GPU).
+  // The result on the device, kept until the first map after its release (so
+  // that its text can be formatted on the GPU).
   struct Device {
     ResultSlab slab;
     int64_t n = 0;

@@ -179,3 +179,39 @@ def test_failed_builds_leave_the_context_usable():
     finally:
         hold.close()
         eng.close()
+
+
+def test_released_results_make_room_for_the_next():
+    """Maps in a loop, each result released before the next: the device never holds
+    two of them, and the memory pool keeps its size."""
+    from cuda.bindings import runtime as rt
+    from cuda.bindings.driver import cuuint64_t
+    rng = np.random.Generator(np.random.PCG64(8))
+    t = synth.make_target(rng, 4_000_000, n_contigs=4, median=900_000)
+    q = synth.make_reads_fixed(rng, t, 400_000, length=60)
+    s = api.Setting(total_db=float(t.offsets[-1]))
+    _, q_loads = api.ram_loads(np.diff(q.offsets), 32_000_000)
+    attr = rt.cudaMemPoolAttr
+    eng = api.Engine(0)
+    _, pool = rt.cudaDeviceGetDefaultMemPool(0)
+
+    def mb(a):
+        return int(rt.cudaMemPoolGetAttribute(pool, a)[1]) / MB
+
+    high, reserved = [], []
+    try:
+        eng.trim()
+        for _ in range(5):
+            rt.cudaMemPoolSetAttribute(pool, attr.cudaMemPoolAttrUsedMemHigh, cuuint64_t(0))
+            T = eng.targets(s, t.bases, t.offsets, [len(t)], 64_000_000)
+            r = eng.map(s, T, q.bases, q.offsets, q_loads, 2_000_000)
+            slab = 48 * len(r["read"]) / MB
+            del r
+            T.close()
+            high.append(mb(attr.cudaMemPoolAttrUsedMemHigh))
+            reserved.append(mb(attr.cudaMemPoolAttrReservedMemCurrent))
+    finally:
+        eng.close()
+    assert slab > 10
+    assert max(high) - high[0] < slab / 2, (high, slab)
+    assert reserved[-1] == reserved[1], reserved
