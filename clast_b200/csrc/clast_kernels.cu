@@ -3173,41 +3173,55 @@ __host__ __device__ __forceinline__ long long dp_bucket_hi(int b) {
   return dp_bucket_lo(b) + (1ll << (x / 16 - 1)) - 1;
 }
 
-// Cost model of the warp / thread split, in SM clock cycles, fitted on the
-// B200 at gap 8 (W = 17): a hit in thread mode takes kDpThreadCellCycles per
-// cell when its warp has the SM sub-partition to itself (a row is W dependent
-// cells), and a full grid runs kDpThreadCellsPerCycle cells per cycle; a hit
-// in warp mode takes kDpWarpRowCycles per row alone (two wavefront steps),
-// and warps run kDpWarpRowsPerCycle rows per cycle over the GPU.  The two
-// kernels run side by side: with L the longer of the two longest hits' times
+// Cost model of the warp / thread split, in SM clock cycles, fitted on the B200
+// at gaps 2 - 16 in both modes to batches of 1 to 13,000 hits of 150 bp - 5 kbp,
+// equal and uneven, every hit one way or the other.
+// Thread mode: a row takes dp_thread_row_cycles where the hit's warp has the SM
+// sub-partition to itself (a row is W dependent cells; below some twenty of them
+// it waits for the letters of the warp's other hits, and a local one also keeps
+// its best cell), the ends and bands of its two passes dp_thread_band_cycles; a
+// full grid runs kDpThreadCellsPerCycle cells per cycle.  Warp mode: a row takes
+// kDpWarpRowCycles alone (two wavefront steps); the GPU runs
+// dp_warp_rows_per_cycle rows per cycle and a hit kDpWarpHitCycles of its own.
+// Two kernels run side by side: with L the longer of the two longest hits' times
 // and I the issue time of both kernels' work, the batch takes max(L + I/2, I)
-// (measured: a lone hit's rows slow down as other warps share its
-// sub-partition, and the GPU cannot issue faster than I).  Forking the second
-// stream and the launch cost kDpLaunchCycles.  Only the split depends on
-// these; results do not.
-constexpr double kDpThreadCellCycles = 26.0;
+// (measured: a lone hit's rows slow down as other warps share its sub-partition,
+// and the GPU cannot issue faster than I), and the second stream kDpForkCycles.
+// Only the split depends on these; results do not.  With 26 cycles per cell and 6
+// rows per cycle everywhere (as fitted at gap 8, global mode), local batches and
+// narrow bands stayed in thread mode too long: 4,000 local reads of 100 - 5,000 bp
+// 1.93 to 0.73 ms at gap 3, 1.16 to 0.75 at gap 8; 3,000 of 150 bp at gap 16 0.118
+// to 0.077.
 constexpr double kDpThreadCellsPerCycle = 1000.0;
 constexpr double kDpWarpRowCycles = 217.0;
-constexpr double kDpWarpRowsPerCycle = 6.0;
-constexpr double kDpLaunchCycles = 10000.0;
+constexpr double kDpWarpHitCycles = 8.4;
+constexpr double kDpForkCycles = 10000.0;
 constexpr long long kDpWarpMinRows = 16;
+__host__ __device__ __forceinline__ double dp_thread_row_cycles(int W, bool local) {
+  return !local ? fmax(480.0, 27.0 * W) : W <= 5 ? 510.0 : 500.0 + 26.0 * W;
+}
+__host__ __device__ __forceinline__ double dp_thread_band_cycles(int W, bool local) {
+  return (local ? 25.0 : 50.0) * W * W;
+}
+__host__ __device__ __forceinline__ double dp_warp_rows_per_cycle(bool local) { return local ? 4.6 : 5.9; }
 
 // Estimated time of the DP with the `s` longest hits (rows summed: sw, the
 // longest r1) one per warp and the rest (rows summed: rest, the longest rn)
 // one per thread.
-__host__ __device__ __forceinline__ double dp_split_cycles(int W, long long s, double r1, double sw, double rn,
-                                                           double rest) {
+__host__ __device__ __forceinline__ double dp_split_cycles(int W, bool local, long long s, double r1, double sw,
+                                                           double rn, double rest) {
   double lat = s > 0 ? r1 * kDpWarpRowCycles : 0.0;
-  if (rest > 0) lat = fmax(lat, rn * W * kDpThreadCellCycles);
-  const double issue = (s > 0 ? sw / kDpWarpRowsPerCycle : 0.0) + rest * W / kDpThreadCellsPerCycle;
-  return fmax(lat + 0.5 * issue, issue) + (s > 0 ? kDpLaunchCycles : 0.0);
+  if (rest > 0) lat = fmax(lat, rn * dp_thread_row_cycles(W, local) + dp_thread_band_cycles(W, local));
+  const double issue = sw / dp_warp_rows_per_cycle(local) + (double)s * kDpWarpHitCycles +
+                       rest * W / kDpThreadCellsPerCycle;
+  return fmax(lat + 0.5 * issue, issue) + (s > 0 && rest > 0 ? kDpForkCycles : 0.0);
 }
 
 // The split on the device: the hits of kDpMaxThreadRows rows or more one per
 // warp; then, with `split`, every bucket boundary (longest first) is a candidate,
 // and the earliest estimated end wins.  One thread; ~500 buckets.
 __global__ void k_dp_warp_split(const unsigned int* __restrict__ count, const unsigned long long* __restrict__ rows,
-                                int W, long long cap, bool split, long long* __restrict__ warp_n) {
+                                int W, bool local, long long cap, bool split, long long* __restrict__ warp_n) {
   if (threadIdx.x != 0) return;
   double total = 0;
   for (int b = 0; b < kDpBuckets; ++b) total += (double)rows[b];
@@ -3220,7 +3234,7 @@ __global__ void k_dp_warp_split(const unsigned int* __restrict__ count, const un
     if (r1 < 0) r1 = rn;
     if (dp_bucket_lo(b) < kDpMaxThreadRows) {
       // candidate: the buckets before b one per warp, b and the rest one per thread
-      const double t = dp_split_cycles(W, s, s > 0 ? r1 : 0, sw, rn, total - sw);
+      const double t = dp_split_cycles(W, local, s, s > 0 ? r1 : 0, sw, rn, total - sw);
       if (!any || t < best) { best = t; best_s = s; }
       any = true;
       if (!split || dp_bucket_lo(b) < kDpWarpMinRows || s + count[b] > cap) {
@@ -3231,7 +3245,7 @@ __global__ void k_dp_warp_split(const unsigned int* __restrict__ count, const un
     s += count[b];
     sw += (double)rows[b];
   }
-  if (all_taken && s > 0 && (!any || dp_split_cycles(W, s, r1, sw, 0, 0) < best)) best_s = s;  // every hit one per warp
+  if (all_taken && s > 0 && (!any || dp_split_cycles(W, local, s, r1, sw, 0, 0) < best)) best_s = s;  // every hit one per warp
   *warp_n = best_s;
 }
 
@@ -3254,20 +3268,23 @@ long long launch_dp_mode(DpKernelArgs a, const DpLaunch& m, cudaStream_t st) {
     return o;
   }();
   const int sms = occ.sms, per_sm = occ.per_sm, warp_per_sm = occ.warp_per_sm;
-  // hits one per warp: at most one wave of the warp kernel's resident warps
-  // (the cost model has no waves)
+  // hits one per warp: at most one wave of the warp kernel's resident warps (the
+  // cost model has no waves); half as many more where all are equal and the issue
+  // rate bounds them (3,245 local hits of 150 bp at gap 16, 285 more than a wave:
+  // 0.077 against 0.118 ms one per thread; 6,509: 0.145 against 0.118)
   const long long cap = (long long)sms * warp_per_sm * (threads / 32);
   a.warp_n = nullptr;
   a.warp_fixed = 0;
   if (m.warp == kDpWarpAll || m.uniform_rows >= kDpMaxThreadRows) {
     a.warp_fixed = a.n;
   } else if (m.buckets.count && m.warp_n && (m.warp == kDpWarpAuto || m.long_hits)) {
-    k_dp_warp_split<<<1, 32, 0, st>>>(m.buckets.count, m.buckets.rows, W, cap, m.warp == kDpWarpAuto, m.warp_n);
+    k_dp_warp_split<<<1, 32, 0, st>>>(m.buckets.count, m.buckets.rows, W, LOCAL, cap, m.warp == kDpWarpAuto,
+                                      m.warp_n);
     CLAST_LAUNCHED();
     a.warp_n = m.warp_n;
-  } else if (m.warp == kDpWarpAuto && m.uniform_rows >= kDpWarpMinRows && a.n <= cap) {
+  } else if (m.warp == kDpWarpAuto && m.uniform_rows >= kDpWarpMinRows && 2 * a.n <= 3 * cap) {
     const double r = (double)m.uniform_rows, rows = r * (double)a.n;
-    if (dp_split_cycles(W, a.n, r, rows, 0, 0) < dp_split_cycles(W, 0, 0, 0, r, rows)) a.warp_fixed = a.n;
+    if (dp_split_cycles(W, LOCAL, a.n, r, rows, 0, 0) < dp_split_cycles(W, LOCAL, 0, 0, 0, r, rows)) a.warp_fixed = a.n;
   }
   const int64_t rest = a.n - (a.warp_n ? 0 : a.warp_fixed);  // hits left for the one-per-thread kernels (at most)
   bool joined = false;
