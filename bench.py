@@ -161,6 +161,17 @@ class ClockSampler:
 # ---------------------------------------------------------------------------
 # CPU baselines (the reference built for the CPU, else the oracle port)
 # ---------------------------------------------------------------------------
+def reference_binary():
+    """The reference built for the CPU (oracle/build_ref.py); an error where it is
+    not: the oracle, a port of ours, never stands in for it."""
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import oracle as O
+    if not O.ref_available():
+        raise RuntimeError("the reference's CPU build is not here (%s), nor sources to make it from" %
+                           os.path.relpath(O.REF, ROOT))
+    return O.REF
+
+
 def cpu_reference_rate(t, q, n_sample, threads=None):
     """Reference CPU throughput on this host, extrapolated to the full job.
 
@@ -168,12 +179,7 @@ def cpu_reference_rate(t, q, n_sample, threads=None):
     the index builds of both target RAM loads) and with the first n_sample
     reads.  The full job needs one pair of index builds per query RAM load, so
     T_full = loads_full * T_fixed + (reads_full / n_sample) * (T_sample - T_fixed)."""
-    sys.path.insert(0, os.path.join(ROOT, "oracle"))
-    import oracle as O
-    kind = "reference" if O.ref_available() else "port"
-    exe = O.REF if kind == "reference" else O.CLI
-    if kind == "port" and not os.path.exists(exe):
-        O.build()
+    exe = reference_binary()
     threads = threads or os.cpu_count()
     env = dict(os.environ, OMP_NUM_THREADS=str(threads))
     with tempfile.TemporaryDirectory() as d:
@@ -195,7 +201,7 @@ def cpu_reference_rate(t, q, n_sample, threads=None):
     t_full = q_loads * times[1] + len(q) * per_read
     mbp = q.offsets[-1] / 1e6
     return {
-        "value": mbp / t_full, "unit": "Mbp/s", "cores": threads, "kind": kind,
+        "value": mbp / t_full, "unit": "Mbp/s", "cores": threads, "kind": "reference",
         "sample": "full target; a 1-read run (%.1f s: FASTA + index builds) and a %d-read run (%.1f s), "
                   "extrapolated to %d query RAM loads and %d reads (%.0f s)" % (
                       times[1], n_sample, times[n_sample], q_loads, len(q), t_full),
@@ -857,6 +863,11 @@ def run_ours(args):
 def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    try:
+        reference_binary()
+    except RuntimeError as e:
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
         return
     t, q = synth.workload(args.workload, seed=args.seed, scale=args.scale)
     vals = []
