@@ -3,10 +3,10 @@
 //
 // One context owns one CUDA stream and a scratch pool.  An index keeps its
 // target window resident in HBM (bases with joints, padded with 'N', plus the
-// key directory, unique keys, bucket ranges and resolved entries).  A search
-// runs the whole hit pipeline of CDeviceHitList (CDeviceHitList.cu:228-423)
-// for a batch of query windows with three host synchronisations (seed total,
-// hit total, result total).
+// hash table, the filter and the resolved entries).  A search runs the whole hit
+// pipeline of CDeviceHitList (CDeviceHitList.cu:228-423) for a batch of query
+// windows against a group of target windows with two host synchronisations (hit
+// total, result total).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1311,10 +1311,9 @@ int clast_last_map_stats(const clast_ctx* ctx, double* device_ms, int64_t* kerne
 
 // ----------------------------------------------------------------------------
 // clast_search_noalloc: clast_search on a fixed scratch buffer, allocating
-// nothing.  It seeds the one query window itself (partitions sized to fit
-// the scratch), then runs search_seeded, the stages clast_search runs, with
-// every device buffer a slot of the static scratch (Workspace arena mode);
-// the hits go from scratch slots straight into the caller's host arrays.
+// nothing.  It runs search_group, as clast_search does, with seed partitions
+// sized to fit the scratch and every device buffer a slot of it (Workspace arena
+// mode); the hits go from scratch slots straight into the caller's host arrays.
 // ----------------------------------------------------------------------------
 namespace {
 

@@ -3,10 +3,10 @@
 // Reference (masayano/CLAST) stages and the kernels that replace them:
 //   SRead2bit/SRepelHasOddBase + CDeviceSeqList_query::createHashIndex -> pack_bases, kmer_at
 //   CDeviceHashTable (sort_by_key, unique, reduce_by_key, scan, cut)   -> sample_keys,
-//       radix_sort_u64, index_*, table_* (hash table + Bloom filter for one-probe lookups)
-//   createRawSeedList (binarySearch, writeSeedList)                     -> seed_fused
-//   deleteSeedsOnSequenceBoundary                                       -> folded into seed_fused
-//   sortSeeds / deletingIsolateSeeds / deleteDuplicateSeeds             -> seed_sort_filter
+//       radix_sort_u64, index_place (hash table + Bloom filter for one-probe lookups)
+//   createRawSeedList (binarySearch, writeSeedList)                     -> seed_reads, seed_fused
+//   deleteSeedsOnSequenceBoundary                                       -> folded into these
+//   sortSeeds / deletingIsolateSeeds / deleteDuplicateSeeds             -> seed_reads, seed_filter
 //   globalAlign* / localAlign* + calculateEvalue + deleteBadHits        -> banded_dp
 //   resultSorting + deleteHits_duplicateResult                          -> final_* (per read)
 #include <cuda_runtime.h>
@@ -2791,8 +2791,8 @@ __device__ __forceinline__ void banded_hit(const DpTab<float2>& tab, const char*
 // banded_hit, same tie rules (the local best is the first maximum in
 // row-major order, the global end node the first maximum in column order),
 // so every output equals banded_hit's.  Results are returned in every lane.
-// A row takes 217 cycles alone (275 before H became a running maximum and the
-// letter pairs were looked up a row ahead): the two shuffles and the selects
+// A row takes some 210 cycles alone (275 before H became a running maximum and
+// the letter pairs were looked up a row ahead): the two shuffles and the selects
 // between them.
 template <int GAP, bool LOCAL>
 __device__ __forceinline__ void banded_hit_warp(const DpTab<int2>& tab, const char* __restrict__ tb,

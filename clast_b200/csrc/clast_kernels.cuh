@@ -176,10 +176,11 @@ struct DpParams {
 // How the DP is launched: one thread per hit over a grid of all hits, in blocks
 // that sort hits of one length (uniform_rows) by the rows of their forward pass.
 //
-// The first hits of the order (the longest, when the
-// order is longest first) may run one per warp (an anti-diagonal wavefront
-// over the band) instead of one per thread: a long hit alone takes about 1/7
-// of the time there, at a lower throughput per cell.  `warp` says how many:
+// The first hits of the order (the longest, when the order is longest first) may
+// run one per warp (an anti-diagonal wavefront over the band) instead of one per
+// thread: a 5 kbp hit alone takes 0.54 against 0.95 ms there at gap 8 (0.56 and
+// 1.65 in local mode, 0.54 and 2.13 at gap 16), at a lower throughput per cell.
+// `warp` says how many:
 // kDpWarpAuto splits where the cost model puts the end of both launches
 // earliest -- on the device from the length buckets' counts and row sums
 // (buckets + warp_n), or, for hits that all have `uniform_rows` rows, all or

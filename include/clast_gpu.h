@@ -248,8 +248,9 @@ int clast_write_file(const char* path, const char* buf, int64_t n, int32_t threa
 
 /* Hands back the device memory a context keeps for reuse between calls: its
  * scratch buffers, the device copies of released results, and the blocks
- * the device's memory pool holds after stream-ordered frees.  Results and
- * targets still in use are kept.  Waits for the device first. */
+ * the device's memory pool holds after stream-ordered frees; also its pinned
+ * staging buffer (at most 16 MB).  Results and targets still in use are kept.
+ * Waits for the device first. */
 int clast_ctx_trim(clast_ctx* ctx);
 
 /* Device-side timing of the last clast_map call in milliseconds (kernels and
