@@ -115,13 +115,14 @@ struct StageTimer {
     return e;
   }
   void begin(cudaStream_t st) {
-    cur_a = take();
+    if (!cur_a) cur_a = take();  // else of a stage that ended by an exception
     CLAST_CK(cudaEventRecord(cur_a, st));
   }
   void end(int stage, cudaStream_t st, int launches = 1) {
     cudaEvent_t b = take();
     CLAST_CK(cudaEventRecord(b, st));
     pending.push_back({stage, cur_a, b});
+    cur_a = nullptr;
     n[stage] += launches;
   }
   void flush() {
@@ -140,6 +141,7 @@ struct StageTimer {
   }
   ~StageTimer() {
     for (auto e : pool) cudaEventDestroy(e);
+    if (cur_a) cudaEventDestroy(cur_a);
     for (auto& p : pending) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
   }
 };
