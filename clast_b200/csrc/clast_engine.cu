@@ -347,7 +347,8 @@ int64_t search_group(clast_ctx* c, Workspace& ws, const clast_params* p, const Q
     tm.end(StageTimer::SEED, st);
     // sortSeeds, deletingIsolateSeeds, deleteDuplicateSeeds
     tm.begin(st);
-    seed_filter(skey, sq, off, cnt, nvalid, first_q, qb.wstart, qb.nwin, nw, p->width, p->gap, nv, lists, hcnt, ctl, st);
+    seed_filter(skey, sq, off, cnt, nvalid, first_q, qb.wstart, qb.nwin, nw, p->width, p->gap, nv, lists, hcnt,
+                g.part_cap * nw, ctl, st);
     tm.end(StageTimer::SORT, st, 4);
     scan_i32_to(hcnt, nv, hoff, state1, &ctl->hits, st);
     const GroupCtl& h = read_ctl(c, ctl, st);
@@ -376,6 +377,9 @@ int64_t search_group(clast_ctx* c, Workspace& ws, const clast_params* p, const Q
                                   " (use clast_search)");
     if (ws.arena) ws.arena_rewind(mark);
     g.part_cap = (most + nw - 1) / nw;  // strands past a full partition wrote nothing: run again
+    // a little more the next time (the workspace takes a quarter more anyway):
+    // few reads with many seeds each fill some partitions far above the mean
+    c->part_hint = std::max(c->part_hint, g.part_cap + g.part_cap / 8);
   }
   if (H >= ((int64_t)1 << 32)) throw TooManyHits("more than 2^32 hits in one window");
   c->stats.hits += H;
@@ -759,7 +763,7 @@ int clast_search(clast_ctx* ctx, const clast_index* ix, const clast_params* p, c
       Group g;
       g.nw = 1;
       g.ix[0] = ix;
-      g.part_cap = first_part_cap(ctx, n_qbases);
+      g.part_cap = std::max(first_part_cap(ctx, n_qbases), ctx->part_hint);
       F = search_group(ctx, ctx->ws, p, qb.ref(), g, sink);
     }
     out->n = F;
@@ -1131,7 +1135,7 @@ static int map_impl(clast_ctx* ctx, const clast_targets* T, const clast_params* 
     for (size_t k = 0; k < groups.size(); ++k) {
       Group g = groups[k];
       std::unique_ptr<SlabSink> sink(new SlabSink(n_loads, groups.size() > 1));
-      g.part_cap = first_part_cap(ctx, qr.n);
+      g.part_cap = std::max(first_part_cap(ctx, qr.n), ctx->part_hint);
       const clast_stats before = S;
       int64_t f = 0;
       bool split = false;
@@ -1150,6 +1154,7 @@ static int map_impl(clast_ctx* ctx, const clast_targets* T, const clast_params* 
         CLAST_CK(cudaStreamSynchronize(st));
         ctx->timer.flush();
         ctx->ws.release_all();  // buffers that grew for the whole group
+        ctx->part_hint = 0;
         groups.erase(groups.begin() + k);
         for (int w = 0; w < g.nw; ++w) {
           Group one;
@@ -1274,6 +1279,7 @@ int clast_ctx_trim(clast_ctx* ctx) {
     for (auto& a : ctx->arenas)
       if (!a->in_use) a->dev.slab.mem.release();
     ctx->ws.release_all();
+    ctx->part_hint = 0;
     ctx->release_staging();
     for (auto& w : ctx->ws_build) w.release_all();
     CLAST_CK(cudaDeviceSynchronize());

@@ -217,6 +217,7 @@ struct clast_ctx {
   clast_stats stats{};
   StageTimer timer;
   int64_t seed_hint = 0;  // seed buffer capacity that sufficed before
+  int64_t part_hint = 0;  // fullest seed partition of a window that overflowed before
   clast::GroupCtl* ctl = nullptr;  // pinned copy of a group's counters
   int32_t* lens = nullptr;         // pinned, behind it: shortest and longest read, when the device looks at them
   // Pinned buffer of up to kStageMax bytes for small tables on their way up and

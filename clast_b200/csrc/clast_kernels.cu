@@ -2131,7 +2131,8 @@ __global__ void __launch_bounds__(TEAM == 1 ? kSeedFusedThreads : 32 * TEAM)
 // first other hit is none if it lies near that seed (first_q's top bit).
 __global__ void k_window_first(int32_t* __restrict__ nvalid, const int32_t* __restrict__ wstart, int nwin, int nw,
                                const int32_t* __restrict__ cnt, const uint32_t* __restrict__ first_q,
-                               int32_t* __restrict__ hcnt) {
+                               int32_t* __restrict__ hcnt, int64_t part_cap, GroupCtl* __restrict__ ctl) {
+  if (blockIdx.x == 0 && threadIdx.x < kSeedParts && (int64_t)ctl->cursor[threadIdx.x] > part_cap) ctl->full = 1;
   const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= nwin * nw) return;
@@ -2160,6 +2161,7 @@ struct SeedFilterCtx {
   const int32_t* nvalid;
   int width, gap;
   int32_t* hcnt;
+  const int* full;  // GroupCtl::full
 };
 __device__ __forceinline__ int valid_seeds(int nvalid) { return nvalid < 0 ? ~nvalid : nvalid; }
 
@@ -2241,7 +2243,7 @@ __global__ void k_seed_filter_small(uint64_t* __restrict__ skey, uint32_t* __res
                                     uint32_t* __restrict__ lists, GroupCtl* __restrict__ ctl) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int x = s < nv ? c.nvalid[s] : 0;
-  const int nvalid = valid_seeds(x);
+  const int nvalid = *c.full ? 0 : valid_seeds(x);
   const int n = nvalid > 0 ? c.cnt[s] : 0;
   const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -2354,6 +2356,10 @@ __global__ void __launch_bounds__(kWarpSmemThreads) k_seed_filter_mid(uint64_t* 
   const int total = *count;
   for (int64_t li = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; li < total; li += nwarps) {
     const int64_t s = list[li];
+    if (*c.full) {
+      if (lane == 0) c.hcnt[s] = 0;
+      continue;
+    }
     const int64_t o = c.off[s];
     const int n = c.cnt[s];
     const int x = c.nvalid[s];
@@ -2407,6 +2413,10 @@ __global__ void __launch_bounds__(SMEM ? 256 : 1024) k_seed_filter_big(uint64_t*
   const int total = *count;
   for (int li = blockIdx.x; li < total; li += gridDim.x) {
     const int64_t s = list[li];
+    if (*c.full) {  // the same for the whole block
+      if (threadIdx.x == 0) c.hcnt[s] = 0;
+      continue;
+    }
     const int64_t o = c.off[s];
     const int n = c.cnt[s];
     if (SMEM) {
@@ -3771,14 +3781,14 @@ void seed_reads(const QueryView& q, const SeedWins& W, int nw, int width, int ga
 
 void seed_filter(uint64_t* skey, uint32_t* sq, const int64_t* off, const int32_t* cnt, int32_t* nvalid,
                  const uint32_t* first_q, const int32_t* win_start, int n_windows, int nw, int width, int gap,
-                 int64_t nv, uint32_t* lists, int32_t* hcnt, GroupCtl* ctl, cudaStream_t st) {
+                 int64_t nv, uint32_t* lists, int32_t* hcnt, int64_t part_cap, GroupCtl* ctl, cudaStream_t st) {
   if (nv <= 0) return;
   if (n_windows > 0) {
     k_window_first<<<blocks_for((int64_t)n_windows * nw * 32, 256), 256, 0, st>>>(nvalid, win_start, n_windows, nw, cnt,
-                                                                                 first_q, hcnt);
+                                                                                 first_q, hcnt, part_cap, ctl);
     CLAST_LAUNCHED();
   }
-  SeedFilterCtx c{off, cnt, nvalid, width, gap, hcnt};
+  SeedFilterCtx c{off, cnt, nvalid, width, gap, hcnt, &ctl->full};
   if (!first_q) {
     k_seed_filter_small<<<blocks_for(nv, 256), 256, 0, st>>>(skey, sq, c, nv, lists, ctl);
     CLAST_LAUNCHED();

@@ -89,6 +89,7 @@ struct GroupCtl {
   long long hits, results;
   long long dp_warp;  // hits the DP's split sends to the one-per-warp kernel
   int bad;            // see DpLaunch::bad
+  int full;           // a seed partition overflowed: the filters write no hits, the search runs again
   int n_seeds[3];     // slots listed for the seed filters' longer tiers
   int n_stored[4];    // reads whose seeds are stored: of one round, longer, and how many of each are taken
   int n_long;         // reads listed for k_final_long
@@ -147,10 +148,10 @@ void seed_reads(const QueryView& q, const SeedWins& W, int nw, int width, int ga
 // hits at off[v] onwards, hcnt[v] of them.  lists: 3 nv words.  With first_q
 // (seed_reads) only the listed slots are left to filter.  The first slot
 // of every (target window, query window) with a valid seed has its nvalid
-// complemented.
+// complemented.  part_cap: seeds that a partition holds (all windows').
 void seed_filter(uint64_t* skey, uint32_t* sq, const int64_t* off, const int32_t* cnt, int32_t* nvalid,
                  const uint32_t* first_q, const int32_t* win_start, int n_windows, int nw, int width, int gap,
-                 int64_t nv, uint32_t* lists, int32_t* hcnt, GroupCtl* ctl, cudaStream_t st);
+                 int64_t nv, uint32_t* lists, int32_t* hcnt, int64_t part_cap, GroupCtl* ctl, cudaStream_t st);
 // First seeds of the slots that seed_reads filtered (key null: none).
 struct FirstSeeds {
   const uint64_t* key;
